@@ -52,6 +52,12 @@ static int alloc_n(emc_plan* p, T** ptr, size_t n) {
 }
 
 // ------------------------------------------------------------- bind ------
+// fp16(k) times a power of two: exact (k's FP16 form has 11 significant bits,
+// and the scale keeps its last one at 2^-17 or above).
+__device__ __forceinline__ __half scaled_count(float k, float scale) {
+  return __float2half_rn(__half2float(__float2half_rn(k)) * scale);
+}
+
 __global__ void gather_coords_kernel(const int* __restrict__ pix, const float* __restrict__ x,
                                      const float* __restrict__ y, const float* __restrict__ z,
                                      float* cx, float* cy, float* cz, int Kp) {
@@ -90,15 +96,14 @@ __global__ void pattern_norm_kernel(const float* __restrict__ images, const int*
 // fast index so that a pattern's row stays in L2 while its blocks run; flags
 // and part[i][block] (the block's sum of k, FP64, fixed order) reduced by
 // warp shuffles and one barrier.  Kraw / Kt / K2 (FP32 path) may be null;
-// with Kh non-null the kernel also writes the tensor path's FP16 operands
-// (the same values as tc_pattern_ops_kernel with scale k2_scale).
+// with Kh non-null the kernel also writes the tensor path's FP16 counts
+// (the same values as tc_pattern_ops_kernel with the same scale).
 __global__ void pattern_ops_kernel(const float* __restrict__ images, const int* __restrict__ pix,
                                    const float* __restrict__ cnorm, int n2, int N, int Kp,
                                    float* __restrict__ Kraw, float* __restrict__ Kt,
                                    float* __restrict__ K2, int* __restrict__ flags,
                                    const int* __restrict__ perm, double* __restrict__ part,
-                                   __half* __restrict__ Kh, __half* __restrict__ K2h,
-                                   __half* __restrict__ K2l, float k2_scale) {
+                                   __half* __restrict__ Kh, float count_scale) {
   const int nqb = (Kp + 255) / 256;
   const int i = (int)(blockIdx.x / nqb);
   const int q = (int)(blockIdx.x % nqb) * 256 + threadIdx.x;
@@ -137,17 +142,7 @@ __global__ void pattern_ops_kernel(const float* __restrict__ images, const int* 
     const float kt = k >= 1e-10f ? k : 0.0f;  // the reference's (double)k > 1e-10
     if (Kt) Kt[o] = kt;
     if (K2) K2[o] = __fmul_rn(kt, kt);
-    if (Kh) {
-      const __half kh = __float2half_rn(v);
-      const float kr = __half2float(kh);
-      const float k2 = kr * kr * k2_scale;
-      const __half hi = __float2half_rn(k2);
-      Kh[o] = kh;
-      if (K2h) {
-        K2h[o] = hi;
-        K2l[o] = __float2half_rn(k2 - __half2float(hi));
-      }
-    }
+    if (Kh) Kh[o] = scaled_count(v, count_scale);
   }
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -187,8 +182,7 @@ __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
     const float* __restrict__ images, const int* __restrict__ pix, const float* __restrict__ cnorm,
     int n2, int N, int Kp, float* __restrict__ Kraw, float* __restrict__ Kt,
     float* __restrict__ K2, int* __restrict__ flags, const int* __restrict__ perm,
-    float* __restrict__ Ksum, __half* __restrict__ Kh, __half* __restrict__ K2h,
-    __half* __restrict__ K2l, float k2_scale) {
+    float* __restrict__ Ksum, __half* __restrict__ Kh, float count_scale) {
   extern __shared__ __align__(16) unsigned char row_smem[];
   float* srow = reinterpret_cast<float*>(row_smem);
   double* wsum = reinterpret_cast<double*>(row_smem + (size_t)n2 * sizeof(float));
@@ -236,22 +230,9 @@ __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
     const float kt1 = k[1] >= 1e-10f ? k[1] : 0.0f;
     if (Kt) *reinterpret_cast<float2*>(Kt + o) = make_float2(kt0, kt1);
     if (K2) *reinterpret_cast<float2*>(K2 + o) = make_float2(__fmul_rn(kt0, kt0), __fmul_rn(kt1, kt1));
-    if (Kh) {
-      __half kh[2], hi[2], lw[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        kh[u] = __float2half_rn(v[u]);
-        const float kr = __half2float(kh[u]);
-        const float k2 = kr * kr * k2_scale;
-        hi[u] = __float2half_rn(k2);
-        lw[u] = __float2half_rn(k2 - __half2float(hi[u]));
-      }
-      *reinterpret_cast<__half2*>(Kh + o) = __halves2half2(kh[0], kh[1]);
-      if (K2h) {
-        *reinterpret_cast<__half2*>(K2h + o) = __halves2half2(hi[0], hi[1]);
-        *reinterpret_cast<__half2*>(K2l + o) = __halves2half2(lw[0], lw[1]);
-      }
-    }
+    if (Kh)
+      *reinterpret_cast<__half2*>(Kh + o) =
+          __halves2half2(scaled_count(v[0], count_scale), scaled_count(v[1], count_scale));
   }
   bits = (int)__reduce_or_sync(0xffffffffu, (unsigned)bits);
   vmax = (int)__reduce_max_sync(0xffffffffu, (unsigned)vmax);
@@ -286,7 +267,6 @@ __global__ void pattern_sums_kernel(const double* __restrict__ part, int N, int 
 }
 
 // ------------------------------------------------------------ expand -----
-constexpr float kPoisC = 0.02f;       // emc_cuda.cu:205
 constexpr float kSliceFloor = 1e-6f;  // true-Poisson floor for unknown voxels
 
 template <int INTERP>
@@ -353,7 +333,7 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
   // go out as 8-byte stores (Kp is a multiple of 128)
   constexpr int kSliceRows = slice_rows_per_block<INTERP>();
   const int r0 = blockIdx.x * kSliceRows;
-  const int gl_end = ops.gl_end ? 32 * __ldg(ops.gl_end) : Kp;  // G lo pixels
+  const int hl_end = ops.hl_end ? 64 * __ldg(ops.hl_end) : Kp;  // H lo pixels
   const int nr = min(kSliceRows, R - r0);
   __shared__ RotMat sR[kSliceRows];
   if (threadIdx.x < nr) sR[threadIdx.x] = quat_to_matrix(rot + 4 * (size_t)(r0 + threadIdx.x));
@@ -370,6 +350,8 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
     const int pv[4] = {pp.x, pp.y, pp.z, pp.w};
     const float xv[4] = {X.x, X.y, X.z, X.w}, yv[4] = {Y.x, Y.y, Y.z, Y.w},
                 zv[4] = {Z.x, Z.y, Z.z, Z.w};
+    const bool live = ops.live && __ldg(ops.live + (q >> 6)) != 0;
+    int odd = 0;  // bit 0: an s <= 0, bit 1: one in (0, 1e-10)
 #pragma unroll
     for (int k = 0; k < kSliceRows; ++k) {
       if (k >= nr) break;  // uniform over the block
@@ -383,6 +365,7 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
         // one division per pixel: h = 1 / (s + c) serves A = s^2 h and the operands
         hv[u] = sv[u] > 0.0f ? 1.0f / (sv[u] + kPoisC) : 0.0f;
         if (pv[u] >= 0) {
+          if (!(sv[u] >= 1e-10f)) odd |= sv[u] > 0.0f ? 2 : 1;
           if (sv[u] > 0.0f) {
             cnt[k] += 1.0f;
             A[k] += sv[u] * sv[u] * hv[u];
@@ -393,10 +376,15 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
       // the tensor path takes its FP16 operands straight from s; the FP32
       // path keeps the slices
       const size_t e = (size_t)(r0 + k) * Kp + q;
-      if (ops.Gh)
-        rot_ops_store4(ops, e, sv, hv, q < gl_end);
+      if (ops.live)
+        rot_ops_store4(ops, e, sv, hv, live, q < hl_end);
       else
         *reinterpret_cast<float4*>(S + e) = make_float4(sv[0], sv[1], sv[2], sv[3]);
+    }
+    if (ops.inv && odd) {  // races store the same value
+      const size_t f = (size_t)(r0 >> 7) * ops.nkb + (q >> 6);
+      if (odd & 1) ops.inv[f] = 1;
+      if (odd & 2) ops.tiny[f] = 1;
     }
   }
   // per row: FP32 warp sums, then FP64 over the warps
@@ -428,6 +416,32 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
     rot_cnt[r0 + k] = (float)a;
     rot_A[r0 + k] = (float)b;
     rot_ssum[r0 + k] = (float)c;
+  }
+}
+
+// The plane T = [0 < s < 1e-10] of the likelihood's rotation operands, in
+// the (rotation tile, 64-pixel block) pairs that hold such a value -- none in
+// most iterations: a block per rotation tile looks at its flags and exits.
+template <int INTERP>
+__global__ void __launch_bounds__(256) tiny_plane_kernel(
+    const float* __restrict__ model, int side, const float* __restrict__ rot,
+    const int* __restrict__ pix, const float* __restrict__ cx, const float* __restrict__ cy,
+    const float* __restrict__ cz, int R, int Kp, const unsigned char* __restrict__ tiny, int nkb,
+    __half* __restrict__ T) {
+  const int rt = blockIdx.x;
+  for (int kb = 0; kb < nkb; ++kb) {
+    if (!__ldg(tiny + (size_t)rt * nkb + kb)) continue;  // uniform over the block
+    for (int e = threadIdx.x; e < 128 * 64; e += blockDim.x) {
+      const int r = rt * 128 + (e >> 6), q = kb * 64 + (e & 63);
+      if (r >= R) break;
+      const int pv = pix[q];
+      float s = 0.0f;
+      if (pv >= 0) {
+        const RotMat Rm = quat_to_matrix(rot + 4 * (size_t)r);
+        s = plan_sample<INTERP>(model, side, Rm, cx[q], cy[q], cz[q]);
+      }
+      T[(size_t)r * Kp + q] = __float2half_rn(s > 0.0f && s < 1e-10f ? 1.0f : 0.0f);
+    }
   }
 }
 
@@ -1396,24 +1410,22 @@ int emc::pattern_side(emc_plan* p, const int* d_perm, bool with_tc) {
   // Kt / K2 exist only for the FP32 path (null: not written).
   const int nqb = ceil_div(p->Kp, 256);
   // once the tensor-core operands exist, their FP16 counts come from the same
-  // pass at the current K^2 scale (bind re-runs them if the new counts need
+  // pass at the current scale (bind re-runs them if the new counts need
   // another scale)
   const bool fused = p->tc != nullptr && p->Kh != nullptr;
-  p->fused_k2_scale = fused ? p->k2_scale : 0.0f;
+  p->fused_scale = fused ? p->count_scale : 0.0f;
   const size_t row_smem = pattern_row_smem(n2, p->Kp);
   if (row_smem <= (size_t)kRowSmemMax) {
     pattern_row_kernel<<<N, kRowThreads, row_smem, ctx->stream>>>(
         p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->K2, p->flags, d_perm,
-        p->Ksum, fused ? p->Kh : nullptr, fused ? p->K2hi : nullptr, fused ? p->K2lo : nullptr,
-        p->k2_scale);
+        p->Ksum, fused ? p->Kh : nullptr, p->count_scale);
     if ((rc = after_launch(ctx, "pattern_row_kernel"))) return rc;
     if (with_tc && p->tc) return tc_pattern_side(p, d_perm, fused);
     return EMC_OK;
   }
   pattern_ops_kernel<<<(unsigned)N * (unsigned)nqb, 256, 0, ctx->stream>>>(
       p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->K2, p->flags, d_perm,
-      p->ksum_part, fused ? p->Kh : nullptr, fused ? p->K2hi : nullptr, fused ? p->K2lo : nullptr,
-      p->k2_scale);
+      p->ksum_part, fused ? p->Kh : nullptr, p->count_scale);
   if ((rc = after_launch(ctx, "pattern_ops_kernel"))) return rc;
   pattern_sums_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(p->ksum_part, N, nqb, p->Ksum);
   if ((rc = after_launch(ctx, "pattern_sums_kernel"))) return rc;
@@ -1533,20 +1545,28 @@ extern "C" int emc_plan_bind(emc_plan* p, const float* d_images, const int* d_ma
   return EMC_OK;
 }
 
+template <int INTERP>
+static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
+  emc_ctx* ctx = p->ctx;
+  slice_rows_kernel<INTERP>
+      <<<ceil_div(p->d.n_rot, slice_rows_per_block<INTERP>()), 256, 0, ctx->stream>>>(
+          model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S,
+          p->rot_cnt, p->rot_A, p->rot_ssum, ops);
+  int rc = after_launch(ctx, "slice_rows_kernel");
+  if (rc || !ops.tiny) return rc;
+  tiny_plane_kernel<INTERP><<<p->n_rt, 256, 0, ctx->stream>>>(
+      model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, ops.tiny, ops.nkb,
+      tc_tiny_plane(p));
+  return after_launch(ctx, "tiny_plane_kernel");
+}
+
 static int plan_expand(emc_plan* p, const float* model) {
   emc_ctx* ctx = p->ctx;
   const RotOps ops = tc_rot_ops(p);
-  if (p->d.interp == EMC_INTERP_NEAREST)
-    slice_rows_kernel<EMC_INTERP_NEAREST>
-        <<<ceil_div(p->d.n_rot, slice_rows_per_block<EMC_INTERP_NEAREST>()), 256, 0, ctx->stream>>>(
-        model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S,
-        p->rot_cnt, p->rot_A, p->rot_ssum, ops);
-  else
-    slice_rows_kernel<EMC_INTERP_TRILINEAR>
-        <<<ceil_div(p->d.n_rot, slice_rows_per_block<EMC_INTERP_TRILINEAR>()), 256, 0, ctx->stream>>>(
-        model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S,
-        p->rot_cnt, p->rot_A, p->rot_ssum, ops);
-  return after_launch(ctx, "slice_rows_kernel");
+  if (ops.inv)
+    EMC_CUDA(ctx, cudaMemsetAsync(p->rot_flags, 0, 2 * (size_t)p->n_rt * ops.nkb, ctx->stream));
+  return p->d.interp == EMC_INTERP_NEAREST ? expand_launch<EMC_INTERP_NEAREST>(p, model, ops)
+                                           : expand_launch<EMC_INTERP_TRILINEAR>(p, model, ops);
 }
 
 static int plan_estep_fp32(emc_plan* p) {
@@ -2022,7 +2042,7 @@ extern "C" int emc_plan_set_option(emc_plan* p, int option, int value) {
   if (option == EMC_OPT_GLO_TAIL) {
     EMC_REQUIRE(ctx, value >= 0 && value <= 1000000, "plan_set_option: G lo tail %d", value);
     p->glo_tail_ppm = value;
-    return p->tc ? tc_glo_extent(p) : EMC_OK;
+    return p->tc ? tc_block_lists(p) : EMC_OK;
   }
   if (option == EMC_OPT_MSTEP_QLO) {
     EMC_REQUIRE(ctx, value == 0 || value == 1, "plan_set_option: q_lo %d", value);

@@ -25,7 +25,9 @@ struct emc_plan {
   bool counts_integer = false;     // every count is an integer in [0, 65504]
   int count_max = 0;               // the largest count
   int counts_round = 0;            // tensor path: counts above 2048 rounded to FP16
-  float k2_scale = 1.0f / 128.0f;  // K^2 operand = k^2 k2_scale (hi + lo), set at bind
+  // the likelihood's count operands are k and k (k - 1) times this power of two
+  // (set at bind; 1 for true Poisson)
+  float count_scale = 1.0f / 128.0f;
 
   // bound inputs (caller owned)
   const float* images = nullptr;
@@ -42,23 +44,31 @@ struct emc_plan {
   float* Kraw = nullptr;  // k (x c_i when normalising); FP32 plans only
   double* ksum_part = nullptr;  // [N][Kp / 256] block sums of k
   std::vector<int> h_mask, h_pix;  // the bound mask and its compacted pixels (re-binds)
-  float fused_k2_scale = 0.0f;  // K^2 scale of FP16 operands written by pattern_ops (0: none)
+  float fused_scale = 0.0f;  // count_scale of FP16 counts written by the pattern pass (0: none)
   float* Kt = nullptr;    // k if k > 1e-10 else 0
   float* K2 = nullptr;    // Kt^2
   float* Ksum = nullptr;  // [N] sum_p k
   float* cnorm = nullptr; // [N] c_i (1 when not normalising)
 
-  // pattern operands (tensor-core path): counts as FP16, rows of Kp
+  // pattern operands (tensor-core path), rows of Kp, times count_scale
   __half* Kh = nullptr;      // k
-  __half* K2hi = nullptr;    // fp16(k^2 * 2^-e)
-  __half* K2lo = nullptr;    // k^2 * 2^-e - K2hi
-  unsigned char* k2lo_any = nullptr;  // [Np/128][Kp/32] block has a nonzero K2lo
-  // [Np/128 + 1] the likelihood's G lo term runs on the k-blocks below glo_kb[pt]
-  // of pattern tile pt: the blocks after it hold at most glo_tail_ppm / 1e6 of
-  // every pattern's counts (EMC_OPT_GLO_TAIL; 0: G lo on every block);
-  // glo_kb[Np/128] is the largest of them
-  int* glo_kb = nullptr;
+  __half* Jh = nullptr;      // fp16(j), j = k (k - 1): written in blocks with a count above 1
+  __half* Jl = nullptr;      // j - Jh: written in blocks where it is not 0
+  float *ktot = nullptr, *k2tot = nullptr;  // [Np] sum k, sum k^2 (exact, then rounded)
+  unsigned char* blk_bits = nullptr;  // [Np/128][Kp/64] what the block holds (es::kJ ..)
+  // the blocks each pattern tile (and pair of tiles) has counts in, with their
+  // bits: index << 8 | bits, in order; never empty
+  uint32_t *pt_list = nullptr, *pp_list = nullptr;
+  int *pt_n = nullptr, *pp_n = nullptr;
+  unsigned char* blk_live = nullptr;  // [Kp/64] some pattern counts there
+  // [Np/128 + 1] K . H takes H's lo half on the 64-pixel blocks below lo_kb[pt]:
+  // the blocks after it hold at most 300 glo_tail_ppm / 1e6 of every pattern's
+  // counts (EMC_OPT_GLO_TAIL; 0: every block); lo_kb[Np/128] is the largest
+  int* lo_kb = nullptr;
   int glo_tail_ppm = 1000;
+  // [2][Rp/128][Kp/64] per iteration: a slice value s <= 0 / in (0, 1e-10) among
+  // the tile's rotations and the block's pixels
+  unsigned char* rot_flags = nullptr;
   __half* KhT = nullptr;     // [Kp][Np] transposed counts for the M-step
 
   // rotation side, per iteration
@@ -193,33 +203,40 @@ void prune_free(emc_plan* p);
 int prune_reset(emc_plan* p);
 int tc_pattern_side(emc_plan* p, const int* d_perm, bool counts_done = false);
 int tc_ensure_qlo(emc_plan* p);
-int tc_glo_extent(emc_plan* p);  // glo_kb from the bound counts and glo_tail_ppm
+int tc_block_lists(emc_plan* p);  // count sums, lo_kb and block lists from the bound counts
+__half* tc_tiny_plane(emc_plan* p);  // 1 where 0 < s < 1e-10 (blocks flagged tiny)
 int pattern_side(emc_plan* p, const int* d_perm, bool with_tc);
+constexpr float kPoisC = 0.02f;  // emc_cuda.cu:205
+
 // Rotation-side FP16 operands of the tensor-core likelihood, written by the
-// expand kernel straight from each slice value s (no FP32 slice buffer):
-// reference likelihood: M' = [s >= 1e-10], M'S * 2^-8, G = s / (s + c) and
-// H = 1 / (s + c) (c = 0.02; zero where s <= 0) as FP16 hi + lo; true Poisson:
-// log max(s, 1e-6) as FP16 hi + lo in Gh / Gl.  flags[0] |= 4 when M'S * 2^-8
-// leaves the FP16 range.
+// expand kernel straight from each slice value s (no FP32 slice buffer).
+// Reference likelihood: M'S = [s >= 1e-10] s 2^-8, H = 1 / (s + 0.02) with 0
+// where s <= 0 (its lo half in Hl where that is read), I = [s <= 0], and the
+// flags of the 64-pixel blocks that hold such pixels or an s in (0, 1e-10);
+// true Poisson: log max(s, 1e-6) as hi + lo in Lh / Ll.  Blocks in which no pattern counts are not
+// written (nothing reads them).  flags[0] |= 4 when M'S leaves the FP16 range.
 struct RotOps {
-  __half *Mp = nullptr, *MSh = nullptr, *Gh = nullptr, *Gl = nullptr, *Hh = nullptr, *Hl = nullptr;
+  __half *MS = nullptr, *Hh = nullptr, *Hl = nullptr, *Iv = nullptr;
+  __half *Lh = nullptr, *Ll = nullptr;
   int* flags = nullptr;
-  int logs = 0;
-  // device int: G lo is read (and written) only in the 32-pixel blocks below
+  const unsigned char* live = nullptr;  // [nkb] (null: no tensor path)
+  unsigned char *inv = nullptr, *tiny = nullptr;  // [n_rt][nkb]
+  int nkb = 0;
+  // device int: H lo is read (and written) only in the 64-pixel blocks below
   // it, the largest count-tail bound of the pattern tiles (null: every block)
-  const int* gl_end = nullptr;
+  const int* hl_end = nullptr;
 };
 
 // The operands of four neighbouring pixels e .. e + 3 (e a multiple of 4) as
-// 8-byte stores; hv = 1 / (s + 0.02) where s > 0 (0 elsewhere), computed by
-// the caller.  The same values as rot_ops_store2, pixel by pixel.
+// 8-byte stores; hv = 1 / (s + 0.02) where s > 0, else 0, computed by the caller.
 __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const float (&sv)[4],
-                                               const float (&hv)[4], bool g_lo) {
+                                               const float (&hv)[4], bool live, bool h_lo) {
   union H4 {
     __half h[4];
     uint2 u;
   };
-  if (o.logs) {
+  if (o.Lh) {
+    if (!live) return;
     H4 hi, lo;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
@@ -227,33 +244,30 @@ __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const 
       hi.h[u] = __float2half_rn(l);
       lo.h[u] = __float2half_rn(l - __half2float(hi.h[u]));
     }
-    *reinterpret_cast<uint2*>(o.Gh + e) = hi.u;
-    *reinterpret_cast<uint2*>(o.Gl + e) = lo.u;
+    *reinterpret_cast<uint2*>(o.Lh + e) = hi.u;
+    *reinterpret_cast<uint2*>(o.Ll + e) = lo.u;
     return;
   }
-  H4 mp4, ms4, gh4, gl4, hh4, hl4;
+  H4 ms4, hh4, hl4, iv4;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const float s = sv[u];
     const bool mp = s >= 1e-10f;
-    const bool m = s > 0.0f;
-    const float ms = mp ? s * (1.0f / 256.0f) : 0.0f;
-    if (ms > 60000.0f) atomicOr(o.flags, 4);
-    const float h = hv[u];
-    const float g = m ? s * h : 0.0f;
-    mp4.h[u] = __float2half_rn(mp ? 1.0f : 0.0f);
+    float ms = mp ? s * (1.0f / 256.0f) : 0.0f;
+    if (ms > 60000.0f) {
+      atomicOr(o.flags, 4);
+      ms = 60000.0f;  // the operand stays finite: later models may skip this block
+    }
     ms4.h[u] = __float2half_rn(ms);
-    gh4.h[u] = __float2half_rn(g);
-    gl4.h[u] = __float2half_rn(g - __half2float(gh4.h[u]));
-    hh4.h[u] = __float2half_rn(h);
-    hl4.h[u] = __float2half_rn(h - __half2float(hh4.h[u]));
+    iv4.h[u] = __float2half_rn(s > 0.0f ? 0.0f : 1.0f);
+    hh4.h[u] = __float2half_rn(hv[u]);
+    hl4.h[u] = __float2half_rn(hv[u] - __half2float(hh4.h[u]));
   }
-  *reinterpret_cast<uint2*>(o.Mp + e) = mp4.u;
-  *reinterpret_cast<uint2*>(o.MSh + e) = ms4.u;
-  *reinterpret_cast<uint2*>(o.Gh + e) = gh4.u;
-  if (o.Gl && g_lo) *reinterpret_cast<uint2*>(o.Gl + e) = gl4.u;
+  if (!live) return;
+  *reinterpret_cast<uint2*>(o.MS + e) = ms4.u;
   *reinterpret_cast<uint2*>(o.Hh + e) = hh4.u;
-  if (o.Hl) *reinterpret_cast<uint2*>(o.Hl + e) = hl4.u;
+  *reinterpret_cast<uint2*>(o.Iv + e) = iv4.u;
+  if (o.Hl && h_lo) *reinterpret_cast<uint2*>(o.Hl + e) = hl4.u;
 }
 
 RotOps tc_rot_ops(emc_plan* p);  // the plan's operand buffers (all null for FP32 plans)

@@ -146,12 +146,17 @@ __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* map) {
 // 2D tiled bulk tensor load into shared memory, completing on `bar`.
 // x = innermost (contiguous) coordinate in elements, y = row.
 __device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y,
-                                            uint64_t* bar) {
+                                            uint32_t bar) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
       " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(smem_dst)),
-      "l"((uint64_t)map), "r"(x), "r"(y), "r"(smem_u32(bar))
+      "l"((uint64_t)map), "r"(x), "r"(y), "r"(bar)
       : "memory");
+}
+
+__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y,
+                                            uint64_t* bar) {
+  tma_load_2d(smem_dst, map, x, y, smem_u32(bar));
 }
 
 // ---- tcgen05 ---------------------------------------------------------------
@@ -216,6 +221,18 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
       : "r"(taddr));
 #pragma unroll
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
+}
+
+// The same for 8 columns.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8]) {
+  uint32_t r[8];
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7])
+      : "r"(taddr));
+#pragma unroll
+  for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(r[i]);
 }
 
 __device__ __forceinline__ void tmem_wait_ld() {
@@ -320,7 +337,21 @@ __device__ __forceinline__ void mma_commit_pair(uint64_t* bar, uint16_t cta_mask
       : "memory");
 }
 
-__device__ __forceinline__ bool elect_one_lane() { return (threadIdx.x & 31) == 0; }
+// True in one lane of a converged warp.  The single threads that issue TMA
+// loads and MMAs are chosen with it rather than by their lane number: the
+// compiler then knows that one lane is active, and forms the uniform operands
+// of these instructions directly instead of in a loop over the active lanes.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t on;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(on)
+      :
+      : "memory");
+  return on != 0;
+}
 
 }  // namespace ptx
 }  // namespace emc

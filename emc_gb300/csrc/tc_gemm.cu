@@ -1,21 +1,18 @@
 // Tensor-core (tcgen05 + TMA) E-step and M-step of the fused iteration.
 //
-// E-step.  For a tile of 128 patterns (M, one TMEM lane each) x 128
-// rotations (N) the reference's "poisson" likelihood with per-pair scaling
-// (emc_cuda.cu:196-216, 438-454) is expanded into four contractions over the
-// compacted pixels, accumulated in TMEM (FP32, 4 x 128 columns = all 512):
-//   num = sum k^2 [s > 1e-10]             (K^2 hi + lo)  x  M'         exact
-//   den = sum k s [s > 1e-10]             K              x  (M' S) hi
-//   B   = sum k s/(s+c) [s > 0]           K              x  (G hi + lo)
-//   C   = sum k^2 /(s+c) [s > 0]          (K^2 hi + lo)  x  (H hi + lo)
+// E-step.  For a tile of patterns (M, one TMEM lane each) x 128 rotations (N)
+// the reference's "poisson" likelihood with per-pair scaling (emc_cuda.cu:
+// 196-216, 438-454) is expanded into four sums over the compacted pixels,
+//   num = sum k^2 [s > 1e-10]        den = sum k s [s > 1e-10]
+//   B   = sum k s/(s+c) [s > 0]      C   = sum k^2 /(s+c) [s > 0]
 // so that with 1/phi = den/num:  S_ri = A_r - 2 B/phi + C/phi^2  and
-// L_ri = log w_r - S_ri / (2 count_r sigma^2).  Counts are integers <= 2048,
-// exact in FP16; K^2 * 2^-7 is split exactly into two FP16 terms; the
-// rotation-side factors are split hi + lo (the lo x lo products are dropped,
-// relative size 2^-22).  The epilogue (4 warps, one pattern row per thread)
-// forms L and phi, stores them coalesced along patterns, and keeps a running
-// (max, sum exp) per pattern over the tile's rotations: the per-tile LSE
-// partials that the FP64 normaliser combines.
+// L_ri = log w_r - S_ri / (2 count_r sigma^2).  They come from contractions of
+// the counts (exact in FP16, with k (k - 1) as two FP16 terms) with M'S, with
+// H = 1/(s+c) and, where a slice has invalid pixels, with their indicator; the
+// section below says how.  The epilogue forms L and phi, stores them coalesced
+// along patterns, and keeps a running (max, sum exp) per pattern over the
+// tile's rotations: the per-tile LSE partials that the FP64 normaliser
+// combines.
 //
 // M-step.  U = Q K^T over the patterns for a tile of 128 rotations x 256
 // pixels, Q = P / phi split hi + lo in FP16 with a per-rotation power-of-two
@@ -84,15 +81,12 @@ static int make_map(emc_ctx* ctx, CUtensorMap* map, const void* base, uint64_t r
 
 // ---------------------------------------------------- pattern operands ---
 
-// Counts -> FP16 operands, rows of Kp (patterns padded to Np with zeros):
+// Counts -> FP16 operand, rows of Kp (patterns padded to Np with zeros):
 // Kh = fp16(k) (k itself up to 2048; larger counts rounded to 11 significant
-// bits), K2h + K2l = Kh^2 * k2_scale exactly (Kh^2 has at most 22 significant
-// bits, and k2_scale keeps the largest below 2^15 and every value a multiple
-// of 2^-24) (K2h == nullptr: Kh only).
+// bits) times the power of two `scale`, exactly.
 __global__ void tc_pattern_ops_kernel(const float* __restrict__ images, const int* __restrict__ pix,
                                       int n2, int N, int Kp, __half* __restrict__ Kh,
-                                      __half* __restrict__ K2h, __half* __restrict__ K2l,
-                                      const int* __restrict__ perm, float k2_scale) {
+                                      const int* __restrict__ perm, float scale) {
   // one block per (pattern row, 256 pixels), pixel blocks the fast index
   const int nqb = (Kp + 255) / 256;
   const int i = (int)(blockIdx.x / nqb);
@@ -103,85 +97,189 @@ __global__ void tc_pattern_ops_kernel(const float* __restrict__ images, const in
     const int p = pix[q];
     if (p >= 0) k = __ldg(images + (size_t)(perm ? perm[i] : i) * n2 + p);
   }
-  const __half kh = __float2half_rn(k);
-  const float kr = __half2float(kh);
-  const float k2 = kr * kr * k2_scale;  // exact in FP32: 22 significant bits
-  const __half hi = __float2half_rn(k2);
-  const __half lo = __float2half_rn(k2 - __half2float(hi));
-  const size_t o = (size_t)i * Kp + q;
-  Kh[o] = kh;
-  if (K2h) {
-    K2h[o] = hi;
-    K2l[o] = lo;
-  }
+  Kh[(size_t)i * Kp + q] = __float2half_rn(__half2float(__float2half_rn(k)) * scale);
 }
 
-// flags[pt][kb] = any K2l != 0 in rows pt*128..+127, cols kb*32..+31.
-__global__ void tc_k2lo_flags_kernel(const __half* __restrict__ K2l, int Kp,
-                                     unsigned char* __restrict__ flags, int nkb) {
-  const int pt = blockIdx.y, kb = blockIdx.x;
-  int any = 0;
-  for (int e = threadIdx.x; e < 128 * 32; e += blockDim.x) {
-    const int r = pt * 128 + e / 32, c = kb * 32 + e % 32;
-    if (__half2float(K2l[(size_t)r * Kp + c]) != 0.0f) any = 1;
-  }
-  any = __syncthreads_or(any);
-  if (threadIdx.x == 0) flags[(size_t)pt * nkb + kb] = (unsigned char)any;
-}
+namespace es {  // bits of a (128-pattern tile, 64-pixel block) in blk_bits and the lists
+constexpr uint32_t kJ = 1;    // a count above 1
+constexpr uint32_t kJlo = 2;  // k (k - 1) has a second FP16 term
+constexpr uint32_t kHlo = 4;  // lists: before the count tail, K . H takes H's lo half
+constexpr uint32_t kAny = 8;  // a count
+}  // namespace es
 
-// The sum of one 32-pixel block of an FP16 count row (64 bytes, 16-byte aligned).
-__device__ __forceinline__ float count_block_sum(const __half* k) {
-  const uint4* v = reinterpret_cast<const uint4*>(k);
-  float s = 0.0f;
+// bits[pt][kb] of the block, and in blocks with a count above 1 the operand
+// j = k (k - 1) as FP16 hi (and lo where some term needs it).  One CTA per block
+// of two pattern tiles: a pair of CTAs multiplies both where one needs it, so
+// j is written for both.  256 rows x 128 B, eight 16-byte loads a thread.
+__global__ void __launch_bounds__(256) tc_count_blocks_kernel(
+    const __half* __restrict__ Kh, int Kp, int nkb, int n_pt, float scale,
+    __half* __restrict__ Jh, __half* __restrict__ Jl, unsigned char* __restrict__ bits) {
+  const int kb = blockIdx.x, pt0 = 2 * blockIdx.y;
+  const int nt = min(2, n_pt - pt0);
+  const float inv = 1.0f / scale;
+  union V {
+    uint4 u;
+    __half h[8];
+  } v[2][4];
+  int any[2] = {0, 0}, two[2] = {0, 0}, low[2] = {0, 0};
+  auto at = [&](int t, int j) {
+    const int e = threadIdx.x + 256 * j;
+    return (size_t)((pt0 + t) * 128 + (e >> 3)) * Kp + kb * 64 + (e & 7) * 8;
+  };
 #pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const uint4 u = v[j];
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+  for (int t = 0; t < 2; ++t) {
+    if (t >= nt) break;
 #pragma unroll
-    for (int h = 0; h < 4; ++h) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[h]));
-      s += f.x + f.y;
+    for (int j = 0; j < 4; ++j) v[t][j].u = *reinterpret_cast<const uint4*>(Kh + at(t, j));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      any[t] |= (v[t][j].u.x | v[t][j].u.y | v[t][j].u.z | v[t][j].u.w) != 0;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) two[t] |= __half2float(v[t][j].h[c]) * inv > 1.0f;
     }
   }
-  return s;
+#pragma unroll
+  for (int t = 0; t < 2; ++t) {
+    any[t] = __syncthreads_or(any[t]);
+    two[t] = __syncthreads_or(two[t]);
+  }
+  if ((two[0] | two[1]) && Jh) {
+    V lo[2][4];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      if (t >= nt) break;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        V hi;
+#pragma unroll
+        for (int c = 0; c < 8; ++c) {
+          const float k = __half2float(v[t][j].h[c]) * inv;
+          const float x = k * (k - 1.0f) * scale;
+          hi.h[c] = __float2half_rn(x);
+          lo[t][j].h[c] = __float2half_rn(x - __half2float(hi.h[c]));
+          low[t] |= __half2float(lo[t][j].h[c]) != 0.0f;
+        }
+        *reinterpret_cast<uint4*>(Jh + at(t, j)) = hi.u;
+      }
+    }
+    low[0] = __syncthreads_or(low[0]);
+    low[1] = __syncthreads_or(low[1]);
+    if (low[0] | low[1])
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        if (t >= nt) break;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(Jl + at(t, j)) = lo[t][j].u;
+      }
+  }
+  if (threadIdx.x < nt) {
+    const int t = threadIdx.x;
+    bits[(size_t)(pt0 + t) * nkb + kb] = (unsigned char)(
+        ((t ? any[1] : any[0]) ? es::kAny : 0u) | ((t ? two[1] : two[0]) ? es::kJ : 0u) |
+        ((t ? low[1] : low[0]) ? es::kJlo : 0u));
+  }
 }
 
-// One warp per pattern row n: the last 32-pixel block b whose suffix (blocks
-// b ..) still holds more than eps of the row's counts; glo_kb[n / 128] (zeroed
-// before) becomes the largest b + 1 over the tile's rows, and glo_kb[n_pt]
-// the largest over all tiles (the expand writes G lo below it).  Lane l takes a
-// contiguous run of blocks: run sums, a warp prefix scan, then a second walk
-// over its run.  Integer counts below 2^24 in total sum exactly in FP32.
-__global__ void __launch_bounds__(256) tc_glo_extent_kernel(const __half* __restrict__ Kh, int Kp,
-                                                            int nkb, int N, float eps,
-                                                            int* __restrict__ glo_kb) {
+// One warp per pattern row n: ktot = sum k and k2tot = sum k^2 (integers, then
+// rounded once), and the last 64-pixel block b whose suffix (blocks b ..) still
+// holds more than eps of the row's counts: lo_kb[n / 128] (zeroed before)
+// becomes the largest b + 1 over the tile's rows, lo_kb[n_pt] the largest of
+// all.  Lane l takes a contiguous run of blocks: run sums, a warp prefix scan,
+// then a second walk over its run.
+__global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __restrict__ Kh, int Kp,
+                                                            int nkb, int N, float scale, float eps,
+                                                            float* __restrict__ ktot,
+                                                            float* __restrict__ k2tot,
+                                                            int* __restrict__ lo_kb) {
   const int n = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (n >= N) return;  // whole warps
+  const float inv = 1.0f / scale;
   const __half* k = Kh + (size_t)n * Kp;
   const int per = (nkb + 31) / 32;
   const int b0 = min(lane * per, nkb), b1 = min(b0 + per, nkb);
-  float c = 0.0f;
-  for (int b = b0; b < b1; ++b) c += count_block_sum(k + 32 * (size_t)b);
-  float inc = c;
+  auto block = [&](int b, unsigned long long& s2) {  // the block's sum of k; k^2 added to s2
+    const uint4* v = reinterpret_cast<const uint4*>(k + 64 * (size_t)b);
+    unsigned s = 0;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint4 u = v[j];
+      if ((u.x | u.y | u.z | u.w) == 0) continue;
+      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+      for (int h = 0; h < 4; ++h) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[h]));
+        const unsigned x = (unsigned)(f.x * inv), y = (unsigned)(f.y * inv);
+        s += x + y;
+        s2 += (unsigned long long)x * x + (unsigned long long)y * y;
+      }
+    }
+    return s;
+  };
+  unsigned long long s2 = 0, dummy = 0, c = 0;
+  for (int b = b0; b < b1; ++b) c += block(b, s2);
+  unsigned long long incl = c;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const float t = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += t;
+    const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
   }
-  const float total = __shfl_sync(0xffffffffu, inc, 31);
-  const float lim = eps * total;
-  float pre = inc - c;  // the counts of the blocks before b0
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  const unsigned long long total = __shfl_sync(0xffffffffu, incl, 31);
+  const float lim = eps * (float)total;
+  unsigned long long pre = incl - c;  // the counts of the blocks before b0
   int last = -1;
   for (int b = b0; b < b1; ++b) {
-    if (total - pre > lim) last = b;  // the suffix from b
-    pre += count_block_sum(k + 32 * (size_t)b);
+    if ((float)(total - pre) > lim) last = b;  // the suffix from b
+    pre += block(b, dummy);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
-  if (lane == 0 && last >= 0) {
-    atomicMax(glo_kb + n / 128, last + 1);
-    atomicMax(glo_kb + (N + 127) / 128, last + 1);
+  if (lane == 0) {
+    ktot[n] = (float)total;
+    k2tot[n] = (float)s2;
+    if (last >= 0) {
+      atomicMax(lo_kb + n / 128, last + 1);
+      atomicMax(lo_kb + (N + 127) / 128, last + 1);
+    }
   }
+}
+
+// List i < n_pt: the blocks of pattern tile i; list n_pt + i: those of tiles 2 i
+// and 2 i + 1 together.  One warp each.  A tile without counts keeps block 0, so
+// that its accumulators are written.  The last warps: live[kb].
+__global__ void __launch_bounds__(32) tc_block_lists_kernel(
+    const unsigned char* __restrict__ bits, int n_pt, int nkb, const int* __restrict__ lo_kb,
+    uint32_t* __restrict__ pt_list, int* __restrict__ pt_n, uint32_t* __restrict__ pp_list,
+    int* __restrict__ pp_n, unsigned char* __restrict__ live) {
+  const int lane = threadIdx.x, n_pp = (n_pt + 1) / 2;
+  int i = blockIdx.x;
+  if (i >= n_pt + n_pp) {
+    const int kb = (i - n_pt - n_pp) * 32 + lane;
+    if (kb >= nkb) return;
+    int any = 0;
+    for (int t = 0; t < n_pt; ++t) any |= bits[(size_t)t * nkb + kb] & es::kAny;
+    live[kb] = any || kb == 0;
+    return;
+  }
+  const bool pair = i >= n_pt;
+  if (pair) i -= n_pt;
+  const int t0 = pair ? 2 * i : i, t1 = pair ? min(2 * i + 1, n_pt - 1) : i;
+  uint32_t* list = (pair ? pp_list : pt_list) + (size_t)i * nkb;
+  const int end = lo_kb ? max(lo_kb[t0], lo_kb[t1]) : 0;
+  int n = 0;
+  for (int kb0 = 0; kb0 < nkb; kb0 += 32) {
+    const int kb = kb0 + lane;
+    uint32_t b = 0;
+    if (kb < nkb) b = bits[(size_t)t0 * nkb + kb] | bits[(size_t)t1 * nkb + kb];
+    const unsigned on = __ballot_sync(0xffffffffu, (b & es::kAny) != 0);
+    if (b & es::kAny)
+      list[n + __popc(on & ((1u << lane) - 1u))] =
+          (uint32_t)kb << 8 | (b & (es::kJ | es::kJlo)) | (kb < end ? es::kHlo : 0u);
+    n += __popc(on);
+  }
+  if (n == 0 && lane == 0) list[0] = 0;
+  if (lane == 0) (pair ? pp_n : pt_n)[i] = max(n, 1);
 }
 
 // [rows][cols] -> [cols][rows], FP16: 64 x 64 tiles, moved with 4-byte
@@ -221,26 +319,66 @@ __global__ void transpose_h_kernel(const __half* __restrict__ in, int rows, int 
 }
 
 // ------------------------------------------------------------ E-step -----
-// One CTA owns 128 patterns x 128 rotations and all four contractions:
-//   B = K . G^T,  den = K . (M'S)^T,  C = K^2 . H^T,  num = K^2 . M'^T.
-// Operands that multiply the same pattern-side tile are stored next to each
-// other in shared memory ([G | M'S] and [H | M']), so each pair is one
-// 128 x 256 MMA: the pattern-side tile is read once per pair, which lowers
-// the shared-memory operand traffic per FLOP that bounds 128 x 128 MMAs.
-// TMEM columns: B 0-127, den 128-255, C 256-383, num 384-511.
+// num, den, B and C from contractions with H = 1/(s + c) only: with I = [s <= 0]
+// (H = 0 there), J = k (k - 1) and s/(s+c) = 1 - c/(s+c),
+//   den = K . (M'S)^T                  B   = k_tot - n_1 - c (K . H^T)
+//   C   = K . H^T + J . H^T            num = k2_tot - n_1 - n_J
+//   n_1 = K . I^T                      n_J = J . I^T
+// with k_tot and k2_tot summed exactly at bind (a pixel with 0 < s < 1e-10
+// counts in B and C but not in num: its k^2 is added to n_J through a plane T).
+// What each 64-pixel block of a pattern tile needs is decided at bind too:
+// nothing where no pattern of the tile counts, K x [M'S | H] where every count
+// is 0 or 1 (J = 0), J x H where one is larger, the products with I only where
+// the rotation tile has an invalid pixel.  The four-contraction form multiplied
+// K and K^2 by four operands on every block: at 128^3 x 20,000 patterns of 5,000
+// photons 4.4 products of 128 columns per block, 1.1 to 2.3 here.
+//
+// TMEM has room for four of the five sums: den and K.H in columns 0-255, n_1 and
+// J.H in 256-383 and 384-511.  Where a tile needs n_J, J x [H | I] runs first (pass
+// A, columns 256-511), and the epilogue warps move both sums out into the tile's
+// own part of phi and L, which they overwrite at the end.  One CTA owns 128 patterns x 128 rotations, or (PAIR) a cluster of
+// two 256 x 128 with 256-row MMAs issued by rank 0: each CTA then holds its own
+// 128 patterns and 64 of the 128 rows of every rotation operand, [M'S | H] (and
+// [H | I]) side by side, so the columns of such a 256-column product come in
+// quarters (den 0-63, K.H 0-63, den 64-127, K.H 64-127).  Per 64-pixel block and
+// CTA that is 32 KB for a 256 x 256 x 64 product (the M-step's ratio).
+//
+// The passes: A as above; C, K x H's lo half on the blocks before the count tail;
+// B, K x [M'S | H], K x I and, in tiles without pass A, J x H.  The tensor core
+// cuts a sum's last bits off at every addition, so small terms come first: C
+// before B, and every pass from the dim outer blocks to the bright inner ones,
+// which keeps the sums small for most of their additions.  Every stage of
+// a tile has the same places in shared memory (six slots of 32 KB to four of 56
+// KB on a pair), so that the threads that issue loads and products spend few
+// instructions on a stage: a plain block's products take 512 clocks, and
+// working out places for stages of many shapes took 750.  For the same reason
+// 256-column products are preferred: four issue in 370 clocks, whatever their
+// width, and run 512 (256 at 128 columns).
 namespace es {
 constexpr int BM = 128;        // patterns per tile (TMEM lanes)
 constexpr int BN = 128;        // rotations per tile
-constexpr int BK = 32;         // pixels per stage (64 B rows, 64B swizzle)
-constexpr int STAGES = 3;
-constexpr int TILE_BYTES = 128 * BK * 2;  // 8 KB, both operand sides
-// stage slots: pattern side, then the two N=256 pairs, then the lo terms
-enum Slot { sK = 0, sK2h, sK2l, sGh, sMS, sHh, sMp, sGl, sHl, kSlots };
-constexpr int STAGE_BYTES = kSlots * TILE_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 8192 + 1024;  // barriers, row data, parts
+constexpr int BK = 64;         // pixels per stage (128 B rows, 128B swizzle)
+constexpr int CHUNK = 8192;    // 64 rows of one operand
+constexpr int CHUNKS = 27;
+constexpr int NB = 8;          // slots at most
+// A thread takes over 100 clocks for each TMA load it issues: one producer for
+// the three to six loads of a stage would set the pace, so three warps share them.
+constexpr int PRODUCERS = 3;   // pattern side | first | second rotation operand
+constexpr int MMA_WARP = PRODUCERS, EPI_WARP0 = PRODUCERS + 1;
 constexpr int EPI_WARPS = 16;  // four per TMEM lane quarter, 32 columns each
 constexpr int EPI_PARTS = EPI_WARPS / 4;
-constexpr int THREADS = 64 + 32 * EPI_WARPS;
+constexpr int THREADS = 32 * (EPI_WARP0 + EPI_WARPS);
+static_assert(EPI_WARP0 % 4 == 0, "epilogue warp w reads TMEM lane quarter w % 4");
+// The block list with the rotation tile's flags is put together in shared
+// memory before the loop.  Entries beyond kList (more than 70,400 pixels with
+// counts) are read from global memory.
+constexpr int kList = 1100;
+constexpr uint32_t kInv = 16, kTiny = 32;  // flags of the rotation tile in an entry
+constexpr uint32_t kNJ = 64;               // of all entries: the tile needs n_J
+// barriers, per-rotation rows (3 x 128 floats), epilogue parts, list
+constexpr int EXTRA = 256 + 3 * BN * 4 + (EPI_PARTS - 1) * BM * 8 + kList * 4 + 16;
+constexpr int SMEM_BYTES = CHUNKS * CHUNK + EXTRA + 1024;
+static_assert(SMEM_BYTES <= 232448, "shared memory of the likelihood kernel");
 }  // namespace es
 
 // Tile of CTA b in a grouped raster over n_pt pattern tiles x n_rt rotation
@@ -269,18 +407,23 @@ __device__ __forceinline__ void raster_tile(int b, int raster, int n_pt, int n_r
 }
 
 struct TcEstepArgs {
-  int N, R, Kp, n_pt, n_rt, nkb;
+  int N, R, n_pt, n_rt, nkb;
   int raster;                     // tile order (raster_tile)
   int tile0;                      // CTA b runs tile tile0 + b of the order
-  int gh_lo;                      // lo terms: bit 0 G, bit 1 H (3: both, 0: hi only)
+  int gh_lo;                      // H lo: bit 0 in K.H before the tail, bit 1 everywhere
   const int2* tiles;              // pruned iteration: (pattern tile, rotation tile) per CTA
-  const unsigned char* k2lo_any;  // [n_pt][nkb]
-  const int* glo_kb;              // [n_pt] G lo runs on k-blocks below glo_kb[pt]
+  const uint32_t* list;           // [tiles][nkb] blocks of each pattern tile (pair)
+  const int* list_n;              // [tiles]
+  const unsigned char* rot_inv;   // [n_rt][nkb] the rotation tile has an s <= 0 there
+  const unsigned char* rot_tiny;  // [n_rt][nkb] ... an s in (0, 1e-10)
   const float* rot_cnt;
   const float* rot_A;
   const float* rotw;
   const float* cnorm;   // c_i (phi is stored as c_i num/den)
-  float k2_inv;         // 1 / k2_scale of the K^2 operand
+  const float* ktot;    // [N] sum k
+  const float* k2tot;   // [N] sum k^2
+  float k_inv;          // 1 / count_scale of the K and J operands
+  int zrow;             // a row past the rotation operands: TMA reads it as zeros
   const float* sigma;   // [1] annealing width (device memory)
   int known_intensity;
   float* L;
@@ -291,63 +434,183 @@ struct TcEstepArgs {
   uint32_t spin;  // polls per pipeline wait (ptx::kSpinLimit unless a debug option lowers it)
 };
 
-// Epilogue of the likelihood kernels (warps 2 .. 2 + EPI_WARPS - 1): EPI_PARTS
-// warps per TMEM lane quarter, each on a part of the 128 columns, so that
-// the expf / divide latency of one hides behind another.  Reads B, den, C and
-// num of this CTA's 128 patterns x 128 rotations from TMEM, writes L and
-// phi and the tile's (max, sum exp) per pattern.
+// The stages of a tile, from the bits of all its entries: where each operand
+// lies, in chunks from the slot's first (the pattern side takes two, a rotation
+// operand RC: 64 rows of a pair's 128, or all).
+template <bool PAIR>
+struct EsStages {
+  static constexpr int RC = PAIR ? 1 : 2;
+  // pass A: J, [H | I]; then what few tiles have: J lo, [H lo | 0], K, [0 | T]
+  static constexpr int aJ = 0, aH = 2, aI = 2 + RC;
+  int aJl, aHl, aK, aT;
+  // pass B: K, [M'S (or H lo) | H], I; in tiles without pass A: J, J lo, H lo
+  static constexpr int bK = 0, bMS = 2, bH = 2 + RC, bI = 2 + 2 * RC;
+  int bJ, bJl, bHl;
+  // pass C: K, [0 | H lo] (256 columns: a pair's K.H lies in two column quarters
+  // that one 128-column product cannot reach, and den starts from the 0)
+  static constexpr int cK = 0, cZ = 2, cHl = 2 + RC;
+  int size, slots;
+  // jh: J x H lo as well; full_h: H lo in M'S's place
+  __device__ __forceinline__ EsStages(uint32_t seen, bool nj, bool jh, bool full_h) {
+    const int jl = (seen & es::kJlo) ? 2 : 0;
+    int o = aI + RC;
+    aJl = o;
+    o += jl;
+    aHl = o;
+    o += jh ? 2 * RC : 0;
+    aK = o;
+    o += (seen & es::kTiny) ? 2 : 0;
+    aT = o;
+    o += (seen & es::kTiny) ? 2 * RC : 0;
+    const bool j = !nj && (seen & es::kJ);
+    int q = bI + ((seen & es::kInv) ? RC : 0);
+    bJ = q;
+    q += j ? 2 : 0;
+    bJl = q;
+    q += j ? jl : 0;
+    bHl = q;
+    q += j && jh && !full_h ? RC : 0;
+    size = max(q, nj ? o : 0);
+    slots = min(es::NB, es::CHUNKS / size);
+  }
+};
+
+// Entry b of a tile's work: its pattern tile's list entry with the rotation
+// tile's flags of that block.
+__device__ __forceinline__ uint32_t es_entry(const uint32_t* list, const unsigned char* inv,
+                                             const unsigned char* tiny, int b) {
+  const uint32_t e = __ldg(list + b);
+  const uint32_t kb = e >> 8;
+  return e | (inv[kb] ? es::kInv : 0u) | (tiny[kb] ? es::kTiny : 0u);
+}
+
+// a / b for normal a and b whose quotient is normal too: the hardware
+// reciprocal, the quotient by it, and one residual correction (Markstein 1990),
+// which leaves at most the last bit.  Half the instructions of the general
+// division, whose range checks num and den do not need.
+__device__ __forceinline__ float quotient(float a, float b) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+  const float q = a * r;
+  return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
+}
+
+// Epilogue of the likelihood kernel (warps EPI_WARP0 ..): EPI_PARTS warps per
+// TMEM lane quarter, each on a part of the 128 columns.  Reads the accumulators
+// of this CTA's 128 patterns x 128 rotations from TMEM, writes L and phi and
+// the tile's (max, sum exp) per pattern.
+template <bool PAIR>
 __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tmem, uint64_t* accum,
-                                               const float* s_A, const float* s_scale,
+                                               uint64_t* jdone, uint32_t jfree, const float* s_A, const float* s_scale,
                                                const float* s_lw, float2* s_half, int warp,
-                                               int lane, int n0, int r0, int rt) {
+                                               int lane, int n0, int r0, int rt, uint32_t seen) {
   using namespace es;
-  // EPI_PARTS warps per TMEM lane quarter, each on a part of the 128
-  // columns, so that the expf / divide latency of one hides behind another
   const int quarter = warp & 3;  // TMEM lanes this warp may access
-  const int half = (warp - 2) >> 2;  // column part
+  const int half = (warp - EPI_WARP0) >> 2;  // column part
   const int row = quarter * 32 + lane;
   const int n = n0 + row;
   const bool nok = n < a.N;
   const float ci = nok ? a.cnorm[n] : 1.0f;
+  const float ktot = nok ? a.ktot[n] : 0.0f, k2tot = nok ? a.k2tot[n] : 0.0f;
+  const bool full_h = a.known_intensity && (a.gh_lo & 2);
+  // which of the sums received a product (their columns hold old data otherwise)
+  const bool nj = seen & kNJ, have_j = !nj && (seen & kJ), have_1 = seen & kInv;
+  const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
+  const int cbeg = half * (BN / EPI_PARTS), cend = cbeg + BN / EPI_PARTS;
+  if (nj) {
+    // pass A's J.H to phi and n_J to L; the columns go back before the stores,
+    // whose completion the arrival would otherwise wait for
+    constexpr int CN = BN / EPI_PARTS;
+    float vj[CN], vn[CN];
+    const bool got = ptx::mbar_wait_sleep(jdone, 0, a.status, 13, 64, a.spin);
+    if (got) {
+      ptx::tc_fence_after();
+      const int cj = 256 + (PAIR ? cbeg + (cbeg & 64) : cbeg);
+      ptx::tmem_ld16(lane_addr + cj, reinterpret_cast<float(&)[16]>(vj[0]));
+      ptx::tmem_ld16(lane_addr + cj + 16, reinterpret_cast<float(&)[16]>(vj[16]));
+      ptx::tmem_ld16(lane_addr + cj + (PAIR ? 64 : 128), reinterpret_cast<float(&)[16]>(vn[0]));
+      ptx::tmem_ld16(lane_addr + cj + (PAIR ? 80 : 144), reinterpret_cast<float(&)[16]>(vn[16]));
+      ptx::tmem_wait_ld();
+      ptx::tc_fence_before();
+    }
+    __syncwarp();
+    if (lane == 0) ptx::mbar_arrive_cluster(jfree);
+    if (got) {
+      const int jn = nok ? min(CN, a.R - (r0 + cbeg)) : 0;
+      float* Lp = a.L + (size_t)(r0 + cbeg) * a.N + n;
+      float* Pp = a.PHI + (size_t)(r0 + cbeg) * a.N + n;
+#pragma unroll
+      for (int j = 0; j < CN; ++j) {
+        if (j < jn) {
+          *Lp = vn[j];
+          *Pp = vj[j];
+        }
+        Lp += a.N;
+        Pp += a.N;
+      }
+    }
+  }
   float m = -INFINITY, ssum = 0.0f;
   int nbad = 0;
   if (ptx::mbar_wait_sleep(accum, 0, a.status, 2, 256, a.spin)) {
     ptx::tc_fence_after();
-    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    for (int c0 = half * (BN / EPI_PARTS); c0 < (half + 1) * (BN / EPI_PARTS); c0 += 16) {
-      float vn[16], vd[16], vb[16], vc[16];
-      ptx::tmem_ld16(lane_addr + 0 + c0, vb);
-      ptx::tmem_ld16(lane_addr + 128 + c0, vd);
-      ptx::tmem_ld16(lane_addr + 256 + c0, vc);
-      ptx::tmem_ld16(lane_addr + 384 + c0, vn);
+    constexpr int CG = 8;
+    for (int c0 = cbeg; c0 < cend; c0 += CG) {
+      float vd[CG], vh[CG], vj[CG], vn[CG];
+      const int cd = PAIR ? c0 + (c0 & 64) : c0;  // column of den; K.H follows
+      ptx::tmem_ld8(lane_addr + cd, vd);
+      ptx::tmem_ld8(lane_addr + cd + (PAIR ? 64 : 128), vh);
+      if (have_1) ptx::tmem_ld8(lane_addr + 256 + c0, vn);
+      if (have_j) ptx::tmem_ld8(lane_addr + 384 + c0, vj);
       ptx::tmem_wait_ld();
+      float mx = m;
+      // eight independent chains, then their exponentials: the running
+      // (max, sum exp) is updated once per eight columns
+      const int jn = nok ? min(CG, a.R - (r0 + c0)) : 0;  // columns that are pairs
+      float* Lp = a.L + (size_t)(r0 + c0) * a.N + n;
+      float* Pp = a.PHI + (size_t)(r0 + c0) * a.N + n;
+      float vq[CG];  // n_J
+      if (nj) {      // this thread's own stores, all loads in flight together
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int cl = c0 + j;
-        const int r = r0 + cl;
-        const float num = vn[j] * a.k2_inv, den = vd[j] * 256.0f;
-        const float B = vb[j], Cc = vc[j] * a.k2_inv;
-        const float sc = s_scale[cl];
-        bool ok = nok && r < a.R && sc > 0.0f;
+        for (int j = 0; j < CG; ++j) {
+          vq[j] = j < jn ? Lp[(size_t)j * a.N] : 0.0f;
+          vj[j] = j < jn ? Pp[(size_t)j * a.N] : 0.0f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < CG; ++j) {
+        const float n1 = have_1 ? vn[j] * a.k_inv : 0.0f;
+        const float kh = (full_h ? vh[j] + vd[j] : vh[j]) * a.k_inv;
+        const float B = __fmaf_rn(-kPoisC, kh, ktot - n1);
+        const float Cc = have_j || nj ? __fmaf_rn(vj[j], a.k_inv, kh) : kh;
+        const float sc = s_scale[c0 + j];
+        bool ok = j < jn && sc > 0.0f;
         float iphi = 1.0f, phi = 1.0f;
         if (!a.known_intensity) {
+          const float num = nj ? __fmaf_rn(-a.k_inv, vq[j], k2tot - n1) : k2tot - n1;
+          const float den = vd[j] * (256.0f * a.k_inv);
           ok = ok && num > 0.0f && den > 0.0f;
-          iphi = den / num;
-          phi = ci * num / den;
+          iphi = quotient(den, num);
+          phi = quotient(ci * num, den);
         }
-        const float Sig = s_A[cl] - 2.0f * B * iphi + Cc * iphi * iphi;
-        const float L = ok ? s_lw[cl] - Sig * sc : -INFINITY;
-        if (nok && r < a.R) {
-          if (!ok) nbad++;
-          a.L[(size_t)r * a.N + n] = L;
-          a.PHI[(size_t)r * a.N + n] = ok ? phi : 1.0f;
+        const float Sig = __fmaf_rn(__fmaf_rn(Cc, iphi, -2.0f * B), iphi, s_A[c0 + j]);
+        const float L = ok ? __fmaf_rn(-Sig, sc, s_lw[c0 + j]) : -INFINITY;
+        if (j < jn) {
+          nbad += ok ? 0 : 1;
+          *Lp = L;
+          *Pp = ok ? phi : 1.0f;
         }
-        if (L > m) {
-          ssum = ssum * expf(m - L) + 1.0f;
-          m = L;
-        } else if (L > -INFINITY) {
-          ssum += expf(L - m);
-        }
+        Lp += a.N;
+        Pp += a.N;
+        vh[j] = L;
+        mx = fmaxf(mx, L);
+      }
+      if (mx > -INFINITY) {
+        float s = 0.0f;
+#pragma unroll
+        for (int j = 0; j < CG; ++j) s += expf(vh[j] - mx);
+        ssum = ssum * expf(m - mx) + s;
+        m = mx;
       }
     }
   }
@@ -370,297 +633,337 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
   if (nbad) atomicAdd(a.bad, nbad);
 }
 
+template <bool PAIR>
 __global__ void __launch_bounds__(es::THREADS, 1)
-    tc_estep_kernel(const __grid_constant__ CUtensorMap mK, const __grid_constant__ CUtensorMap mK2h,
-                    const __grid_constant__ CUtensorMap mK2l, const __grid_constant__ CUtensorMap mMp,
-                    const __grid_constant__ CUtensorMap mMS, const __grid_constant__ CUtensorMap mGh,
-                    const __grid_constant__ CUtensorMap mGl, const __grid_constant__ CUtensorMap mHh,
-                    const __grid_constant__ CUtensorMap mHl, TcEstepArgs a) {
+    tc_estep_kernel(const __grid_constant__ CUtensorMap mK, const __grid_constant__ CUtensorMap mJ,
+                    const __grid_constant__ CUtensorMap mJl, const __grid_constant__ CUtensorMap mMS,
+                    const __grid_constant__ CUtensorMap mHh, const __grid_constant__ CUtensorMap mHl,
+                    const __grid_constant__ CUtensorMap mIv, const __grid_constant__ CUtensorMap mTv,
+                    TcEstepArgs a) {
   using namespace es;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* accum = empty + STAGES;
+  uint64_t* full = (uint64_t*)(smem + CHUNKS * CHUNK);
+  uint64_t* empty = full + NB;
+  uint64_t* accum = empty + NB;
   uint64_t* drain = accum + 1;  // the MMA issuer's own completion wait before TMEM is freed
-  uint32_t* tmem_slot = (uint32_t*)(drain + 1);
-  float* s_A = (float*)(smem + STAGES * STAGE_BYTES + 256);
+  uint64_t* jdone = drain + 1;  // pass A's products are complete
+  uint64_t* jfree = jdone + 1;  // (rank 0) J.H and n_J have been moved out of TMEM
+  uint32_t* tmem_slot = (uint32_t*)(jfree + 1);
+  float* s_A = (float*)(smem + CHUNKS * CHUNK + 256);
   float* s_scale = s_A + BN;
   float* s_lw = s_scale + BN;
   float2* s_half = (float2*)(s_lw + BN);  // [EPI_PARTS-1][BM] (max, sum exp) of column parts 1..
+  uint32_t* s_list = (uint32_t*)(s_half + (EPI_PARTS - 1) * BM);  // [kList]
+  uint32_t* s_seen = s_list + kList;  // the bits of all entries; entries passes A and C look at
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
   const float sg = *a.sigma;
   const float inv2s2 = 1.0f / (2.0f * sg * sg);
-  int pt, rt;
-  if (a.tiles) {  // pruned: the listed tiles only
+  int pt, rt;  // pattern tile (pair of tiles), rotation tile
+  if (!PAIR && a.tiles) {  // pruned: the listed tiles only
     const int2 t = a.tiles[blockIdx.x];
     pt = t.x;
     rt = t.y;
   } else {
-    raster_tile(blockIdx.x + a.tile0, a.raster, a.n_pt, a.n_rt, pt, rt);
+    raster_tile((int)(PAIR ? blockIdx.x >> 1 : blockIdx.x) + a.tile0, a.raster,
+                PAIR ? (a.n_pt + 1) / 2 : a.n_pt, a.n_rt, pt, rt);
   }
-  const int n0 = pt * BM, r0 = rt * BN;
+  // a pair's second tile may be n_pt (no patterns) when n_pt is odd
+  const int n0 = (PAIR ? 2 * pt + (int)rank : pt) * BM, r0 = rt * BN;
+  const uint32_t* list = a.list + (size_t)pt * a.nkb;
+  const int cnt = a.list_n[pt];
+  const unsigned char* inv = a.rot_inv + (size_t)rt * a.nkb;
+  const unsigned char* tiny = a.rot_tiny + (size_t)rt * a.nkb;
+  const bool full_h = a.known_intensity && (a.gh_lo & 2);  // phi = 1: no den, H lo throughout
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
+    for (int s = 0; s < NB; ++s) {
       ptx::mbar_init(&full[s], 1);
       ptx::mbar_init(&empty[s], 1);
     }
     ptx::mbar_init(accum, 1);
     ptx::mbar_init(drain, 1);
+    ptx::mbar_init(jdone, 1);
+    ptx::mbar_init(jfree, EPI_WARPS * (PAIR ? 2 : 1));
     ptx::fence_mbar_init();
+    s_seen[0] = s_seen[1] = s_seen[2] = 0;
+  }
+  uint32_t seen = 0, last_a = 0, last_c = 0;
+  for (int b = threadIdx.x; b < cnt; b += THREADS) {
+    const uint32_t e = es_entry(list, inv, tiny, b);
+    if (b < kList) s_list[b] = e;
+    seen |= e & 0xff;
+    // n_J is needed: invalid pixels where counts exceed 1, or an s in (0, 1e-10)
+    if (((e & (kJ | kInv)) == (kJ | kInv) || (e & kTiny)) && !a.known_intensity) seen |= kNJ;
+    if (e & (kJ | kTiny)) last_a = b + 1;
+    if (e & kHlo) last_c = b + 1;
   }
   if (threadIdx.x < BN) {
     const int r = r0 + threadIdx.x;
-    const float cnt = r < a.R ? a.rot_cnt[r] : 0.0f;
+    const float c = r < a.R ? a.rot_cnt[r] : 0.0f;
     s_A[threadIdx.x] = r < a.R ? a.rot_A[r] : 0.0f;
-    s_scale[threadIdx.x] = cnt > 0.0f ? inv2s2 / cnt : -1.0f;  // < 0: invalid rotation
+    s_scale[threadIdx.x] = c > 0.0f ? inv2s2 / c : -1.0f;  // < 0: invalid rotation
     s_lw[threadIdx.x] = r < a.R ? logf(a.rotw[r]) : 0.0f;
   }
-  if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, 512);
-    ptx::tmem_relinquish();
+  if (warp == MMA_WARP) {
+    if (PAIR) {
+      ptx::tmem_alloc_pair(tmem_slot, 512);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(tmem_slot, 512);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  seen = __reduce_or_sync(0xffffffffu, seen);
+  last_a = __reduce_max_sync(0xffffffffu, last_a);
+  if (lane == 0 && seen) atomicOr(s_seen, seen);
+  last_c = __reduce_max_sync(0xffffffffu, last_c);
+  if (lane == 0 && last_a) atomicMax(s_seen + 1, last_a);
+  if (lane == 0 && last_c) atomicMax(s_seen + 2, last_c);
+  __syncthreads();
+  if (PAIR) ptx::cluster_sync();  // both CTAs' barriers initialised and TMEM allocated
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const unsigned char* flags = a.k2lo_any + (size_t)pt * a.nkb;
-  const bool hlo = (a.gh_lo & 2) != 0;
-  const int glo_end = (a.gh_lo & 1) ? a.glo_kb[pt] : 0;  // G lo on k-blocks below it
+  auto entry = [&](uint32_t b) { return b < kList ? s_list[b] : es_entry(list, inv, tiny, (int)b); };
+  const bool known = a.known_intensity != 0;
+  const bool jh = (a.gh_lo & 2) != 0;  // H lo in every product
+  const uint32_t all = *s_seen;
+  const bool nj = all & kNJ;  // the tile has a pass A
+  const EsStages<PAIR> st(known ? all & ~kTiny : all, nj, jh, full_h);
+  // entries of each pass: A those with J (or T), B all, C those before the count tail
+  const uint32_t n_a = nj ? s_seen[1] : 0u, n_b = (uint32_t)cnt;
+  const uint32_t n_c = full_h || !a.gh_lo ? 0u : (jh ? n_b : s_seen[2]);
+  const uint32_t in_c = jh ? ~0u : kHlo;
 
-  if (warp == 0) {
-    // ------------------------------------------------ TMA producer
-    if (lane == 0) {
-      const CUtensorMap* maps[kSlots] = {&mK, &mK2h, &mK2l, &mGh, &mMS, &mHh, &mMp, &mGl, &mHl};
-      int kb = 0;
-      for (; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 0, a.spin)) break;
-        const bool lo = flags[kb] != 0;
-        const bool glo = kb < glo_end;
-        const int ntiles = kSlots - (lo ? 0 : 1) - (glo ? 0 : 1) - (hlo ? 0 : 1);
-        ptx::mbar_arrive_expect_tx(&full[s], ntiles * TILE_BYTES);
-        unsigned char* st = smem + s * STAGE_BYTES;
-        for (int j = 0; j < kSlots; ++j) {
-          if (j == sK2l && !lo) continue;
-          if ((j == sGl && !glo) || (j == sHl && !hlo)) continue;
-          ptx::tma_load_2d(st + j * TILE_BYTES, maps[j], kb * BK, j < sGh ? n0 : r0, &full[s]);
+  if (warp < PRODUCERS) {
+    // ------------------------------------------------ TMA producers (both CTAs of a pair)
+    if (ptx::elect_one()) {
+      constexpr int RC = EsStages<PAIR>::RC;
+      const int rr = r0 + 64 * (int)rank;  // this CTA's rows of the rotation operands
+      const uint32_t full0 = ptx::smem_u32(full);
+      const uint32_t fb0 = PAIR ? ptx::mapa_shared(full0, 0) : full0;
+      uint32_t it = 0, slot = 0, phase = 1;  // stages issued; the next one's slot and parity
+      bool run = true;
+      auto ld = [&](int o, const CUtensorMap* m, uint32_t e, int y) {
+        unsigned char* to = smem + ((int)slot * st.size + o) * CHUNK;
+        const int x = (int)(e >> 8) * BK;
+        if (PAIR)
+          ptx::tma_load_2d_pair(to, m, x, y, fb0 + 8 * slot);
+        else
+          ptx::tma_load_2d(to, m, x, y, fb0 + 8 * slot);
+      };
+      auto ldr = [&](int o, const CUtensorMap* m, uint32_t e) {  // 64 rotation rows, or 128 in two boxes
+        ld(o, m, e, rr);
+        if (!PAIR) ld(o + 1, m, e, rr + 64);
+      };
+      auto ldz = [&](int o, const CUtensorMap* m, uint32_t e) {  // as many rows of zeros
+        ld(o, m, e, a.zrow);
+        if (!PAIR) ld(o + 1, m, e, a.zrow);
+      };
+      // a free slot, armed by the first producer for a stage of `chunks`
+      // (rank 0's barriers count both CTAs' bytes)
+      auto open = [&](int chunks) {
+        if (!ptx::mbar_wait(&empty[slot], phase, a.status, 0, a.spin)) return run = false;
+        if (warp == 0 && rank == 0)
+          ptx::mbar_arrive_expect_tx(&full[slot], (uint32_t)chunks * (CHUNK * (PAIR ? 2 : 1)));
+        return true;
+      };
+      auto next = [&]() {
+        ++it;
+        if (++slot == (uint32_t)st.slots) {
+          slot = 0;
+          phase ^= 1;
         }
+      };
+      for (uint32_t u = n_a; u-- > 0;) {  // pass A
+        const uint32_t e = entry(u);
+        if (!(e & (kJ | kTiny))) continue;
+        const bool j = e & kJ, jl = j && (e & kJlo), hl = j && jh, t = e & kTiny;
+        if (!open((j ? 2 + 2 * RC : 0) + (jl ? 2 : 0) + (hl ? 2 * RC : 0) + (t ? 2 + 2 * RC : 0)))
+          break;
+        if (warp == 0) {
+          if (j) ld(st.aJ, &mJ, e, n0);
+          if (jl) ld(st.aJl, &mJl, e, n0);
+          if (t) ld(st.aK, &mK, e, n0);
+        } else if (warp == 1) {
+          if (j) ldr(st.aH, &mHh, e);
+          if (hl) ldr(st.aHl, &mHl, e);
+          if (t) ldz(st.aT, &mTv, e);
+        } else {
+          if (j) ldr(st.aI, &mIv, e);
+          if (hl) ldz(st.aHl + RC, &mHl, e);
+          if (t) ldr(st.aT + RC, &mTv, e);
+        }
+        next();
       }
-      // no copy may still be landing in shared memory when the CTA exits
-      // (after a normal run the MMAs have consumed them all: no wait)
-      ptx::drain_loads(full, STAGES, (uint32_t)kb, a.status, 11);
+      for (uint32_t u = n_c; run && u-- > 0;) {  // pass C
+        const uint32_t e = entry(u);
+        if (!(e & in_c)) continue;
+        if (!open(2 + 2 * RC)) break;
+        if (warp == 0) {
+          ld(st.cK, &mK, e, n0);
+        } else if (warp == 1) {
+          ldz(st.cZ, &mHl, e);
+        } else {
+          ldr(st.cHl, &mHl, e);
+        }
+        next();
+      }
+      for (uint32_t u = n_b; run && u-- > 0;) {  // pass B
+        const uint32_t e = entry(u);
+        const bool j = !nj && (e & kJ), jl = j && (e & kJlo);
+        const bool hl = j && jh && !full_h;
+        if (!open(2 + 2 * RC + ((e & kInv) ? RC : 0) + (j ? 2 : 0) + (jl ? 2 : 0) + (hl ? RC : 0)))
+          break;
+        if (warp == 0) {
+          ld(st.bK, &mK, e, n0);
+          if (jl) ld(st.bJl, &mJl, e, n0);
+          if (hl) ldr(st.bHl, &mHl, e);
+        } else if (warp == 1) {
+          ldr(st.bMS, full_h ? &mHl : &mMS, e);
+          if (j) ld(st.bJ, &mJ, e, n0);
+        } else {
+          ldr(st.bH, &mHh, e);
+          if (e & kInv) ldr(st.bI, &mIv, e);
+        }
+        next();
+      }
+      // no copy may still be landing in shared memory when the CTA exits: after
+      // a normal run the MMAs have consumed them all (no wait)
+      if (warp == 0 && rank == 0) ptx::drain_loads(full, st.slots, it, a.status, 11);
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc2 = ptx::idesc_f16(BM, 2 * BN);  // the N = 256 pairs
-      constexpr uint32_t idesc1 = ptx::idesc_f16(BM, BN);
-      for (int kb = 0; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&full[s], ph, a.status, 1, a.spin)) break;
-        ptx::tc_fence_after();
-        const bool lo = flags[kb] != 0;
-        const bool glo = kb < glo_end;
-        const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
+  } else if (warp == MMA_WARP) {
+    // ------------------------------------------------ MMA issuer (rank 0 of a pair)
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr int M = PAIR ? 2 * BM : BM;
+      constexpr uint32_t idesc2 = ptx::idesc_f16(M, 2 * BN);
+      constexpr uint32_t idesc1 = ptx::idesc_f16(M, BN);
+      auto mma = [&](uint32_t d, uint64_t x, uint64_t y, uint32_t id, uint32_t acc) {
+        if (PAIR)
+          ptx::mma_f16_pair(d, x, y, id, acc);
+        else
+          ptx::mma_f16(d, x, y, id, acc);
+      };
+      const uint32_t t256 = tmem + 256, t384 = tmem + 384;
+      const uint64_t desc0 = ptx::smem_desc(ptx::smem_u32(smem), 1024, 2);
+      uint32_t slot = 0, phase = 0;
+      uint64_t base = 0;
+      bool run = true;
+      // descriptors count 16-byte units (no carry past the 14-bit address field)
+      auto d = [&](int o, int ks) { return base + (uint64_t)(o * (CHUNK / 16) + ks * 2); };
+      auto mma4 = [&](uint32_t t, int x, int y, uint32_t id, uint32_t acc) {
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {
-          // 8-row core-matrix groups 512 B apart: a 256-row operand runs
-          // through two adjacent 128-row slots
-          auto d = [&](int j) { return ptx::smem_desc(base + j * TILE_BYTES + ks * 32, 512, 4); };
-          const uint32_t acc = (kb | ks) ? 1u : 0u;
-          ptx::mma_f16(tmem + 0, d(sK), d(sGh), idesc2, acc);      // B hi | den
-          ptx::mma_f16(tmem + 256, d(sK2h), d(sHh), idesc2, acc);  // C hi | num
-          if (glo) ptx::mma_f16(tmem + 0, d(sK), d(sGl), idesc1, 1u);     // B lo
-          if (hlo) ptx::mma_f16(tmem + 256, d(sK2h), d(sHl), idesc1, 1u); // C lo
-          if (lo) ptx::mma_f16(tmem + 256, d(sK2l), d(sHh), idesc2, 1u);  // K^2 lo: C | num
+        for (int ks = 0; ks < BK / 16; ++ks) mma(t, d(x, ks), d(y, ks), id, ks ? 1u : acc);
+      };
+      auto open = [&]() {
+        if (!ptx::mbar_wait(&full[slot], phase, a.status, 1, a.spin)) return run = false;
+        ptx::tc_fence_after();
+        base = desc0 + (uint64_t)(slot * (uint32_t)st.size * (CHUNK / 16));
+        return true;
+      };
+      auto close = [&]() {
+        if (PAIR)
+          ptx::mma_commit_pair(&empty[slot], 0x3);
+        else
+          ptx::mma_commit(&empty[slot]);
+        if (++slot == (uint32_t)st.slots) {
+          slot = 0;
+          phase ^= 1;
         }
-        ptx::mma_commit(&empty[s]);
+      };
+      uint32_t accA = 0;  // pass A's columns hold a product
+      for (uint32_t u = n_a; u-- > 0;) {
+        const uint32_t e = entry(u);
+        if (!(e & (kJ | kTiny))) continue;
+        if (!open()) break;
+        const bool j = e & kJ, jl = j && (e & kJlo);
+        if (j) {
+          mma4(t256, st.aJ, st.aH, idesc2, accA);  // J.H | n_J
+          accA = 1;
+          if (jl) mma4(t256, st.aJl, st.aH, idesc2, 1u);
+          if (jh) mma4(t256, st.aJ, st.aHl, idesc2, 1u);
+        }
+        if (e & kTiny) {
+          mma4(t256, st.aK, st.aT, idesc2, accA);
+          accA = 1;
+          if (j) mma4(t256, st.aJ, st.aT, idesc2, 1u);
+          if (jl) mma4(t256, st.aJl, st.aT, idesc2, 1u);
+        }
+        close();
       }
-      // fires when every MMA issued above has completed; after a timeout the
-      // epilogue's own bounded wait reports it
-      ptx::mma_commit(accum);
-      // TMEM is freed only after every MMA issued here has completed, also
-      // when the epilogue stopped waiting
-      ptx::mma_commit(drain);
+      if (nj) {
+        if (PAIR)
+          ptx::mma_commit_pair(jdone, 0x3);
+        else
+          ptx::mma_commit(jdone);
+      }
+      uint32_t accB = 0;  // den | K.H holds a product
+      for (uint32_t u = n_c; run && u-- > 0;) {  // pass C
+        const uint32_t e = entry(u);
+        if (!(e & in_c)) continue;
+        if (!open()) break;
+        mma4(tmem, st.cK, st.cZ, idesc2, accB);
+        accB = 1;
+        close();
+      }
+      uint32_t accJ = 0, acc1 = 0;  // J.H, n_1 hold a product of this pass
+      bool taken = nj;              // pass A's sums are still there
+      for (uint32_t u = n_b; run && u-- > 0;) {
+        const uint32_t e = entry(u);
+        const bool j = !nj && (e & kJ);
+        if (!open()) break;
+        mma4(tmem, st.bK, st.bMS, idesc2, accB);  // den | K.H
+        accB = 1;
+        if (taken && (j || (e & kInv))) {
+          if (!ptx::mbar_wait_cluster(jfree, 0, a.status, 13, a.spin)) break;
+          ptx::tc_fence_after();
+          taken = false;
+        }
+        if (j) {
+          mma4(t384, st.bJ, st.bH, idesc1, accJ);
+          accJ = 1;
+          if (e & kJlo) mma4(t384, st.bJl, st.bH, idesc1, 1u);
+          if (jh) mma4(t384, st.bJ, full_h ? st.bMS : st.bHl, idesc1, 1u);
+        }
+        if (e & kInv) {
+          mma4(t256, st.bK, st.bI, idesc1, acc1);
+          acc1 = 1;
+        }
+        close();
+      }
+      // accum fires when every MMA issued above has completed (after a timeout
+      // the epilogue's own bounded wait reports it); drain: TMEM is freed only
+      // after every MMA issued here has completed, also when the epilogue
+      // stopped waiting (both CTAs' TMEM is written by a pair's MMAs)
+      if (PAIR) {
+        ptx::mma_commit_pair(accum, 0x3);
+        ptx::mma_commit_pair(drain, 0x1);
+      } else {
+        ptx::mma_commit(accum);
+        ptx::mma_commit(drain);
+      }
       ptx::mbar_wait(drain, 0, a.status, 12);
     }
   } else {
-    // ------------------------------------------------ epilogue (warps 2-17)
-    estep_epilogue(a, tmem, accum, s_A, s_scale, s_lw, s_half, warp, lane, n0, r0, rt);
+    // ------------------------------------------------ epilogue
+    estep_epilogue<PAIR>(a, tmem, accum, jdone, ptx::mapa_shared(ptx::smem_u32(jfree), 0), s_A, s_scale, s_lw, s_half, warp, lane, n0, r0, rt,
+                         *s_seen);
   }
   ptx::tc_fence_before();
   __syncthreads();
-  if (threadIdx.x == 32) ptx::settle_after_timeout(a.status);
+  if (PAIR) ptx::cluster_sync();  // the pair's MMAs and barrier traffic are over in both CTAs
+  if (threadIdx.x == 32 * MMA_WARP) ptx::settle_after_timeout(a.status);
   __syncthreads();
-  if (warp == 1) {
+  if (warp == MMA_WARP) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, 512);
-  }
-}
-
-// ------------------------------------------------ E-step on CTA pairs -----
-// The same contractions over 256 patterns x 128 rotations per cluster of two
-// CTAs, with 256-row MMAs (cta_group::2) issued by rank 0.  Each CTA keeps
-// its own 128 patterns' tiles (K, K^2 hi, K^2 lo) and one half of every
-// rotation-side operand: rank 0 the G and H columns of the [G | M'S] and
-// [H | M'] pairs, rank 1 the M'S and M' columns, and 64 of the 128 G lo rows
-// each.  Per 32-pixel stage a CTA loads 36 KB (44 KB with K^2 lo) instead of
-// 56-64 KB for the same MMA work, and five stages fit in shared memory: the
-// loads in flight cover more of the L2 / HBM latency that stalls the MMAs.  Both CTAs' loads complete
-// on rank 0's `full` barriers; rank 0's commits arrive on both CTAs' `empty`
-// and `accum` barriers.  The epilogue is the single-CTA kernel's, per CTA.
-namespace es2 {
-constexpr int STAGES = 5;
-constexpr int TILE = 128 * es::BK * 2;  // 8 KB: 128 rows of one operand
-constexpr int HALF = TILE / 2;          // 64 rows (G lo half)
-constexpr int oK = 0, oK2h = TILE, oK2l = 2 * TILE, oB1 = 3 * TILE, oB2 = 4 * TILE,
-              oGl = 5 * TILE;
-constexpr int STAGE_BYTES = 5 * TILE + HALF;  // 44 KB; no H lo (known intensity runs single CTAs)
-// barriers (256 B), per-rotation rows (3 x 128 floats), epilogue parts
-constexpr int EXTRA = 256 + 3 * es::BN * 4 + (es::EPI_PARTS - 1) * es::BM * 8;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EXTRA + 1024;
-static_assert(SMEM_BYTES <= 232448, "shared memory of the pair kernel");
-}  // namespace es2
-
-__global__ void __launch_bounds__(es::THREADS, 1)
-    tc_estep_pair_kernel(const __grid_constant__ CUtensorMap mK,
-                         const __grid_constant__ CUtensorMap mK2h,
-                         const __grid_constant__ CUtensorMap mK2l,
-                         const __grid_constant__ CUtensorMap mMp,
-                         const __grid_constant__ CUtensorMap mMS,
-                         const __grid_constant__ CUtensorMap mGh,
-                         const __grid_constant__ CUtensorMap mGl64,
-                         const __grid_constant__ CUtensorMap mHh, TcEstepArgs a) {
-  using namespace es;
-  using es2::STAGES;
-  using es2::STAGE_BYTES;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
-  uint64_t* empty = full + STAGES;
-  uint64_t* accum = empty + STAGES;
-  uint64_t* drain = accum + 1;  // rank 0's MMA issuer waits on it before TMEM is freed
-  uint32_t* tmem_slot = (uint32_t*)(drain + 1);
-  float* s_A = (float*)(smem + STAGES * STAGE_BYTES + 256);
-  float* s_scale = s_A + BN;
-  float* s_lw = s_scale + BN;
-  float2* s_half = (float2*)(s_lw + BN);
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = ptx::cluster_ctarank();
-  const float sg = *a.sigma;
-  const float inv2s2 = 1.0f / (2.0f * sg * sg);
-  const int n_ptp = (a.n_pt + 1) / 2;
-  int ptp, rt;
-  raster_tile((int)(blockIdx.x >> 1) + a.tile0, a.raster, n_ptp, a.n_rt, ptp, rt);
-  const int pt = 2 * ptp + (int)rank;  // may be n_pt (no patterns) when n_pt is odd
-  const int n0 = pt * BM, r0 = rt * BN;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < STAGES; ++s) {
-      ptx::mbar_init(&full[s], 1);
-      ptx::mbar_init(&empty[s], 1);
-    }
-    ptx::mbar_init(accum, 1);
-    ptx::mbar_init(drain, 1);
-    ptx::fence_mbar_init();
-  }
-  if (threadIdx.x < BN) {
-    const int r = r0 + threadIdx.x;
-    const float cnt = r < a.R ? a.rot_cnt[r] : 0.0f;
-    s_A[threadIdx.x] = r < a.R ? a.rot_A[r] : 0.0f;
-    s_scale[threadIdx.x] = cnt > 0.0f ? inv2s2 / cnt : -1.0f;
-    s_lw[threadIdx.x] = r < a.R ? logf(a.rotw[r]) : 0.0f;
-  }
-  if (warp == 1) {
-    ptx::tmem_alloc_pair(tmem_slot, 512);
-    ptx::tmem_relinquish_pair();
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::cluster_sync();  // both CTAs' barriers initialised and TMEM allocated
-  ptx::tc_fence_after();
-  const uint32_t tmem = *tmem_slot;
-  // the K^2 lo MMA runs for a k-block when either pattern tile needs it
-  const int pt0 = 2 * ptp, pt1 = 2 * ptp + 1;
-  const unsigned char* flags0 = a.k2lo_any + (size_t)pt0 * a.nkb;
-  const unsigned char* flags1 = pt1 < a.n_pt ? a.k2lo_any + (size_t)pt1 * a.nkb : nullptr;
-  // G lo on the k-blocks either pattern tile needs (H lo, gh_lo bit 1, runs on single CTAs)
-  const int glo_end =
-      (a.gh_lo & 1) ? max(a.glo_kb[pt0], pt1 < a.n_pt ? a.glo_kb[pt1] : 0) : 0;
-
-  if (warp == 0) {
-    // ------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
-      const CUtensorMap* mb1 = rank ? &mMS : &mGh;
-      const CUtensorMap* mb2 = rank ? &mMp : &mHh;
-      int kb = 0;
-      for (; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 0, a.spin)) break;
-        const bool lo = flags0[kb] != 0 || (flags1 && flags1[kb] != 0);
-        const bool glo = kb < glo_end;
-        const uint32_t bytes = (lo ? 5 : 4) * es2::TILE + (glo ? es2::HALF : 0);
-        if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * bytes);  // both CTAs' loads
-        const uint32_t fb = ptx::mapa_shared(ptx::smem_u32(&full[s]), 0);
-        unsigned char* st = smem + s * STAGE_BYTES;
-        const int x = kb * BK;
-        ptx::tma_load_2d_pair(st + es2::oK, &mK, x, n0, fb);
-        ptx::tma_load_2d_pair(st + es2::oK2h, &mK2h, x, n0, fb);
-        if (lo) ptx::tma_load_2d_pair(st + es2::oK2l, &mK2l, x, n0, fb);
-        ptx::tma_load_2d_pair(st + es2::oB1, mb1, x, r0, fb);
-        ptx::tma_load_2d_pair(st + es2::oB2, mb2, x, r0, fb);
-        if (glo) ptx::tma_load_2d_pair(st + es2::oGl, &mGl64, x, r0 + 64 * (int)rank, fb);
-      }
-      // rank 0's barriers count both CTAs' bytes of the stages it armed
-      if (rank == 0) ptx::drain_loads(full, STAGES, (uint32_t)kb, a.status, 11);
-    }
-  } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer (rank 0)
-    if (rank == 0 && lane == 0) {
-      constexpr uint32_t idesc2 = ptx::idesc_f16(2 * BM, 2 * BN);  // 256 x 256 pairs
-      constexpr uint32_t idesc1 = ptx::idesc_f16(2 * BM, BN);      // 256 x 128 lo terms
-      for (int kb = 0; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&full[s], ph, a.status, 1, a.spin)) break;
-        ptx::tc_fence_after();
-        const bool lo = flags0[kb] != 0 || (flags1 && flags1[kb] != 0);
-        const bool glo = kb < glo_end;
-        const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
-#pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {
-          auto d = [&](int off) { return ptx::smem_desc(base + off + ks * 32, 512, 4); };
-          const uint32_t acc = (kb | ks) ? 1u : 0u;
-          ptx::mma_f16_pair(tmem + 0, d(es2::oK), d(es2::oB1), idesc2, acc);      // B hi | den
-          ptx::mma_f16_pair(tmem + 256, d(es2::oK2h), d(es2::oB2), idesc2, acc);  // C hi | num
-          if (glo) ptx::mma_f16_pair(tmem + 0, d(es2::oK), d(es2::oGl), idesc1, 1u);
-          if (lo) ptx::mma_f16_pair(tmem + 256, d(es2::oK2l), d(es2::oB2), idesc2, 1u);
-        }
-        ptx::mma_commit_pair(&empty[s], 0x3);
-      }
-      ptx::mma_commit_pair(accum, 0x3);
-      ptx::mma_commit_pair(drain, 0x1);  // both CTAs' TMEM is written by these MMAs
-      ptx::mbar_wait(drain, 0, a.status, 12);
-    }
-  } else {
-    // ------------------------------------------------ epilogue (warps 2-17)
-    estep_epilogue(a, tmem, accum, s_A, s_scale, s_lw, s_half, warp, lane, n0, r0, rt);
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::cluster_sync();  // the pair's MMAs and barrier traffic are over in both CTAs
-  if (threadIdx.x == 32) ptx::settle_after_timeout(a.status);
-  __syncthreads();
-  if (warp == 1) {
-    ptx::tc_fence_after();
-    ptx::tmem_dealloc_pair(tmem, 512);
+    if (PAIR)
+      ptx::tmem_dealloc_pair(tmem, 512);
+    else
+      ptx::tmem_dealloc(tmem, 512);
   }
 }
 
@@ -753,7 +1056,7 @@ __global__ void __launch_bounds__(ep::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       int kb = 0;
       for (; kb < a.nkb; ++kb) {
         const int s = kb % STAGES;
@@ -769,7 +1072,7 @@ __global__ void __launch_bounds__(ep::THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       constexpr uint32_t idesc = ptx::idesc_f16(BM, BN);
       for (int kb = 0; kb < a.nkb; ++kb) {
         const int s = kb % STAGES;
@@ -869,6 +1172,7 @@ struct TcMstepArgs {
   int raster;  // tile order (raster_tile over pixel tiles x rotation tiles)
   const float* T;
   const float* qscale;  // [R] 2^-e_r
+  float k_inv;          // 1 / count_scale of the K^T operand
   const float* rot;
   const float *cx, *cy, *cz;
   int side, interp, deterministic;
@@ -1030,7 +1334,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x) {
@@ -1056,7 +1360,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       constexpr uint32_t idesc = ptx::idesc_f16(BM, BN);
       uint32_t it = 0;
       bool ok = true;
@@ -1108,7 +1412,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       const int r = r0 + rl;
       const bool rok = r < a.R;
       const float Tr = rok ? a.T[r] : 0.0f;
-      const float qs = rok ? a.qscale[r] : 0.0f;
+      const float qs = rok ? a.qscale[r] * a.k_inv : 0.0f;
       const bool live = rok && Tr > 1e-10f;
       RotMat Rm = {};
       if (rok) Rm = quat_to_matrix(a.rot + 4 * (size_t)r);
@@ -1225,7 +1529,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       uint32_t it = 0;
       bool ok = true;
       const uint32_t bytes = STAGE_BYTES;
@@ -1253,7 +1557,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
     }
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer (rank 0)
-    if (rank == 0 && lane == 0) {
+    if (rank == 0 && ptx::elect_one()) {
       constexpr uint32_t idesc = ptx::idesc_f16(2 * BM, BN);  // 256 x 256
       uint32_t it = 0;
       bool ok = true;
@@ -1302,7 +1606,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       const int r = r0 + rl;
       const bool rok = r < a.R;
       const float Tr = rok ? a.T[r] : 0.0f;
-      const float qs = rok ? a.qscale[r] : 0.0f;
+      const float qs = rok ? a.qscale[r] * a.k_inv : 0.0f;
       const bool live = rok && Tr > 1e-10f;
       RotMat Rm = {};
       if (rok) Rm = quat_to_matrix(a.rot + 4 * (size_t)r);
@@ -1353,12 +1657,11 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 
 // ------------------------------------------------------------ host -------
 struct TcState {
-  CUtensorMap mK, mK2h, mK2l, mQh, mQl, mKt;
+  CUtensorMap mK, mJ, mJl, mQh, mQl, mKt;
   CUtensorMap mKt128;  // K^T in 128-row boxes (pair M-step halves)
-  CUtensorMap rot[6];    // M', MS, Gh, Gl, Hh, Hl: 128-row boxes
-  CUtensorMap gl64;        // G lo: 64-row boxes (CTA-pair halves)
-  CUtensorMap mLh, mLl;  // true Poisson: log-slices hi / lo (in Gh, Gl), 256-row boxes
-  __half *Mp, *MSh, *Gh, *Gl, *Hh, *Hl;
+  CUtensorMap mMS, mHh, mHl, mIv, mTv;  // rotation operands: 64-row boxes
+  CUtensorMap mLh, mLl;  // true Poisson: log-slices hi / lo, 256-row boxes
+  __half *MS, *Hh, *Hl, *Iv, *Tv, *Lh, *Ll;
   int* status;
 };
 
@@ -1370,18 +1673,20 @@ int tc_bind(emc_plan* p) {
     return fail(ctx, EMC_ERR_UNSUPPORTED,
                 "mixed precision needs integer counts in [0, 2048] (exact in FP16), or in [0, "
                 "65504] with EMC_OPT_COUNTS_ROUND (largest count here %d)", p->count_max);
-  {
-    // K^2 scale: the largest FP16 count squared times k2_scale stays below 2^15
-    const float km = __half2float(__float2half_rn((float)p->count_max));
-    int e = 7;
-    while (km * km * std::ldexp(1.0f, -e) > 32768.0f) ++e;
-    p->k2_scale = std::ldexp(1.0f, -e);
-  }
   if (p->d.diff != EMC_DIFF_POISSON && p->d.diff != EMC_DIFF_TRUE_POISSON)
     return fail(ctx, EMC_ERR_UNSUPPORTED,
                 "mixed precision implements the poisson and true-poisson likelihoods");
   const bool pois = p->d.diff == EMC_DIFF_TRUE_POISSON;
-  const int N = p->d.n_images, Np = p->Np, Kp = p->Kp, Rp = p->Rp;
+  const int Np = p->Np, Kp = p->Kp, Rp = p->Rp;
+  if (pois) {
+    p->count_scale = 1.0f;
+  } else {
+    // the largest FP16 count squared times the scale stays below 2^15
+    const float km = __half2float(__float2half_rn((float)p->count_max));
+    int e = 7;
+    while (km * km * std::ldexp(1.0f, -e) > 32768.0f) ++e;
+    p->count_scale = std::ldexp(1.0f, -e);
+  }
   int rc = EMC_OK;
   if (!p->tc) {
     TcState* st = new TcState();
@@ -1390,17 +1695,28 @@ int tc_bind(emc_plan* p) {
     const size_t pk = (size_t)Np * Kp, rk = (size_t)Rp * Kp;
     if (!rc) rc = plan_alloc(p, (void**)&p->Kh, pk * 2);
     if (!rc) rc = plan_alloc(p, (void**)&p->KhT, pk * 2);
+    const size_t n_pt = (size_t)(Np / 128), nkb = (size_t)(Kp / 64), n_pp = (n_pt + 1) / 2;
+    if (!rc) rc = plan_alloc(p, (void**)&p->blk_bits, n_pt * nkb);
+    if (!rc) rc = plan_alloc(p, (void**)&p->blk_live, nkb);
+    if (!rc) rc = plan_alloc(p, (void**)&p->pt_list, n_pt * nkb * 4);
+    if (!rc) rc = plan_alloc(p, (void**)&p->pt_n, n_pt * 4);
+    if (!rc) rc = plan_alloc(p, (void**)&p->pp_list, n_pp * nkb * 4);
+    if (!rc) rc = plan_alloc(p, (void**)&p->pp_n, n_pp * 4);
     if (!pois) {
-      if (!rc) rc = plan_alloc(p, (void**)&p->K2hi, pk * 2);
-      if (!rc) rc = plan_alloc(p, (void**)&p->K2lo, pk * 2);
-      if (!rc) rc = plan_alloc(p, (void**)&p->k2lo_any, (size_t)(Np / 128) * (Kp / 32));
-      if (!rc) rc = plan_alloc(p, (void**)&p->glo_kb, sizeof(int) * (size_t)(Np / 128 + 1));
+      if (!rc) rc = plan_alloc(p, (void**)&p->Jh, pk * 2);
+      if (!rc) rc = plan_alloc(p, (void**)&p->Jl, pk * 2);
+      if (!rc) rc = plan_alloc(p, (void**)&p->ktot, (size_t)Np * 4);
+      if (!rc) rc = plan_alloc(p, (void**)&p->k2tot, (size_t)Np * 4);
+      if (!rc) rc = plan_alloc(p, (void**)&p->lo_kb, sizeof(int) * (n_pt + 1));
+      if (!rc) rc = plan_alloc(p, (void**)&p->rot_flags, 2 * (size_t)p->n_rt * nkb);
     }
-    __half** rot_ops[6] = {&st->Gh, &st->Gl, &st->Mp, &st->MSh, &st->Hh, &st->Hl};
-    for (int j = 0; j < (pois ? 2 : 6); ++j) {
-      if (!rc) rc = plan_alloc(p, (void**)rot_ops[j], rk * 2);
+    __half** pois_ops[] = {&st->Lh, &st->Ll};
+    __half** rot_ops[] = {&st->MS, &st->Hh, &st->Hl, &st->Iv, &st->Tv};
+    for (int j = 0; j < (pois ? 2 : 5); ++j) {
+      __half** op = pois ? pois_ops[j] : rot_ops[j];
+      if (!rc) rc = plan_alloc(p, (void**)op, rk * 2);
       // rows R..Rp stay zero: the expand writes the operands of rows < R
-      if (!rc) EMC_CUDA(ctx, cudaMemsetAsync(*rot_ops[j], 0, rk * 2, ctx->stream));
+      if (!rc) EMC_CUDA(ctx, cudaMemsetAsync(*op, 0, rk * 2, ctx->stream));
     }
     if (!rc) rc = plan_alloc(p, (void**)&p->Qh, (size_t)Rp * Np * 2);
     if (!rc) rc = plan_alloc(p, (void**)&p->qscale, (size_t)Rp * 4);
@@ -1409,26 +1725,27 @@ int tc_bind(emc_plan* p) {
     EMC_CUDA(ctx, cudaMemsetAsync(st->status, 0, 64, ctx->stream));
     EMC_CUDA(ctx, cudaMemsetAsync(p->Qh, 0, (size_t)Rp * Np * 2, ctx->stream));
     // tensor maps (fixed addresses for the plan's lifetime)
-    if (!rc) rc = make_map(ctx, &st->mK, p->Kh, Np, Kp, 128, 32);
     if (pois) {
-      if (!rc) rc = make_map(ctx, &st->mLh, st->Gh, Rp, Kp, 256, 32);
-      if (!rc) rc = make_map(ctx, &st->mLl, st->Gl, Rp, Kp, 256, 32);
+      if (!rc) rc = make_map(ctx, &st->mK, p->Kh, Np, Kp, 128, 32);
+      if (!rc) rc = make_map(ctx, &st->mLh, st->Lh, Rp, Kp, 256, 32);
+      if (!rc) rc = make_map(ctx, &st->mLl, st->Ll, Rp, Kp, 256, 32);
     } else {
-      if (!rc) rc = make_map(ctx, &st->mK2h, p->K2hi, Np, Kp, 128, 32);
-      if (!rc) rc = make_map(ctx, &st->mK2l, p->K2lo, Np, Kp, 128, 32);
-      const __half* ro[6] = {st->Mp, st->MSh, st->Gh, st->Gl, st->Hh, st->Hl};
-      for (int j = 0; j < 6 && !rc; ++j) rc = make_map(ctx, &st->rot[j], ro[j], Rp, Kp, 128, 32);
-      if (!rc) rc = make_map(ctx, &st->gl64, st->Gl, Rp, Kp, 64, 32);
+      if (!rc) rc = make_map(ctx, &st->mK, p->Kh, Np, Kp, 128, 64);
+      if (!rc) rc = make_map(ctx, &st->mJ, p->Jh, Np, Kp, 128, 64);
+      if (!rc) rc = make_map(ctx, &st->mJl, p->Jl, Np, Kp, 128, 64);
+      CUtensorMap* rm[] = {&st->mMS, &st->mHh, &st->mHl, &st->mIv, &st->mTv};
+      for (int j = 0; j < 5 && !rc; ++j) rc = make_map(ctx, rm[j], *rot_ops[j], Rp, Kp, 64, 64);
     }
     if (!rc) rc = make_map(ctx, &st->mQh, p->Qh, Rp, Np, 128, 64);
     if (!rc) rc = make_map(ctx, &st->mKt, p->KhT, Kp, Np, 256, 64);
     if (!rc) rc = make_map(ctx, &st->mKt128, p->KhT, Kp, Np, 128, 64);
     if (rc) return rc;
-    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       es::SMEM_BYTES));
-    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pair_kernel,
+    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       es2::SMEM_BYTES));
+                                       es::SMEM_BYTES));
+    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       es::SMEM_BYTES));
     EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pois_kernel,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, ep::SMEM_BYTES));
     EMC_CUDA(ctx, cudaFuncSetAttribute(tc_mstep_kernel<0>,
@@ -1446,28 +1763,27 @@ int tc_bind(emc_plan* p) {
   }
   if (p->mstep_q_lo && (rc = tc_ensure_qlo(p))) return rc;
   // counts already in FP16 from the bind's pattern pass when its scale holds
-  return tc_pattern_side(p, nullptr, p->fused_k2_scale == p->k2_scale);
+  return tc_pattern_side(p, nullptr, p->fused_scale == p->count_scale);
 }
 
 // FP16 pattern operands for the pattern order perm (position -> input
 // pattern; nullptr: input order).
-// counts_done: pattern_ops_kernel already wrote Kh / K2h / K2l at the
-// current scale (rows < N; the padding rows stay zero from the first bind).
+// counts_done: the pattern pass already wrote Kh at the current scale (rows
+// < N; the padding rows stay zero from the first bind).
 int tc_pattern_side(emc_plan* p, const int* d_perm, bool counts_done) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images, Np = p->Np, Kp = p->Kp;
-  const bool pois = p->d.diff == EMC_DIFF_TRUE_POISSON;
   int rc;
   if (!counts_done) {
     tc_pattern_ops_kernel<<<(unsigned)Np * (unsigned)ceil_div(Kp, 256), 256, 0, ctx->stream>>>(
-        p->images, p->pix, p->n2, N, Kp, p->Kh, pois ? nullptr : p->K2hi, p->K2lo, d_perm,
-        p->k2_scale);
+        p->images, p->pix, p->n2, N, Kp, p->Kh, d_perm, p->count_scale);
     if ((rc = after_launch(ctx, "tc_pattern_ops_kernel"))) return rc;
   }
-  if (!pois) tc_k2lo_flags_kernel<<<dim3(Kp / 32, Np / 128), 256, 0, ctx->stream>>>(p->K2lo, Kp, p->k2lo_any,
-                                                                         Kp / 32);
-  if ((rc = after_launch(ctx, "tc_k2lo_flags_kernel"))) return rc;
-  if (!pois && (rc = tc_glo_extent(p))) return rc;
+  const int n_pt = Np / es::BM;
+  tc_count_blocks_kernel<<<dim3(Kp / es::BK, (n_pt + 1) / 2), 256, 0, ctx->stream>>>(
+      p->Kh, Kp, Kp / es::BK, n_pt, p->count_scale, p->Jh, p->Jl, p->blk_bits);
+  if ((rc = after_launch(ctx, "tc_count_blocks_kernel"))) return rc;
+  if ((rc = tc_block_lists(p))) return rc;
   transpose_h_kernel<<<dim3(ceil_div(Kp, 64), ceil_div(Np, 64)), dim3(32, 8), 0, ctx->stream>>>(
       p->Kh, Np, Kp, p->KhT);
   return after_launch(ctx, "transpose_h_kernel");
@@ -1475,14 +1791,22 @@ int tc_pattern_side(emc_plan* p, const int* d_perm, bool counts_done) {
 
 int* tc_status(emc_plan* p) { return p->tc ? state(p)->status : nullptr; }
 
-int tc_glo_extent(emc_plan* p) {
-  if (!p->glo_kb) return EMC_OK;  // true Poisson: no G operand
+__half* tc_tiny_plane(emc_plan* p) { return state(p)->Tv; }
+
+int tc_block_lists(emc_plan* p) {
   emc_ctx* ctx = p->ctx;
   const int nkb = p->Kp / es::BK, n_pt = p->Np / es::BM;
-  EMC_CUDA(ctx, cudaMemsetAsync(p->glo_kb, 0, sizeof(int) * (size_t)(n_pt + 1), ctx->stream));
-  tc_glo_extent_kernel<<<ceil_div(p->d.n_images, 8), 256, 0, ctx->stream>>>(
-      p->Kh, p->Kp, nkb, p->d.n_images, (float)p->glo_tail_ppm * 1e-6f, p->glo_kb);
-  return after_launch(ctx, "tc_glo_extent_kernel");
+  int rc;
+  if (p->lo_kb) {
+    EMC_CUDA(ctx, cudaMemsetAsync(p->lo_kb, 0, sizeof(int) * (size_t)(n_pt + 1), ctx->stream));
+    tc_count_rows_kernel<<<ceil_div(p->d.n_images, 8), 256, 0, ctx->stream>>>(
+        p->Kh, p->Kp, nkb, p->d.n_images, p->count_scale, (float)p->glo_tail_ppm * 3e-4f, p->ktot,
+        p->k2tot, p->lo_kb);
+    if ((rc = after_launch(ctx, "tc_count_rows_kernel"))) return rc;
+  }
+  tc_block_lists_kernel<<<n_pt + (n_pt + 1) / 2 + ceil_div(nkb, 32), 32, 0, ctx->stream>>>(
+      p->blk_bits, n_pt, nkb, p->lo_kb, p->pt_list, p->pt_n, p->pp_list, p->pp_n, p->blk_live);
+  return after_launch(ctx, "tc_block_lists_kernel");
 }
 
 // The FP16 lo half of the M-step operand and its tensor map, allocated the
@@ -1532,6 +1856,13 @@ static int estep_pois_launch(emc_plan* p, int raster, int first, int count, bool
   return after_launch(ctx, "tc_estep_pois_kernel");
 }
 
+// The halves of H in force: bit 0 H lo in K . H before the count tail, bit 1 in
+// every product (auto: when the intensity is known -- phi = 1 leaves the
+// C = K^2 . H term unbalanced, and its rounding then shows in the likelihood).
+static int estep_gh_lo(const emc_plan* p) {
+  return p->estep_gh_lo >= 0 ? p->estep_gh_lo : (p->d.known_intensity ? 3 : 1);
+}
+
 static int estep_launch(emc_plan* p, int raster, int first, int count, bool full) {
   if (p->d.diff == EMC_DIFF_TRUE_POISSON) return estep_pois_launch(p, raster, first, count, full);
   emc_ctx* ctx = p->ctx;
@@ -1539,22 +1870,22 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
   TcEstepArgs a;
   a.N = p->d.n_images;
   a.R = p->d.n_rot;
-  a.Kp = p->Kp;
   a.n_pt = p->Np / es::BM;
   a.n_rt = p->Rp / es::BN;
   a.nkb = p->Kp / es::BK;
   a.raster = raster;
-  // auto: G lo always; H lo too when the intensity is known (phi = 1 leaves
-  // the C = K^2 . H term unbalanced, and its rounding shows in the likelihood)
-  a.gh_lo = p->estep_gh_lo >= 0 ? p->estep_gh_lo : (p->d.known_intensity ? 3 : 1);
+  a.gh_lo = estep_gh_lo(p);
   a.tiles = full ? nullptr : p->prune_tiles;
-  a.k2lo_any = p->k2lo_any;
-  a.glo_kb = p->glo_kb;
-  a.k2_inv = 1.0f / p->k2_scale;
+  a.rot_inv = p->rot_flags;
+  a.rot_tiny = p->rot_flags + (size_t)a.n_rt * a.nkb;
   a.rot_cnt = p->rot_cnt;
   a.rot_A = p->rot_A;
   a.rotw = p->rotw;
   a.cnorm = p->cnorm;
+  a.ktot = p->ktot;
+  a.k2tot = p->k2tot;
+  a.k_inv = 1.0f / p->count_scale;
+  a.zrow = p->Rp;
   a.sigma = p->sigma_dev;
   a.known_intensity = p->d.known_intensity;
   a.L = p->L;
@@ -1563,9 +1894,10 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
   a.bad = p->flags + 4;
   a.status = st->status;
   a.spin = p->debug_spin ? p->debug_spin : ptx::kSpinLimit;
-  const CUtensorMap* rm = st->rot;
-  if (p->estep_pair && !a.tiles && !(a.gh_lo & 2)) {
+  if (p->estep_pair && !a.tiles) {
     // CTA pairs: tiles are (pattern-tile pair, rotation tile)
+    a.list = p->pp_list;
+    a.list_n = p->pp_n;
     const int total = ((a.n_pt + 1) / 2) * a.n_rt;
     first = std::max(0, std::min(first, total));
     const int pairs = std::min(total - first, count);
@@ -1574,7 +1906,7 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * pairs);
     cfg.blockDim = dim3(es::THREADS);
-    cfg.dynamicSmemBytes = es2::SMEM_BYTES;
+    cfg.dynamicSmemBytes = es::SMEM_BYTES;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -1583,9 +1915,9 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_estep_pair_kernel, st->mK, st->mK2h, st->mK2l,
-                                             rm[0], rm[1], rm[2], st->gl64, rm[4], a);
-    if (e == cudaSuccess) return after_launch(ctx, "tc_estep_pair_kernel");
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_estep_kernel<true>, st->mK, st->mJ, st->mJl,
+                                             st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
+    if (e == cudaSuccess) return after_launch(ctx, "tc_estep_kernel (pairs)");
     // a refused launch configuration (a GPU or partition that cannot
     // co-schedule the pairs) is not a sticky error: single CTAs from now on
     (void)cudaGetLastError();
@@ -1593,13 +1925,15 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     first *= 2;  // about the same part of the grid, in single-CTA tiles
     count = count > INT_MAX / 2 ? INT_MAX : 2 * count;
   }
+  a.list = p->pt_list;
+  a.list_n = p->pt_n;
   const int total = a.n_pt * a.n_rt;
   first = a.tiles ? 0 : std::max(0, std::min(first, total));
   const int grid = a.tiles ? p->prune_n_tiles : std::min(total - first, count);
   a.tile0 = first;
   if (grid == 0) return EMC_OK;
-  tc_estep_kernel<<<grid, es::THREADS, es::SMEM_BYTES, ctx->stream>>>(
-      st->mK, st->mK2h, st->mK2l, rm[0], rm[1], rm[2], rm[3], rm[4], rm[5], a);
+  tc_estep_kernel<false><<<grid, es::THREADS, es::SMEM_BYTES, ctx->stream>>>(
+      st->mK, st->mJ, st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tc_estep_kernel launch");
   return after_launch(ctx, "tc_estep_kernel");
@@ -1613,34 +1947,27 @@ RotOps tc_rot_ops(emc_plan* p) {
   if (!p->tc) return o;
   TcState* st = state(p);
   o.flags = p->flags;
-  o.Gh = st->Gh;
-  o.Gl = st->Gl;
+  o.live = p->blk_live;
+  o.nkb = p->Kp / es::BK;
   if (p->d.diff == EMC_DIFF_TRUE_POISSON) {
-    o.logs = 1;
-  } else {
-    // the lo planes only where the likelihood reads them (EMC_OPT_ESTEP_GHLO;
-    // auto: G lo, and H lo when the intensity is known)
-    const int gh = p->estep_gh_lo >= 0 ? p->estep_gh_lo : (p->d.known_intensity ? 3 : 1);
-    o.Mp = st->Mp;
-    o.MSh = st->MSh;
-    o.Hh = st->Hh;
-    o.Gl = (gh & 1) ? st->Gl : nullptr;
-    o.Hl = (gh & 2) ? st->Hl : nullptr;
-    if (o.Gl && p->glo_kb) o.gl_end = p->glo_kb + p->Np / es::BM;
+    o.Lh = st->Lh;
+    o.Ll = st->Ll;
+    return o;
   }
+  const int gh = estep_gh_lo(p);
+  o.MS = st->MS;
+  o.Hh = st->Hh;
+  o.Iv = st->Iv;
+  o.inv = p->rot_flags;
+  o.tiny = p->rot_flags + (size_t)p->n_rt * o.nkb;
+  o.Hl = gh ? st->Hl : nullptr;
+  if (gh == 1) o.hl_end = p->lo_kb + p->Np / es::BM;
   return o;
 }
 
-// The likelihood lo terms in force: bit 0 G lo, bit 1 H lo (auto: H lo when
-// the intensity is known).
-static int estep_gh_lo(const emc_plan* p) {
-  return p->estep_gh_lo >= 0 ? p->estep_gh_lo : (p->d.known_intensity ? 3 : 1);
-}
-
-// Full scans of the reference likelihood run on CTA pairs unless switched
-// off or H lo is needed (the pair kernel has no H lo slot).
+// Full scans of the reference likelihood run on CTA pairs unless switched off.
 static bool estep_uses_pair(const emc_plan* p) {
-  return p->estep_pair && p->d.diff != EMC_DIFF_TRUE_POISSON && !(estep_gh_lo(p) & 2);
+  return p->estep_pair && p->d.diff != EMC_DIFF_TRUE_POISSON;
 }
 
 // One timed launch of the likelihood kernel over tiles [first, first + count)
@@ -1769,6 +2096,7 @@ int tc_mstep(emc_plan* p, float* model, float* weight) {
   a.raster = p->mstep_raster;
   a.T = p->T;
   a.qscale = p->qscale;
+  a.k_inv = 1.0f / p->count_scale;
   a.rot = p->rot;
   a.cx = p->cx;
   a.cy = p->cy;
