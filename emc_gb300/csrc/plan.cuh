@@ -61,6 +61,10 @@ struct emc_plan {
   uint32_t *pt_list = nullptr, *pp_list = nullptr;
   int *pt_n = nullptr, *pp_n = nullptr;
   unsigned char* blk_live = nullptr;  // [Kp/64] some pattern counts there
+  // M-step: [Kp/64][Np/64] the (64-pixel, 64-pattern) block holds a count; per
+  // 256-pixel tile the pattern blocks that hold one (never none) as a map and a list
+  unsigned char *sub_any = nullptr, *ms_map = nullptr;
+  int *ms_list = nullptr, *ms_n = nullptr;
   // [Np/128 + 1] K . H takes H's lo half on the 64-pixel blocks below lo_kb[pt]:
   // the blocks after it hold at most 300 glo_tail_ppm / 1e6 of every pattern's
   // counts (EMC_OPT_GLO_TAIL; 0: every block); lo_kb[Np/128] is the largest
@@ -87,6 +91,7 @@ struct emc_plan {
   float2* part = nullptr;  // [n_rt][N] (max, sumexp) per rotation tile
   double* lse = nullptr;   // [N]
   float2* lse2 = nullptr;  // [N] lse as float hi + lo
+  double* ll_part = nullptr;  // [N/32] sums of lse
   float* T = nullptr;      // [Rp] rotation totals
   double* red = nullptr;   // reduction scratch (small)
   unsigned long long* fix_m = nullptr;  // [s^3] fixed-point model (deterministic insert)

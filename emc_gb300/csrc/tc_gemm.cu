@@ -113,7 +113,8 @@ constexpr uint32_t kAny = 8;  // a count
 // j is written for both.  256 rows x 128 B, eight 16-byte loads a thread.
 __global__ void __launch_bounds__(256) tc_count_blocks_kernel(
     const __half* __restrict__ Kh, int Kp, int nkb, int n_pt, float scale,
-    __half* __restrict__ Jh, __half* __restrict__ Jl, unsigned char* __restrict__ bits) {
+    __half* __restrict__ Jh, __half* __restrict__ Jl, unsigned char* __restrict__ bits,
+    unsigned char* __restrict__ sub_any) {
   const int kb = blockIdx.x, pt0 = 2 * blockIdx.y;
   const int nt = min(2, n_pt - pt0);
   const float inv = 1.0f / scale;
@@ -122,6 +123,7 @@ __global__ void __launch_bounds__(256) tc_count_blocks_kernel(
     __half h[8];
   } v[2][4];
   int any[2] = {0, 0}, two[2] = {0, 0}, low[2] = {0, 0};
+  int sub[2][2] = {};  // of the tile's two halves of 64 patterns
   auto at = [&](int t, int j) {
     const int e = threadIdx.x + 256 * j;
     return (size_t)((pt0 + t) * 128 + (e >> 3)) * Kp + kb * 64 + (e & 7) * 8;
@@ -133,14 +135,16 @@ __global__ void __launch_bounds__(256) tc_count_blocks_kernel(
     for (int j = 0; j < 4; ++j) v[t][j].u = *reinterpret_cast<const uint4*>(Kh + at(t, j));
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      any[t] |= (v[t][j].u.x | v[t][j].u.y | v[t][j].u.z | v[t][j].u.w) != 0;
+      sub[t][j >> 1] |= (v[t][j].u.x | v[t][j].u.y | v[t][j].u.z | v[t][j].u.w) != 0;
 #pragma unroll
       for (int c = 0; c < 8; ++c) two[t] |= __half2float(v[t][j].h[c]) * inv > 1.0f;
     }
   }
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    any[t] = __syncthreads_or(any[t]);
+    sub[t][0] = __syncthreads_or(sub[t][0]);
+    sub[t][1] = __syncthreads_or(sub[t][1]);
+    any[t] = sub[t][0] | sub[t][1];
     two[t] = __syncthreads_or(two[t]);
   }
   if ((two[0] | two[1]) && Jh) {
@@ -171,6 +175,11 @@ __global__ void __launch_bounds__(256) tc_count_blocks_kernel(
 #pragma unroll
         for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(Jl + at(t, j)) = lo[t][j].u;
       }
+  }
+  if (threadIdx.x < 2 * nt) {
+    const int t = threadIdx.x >> 1, h = threadIdx.x & 1;
+    sub_any[(size_t)kb * (2 * n_pt) + 2 * pt0 + threadIdx.x] = (unsigned char)(
+        (t ? (h ? sub[1][1] : sub[1][0]) : (h ? sub[0][1] : sub[0][0])) != 0);
   }
   if (threadIdx.x < nt) {
     const int t = threadIdx.x;
@@ -245,15 +254,36 @@ __global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __rest
   }
 }
 
-// List i < n_pt: the blocks of pattern tile i; list n_pt + i: those of tiles 2 i
-// and 2 i + 1 together.  One warp each.  A tile without counts keeps block 0, so
-// that its accumulators are written.  The last warps: live[kb].
+// First n_qt warps: the M-step's lists.  Then list i < n_pt: the blocks of pattern
+// tile i; list n_pt + i: those of tiles 2 i and 2 i + 1 together.  One warp each.
+// A tile without counts keeps block 0, so that its accumulators are written.  The
+// last warps: live[kb].
 __global__ void __launch_bounds__(32) tc_block_lists_kernel(
     const unsigned char* __restrict__ bits, int n_pt, int nkb, const int* __restrict__ lo_kb,
     uint32_t* __restrict__ pt_list, int* __restrict__ pt_n, uint32_t* __restrict__ pp_list,
-    int* __restrict__ pp_n, unsigned char* __restrict__ live) {
+    int* __restrict__ pp_n, unsigned char* __restrict__ live,
+    const unsigned char* __restrict__ sub_any, int n_qt, unsigned char* __restrict__ ms_map,
+    int* __restrict__ ms_list, int* __restrict__ ms_n) {
   const int lane = threadIdx.x, n_pp = (n_pt + 1) / 2;
   int i = blockIdx.x;
+  if (i < n_qt) {  // the M-step's list of pixel tile i
+    const int nb = 2 * n_pt;
+    int n = 0;
+    for (int b0 = 0; b0 < nb; b0 += 32) {
+      const int b = b0 + lane;
+      int any = 0;
+      for (int k = 4 * i; k < min(4 * i + 4, nkb); ++k)
+        any |= b < nb ? sub_any[(size_t)k * nb + b] : 0;
+      const unsigned on = __ballot_sync(0xffffffffu, any);
+      if (b < nb) ms_map[(size_t)i * nb + b] = (unsigned char)any;
+      if (any) ms_list[(size_t)i * nb + n + __popc(on & ((1u << lane) - 1u))] = b;
+      n += __popc(on);
+    }
+    if (n == 0 && lane == 0) ms_list[(size_t)i * nb] = 0;
+    if (lane == 0) ms_n[i] = max(n, 1);
+    return;
+  }
+  i -= n_qt;
   if (i >= n_pt + n_pp) {
     const int kb = (i - n_pt - n_pp) * 32 + lane;
     if (kb >= nkb) return;
@@ -1163,8 +1193,10 @@ constexpr int BN = 256;   // pixels per tile
 constexpr int BK = 64;    // patterns per stage (128 B rows, 128B swizzle)
 constexpr int A_BYTES = BM * BK * 2;  // 16 KB
 constexpr int B_BYTES = BN * BK * 2;  // 32 KB
-constexpr int EPI_WARPS = 8;          // two per TMEM lane quarter, 128 columns each
+constexpr int EPI_WARPS = 16;         // four per TMEM lane quarter, 64 columns each
+constexpr int EPI_COLS = BN / (EPI_WARPS / 4);
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
+constexpr int XYZ_BYTES = 2 * BN * 16;  // pixel coordinates of two tiles
 }  // namespace ms
 
 struct TcMstepArgs {
@@ -1190,17 +1222,14 @@ struct TcMstepArgs {
   // kb_list[kb_off[rt] .. kb_off[rt+1]) (Q is zero elsewhere); nullptr: all
   const int* kb_off;
   const int* kb_list;
+  // per pixel tile, the pattern k-blocks in which it has counts (list, count,
+  // map; K is zero elsewhere)
+  const int* ms_list;
+  const int* ms_n;
+  const unsigned char* ms_map;
   int* status;
   uint32_t spin;  // polls per pipeline wait
 };
-
-// The k-blocks of rotation tile rt: count, and the j-th of them.
-__device__ __forceinline__ int ms_nkb(const TcMstepArgs& a, int rt) {
-  return a.kb_off ? a.kb_off[rt + 1] - a.kb_off[rt] : a.nkb;
-}
-__device__ __forceinline__ int ms_kb(const TcMstepArgs& a, int rt, int j) {
-  return a.kb_off ? a.kb_list[a.kb_off[rt] + j] : j;
-}
 
 __device__ __forceinline__ void tc_add(const TcMstepArgs& a, size_t v, float val, float w) {
   if (a.deterministic) {
@@ -1240,31 +1269,83 @@ __device__ __forceinline__ void tc_insert_nearest(const TcMstepArgs& a, bool on,
   if (on) tc_add(a, (size_t)v, val, w);
 }
 
-__device__ __forceinline__ void tc_insert(const TcMstepArgs& a, const RotMat& R, bool on, float x,
-                                          float y, float z, float val, float w) {
+// Trilinear insertion of one value.
+__device__ __forceinline__ void tc_insert_trilinear(const TcMstepArgs& a, const RotMat& R, float x,
+                                                    float y, float z, float val, float w) {
   const int side = a.side;
-  if (a.interp == EMC_INTERP_NEAREST) {
-    const long ix = voxel_round(voxel_coord(side, rotate_row(R, 0, x, y, z)));
-    const long iy = voxel_round(voxel_coord(side, rotate_row(R, 1, x, y, z)));
-    const long iz = voxel_round(voxel_coord(side, rotate_row(R, 2, x, y, z)));
-    const bool in = on && ix >= 0 && ix < side && iy >= 0 && iy < side && iz >= 0 && iz < side;
-    tc_insert_nearest(a, in, in ? ((long long)iz * side + iy) * side + ix : -1, val, w);
-  } else {
-    if (!on) return;
-    const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
-    const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
-    const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
-    const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
-    const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-    const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
+  const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
+  const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
+  const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
+  const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
+  const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
+  const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int xi = x0 + (k & 1), yi = y0 + ((k >> 1) & 1), zi = z0 + (k >> 2);
-      if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
-      const float f = ((k & 1) ? tx : 1.0f - tx) * (((k >> 1) & 1) ? ty : 1.0f - ty) *
-                      ((k >> 2) ? tz : 1.0f - tz);
-      if (f <= 0.0f) continue;
-      tc_add(a, ((size_t)zi * side + yi) * side + xi, val * f, w * f);
+  for (int k = 0; k < 8; ++k) {
+    const int xi = x0 + (k & 1), yi = y0 + ((k >> 1) & 1), zi = z0 + (k >> 2);
+    if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
+    const float f = ((k & 1) ? tx : 1.0f - tx) * (((k >> 1) & 1) ? ty : 1.0f - ty) *
+                    ((k >> 2) ? tz : 1.0f - tz);
+    if (f <= 0.0f) continue;
+    tc_add(a, ((size_t)zi * side + yi) * side + xi, val * f, w * f);
+  }
+}
+
+// The coordinates of a tile's 256 pixels into shared memory, by the first 256 of
+// the epilogue's threads; read by all of them after the barrier.  Two buffers: a
+// thread that writes the tile after next has passed the next tile's barrier, so
+// every thread is done with this one.
+__device__ __forceinline__ const float4* ms_stage_pixels(const TcMstepArgs& a, float4* s_xyz,
+                                                         int tile, int q0) {
+  float4* dst = s_xyz + (tile & 1) * ms::BN;
+  const int e = (int)threadIdx.x - 64;
+  if (e < ms::BN && q0 + e < a.P_eff)
+    dst[e] = make_float4(__ldg(a.cx + q0 + e), __ldg(a.cy + q0 + e), __ldg(a.cz + q0 + e), 0.0f);
+  asm volatile("bar.sync 1, %0;" ::"n"(ms::EPI_WARPS * 32) : "memory");
+  return dst;
+}
+
+// The insertion of one tile by one epilogue warp: rotation r0 + its lane's row,
+// TMEM columns c_beg .. + EPI_COLS (pixels q0 + column).  Sixteen voxels are
+// worked out before the first of their atomics: with one pixel at a time, its
+// coordinates loaded from global memory between two atomics and U divided by
+// T_r and multiplied again, a column took a warp 1,050 clocks (73 us for a tile,
+// all of a small problem's M-step and most of a pruned one's).
+__device__ __forceinline__ void ms_insert(const TcMstepArgs& a, uint32_t taddr, const float4* xyz,
+                                          int q0, int c_beg, int r, bool rok, float Tr, float qs,
+                                          const RotMat& Rm) {
+  const bool live = rok && Tr > 1e-10f;
+  const int side = a.side;
+  for (int c0 = c_beg; c0 < c_beg + ms::EPI_COLS; c0 += 16) {
+    const int nc = a.P_eff - (q0 + c0);  // columns that are pixels (uniform over the warp)
+    if (nc <= 0) break;
+    float u[16];
+    ptx::tmem_ld16(taddr + c0, u);
+    ptx::tmem_wait_ld();
+    if (a.u) {  // sorted mode: a coalesced store per column (lanes: rotations)
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (rok && j < nc) a.u[(size_t)(q0 + c0 + j) * a.ldu + r] = live ? u[j] * qs : 0.0f;
+    } else if (a.interp == EMC_INTERP_NEAREST) {
+      int v[16];
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float4 p = xyz[c0 + j];
+        const int ix = voxel_round(voxel_coord(side, rotate_row(Rm, 0, p.x, p.y, p.z)));
+        const int iy = voxel_round(voxel_coord(side, rotate_row(Rm, 1, p.x, p.y, p.z)));
+        const int iz = voxel_round(voxel_coord(side, rotate_row(Rm, 2, p.x, p.y, p.z)));
+        const bool in = live && j < nc && (unsigned)ix < (unsigned)side &&
+                        (unsigned)iy < (unsigned)side && (unsigned)iz < (unsigned)side;
+        v[j] = in ? (iz * side + iy) * side + ix : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) tc_insert_nearest(a, v[j] >= 0, v[j], u[j] * qs, Tr);
+    } else if (live) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j)
+        if (j < nc) {
+          const float4 p = xyz[c0 + j];
+          tc_insert_trilinear(a, Rm, p.x, p.y, p.z, u[j] * qs, Tr);
+        }
     }
   }
 }
@@ -1291,7 +1372,7 @@ struct MsRing {
   static constexpr int kStageBytes = (QLO ? 2 : 1) * ms::A_BYTES + ms::B_BYTES;
   static constexpr int kStages = QLO ? 3 : 4;
   static constexpr int kOffK = (QLO ? 2 : 1) * ms::A_BYTES;  // K^T tile in a stage
-  static constexpr int kSmem = kStages * kStageBytes + 256 + 1024;
+  static constexpr int kSmem = kStages * kStageBytes + 256 + ms::XYZ_BYTES + 1024;
   static_assert(kSmem <= 232448, "shared memory of the M-step ring");
 };
 
@@ -1309,6 +1390,17 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
   uint64_t* tempty = tfull + 2;      // [2] accumulator drained (one arrival per epilogue warp)
   uint64_t* drain = tempty + 2;      // the MMA issuer's own completion wait before TMEM is freed
   uint32_t* tmem_slot = (uint32_t*)(drain + 1);
+  float4* s_xyz = (float4*)(smem + Ring::kStages * Ring::kStageBytes + 256);
+  // the k-blocks of tile (rt, qt): those with counts, of all or (pruned) of the
+  // rotation tile's; the first one always, so that the accumulator is written
+  auto blocks = [&](int rt, int qt) {
+    return a.kb_off ? a.kb_off[rt + 1] - a.kb_off[rt] : a.ms_n[qt];
+  };
+  auto block = [&](int rt, int qt, int j) {  // -1: passed over
+    if (!a.kb_off) return a.ms_list[(size_t)qt * a.nkb + j];
+    const int kb = a.kb_list[a.kb_off[rt] + j];
+    return j == 0 || a.ms_map[(size_t)qt * a.nkb + kb] ? kb : -1;
+  };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -1340,9 +1432,10 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x) {
         int r0, q0;
         ms_tile(a, t, r0, q0);
-        const int nk = ms_nkb(a, r0 / BM);
-        for (int j = 0; j < nk; ++j, ++it) {
-          const int kb = ms_kb(a, r0 / BM, j);
+        const int nk = blocks(r0 / BM, q0 / BN);
+        for (int j = 0; j < nk; ++j) {
+          const int kb = block(r0 / BM, q0 / BN, j);
+          if (kb < 0) continue;
           const int s = it % Ring::kStages;
           const uint32_t ph = (it / Ring::kStages) & 1;
           if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 4, a.spin)) {
@@ -1354,6 +1447,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
           ptx::tma_load_2d(st, &mQh, kb * BK, r0, &full[s]);
           if (QLO) ptx::tma_load_2d(st + A_BYTES, &mQl, kb * BK, r0, &full[s]);
           ptx::tma_load_2d(st + Ring::kOffK, &mKt, kb * BK, q0, &full[s]);
+          ++it;
         }
       }
       ptx::drain_loads(full, Ring::kStages, it, a.status, 11);  // none in flight at exit
@@ -1374,8 +1468,9 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
         ms_tile(a, t, r0t, q0t);
         // a tile with no k-block leaves the buffer as it was: its rotations
         // have no responsibility (T_r = 0), so the epilogue inserts nothing
-        const int nk = ms_nkb(a, r0t / BM);
-        for (int kb = 0; kb < nk; ++kb, ++it) {
+        const int nk = blocks(r0t / BM, q0t / BN);
+        for (int j2 = 0; j2 < nk; ++j2) {
+          if (a.kb_off && block(r0t / BM, q0t / BN, j2) < 0) continue;
           const int s = it % Ring::kStages;
           const uint32_t ph = (it / Ring::kStages) & 1;
           if (!ptx::mbar_wait(&full[s], ph, a.status, 5, a.spin)) {
@@ -1389,9 +1484,10 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
             const uint64_t dQh = ptx::smem_desc(base + ks * 32, 1024, 2);
             const uint64_t dQl = ptx::smem_desc(base + A_BYTES + ks * 32, 1024, 2);
             const uint64_t dK = ptx::smem_desc(base + Ring::kOffK + ks * 32, 1024, 2);
-            ptx::mma_f16(d, dQh, dK, idesc, (kb | ks) ? 1u : 0u);
+            ptx::mma_f16(d, dQh, dK, idesc, (j2 | ks) ? 1u : 0u);
             if (QLO) ptx::mma_f16(d, dQl, dK, idesc, 1u);
           }
+          ++it;
           ptx::mma_commit(&empty[s]);
         }
         ptx::mma_commit(&tfull[b]);  // fires when this tile's MMAs have completed
@@ -1400,10 +1496,11 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       ptx::mbar_wait(drain, 0, a.status, 12);
     }
   } else {
-    // ------------------------------------------------ insertion epilogue (warps 2-9)
+    // ------------------------------------------------ insertion epilogue
     const int quarter = warp & 3;       // TMEM lanes this warp may access
-    const int half = (warp - 2) >> 2;   // which 128 of the tile's 256 columns
+    const int part = (warp - 2) >> 2;   // which of the tile's columns
     const int rl = quarter * 32 + lane;
+    bool ok = true;
     int j = 0;
     for (int t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++j) {
       const int b = j & 1;
@@ -1413,31 +1510,15 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       const bool rok = r < a.R;
       const float Tr = rok ? a.T[r] : 0.0f;
       const float qs = rok ? a.qscale[r] * a.k_inv : 0.0f;
-      const bool live = rok && Tr > 1e-10f;
       RotMat Rm = {};
       if (rok) Rm = quat_to_matrix(a.rot + 4 * (size_t)r);
-      if (!ptx::mbar_wait_sleep(&tfull[b], (j >> 1) & 1, a.status, 6, 128, a.spin)) break;
-      ptx::tc_fence_after();
-      const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
-      for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 16) {
-        float u[16];
-        ptx::tmem_ld16(lane_addr + c0, u);
-        ptx::tmem_wait_ld();
-        if (q0 + c0 >= a.P_eff) continue;  // padding columns (uniform over the warp)
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {  // fully unrolled: u[] stays in registers
-          const int q = q0 + c0 + jj;
-          if (q < a.P_eff) {  // uniform over the warp
-            const float U = u[jj] * qs;
-            const float slice = live ? U / Tr : 0.0f;
-            if (a.u) {  // sorted mode: a coalesced store per column (lanes: rotations)
-              if (rok) a.u[(size_t)q * a.ldu + r] = Tr * slice;
-            } else {
-              tc_insert(a, Rm, live, __ldg(a.cx + q), __ldg(a.cy + q), __ldg(a.cz + q),
-                        Tr * slice, Tr);
-            }
-          }
-        }
+      const float4* xyz = ms_stage_pixels(a, s_xyz, j, q0);
+      // after a wait that gave up the warp only keeps the other warps' barrier going
+      ok = ok && ptx::mbar_wait_sleep(&tfull[b], (j >> 1) & 1, a.status, 6, 128, a.spin);
+      if (ok) {
+        ptx::tc_fence_after();
+        ms_insert(a, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN), xyz, q0,
+                  part * EPI_COLS, r, rok, Tr, qs, Rm);
       }
       // this warp's reads of buffer b are complete: hand it back to the MMA warp
       ptx::tc_fence_before();
@@ -1477,7 +1558,7 @@ struct Ring {
   static constexpr int kStageBytes = (QLO ? 2 : 1) * A_BYTES + B_BYTES;
   static constexpr int kStages = QLO ? 4 : 6;
   static constexpr int kOffK = (QLO ? 2 : 1) * A_BYTES;
-  static constexpr int kSmem = kStages * kStageBytes + 256 + 1024;
+  static constexpr int kSmem = kStages * kStageBytes + 256 + ms::XYZ_BYTES + 1024;
   static_assert(kSmem <= 232448, "shared memory of the pair M-step");
 };
 }  // namespace ms2
@@ -1499,6 +1580,7 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
   uint64_t* tempty = tfull + 2;      // [2] rank 0: accumulator drained by both CTAs
   uint64_t* drain = tempty + 2;      // rank 0's MMA issuer waits on it before TMEM is freed
   uint32_t* tmem_slot = (uint32_t*)(drain + 1);
+  float4* s_xyz = (float4*)(smem + STAGES * STAGE_BYTES + 256);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = ptx::cluster_ctarank();
@@ -1537,7 +1619,12 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
         int qt, rp;
         raster_tile(t, a.raster, a.n_qt, n_rp, qt, rp);
         const int r0 = (2 * rp + (int)rank) * BM, q0 = qt * BN + 128 * (int)rank;
-        for (int kb = 0; kb < a.nkb; ++kb, ++it) {
+        const int nk = a.ms_n[qt];
+        const int* list = a.ms_list + (size_t)qt * a.nkb;
+        int kb_next = __ldg(list);
+        for (int j = 0; j < nk; ++j, ++it) {
+          const int kb = kb_next;
+          if (j + 1 < nk) kb_next = __ldg(list + j + 1);
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 4, a.spin)) {
@@ -1565,9 +1652,12 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       for (int t = cl; t < n_tiles && ok; t += ncl, ++j) {
         const int b = j & 1;
         const uint32_t d = tmem + (uint32_t)(b * BN);
+        int qt, rp;
+        raster_tile(t, a.raster, a.n_qt, n_rp, qt, rp);
+        const int nk = a.ms_n[qt];
         if (!ptx::mbar_wait_cluster(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin)) break;
         ptx::tc_fence_after();
-        for (int kb = 0; kb < a.nkb; ++kb, ++it) {
+        for (int kb = 0; kb < nk; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1;
           if (!ptx::mbar_wait(&full[s], ph, a.status, 5, a.spin)) {
@@ -1592,10 +1682,11 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       ptx::mbar_wait(drain, 0, a.status, 12);
     }
   } else {
-    // ------------------------------------------------ insertion epilogue (warps 2-9)
+    // ------------------------------------------------ insertion epilogue
     const int quarter = warp & 3;      // TMEM lanes this warp may access
-    const int half = (warp - 2) >> 2;  // which 128 of the tile's 256 columns
+    const int part = (warp - 2) >> 2;  // which of the tile's columns
     const int rl = quarter * 32 + lane;
+    bool ok = true;
     const uint32_t back = rank == 0 ? 0u : 1u;
     int j = 0;
     for (int t = cl; t < n_tiles; t += ncl, ++j) {
@@ -1607,31 +1698,15 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
       const bool rok = r < a.R;
       const float Tr = rok ? a.T[r] : 0.0f;
       const float qs = rok ? a.qscale[r] * a.k_inv : 0.0f;
-      const bool live = rok && Tr > 1e-10f;
       RotMat Rm = {};
       if (rok) Rm = quat_to_matrix(a.rot + 4 * (size_t)r);
-      if (!ptx::mbar_wait_sleep(&tfull[b], (j >> 1) & 1, a.status, 6, 128, a.spin)) break;
-      ptx::tc_fence_after();
-      const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
-      for (int c0 = half * 128; c0 < half * 128 + 128; c0 += 16) {
-        float u[16];
-        ptx::tmem_ld16(lane_addr + c0, u);
-        ptx::tmem_wait_ld();
-        if (q0 + c0 >= a.P_eff) continue;  // padding columns (uniform over the warp)
-#pragma unroll
-        for (int jj = 0; jj < 16; ++jj) {
-          const int q = q0 + c0 + jj;
-          if (q < a.P_eff) {
-            const float U = u[jj] * qs;
-            const float slice = live ? U / Tr : 0.0f;
-            if (a.u) {  // sorted mode: a coalesced store per column (lanes: rotations)
-              if (rok) a.u[(size_t)q * a.ldu + r] = Tr * slice;
-            } else {
-              tc_insert(a, Rm, live, __ldg(a.cx + q), __ldg(a.cy + q), __ldg(a.cz + q),
-                        Tr * slice, Tr);
-            }
-          }
-        }
+      const float4* xyz = ms_stage_pixels(a, s_xyz, j, q0);
+      // after a wait that gave up the warp only keeps the other warps' barrier going
+      ok = ok && ptx::mbar_wait_sleep(&tfull[b], (j >> 1) & 1, a.status, 6, 128, a.spin);
+      if (ok) {
+        ptx::tc_fence_after();
+        ms_insert(a, tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN), xyz, q0,
+                  part * EPI_COLS, r, rok, Tr, qs, Rm);
       }
       // this warp's reads of buffer b are complete: hand it back to rank 0's MMA warp
       ptx::tc_fence_before();
@@ -1702,6 +1777,11 @@ int tc_bind(emc_plan* p) {
     if (!rc) rc = plan_alloc(p, (void**)&p->pt_n, n_pt * 4);
     if (!rc) rc = plan_alloc(p, (void**)&p->pp_list, n_pp * nkb * 4);
     if (!rc) rc = plan_alloc(p, (void**)&p->pp_n, n_pp * 4);
+    const size_t n_qt = (size_t)ceil_div(Kp, ms::BN), npb = 2 * n_pt;
+    if (!rc) rc = plan_alloc(p, (void**)&p->sub_any, nkb * npb);
+    if (!rc) rc = plan_alloc(p, (void**)&p->ms_map, n_qt * npb);
+    if (!rc) rc = plan_alloc(p, (void**)&p->ms_list, n_qt * npb * 4);
+    if (!rc) rc = plan_alloc(p, (void**)&p->ms_n, n_qt * 4);
     if (!pois) {
       if (!rc) rc = plan_alloc(p, (void**)&p->Jh, pk * 2);
       if (!rc) rc = plan_alloc(p, (void**)&p->Jl, pk * 2);
@@ -1781,7 +1861,7 @@ int tc_pattern_side(emc_plan* p, const int* d_perm, bool counts_done) {
   }
   const int n_pt = Np / es::BM;
   tc_count_blocks_kernel<<<dim3(Kp / es::BK, (n_pt + 1) / 2), 256, 0, ctx->stream>>>(
-      p->Kh, Kp, Kp / es::BK, n_pt, p->count_scale, p->Jh, p->Jl, p->blk_bits);
+      p->Kh, Kp, Kp / es::BK, n_pt, p->count_scale, p->Jh, p->Jl, p->blk_bits, p->sub_any);
   if ((rc = after_launch(ctx, "tc_count_blocks_kernel"))) return rc;
   if ((rc = tc_block_lists(p))) return rc;
   transpose_h_kernel<<<dim3(ceil_div(Kp, 64), ceil_div(Np, 64)), dim3(32, 8), 0, ctx->stream>>>(
@@ -1804,8 +1884,10 @@ int tc_block_lists(emc_plan* p) {
         p->k2tot, p->lo_kb);
     if ((rc = after_launch(ctx, "tc_count_rows_kernel"))) return rc;
   }
-  tc_block_lists_kernel<<<n_pt + (n_pt + 1) / 2 + ceil_div(nkb, 32), 32, 0, ctx->stream>>>(
-      p->blk_bits, n_pt, nkb, p->lo_kb, p->pt_list, p->pt_n, p->pp_list, p->pp_n, p->blk_live);
+  const int n_qt = ceil_div(p->Kp, ms::BN);
+  tc_block_lists_kernel<<<n_qt + n_pt + (n_pt + 1) / 2 + ceil_div(nkb, 32), 32, 0, ctx->stream>>>(
+      p->blk_bits, n_pt, nkb, p->lo_kb, p->pt_list, p->pt_n, p->pp_list, p->pp_n, p->blk_live,
+      p->sub_any, n_qt, p->ms_map, p->ms_list, p->ms_n);
   return after_launch(ctx, "tc_block_lists_kernel");
 }
 
@@ -2111,6 +2193,9 @@ int tc_mstep(emc_plan* p, float* model, float* weight) {
   a.acc2 = p->acc2;
   a.q_lo = p->mstep_q_lo;
   a.aggregate = p->mstep_aggregate;
+  a.ms_list = p->ms_list;
+  a.ms_n = p->ms_n;
+  a.ms_map = p->ms_map;
   a.kb_off = p->prune_kb_off;
   a.kb_list = p->prune_kb_list;
   a.fix_scale = reinterpret_cast<const float2*>(p->red + kRedFixScale);
