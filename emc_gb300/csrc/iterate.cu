@@ -761,28 +761,62 @@ __global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
 }
 
 // ------------------------------------------------------- normalise -------
-// lse_i = M + log(sum_t s_t exp(m_t - M)) over the rotation tiles, FP64,
-// also as two floats hi + lo (hi = fl(lse), lo = fl(lse - hi)) so that
-// consumers form L - lse in FP32 to the same accuracy.  Patterns with no
-// valid pair get lse = +inf (all responsibilities 0).
-__global__ void lse_combine_kernel(const float2* __restrict__ part, int n_rt, int N,
-                                   double* __restrict__ lse, float2* __restrict__ lse2) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float M = -INFINITY;
-  for (int t = 0; t < n_rt; ++t) M = fmaxf(M, part[(size_t)t * N + n].x);
-  double l = INFINITY;
-  if (M > -INFINITY) {
-    double s = 0.0;
-    for (int t = 0; t < n_rt; ++t) {
+// Per pattern, over the rotation tiles' (max, sum exp) pairs: M = the largest max
+// and s = sum_t s_t exp(m_t - M), FP64.  A block takes 32 patterns; its eight
+// warps share the tiles (one thread per pattern left a small problem on a few
+// SMs, and its two serial walks over the tiles took 22 to 44 us there), and their
+// sums are added in warp order.  Results in warp 0, lane = pattern.
+constexpr int kLseWarps = 8;
+__device__ __forceinline__ void lse_tiles(const float2* __restrict__ part, int n_rt, int N, int n,
+                                          float& M, double& s) {
+  __shared__ float sm[kLseWarps][32];
+  __shared__ double ss[kLseWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  float m = -INFINITY;
+  if (n < N)
+    for (int t = warp; t < n_rt; t += kLseWarps) m = fmaxf(m, part[(size_t)t * N + n].x);
+  sm[warp][lane] = m;
+  __syncthreads();
+  M = -INFINITY;
+#pragma unroll
+  for (int w = 0; w < kLseWarps; ++w) M = fmaxf(M, sm[w][lane]);
+  double a = 0.0;
+  if (n < N && M > -INFINITY)
+    for (int t = warp; t < n_rt; t += kLseWarps) {
       const float2 v = part[(size_t)t * N + n];
-      if (v.x > -INFINITY) s += (double)v.y * exp((double)v.x - (double)M);
+      if (v.x > -INFINITY) a += (double)v.y * exp((double)v.x - (double)M);
     }
-    l = (double)M + log(s);
+  ss[warp][lane] = a;
+  __syncthreads();
+  s = 0.0;
+  if (warp == 0)
+#pragma unroll
+    for (int w = 0; w < kLseWarps; ++w) s += ss[w][lane];
+}
+
+// lse_i = M + log(s), FP64, also as two floats hi + lo (hi = fl(lse), lo =
+// fl(lse - hi)) so that consumers form L - lse in FP32 to the same accuracy.
+// Patterns with no valid pair get lse = +inf (all responsibilities 0).
+// ll_part[block] = the sum of the block's finite lse.
+__global__ void __launch_bounds__(32 * kLseWarps) lse_combine_kernel(
+    const float2* __restrict__ part, int n_rt, int N, double* __restrict__ lse,
+    float2* __restrict__ lse2, double* __restrict__ ll_part) {
+  const int n = blockIdx.x * 32 + (threadIdx.x & 31);
+  float M;
+  double s;
+  lse_tiles(part, n_rt, N, n, M, s);
+  if (threadIdx.x >= 32) return;
+  double l = INFINITY;
+  if (n < N) {
+    if (M > -INFINITY) l = (double)M + log(s);
+    lse[n] = l;
+    const float hi = (float)l;
+    lse2[n] = make_float2(hi, isfinite(l) ? (float)(l - (double)hi) : 0.0f);
   }
-  lse[n] = l;
-  const float hi = (float)l;
-  lse2[n] = make_float2(hi, isfinite(l) ? (float)(l - (double)hi) : 0.0f);
+  double t = isfinite(l) ? l : 0.0;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+  if (threadIdx.x == 0) ll_part[blockIdx.x] = t;
 }
 
 __global__ void fill_part_kernel(float2* __restrict__ part, size_t n) {
@@ -793,18 +827,13 @@ __global__ void fill_part_kernel(float2* __restrict__ part, size_t n) {
 
 // Deterministic FP64 sum of the finite entries of x[0..n) into out[0]
 // (one block; the order of additions is fixed).
-__global__ void finite_sum_kernel(const double* __restrict__ x, int n, double* __restrict__ out) {
-  __shared__ double sh[256];
-  double s = 0.0;
+__global__ void __launch_bounds__(1024) finite_sum_kernel(const double* __restrict__ x, int n,
+                                                          double* __restrict__ out) {
+  double s = 0.0, none = 0.0;
   for (int i = threadIdx.x; i < n; i += blockDim.x)
     if (isfinite(x[i])) s += x[i];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[0] = sh[0];
+  block_sum2(s, none);
+  if (threadIdx.x == 0) out[0] = s;
 }
 
 // One block per rotation row: P = exp(L - lse) (in place), Q = P / phi,
@@ -1202,14 +1231,17 @@ __global__ void insert_bounds_kernel(const double* __restrict__ row_mass,
 
 // Inserted sums -> weight and model / weight (-1 where the weight is 0,
 // emc_cuda.cu:758-768), from the fixed-point (deterministic) or the
-// interleaved float accumulators.
+// interleaved float accumulators; part: the blocks' {sum, count} of its positive
+// voxels, for the normalisation.
 __global__ void finish_insert_kernel(const unsigned long long* __restrict__ fm,
                                      const unsigned long long* __restrict__ fw,
                                      const float2* __restrict__ fix_scale,
                                      const float2* __restrict__ acc2, float* __restrict__ model,
-                                     float* __restrict__ weight, long long n) {
+                                     float* __restrict__ weight, long long n,
+                                     double* __restrict__ part) {
   const float2 sc = fm ? *fix_scale : make_float2(1.0f, 1.0f);
   const double inv_m = 1.0 / (double)sc.x, inv_w = 1.0 / (double)sc.y;  // powers of two
+  double s = 0.0, c = 0.0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     float m, w;
@@ -1222,27 +1254,33 @@ __global__ void finish_insert_kernel(const unsigned long long* __restrict__ fm,
       w = a.y;
     }
     weight[v] = w;
-    model[v] = w > 0.0f ? __fdiv_rn(m, w) : -1.0f;
+    const float q = w > 0.0f ? __fdiv_rn(m, w) : -1.0f;
+    model[v] = q;
+    if (q > 0.0f) {
+      s += (double)q;
+      c += 1.0;
+    }
+  }
+  block_sum2(s, c);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = s;
+    part[2 * blockIdx.x + 1] = c;
   }
 }
 
 // ---- one rank of a rotation split --------------------------------------
 // Per pattern, over this plan's rotations: the largest log-likelihood and the
 // sum of exp(L - max) (FP64), from the per-tile partials.
-__global__ void rank_partial_kernel(const float2* __restrict__ part, int n_rt, int N,
-                                    float* __restrict__ out_max, double* __restrict__ out_sum) {
-  const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  float M = -INFINITY;
-  for (int t = 0; t < n_rt; ++t) M = fmaxf(M, part[(size_t)t * N + n].x);
-  double sum = 0.0;
-  if (M > -INFINITY)
-    for (int t = 0; t < n_rt; ++t) {
-      const float2 v = part[(size_t)t * N + n];
-      if (v.x > -INFINITY) sum += (double)v.y * exp((double)v.x - (double)M);
-    }
+__global__ void __launch_bounds__(32 * kLseWarps) rank_partial_kernel(
+    const float2* __restrict__ part, int n_rt, int N, float* __restrict__ out_max,
+    double* __restrict__ out_sum) {
+  const int n = blockIdx.x * 32 + (threadIdx.x & 31);
+  float M;
+  double s;
+  lse_tiles(part, n_rt, N, n, M, s);
+  if (threadIdx.x >= 32 || n >= N) return;
   out_max[n] = M;
-  out_sum[n] = sum;
+  out_sum[n] = s;
 }
 
 // The normaliser combined over all ranks, in the plan's own form (FP64 and
@@ -1260,7 +1298,7 @@ __global__ void lse_from_global_kernel(const double* __restrict__ lse_in, int N,
 // The inserted sums as floats (model sum of T_r x slice, weight sum of T_r),
 // exactly as finish_insert_kernel reads them.
 __global__ void sums_out_kernel(const unsigned long long* __restrict__ fm,
-                                const unsigned long long* __restrict__ fw,
+                                     const unsigned long long* __restrict__ fw,
                                 const float2* __restrict__ fix_scale,
                                 const float2* __restrict__ acc2,
                                 float* __restrict__ msum, float* __restrict__ wsum, long long n) {
@@ -1284,12 +1322,23 @@ __global__ void sums_out_kernel(const unsigned long long* __restrict__ fm,
 __global__ void model_from_sums_kernel(const float* __restrict__ msum,
                                        const float* __restrict__ wsum, float n_ranks,
                                        float* __restrict__ model, float* __restrict__ weight,
-                                       long long n) {
+                                       long long n, double* __restrict__ part) {
+  double s = 0.0, c = 0.0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     const float m = __fdiv_rn(msum[v], n_ranks), w = __fdiv_rn(wsum[v], n_ranks);
     weight[v] = w;
-    model[v] = w > 0.0f ? __fdiv_rn(m, w) : -1.0f;
+    const float q = w > 0.0f ? __fdiv_rn(m, w) : -1.0f;
+    model[v] = q;
+    if (q > 0.0f) {
+      s += (double)q;
+      c += 1.0;
+    }
+  }
+  block_sum2(s, c);
+  if (threadIdx.x == 0) {
+    part[2 * blockIdx.x] = s;
+    part[2 * blockIdx.x + 1] = c;
   }
 }
 
@@ -1333,6 +1382,7 @@ extern "C" int emc_plan_create(emc_ctx* ctx, const emc_plan_desc* desc, emc_plan
   if (!rc) rc = alloc_n(p, &p->part, (size_t)p->n_rt * d.n_images);
   if (!rc) rc = alloc_n(p, &p->lse, d.n_images);
   if (!rc) rc = alloc_n(p, &p->lse2, d.n_images);
+  if (!rc) rc = alloc_n(p, &p->ll_part, ceil_div(d.n_images, 32));
   if (!rc) {
     cudaError_t e = cudaFuncSetAttribute(mprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(sizeof(float) * kMprepStageMax));
@@ -1643,7 +1693,14 @@ static int plan_mstep_fp32(emc_plan* p, float* model, float* weight, const Inser
 // E-step reads sigma from p->sigma_dev.  A full iteration runs them in order;
 // one rank of a rotation split (emc_rank_*) runs the E-step, exports its
 // per-pattern partials, and resumes at the M-step with the global normaliser.
-static int enqueue_normalise(emc_plan* p, float* d_model);
+static int enqueue_normalise(emc_plan* p, float* d_model, int nb);
+
+// Blocks of a pass over the model that leaves mean partials behind, and where
+// they go (the reduction buffer's tail).
+static int mean_blocks(const emc_plan* p, long long n) {
+  return (int)std::min<long long>(ceil_div(n, 1024), std::min(kMeanBlocks, p->ctx->sm_count * 4));
+}
+static double* mean_parts(const emc_plan* p) { return p->red + kRedSlots + 2 * (size_t)p->Rp + 2; }
 
 static int mark_phase(emc_plan* p, int i) {
   emc_ctx* ctx = p->ctx;
@@ -1678,10 +1735,11 @@ static int enqueue_lse(emc_plan* p) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images;
   int rc;
-  lse_combine_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(p->part, p->n_rt, N, p->lse,
-                                                                p->lse2);
+  const int nb = ceil_div(N, 32);
+  lse_combine_kernel<<<nb, 32 * kLseWarps, 0, ctx->stream>>>(p->part, p->n_rt, N, p->lse, p->lse2,
+                                                             p->ll_part);
   if ((rc = after_launch(ctx, "lse_combine_kernel"))) return rc;
-  finite_sum_kernel<<<1, 256, 0, ctx->stream>>>(p->lse, N, p->red + kRedLL);
+  finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->ll_part, nb, p->red + kRedLL);
   if ((rc = after_launch(ctx, "finite_sum_kernel"))) return rc;
   return mark_phase(p, 3);
 }
@@ -1737,31 +1795,23 @@ static int enqueue_finish(emc_plan* p, float* d_model, float* d_weight) {
   const long long n3 = (long long)p->d.side * p->d.side * p->d.side;
   const bool det = p->d.insert_mode == EMC_INSERT_DETERMINISTIC;
   int rc;
-  {
-    const int nb = (int)std::min<long long>(ceil_div(n3, 256), (long long)ctx->sm_count * 8);
-    finish_insert_kernel<<<nb, 256, 0, ctx->stream>>>(det ? p->fix_m : nullptr, p->fix_w,
-                                                       reinterpret_cast<const float2*>(p->red + kRedFixScale),
-                                                       p->acc2, d_model,
-                                                       d_weight, n3);
-    if ((rc = after_launch(ctx, "finish_insert_kernel"))) return rc;
-  }
+  const int nb = mean_blocks(p, n3);
+  finish_insert_kernel<<<nb, 256, 0, ctx->stream>>>(
+      det ? p->fix_m : nullptr, p->fix_w, reinterpret_cast<const float2*>(p->red + kRedFixScale),
+      p->acc2, d_model, d_weight, n3, mean_parts(p));
+  if ((rc = after_launch(ctx, "finish_insert_kernel"))) return rc;
   if ((rc = mark_phase(p, 5))) return rc;
-  return enqueue_normalise(p, d_model);
+  return enqueue_normalise(p, d_model, nb);
 }
 
-// model / positive mean (the reference's normalize_model), then the blur
-static int enqueue_normalise(emc_plan* p, float* d_model) {
+// model / positive mean (the reference's normalize_model) from the nb mean
+// partials of the pass that formed the model, then the blur
+static int enqueue_normalise(emc_plan* p, float* d_model, int nb) {
   emc_ctx* ctx = p->ctx;
   const long long n3 = (long long)p->d.side * p->d.side * p->d.side;
   int rc;
-  double* mean_stats = p->red + kRedMean;
-  // launch_positive_mean writes {sum, count} then its partials after them;
-  // kRedMean + 2 + 2*1024 fits in the reduction buffer tail.
-  double* tail = p->red + kRedSlots + 2 * (size_t)p->Rp;
-  if ((rc = launch_positive_mean(ctx, d_model, n3, tail))) return rc;
-  EMC_CUDA(ctx, cudaMemcpyAsync(mean_stats, tail, 2 * sizeof(double), cudaMemcpyDeviceToDevice,
-                                ctx->stream));
-  if ((rc = launch_scale_by_inverse_mean(ctx, d_model, n3, tail))) return rc;
+  if ((rc = launch_scale_by_partials(ctx, d_model, n3, mean_parts(p), nb, p->red + kRedMean)))
+    return rc;
   if (p->d.blur_sigma > 0.0f) {
     if ((rc = blur_run(ctx, d_model, p->blur))) return rc;
   }
@@ -2137,8 +2187,8 @@ extern "C" int emc_rank_estep(emc_plan* p, float* d_model, float sigma, float* d
   if (rc) return rc;
   if ((rc = enqueue_estep(p, d_model))) return rc;
   const int N = p->d.n_images;
-  rank_partial_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(p->part, p->n_rt, N, d_max,
-                                                                 d_sumexp);
+  rank_partial_kernel<<<ceil_div(N, 32), 32 * kLseWarps, 0, ctx->stream>>>(p->part, p->n_rt, N,
+                                                                          d_max, d_sumexp);
   return after_launch(ctx, "rank_partial_kernel");
 }
 
@@ -2154,7 +2204,7 @@ extern "C" int emc_rank_mstep(emc_plan* p, const double* d_lse, float* d_model_s
   lse_from_global_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(d_lse, N, p->lse, p->lse2);
   int rc = after_launch(ctx, "lse_from_global_kernel");
   if (rc) return rc;
-  finite_sum_kernel<<<1, 256, 0, ctx->stream>>>(p->lse, N, p->red + kRedLL);
+  finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->lse, N, p->red + kRedLL);
   if ((rc = after_launch(ctx, "finite_sum_kernel"))) return rc;
   if ((rc = mark_phase(p, 3))) return rc;
   if ((rc = enqueue_mstep(p, d_model_sum, d_weight_sum))) return rc;
@@ -2175,11 +2225,11 @@ extern "C" int emc_model_from_sums(emc_plan* p, const float* d_model_sum,
   EMC_REQUIRE(ctx, d_model_sum && d_weight_sum && d_model && d_weight && n_ranks >= 1,
               "model_from_sums: bad argument");
   const long long n3 = (long long)p->d.side * p->d.side * p->d.side;
-  const int nb = (int)std::min<long long>(ceil_div(n3, 256), (long long)ctx->sm_count * 8);
+  const int nb = mean_blocks(p, n3);
   model_from_sums_kernel<<<nb, 256, 0, ctx->stream>>>(d_model_sum, d_weight_sum, (float)n_ranks,
-                                                       d_model, d_weight, n3);
+                                                       d_model, d_weight, n3, mean_parts(p));
   int rc = after_launch(ctx, "model_from_sums_kernel");
   if (rc) return rc;
   if ((rc = mark_phase(p, 5))) return rc;
-  return enqueue_normalise(p, d_model);
+  return enqueue_normalise(p, d_model, nb);
 }

@@ -35,12 +35,6 @@ __global__ void divide_by_weight_kernel(float* __restrict__ model, const float* 
   }
 }
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-  for (int o = 16; o >= 1; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  return v;
-}
-
 // Per-block FP64 partial sum and count of x > 0.
 __global__ void __launch_bounds__(kRedThreads) positive_partial_kernel(const float* __restrict__ x,
                                                                        long long n,
@@ -54,35 +48,54 @@ __global__ void __launch_bounds__(kRedThreads) positive_partial_kernel(const flo
       c += 1.0;
     }
   }
-  __shared__ double ss[kRedThreads / 32], sc[kRedThreads / 32];
-  s = warp_sum_d(s);
-  c = warp_sum_d(c);
-  if ((threadIdx.x & 31) == 0) {
-    ss[threadIdx.x >> 5] = s;
-    sc[threadIdx.x >> 5] = c;
-  }
-  __syncthreads();
+  block_sum2(s, c);
   if (threadIdx.x == 0) {
-    double ts = 0.0, tc = 0.0;
-    for (int w = 0; w < kRedThreads / 32; ++w) {
-      ts += ss[w];
-      tc += sc[w];
-    }
-    part[2 * blockIdx.x] = ts;
-    part[2 * blockIdx.x + 1] = tc;
+    part[2 * blockIdx.x] = s;
+    part[2 * blockIdx.x + 1] = c;
   }
 }
 
-__global__ void positive_final_kernel(const double* __restrict__ part, int nb,
-                                      double* __restrict__ out) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double s = 0.0, c = 0.0;
-  for (int b = 0; b < nb; ++b) {
+// {sum, count} of nb partials by one block, in thread 0.  (One thread adding 608
+// pairs took 57 us, as long as four passes over a 128^3 model.)
+__device__ __forceinline__ void sum_partials(const double* __restrict__ part, int nb, double& s,
+                                             double& c) {
+  s = c = 0.0;
+  for (int b = threadIdx.x; b < nb; b += blockDim.x) {
     s += part[2 * b];
     c += part[2 * b + 1];
   }
-  out[0] = s;
-  out[1] = c;
+  block_sum2(s, c);
+}
+
+__global__ void __launch_bounds__(kRedThreads) positive_final_kernel(
+    const double* __restrict__ part, int nb, double* __restrict__ out) {
+  double s, c;
+  sum_partials(part, nb, s, c);
+  if (threadIdx.x == 0) {
+    out[0] = s;
+    out[1] = c;
+  }
+}
+
+__global__ void __launch_bounds__(kRedThreads) scale_by_partials_kernel(
+    float* __restrict__ x, long long n, const double* __restrict__ part, int nb,
+    double* __restrict__ out) {
+  __shared__ float s_inv;
+  double s, c;
+  sum_partials(part, nb, s, c);
+  if (threadIdx.x == 0) {
+    const float mean = c > 0.0 ? (float)(s / c) : 0.0f;
+    s_inv = 1.0f / mean;  // the reference's constant factor (Inf when mean == 0)
+    if (blockIdx.x == 0) {
+      out[0] = s;
+      out[1] = c;
+    }
+  }
+  __syncthreads();
+  const float inv = s_inv;
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
+    x[i] = __fmul_rn(x[i], inv);
 }
 
 __global__ void scale_by_inverse_mean_kernel(float* __restrict__ x, long long n,
@@ -124,7 +137,7 @@ int launch_positive_mean(emc_ctx* ctx, const float* x, long long n, double* out)
   positive_partial_kernel<<<nb, kRedThreads, 0, ctx->stream>>>(x, n, part);
   int rc = after_launch(ctx, "positive_partial_kernel");
   if (rc) return rc;
-  positive_final_kernel<<<1, 32, 0, ctx->stream>>>(part, nb, out);
+  positive_final_kernel<<<1, kRedThreads, 0, ctx->stream>>>(part, nb, out);
   return after_launch(ctx, "positive_final_kernel");
 }
 
@@ -132,6 +145,14 @@ int launch_scale_by_inverse_mean(emc_ctx* ctx, float* x, long long n, const doub
   const int nb = (int)std::min<long long>(ceil_div(n, 256), (long long)ctx->sm_count * 8);
   scale_by_inverse_mean_kernel<<<nb, 256, 0, ctx->stream>>>(x, n, stats);
   return after_launch(ctx, "scale_by_inverse_mean_kernel");
+}
+
+int launch_scale_by_partials(emc_ctx* ctx, float* x, long long n, const double* part, int nb,
+                             double* out) {
+  // every block sums the partials again: few blocks, each with enough of x to hide that
+  const int grid = (int)std::min<long long>(ceil_div(n, 4 * kRedThreads), (long long)ctx->sm_count * 4);
+  scale_by_partials_kernel<<<grid, kRedThreads, 0, ctx->stream>>>(x, n, part, nb, out);
+  return after_launch(ctx, "scale_by_partials_kernel");
 }
 
 int launch_divide_by_weight(emc_ctx* ctx, float* model, const float* weight, long long n) {
