@@ -35,9 +35,10 @@ constexpr int CH = 64;             // channels of every convolution
 constexpr int NCONV = 4;
 constexpr int FC_IN = CH * 4 * 4;  // 1024
 constexpr int OUT = 6;
-constexpr int TILE = 64;           // GEMM tile (rows x columns) of the convolution kernels
-constexpr int KCH = 32;            // reduction chunk of the convolution kernels
-constexpr int WG_COLS = 1024;      // columns per partial of the weight-gradient kernel
+constexpr int CC = 8;              // channels per reduction chunk of the convolution kernels
+constexpr int WS = CH + 4;         // padded row of 64 channels in shared memory
+constexpr int WG_BLOCKS = 304;     // blocks of a weight-gradient launch, two per SM
+constexpr int FC_ROWS = 16;        // samples per block of the linear head's backward pass
 
 __host__ __device__ constexpr int cin(int l) { return l == 0 ? 1 : CH; }
 __host__ __device__ constexpr int hin(int l) { return D >> l; }  // 64, 32, 16, 8
@@ -59,7 +60,7 @@ struct ProposalNet {
   float* out = nullptr;            // [cap][6]
   float *g0 = nullptr, *g1 = nullptr;  // ping-pong activation gradients (largest layer)
   float* gout = nullptr;               // [cap][6]
-  float* wpart = nullptr;              // weight-gradient partials
+  float* wpart = nullptr;              // weight- and bias-gradient partials
   size_t wpart_cap = 0;
   float* loss = nullptr;               // [cap]
   int* idx = nullptr;                  // [cap] sample -> data row
@@ -153,194 +154,463 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, const int* __res
 }
 
 // ------------------------------------------------------- convolutions ----
-// Forward: out[b][co][p] = relu(bias[co] + sum_{ci,t} W[co][ci*9+t] in[b][ci][tap(p,t)])
-// as a GEMM of W (64 x Cin*9) by the implicit column matrix (Cin*9 x B*Ho*Ho).
-// Block: 64 output channels x 64 columns, 256 threads with 4 x 4 outputs each.
-__global__ void __launch_bounds__(256) conv_fwd_kernel(const float* __restrict__ in,
-                                                       const float* __restrict__ W,
-                                                       const float* __restrict__ bias,
-                                                       float* __restrict__ out, int B, int Cin,
-                                                       int Hin) {
-  const int Ho = Hin / 2, npx = Ho * Ho, ncol = B * npx, K = Cin * 9;
-  const int n0 = blockIdx.x * pn::TILE;
-  __shared__ float sW[pn::KCH][pn::TILE + 4];  // [k][co]
-  __shared__ float sX[pn::KCH][pn::TILE + 4];  // [k][column]
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += pn::KCH) {
-    for (int e = threadIdx.x; e < pn::KCH * pn::TILE; e += 256) {
-      const int kk = e / pn::TILE, c = e % pn::TILE;  // c: co for sW, column for sX
-      const int k = k0 + kk;
-      sW[kk][c] = k < K ? W[(size_t)c * K + k] : 0.0f;
-      float v = 0.0f;
-      const int n = n0 + c;
-      if (k < K && n < ncol) {
-        const int b = n / npx, p = n % npx;
-        const int ci = k / 9, t = k % 9;
-        const int yi = 2 * (p / Ho) + t / 3 - 1, xi = 2 * (p % Ho) + t % 3 - 1;
-        if (yi >= 0 && yi < Hin && xi >= 0 && xi < Hin)
-          v = in[(((size_t)b * Cin + ci) * Hin + yi) * Hin + xi];
-      }
-      sX[kk][c] = v;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < pn::KCH; ++kk) {
-      float a[4], x[4];
-      for (int i = 0; i < 4; ++i) a[i] = sW[kk][ty * 4 + i];
-      for (int j = 0; j < 4; ++j) x[j] = sX[kk][tx * 4 + j];
-      for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], x[j], acc[i][j]);
-    }
-    __syncthreads();
+// All of them keep a patch of the input (or of the output gradient) and eight
+// channels' weights in shared memory and 64 to 72 sums per thread in registers,
+// so that a value from shared memory serves eight multiply-adds; what bounds them
+// is FP32 issue.  The GEMM form before, with 4 x 4 sums per thread and every
+// element of the implicit column matrix addressed by divisions, reached 14 TFLOP/s
+// forward: 4,107 us for 2,250 patterns, now 1,456 (47 TFLOP/s in the layer with 16 x
+// 16 outputs); the gradients of 250 patterns took 3,271 us, now 590.
+
+// A stride-2 row of the input in shared memory: the even columns 0, 2, .. at 0,
+// the odd ones -1, 1, 3, .. at HO, so that the eight outputs of a thread read
+// neighbours.  Rows -1 .. 2 HO - 1 at 0 .. 2 HO; what lies outside is zero.
+template <int HO>
+struct ConvPatch {
+  static constexpr int HI = 2 * HO, ROWS = HI + 1, RS = 2 * HO + 4, SIZE = ROWS * RS;
+  static __device__ __forceinline__ int at(int y, int x) {
+    return (y + 1) * RS + ((x & 1) ? HO + (x + 1) / 2 : x / 2);
   }
-  for (int j = 0; j < 4; ++j) {
-    const int n = n0 + tx * 4 + j;
-    if (n >= ncol) continue;
-    const int b = n / npx, p = n % npx;
-    for (int i = 0; i < 4; ++i) {
-      const int co = ty * 4 + i;
-      out[((size_t)b * pn::CH + co) * npx + p] = fmaxf(acc[i][j] + bias[co], 0.0f);
+  // pixels 4 q .. 4 q + 3 of an image into its patch
+  static __device__ __forceinline__ void put4(float* patch, int q, float4 v) {
+    const int y = q / (HI / 4), x = (q % (HI / 4)) * 4;
+    float* row = patch + (y + 1) * RS + x / 2;
+    *reinterpret_cast<float2*>(row) = make_float2(v.x, v.z);
+    row[HO + 1] = v.y;
+    row[HO + 2] = v.w;
+  }
+};
+
+// Channel i of the eight that channel group cg of a block's eight takes: four and
+// four, so that the groups' 16-byte loads meet all banks once.
+__device__ __forceinline__ int own_channel(int cg, int i) {
+  return (i & 4) * 8 + cg * 4 + (i & 3);
+}
+
+__device__ __forceinline__ float4 relu_grad(float4 out, float4 g) {
+  return make_float4(out.x > 0.0f ? g.x : 0.0f, out.y > 0.0f ? g.y : 0.0f,
+                     out.z > 0.0f ? g.z : 0.0f, out.w > 0.0f ? g.w : 0.0f);
+}
+
+__device__ __forceinline__ float4 ldg4(const float* p) {
+  return __ldg(reinterpret_cast<const float4*>(p));
+}
+
+// First convolution (one input channel, 64 -> 32 pixels): one thread per output
+// pixel, all 64 channels.
+__global__ void __launch_bounds__(256) conv0_fwd_kernel(const float* __restrict__ in,
+                                                        const float* __restrict__ W,
+                                                        const float* __restrict__ bias,
+                                                        float* __restrict__ out) {
+  constexpr int HI = pn::D, HO = HI / 2, NPX = HO * HO;
+  __shared__ __align__(16) float sW[9][pn::CH], sB[pn::CH];
+  for (int e = threadIdx.x; e < 9 * pn::CH; e += 256) sW[e % 9][e / 9] = W[e];
+  if (threadIdx.x < pn::CH) sB[threadIdx.x] = bias[threadIdx.x];
+  __syncthreads();
+  const int b = blockIdx.x / (NPX / 256), p = (blockIdx.x % (NPX / 256)) * 256 + threadIdx.x;
+  const int oy = p / HO, ox = p % HO;
+  const float* src = in + (size_t)b * HI * HI;
+  float v[9];
+#pragma unroll
+  for (int t = 0; t < 9; ++t) {
+    const int y = 2 * oy + t / 3 - 1, x = 2 * ox + t % 3 - 1;
+    v[t] = y >= 0 && x >= 0 ? src[y * HI + x] : 0.0f;  // never past the other edge
+  }
+  float* dst = out + (size_t)b * pn::CH * NPX + p;
+#pragma unroll 4
+  for (int c = 0; c < pn::CH; c += 4) {
+    float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 9; ++t) {
+      const float4 w = *reinterpret_cast<const float4*>(&sW[t][c]);
+      a.x = fmaf(w.x, v[t], a.x);
+      a.y = fmaf(w.y, v[t], a.y);
+      a.z = fmaf(w.z, v[t], a.z);
+      a.w = fmaf(w.w, v[t], a.w);
     }
+    const float o[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) dst[(size_t)(c + u) * NPX] = fmaxf(o[u] + sB[c + u], 0.0f);
+  }
+}
+
+// out[b][co][p] = relu(bias[co] + sum_{ci,t} W[co][ci*9+t] in[b][ci][tap(p,t)]),
+// 64 input channels, in the order of (ci, t).  256 threads: 8 groups of 8 output
+// channels x 32 groups of PX neighbouring outputs, over SPB samples.
+template <int HO>
+struct ConvFwd {
+  using Patch = ConvPatch<HO>;
+  static constexpr int PX = HO >= 8 ? 8 : 4;
+  static constexpr int GROUPS = HO * HO / PX, SPB = 32 / GROUPS;
+  static constexpr int X = pn::CC * SPB * Patch::SIZE, W = pn::CC * 9 * pn::WS;
+  static constexpr int SMEM = (X + W) * 4;
+};
+
+template <int HO>
+__global__ void __launch_bounds__(256, 2) conv_fwd_kernel(const float* __restrict__ in,
+                                                          const float* __restrict__ W,
+                                                          const float* __restrict__ bias,
+                                                          float* __restrict__ out, int B) {
+  using F = ConvFwd<HO>;
+  using Patch = typename F::Patch;
+  constexpr int PX = F::PX, HI = Patch::HI, K = pn::CH * 9;
+  extern __shared__ __align__(16) float sm[];
+  float *sX = sm, *sW = sm + F::X;
+  const int cg = threadIdx.x & 7, pg = threadIdx.x >> 3;
+  const int smp = pg / F::GROUPS, g = pg % F::GROUPS;
+  const int oy = g / (HO / PX), ox = (g % (HO / PX)) * PX;
+  const int b0 = blockIdx.x * F::SPB;
+  for (int e = threadIdx.x; e < F::X; e += 256) sX[e] = 0.0f;  // the borders stay zero
+  float acc[8][PX];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < PX; ++j) acc[i][j] = 0.0f;
+  for (int c0 = 0; c0 < pn::CH; c0 += pn::CC) {
+    __syncthreads();
+    constexpr int Q = HI * HI / 4;
+#pragma unroll 8
+    for (int e = threadIdx.x; e < pn::CC * F::SPB * Q; e += 256) {
+      const int q = e % Q, u = e / Q, c = u % pn::CC, sp = u / pn::CC;
+      if (b0 + sp < B)
+        Patch::put4(sX + (c * F::SPB + sp) * Patch::SIZE, q,
+                    ldg4(in + ((size_t)(b0 + sp) * pn::CH + c0 + c) * (HI * HI) + 4 * q));
+    }
+#pragma unroll 5
+    for (int e = threadIdx.x; e < pn::CH * pn::CC * 9 / 4; e += 256) {
+      const int co = e % pn::CH, k = e / pn::CH * 4;
+      const float4 w = ldg4(W + (size_t)co * K + c0 * 9 + k);
+      float* dst = sW + k * pn::WS + co;
+      dst[0] = w.x;
+      dst[pn::WS] = w.y;
+      dst[2 * pn::WS] = w.z;
+      dst[3 * pn::WS] = w.w;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < pn::CC; ++c) {
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) {
+        const float* row = sX + (c * F::SPB + smp) * Patch::SIZE + (2 * oy + ky) * Patch::RS + ox;
+        float ev[PX], od[PX + 1];
+#pragma unroll
+        for (int j = 0; j < PX; j += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(row + j);
+          const float4 o = *reinterpret_cast<const float4*>(row + HO + j);
+          ev[j] = a.x; ev[j + 1] = a.y; ev[j + 2] = a.z; ev[j + 3] = a.w;
+          od[j] = o.x; od[j + 1] = o.y; od[j + 2] = o.z; od[j + 3] = o.w;
+        }
+        od[PX] = row[HO + PX];
+#pragma unroll
+        for (int kx = 0; kx < 3; ++kx) {
+          const float* wp = sW + (c * 9 + ky * 3 + kx) * pn::WS + cg * 4;
+          const float4 w0 = *reinterpret_cast<const float4*>(wp);
+          const float4 w1 = *reinterpret_cast<const float4*>(wp + 32);
+          const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < PX; ++j)
+              acc[i][j] = fmaf(w[i], kx == 1 ? ev[j] : od[j + (kx >> 1)], acc[i][j]);
+        }
+      }
+    }
+  }
+  const int b = b0 + smp;
+  if (b >= B) return;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int co = own_channel(cg, i);
+    const float bi = bias[co];
+    float* dst = out + (((size_t)b * pn::CH + co) * HO + oy) * HO + ox;
+#pragma unroll
+    for (int j = 0; j < PX; j += 4)
+      *reinterpret_cast<float4*>(dst + j) =
+          make_float4(fmaxf(acc[i][j] + bi, 0.0f), fmaxf(acc[i][j + 1] + bi, 0.0f),
+                      fmaxf(acc[i][j + 2] + bi, 0.0f), fmaxf(acc[i][j + 3] + bi, 0.0f));
   }
 }
 
 // Backward through ReLU and the convolution to its input:
 // gin[b][ci][q] = sum_{co,t} W[co][ci*9+t] d[b][co][p(q,t)], d = gout * (out > 0),
-// over the output pixels p whose tap t reads input pixel q.  GEMM of W^T
-// (Cin x 64*9) by the gathered d (64*9 x B*Hin*Hin).
-__global__ void __launch_bounds__(256) conv_bwd_data_kernel(const float* __restrict__ gout,
-                                                            const float* __restrict__ out,
-                                                            const float* __restrict__ W,
-                                                            float* __restrict__ gin, int B,
-                                                            int Cin, int Hin) {
-  const int Ho = Hin / 2, npx = Ho * Ho, nin = Hin * Hin, ncol = B * nin, K = pn::CH * 9;
-  const int n0 = blockIdx.x * pn::TILE, c0 = blockIdx.y * pn::TILE;
-  __shared__ float sW[pn::KCH][pn::TILE + 4];  // [k = co*9 + t][ci]
-  __shared__ float sG[pn::KCH][pn::TILE + 4];  // [k][column]
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int k0 = 0; k0 < K; k0 += pn::KCH) {
-    for (int e = threadIdx.x; e < pn::KCH * pn::TILE; e += 256) {
-      const int kk = e / pn::TILE, c = e % pn::TILE;
-      const int k = k0 + kk, co = k / 9, t = k % 9;
-      const int ci = c0 + c;
-      sW[kk][c] = ci < Cin ? W[(size_t)co * Cin * 9 + ci * 9 + t] : 0.0f;
-      float v = 0.0f;
-      const int n = n0 + c;
-      if (n < ncol) {
-        const int b = n / nin, q = n % nin;
-        const int ty2 = q / Hin + 1 - t / 3, tx2 = q % Hin + 1 - t % 3;  // 2y, 2x
-        if (ty2 >= 0 && tx2 >= 0 && !(ty2 & 1) && !(tx2 & 1) && ty2 / 2 < Ho && tx2 / 2 < Ho) {
-          const size_t o = ((size_t)b * pn::CH + co) * npx + (ty2 / 2) * Ho + tx2 / 2;
-          v = out[o] > 0.0f ? gout[o] : 0.0f;
-        }
-      }
-      sG[kk][c] = v;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int kk = 0; kk < pn::KCH; ++kk) {
-      float a[4], x[4];
-      for (int i = 0; i < 4; ++i) a[i] = sW[kk][ty * 4 + i];
-      for (int j = 0; j < 4; ++j) x[j] = sG[kk][tx * 4 + j];
-      for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], x[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
-  for (int j = 0; j < 4; ++j) {
-    const int n = n0 + tx * 4 + j;
-    if (n >= ncol) continue;
-    const int b = n / nin, q = n % nin;
-    for (int i = 0; i < 4; ++i) {
-      const int ci = c0 + ty * 4 + i;
-      if (ci < Cin) gin[((size_t)b * Cin + ci) * nin + q] = acc[i][j];
-    }
-  }
-}
+// over the output pixels p whose tap t reads input pixel q, in the order of
+// (co, t).  Of the nine taps an input pixel meets one, two, two or four, by the
+// parity of its row and column: a thread takes the 2 x 2 input pixels of four
+// neighbouring output positions for 4 input channels, 9 products per position,
+// channel and co.  256 threads: 16 channel groups x 16 position groups.
+template <int HO>
+struct ConvBwd {
+  static constexpr int ROWS = HO == 16 ? 4 : HO;  // output rows per block and sample
+  static constexpr int SPB = 64 / (ROWS * HO), PARTS = HO / ROWS;
+  static constexpr int RS = HO + 4, SIZE = (ROWS + 1) * RS;  // one row and column more
+  static constexpr int DSZ = pn::CC * SPB * SIZE, W = pn::CC * 9 * pn::WS;
+  static constexpr int SMEM = (DSZ + W) * 4;
+};
 
-// Weight gradient partials: part[s][co][k] = sum over columns n of chunk s of
-// d[co][n] col[k][n] (d = gout * (out > 0), col the implicit input columns);
-// chunk s covers columns [s * WG_COLS, (s + 1) * WG_COLS).  Block: 64 co x 64
-// k for one chunk.
-__global__ void __launch_bounds__(256) conv_wgrad_kernel(const float* __restrict__ gout,
-                                                         const float* __restrict__ out,
-                                                         const float* __restrict__ in,
-                                                         float* __restrict__ part, int B, int Cin,
-                                                         int Hin) {
-  const int Ho = Hin / 2, npx = Ho * Ho, ncol = B * npx, K = Cin * 9;
-  const int k0 = blockIdx.x * pn::TILE, s = blockIdx.y;
-  const int nb = s * pn::WG_COLS, ne = min(ncol, nb + pn::WG_COLS);
-  __shared__ float sD[pn::KCH][pn::TILE + 4];  // [n][co]
-  __shared__ float sC[pn::KCH][pn::TILE + 4];  // [n][k]
-  const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-  float acc[4][4] = {};
-  for (int c0 = nb; c0 < ne; c0 += pn::KCH) {
-    for (int e = threadIdx.x; e < pn::KCH * pn::TILE; e += 256) {
-      const int nn = e / pn::TILE, c = e % pn::TILE;
-      const int n = c0 + nn;
-      float dv = 0.0f, cv = 0.0f;
-      if (n < ne) {
-        const int b = n / npx, p = n % npx;
-        const size_t o = ((size_t)b * pn::CH + c) * npx + p;
-        dv = out[o] > 0.0f ? gout[o] : 0.0f;
-        const int k = k0 + c;
-        if (k < K) {
-          const int ci = k / 9, t = k % 9;
-          const int yi = 2 * (p / Ho) + t / 3 - 1, xi = 2 * (p % Ho) + t % 3 - 1;
-          if (yi >= 0 && yi < Hin && xi >= 0 && xi < Hin)
-            cv = in[(((size_t)b * Cin + ci) * Hin + yi) * Hin + xi];
-        }
-      }
-      sD[nn][c] = dv;
-      sC[nn][c] = cv;
-    }
-    __syncthreads();
-#pragma unroll 8
-    for (int nn = 0; nn < pn::KCH; ++nn) {
-      float a[4], x[4];
-      for (int i = 0; i < 4; ++i) a[i] = sD[nn][ty * 4 + i];
-      for (int j = 0; j < 4; ++j) x[j] = sC[nn][tx * 4 + j];
-      for (int i = 0; i < 4; ++i)
-        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], x[j], acc[i][j]);
-    }
-    __syncthreads();
-  }
+template <int HO>
+__global__ void __launch_bounds__(256, 2) conv_bwd_data_kernel(const float* __restrict__ gout,
+                                                               const float* __restrict__ out,
+                                                               const float* __restrict__ W,
+                                                               float* __restrict__ gin, int B) {
+  using F = ConvBwd<HO>;
+  constexpr int HI = 2 * HO, K = pn::CH * 9;
+  extern __shared__ __align__(16) float sm[];
+  float *sD = sm, *sW = sm + F::DSZ;
+  const int cg = threadIdx.x & 15, pp = threadIdx.x >> 4;
+  constexpr int GROUPS = F::ROWS * HO / 4;
+  const int smp = pp / GROUPS, g = pp % GROUPS;
+  const int ry = g / (HO / 4), px = (g % (HO / 4)) * 4;
+  const int b0 = (blockIdx.x / F::PARTS) * F::SPB, y0 = (blockIdx.x % F::PARTS) * F::ROWS;
+  for (int e = threadIdx.x; e < F::DSZ; e += 256) sD[e] = 0.0f;  // the borders stay zero
+  float acc[4][4][4];  // pixel (2 y, 2 x), (2 y, 2 x + 1), (2 y + 1, 2 x), (2 y + 1, 2 x + 1)
+#pragma unroll
   for (int i = 0; i < 4; ++i)
-    for (int j = 0; j < 4; ++j) {
-      const int co = ty * 4 + i, k = k0 + tx * 4 + j;
-      if (k < K) part[((size_t)s * pn::CH + co) * K + k] = acc[i][j];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int u = 0; u < 4; ++u) acc[i][j][u] = 0.0f;
+  for (int c0 = 0; c0 < pn::CH; c0 += pn::CC) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < pn::CC * F::SPB * (F::ROWS + 1) * (HO / 4); e += 256) {
+      const int x = e % (HO / 4) * 4, u = e / (HO / 4), r = u % (F::ROWS + 1), v = u / (F::ROWS + 1);
+      const int c = v % pn::CC, sp = v / pn::CC;
+      if (b0 + sp < B && y0 + r < HO) {
+        const size_t o = (((size_t)(b0 + sp) * pn::CH + c0 + c) * HO + y0 + r) * HO + x;
+        *reinterpret_cast<float4*>(sD + (c * F::SPB + sp) * F::SIZE + r * F::RS + x) =
+            relu_grad(ldg4(out + o), ldg4(gout + o));
+      }
+    }
+#pragma unroll 6
+    for (int e = threadIdx.x; e < pn::CC * K; e += 256) {
+      const int c = e / K, k = e % K;  // k = ci * 9 + t
+      sW[(c * 9 + k % 9) * pn::WS + k / 9] = W[(size_t)(c0 + c) * K + k];
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c < pn::CC; ++c) {
+      const float* r0 = sD + (c * F::SPB + smp) * F::SIZE + ry * F::RS + px;
+      const float* r1 = r0 + F::RS;
+      const float4 e0 = *reinterpret_cast<const float4*>(r0);
+      const float4 e1 = *reinterpret_cast<const float4*>(r1);
+      const float d0[5] = {e0.x, e0.y, e0.z, e0.w, r0[4]};
+      const float d1[5] = {e1.x, e1.y, e1.z, e1.w, r1[4]};
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        const float4 w0 = *reinterpret_cast<const float4*>(sW + (c * 9 + t) * pn::WS + cg * 4);
+        const float w[4] = {w0.x, w0.y, w0.z, w0.w};
+        const int ky = t / 3, kx = t % 3;
+        const int cls = (ky != 1 ? 2 : 0) + (kx != 1 ? 1 : 0);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            acc[i][j][cls] = fmaf(w[i], (ky == 0 ? d1 : d0)[j + (kx == 0 ? 1 : 0)], acc[i][j][cls]);
+      }
+    }
+  }
+  const int b = b0 + smp;
+  if (b >= B) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float* dst = gin + (((size_t)b * pn::CH + cg * 4 + i) * HI + 2 * (y0 + ry)) * HI + 2 * px;
+#pragma unroll
+    for (int j = 0; j < 4; j += 2) {
+      *reinterpret_cast<float4*>(dst + 2 * j) =
+          make_float4(acc[i][j][0], acc[i][j][1], acc[i][j + 1][0], acc[i][j + 1][1]);
+      *reinterpret_cast<float4*>(dst + HI + 2 * j) =
+          make_float4(acc[i][j][2], acc[i][j][3], acc[i][j + 1][2], acc[i][j + 1][3]);
+    }
+  }
+}
+
+// Weight and bias gradient partials of one block's samples: part[s][co][k] = sum
+// over them and the output pixels of d[co] in[tap], bpart[s][co] = sum of d.  A
+// block takes 8 input channels (72 of the k); 256 threads: 8 groups of 8 output
+// channels x 8 input channels x 4 splits of the output rows, each with 8 x 9
+// sums; the splits are added in order at the end.
+template <int HO>
+struct ConvWgrad {
+  using Patch = ConvPatch<HO>;
+  static constexpr int X = pn::CC * Patch::SIZE, DSZ = HO * HO * pn::WS;
+  static constexpr int RED = 3 * 64 * 72;
+  static constexpr int SMEM = 4 * (X + DSZ > RED ? X + DSZ : RED);
+};
+
+template <int HO>
+__global__ void __launch_bounds__(256, 2) conv_wgrad_kernel(const float* __restrict__ gout,
+                                                            const float* __restrict__ out,
+                                                            const float* __restrict__ in,
+                                                            float* __restrict__ part,
+                                                            float* __restrict__ bpart, int B,
+                                                            int per) {
+  using F = ConvWgrad<HO>;
+  using Patch = typename F::Patch;
+  constexpr int HI = Patch::HI, NPX = HO * HO, K = pn::CH * 9;
+  extern __shared__ __align__(16) float sm[];
+  float *sX = sm, *sD = sm + F::X;
+  const int cg = threadIdx.x & 7, ci = (threadIdx.x >> 3) & 7, sp = threadIdx.x >> 6;
+  const int c0 = blockIdx.x * pn::CC, s = blockIdx.y;
+  const int bend = min(B, (s + 1) * per);
+  float acc[8][9];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int t = 0; t < 9; ++t) acc[i][t] = 0.0f;
+  float bsum = 0.0f;  // block 0: channel threadIdx.x & 63, split sp of the pixels
+  for (int e = threadIdx.x; e < F::X; e += 256) sX[e] = 0.0f;
+  for (int b = s * per; b < bend; ++b) {
+    __syncthreads();
+    constexpr int Q = HI * HI / 4;
+#pragma unroll 4
+    for (int e = threadIdx.x; e < pn::CC * Q; e += 256)
+      Patch::put4(sX + e / Q * Patch::SIZE, e % Q,
+                  ldg4(in + ((size_t)b * pn::CH + c0) * (HI * HI) + 4 * e));
+#pragma unroll 4
+    for (int e = threadIdx.x; e < pn::CH * NPX / 4; e += 256) {
+      const int co = e % pn::CH, px = e / pn::CH * 4;
+      const size_t o = ((size_t)b * pn::CH + co) * NPX + px;
+      const float4 d = relu_grad(ldg4(out + o), ldg4(gout + o));
+      float* dst = sD + px * pn::WS + co;
+      dst[0] = d.x;
+      dst[pn::WS] = d.y;
+      dst[2 * pn::WS] = d.z;
+      dst[3 * pn::WS] = d.w;
+    }
+    __syncthreads();
+    for (int oy = sp; oy < HO; oy += 4) {
+      const float* row = sX + ci * Patch::SIZE + 2 * oy * Patch::RS;
+      float lft[3];
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) lft[ky] = row[ky * Patch::RS + HO];
+#pragma unroll 2
+      for (int ox = 0; ox < HO; ++ox) {
+        const float* dp = sD + (oy * HO + ox) * pn::WS + cg * 4;
+        const float4 a = *reinterpret_cast<const float4*>(dp);
+        const float4 c = *reinterpret_cast<const float4*>(dp + 32);
+        const float d[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
+        float x[9];
+#pragma unroll
+        for (int ky = 0; ky < 3; ++ky) {
+          x[3 * ky] = lft[ky];
+          x[3 * ky + 1] = row[ky * Patch::RS + ox];
+          x[3 * ky + 2] = lft[ky] = row[ky * Patch::RS + HO + ox + 1];
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int t = 0; t < 9; ++t) acc[i][t] = fmaf(d[i], x[t], acc[i][t]);
+      }
+    }
+    if (blockIdx.x == 0)
+      for (int p = sp; p < NPX; p += 4) bsum += sD[p * pn::WS + (threadIdx.x & 63)];
+  }
+  __syncthreads();
+  const int lane64 = threadIdx.x & 63;
+  if (sp > 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int t = 0; t < 9; ++t) sm[((sp - 1) * 72 + i * 9 + t) * 64 + lane64] = acc[i][t];
+  }
+  __syncthreads();
+  if (sp == 0) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int t = 0; t < 9; ++t) {
+        float v = acc[i][t];
+#pragma unroll
+        for (int u = 0; u < 3; ++u) v += sm[(u * 72 + i * 9 + t) * 64 + lane64];
+        part[((size_t)s * pn::CH + own_channel(cg, i)) * K + (c0 + ci) * 9 + t] = v;
+      }
+  }
+  if (blockIdx.x == 0) {
+    __syncthreads();
+    sm[threadIdx.x] = bsum;
+    __syncthreads();
+    if (threadIdx.x < 64) {
+      float v = 0.0f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) v += sm[u * 64 + threadIdx.x];
+      bpart[(size_t)s * pn::CH + threadIdx.x] = v;
+    }
+  }
+}
+
+// The same for the first convolution (one input channel): a warp takes 8 output
+// channels, its lanes neighbouring pixels; the lanes' sums are added at the end.
+__global__ void __launch_bounds__(256) conv0_wgrad_kernel(const float* __restrict__ gout,
+                                                          const float* __restrict__ out,
+                                                          const float* __restrict__ in,
+                                                          float* __restrict__ part,
+                                                          float* __restrict__ bpart, int B,
+                                                          int per) {
+  constexpr int HI = pn::D, HO = HI / 2, NPX = HO * HO;
+  using Patch = ConvPatch<HO>;
+  __shared__ float sX[Patch::SIZE];
+  const int lane = threadIdx.x & 31, cw = (threadIdx.x >> 5) * 8, s = blockIdx.x;
+  const int bend = min(B, (s + 1) * per);
+  float acc[8][10];  // nine taps and the bias
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int t = 0; t < 10; ++t) acc[i][t] = 0.0f;
+  for (int e = threadIdx.x; e < Patch::SIZE; e += 256) sX[e] = 0.0f;
+  for (int b = s * per; b < bend; ++b) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < HI * HI; e += 256)
+      sX[Patch::at(e / HI, e % HI)] = in[(size_t)b * HI * HI + e];
+    __syncthreads();
+    for (int oy = 0; oy < HO; ++oy) {  // 32 pixels: one row
+      float x[9];
+#pragma unroll
+      for (int ky = 0; ky < 3; ++ky) {
+        const float* row = sX + (2 * oy + ky) * Patch::RS;
+        x[3 * ky] = row[HO + lane];
+        x[3 * ky + 1] = row[lane];
+        x[3 * ky + 2] = row[HO + lane + 1];
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const size_t o = ((size_t)b * pn::CH + cw + i) * NPX + oy * HO + lane;
+        const float d = out[o] > 0.0f ? gout[o] : 0.0f;
+#pragma unroll
+        for (int t = 0; t < 9; ++t) acc[i][t] = fmaf(d, x[t], acc[i][t]);
+        acc[i][9] += d;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int t = 0; t < 10; ++t) {
+      float v = acc[i][t];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) {
+        if (t < 9)
+          part[((size_t)s * pn::CH + cw + i) * 9 + t] = v;
+        else
+          bpart[(size_t)s * pn::CH + cw + i] = v;
+      }
     }
 }
 
-// grad[e] = sum_s part[s][e] (fixed order), e < n.
-__global__ void sum_parts_kernel(const float* __restrict__ part, int S, int n,
-                                 float* __restrict__ grad) {
+// grad[e] = sum_s part[s][e] (fixed order), e < n; then the n2 of part2 the same.
+__global__ void sum_parts_kernel(const float* __restrict__ part, const float* __restrict__ part2,
+                                 int S, int n, int n2, float* __restrict__ grad,
+                                 float* __restrict__ grad2) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
+  if (e >= n + n2) return;
+  const float* src = e < n ? part + e : part2 + (e - n);
+  const int m = e < n ? n : n2;
   float a = 0.0f;
-  for (int s = 0; s < S; ++s) a += part[(size_t)s * n + e];
-  grad[e] = a;
-}
-
-// gbias[co] = sum_{b,p} gout * (out > 0); one block per channel.
-__global__ void conv_bgrad_kernel(const float* __restrict__ gout, const float* __restrict__ out,
-                                  int B, int npx, float* __restrict__ gbias) {
-  const int co = blockIdx.x;
-  float a = 0.0f;
-  for (int n = threadIdx.x; n < B * npx; n += 256) {
-    const size_t o = ((size_t)(n / npx) * pn::CH + co) * npx + n % npx;
-    if (out[o] > 0.0f) a += gout[o];
-  }
-  __shared__ float red[256];
-  red[threadIdx.x] = a;
-  __syncthreads();
-  for (int h = 128; h > 0; h >>= 1) {
-    if (threadIdx.x < h) red[threadIdx.x] += red[threadIdx.x + h];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) gbias[co] = red[0];
+#pragma unroll 16
+  for (int s = 0; s < S; ++s) a += src[(size_t)s * m];
+  if (e < n)
+    grad[e] = a;
+  else
+    grad2[e - n] = a;
 }
 
 // ---------------------------------------------------------- linear head --
@@ -364,30 +634,37 @@ __global__ void fc_fwd_kernel(const float* __restrict__ h, const float* __restri
   if (threadIdx.x < pn::OUT) o[b * pn::OUT + threadIdx.x] = red[threadIdx.x][0] + fb[threadIdx.x];
 }
 
-// gh[b][k] = sum_j fw[j][k] go[b][j]; gfw[j][k] = sum_b go[b][j] h[b][k];
-// gfb[j] = sum_b go[b][j].  One thread per k (all samples).
-__global__ void fc_bwd_kernel(const float* __restrict__ h, const float* __restrict__ fw,
-                              const float* __restrict__ go, int B, float* __restrict__ gh,
-                              float* __restrict__ gfw, float* __restrict__ gfb) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k < pn::FC_IN) {
-    float g[pn::OUT] = {};
-    for (int b = 0; b < B; ++b) {
-      const float hv = h[(size_t)b * pn::FC_IN + k];
-      float a = 0.0f;
-      for (int j = 0; j < pn::OUT; ++j) {
-        const float gj = go[b * pn::OUT + j];
-        g[j] = fmaf(gj, hv, g[j]);
-        a = fmaf(fw[j * pn::FC_IN + k], gj, a);
-      }
-      gh[(size_t)b * pn::FC_IN + k] = a;
+// gh[b][k] = sum_j fw[j][k] go[b][j]; part[s][j][k] = sum_b go[b][j] h[b][k] and
+// bpart[s][j] = sum_b go[b][j] over the FC_ROWS samples of block row s.
+__global__ void __launch_bounds__(256) fc_bwd_kernel(const float* __restrict__ h,
+                                                     const float* __restrict__ fw,
+                                                     const float* __restrict__ go, int B,
+                                                     float* __restrict__ gh,
+                                                     float* __restrict__ part,
+                                                     float* __restrict__ bpart) {
+  const int k = blockIdx.x * 256 + threadIdx.x, s = blockIdx.y;
+  const int b0 = s * pn::FC_ROWS, b1 = min(B, b0 + pn::FC_ROWS);
+  float w[pn::OUT], g[pn::OUT] = {};
+#pragma unroll
+  for (int j = 0; j < pn::OUT; ++j) w[j] = fw[j * pn::FC_IN + k];
+#pragma unroll 4
+  for (int b = b0; b < b1; ++b) {
+    const float hv = h[(size_t)b * pn::FC_IN + k];
+    float a = 0.0f;
+#pragma unroll
+    for (int j = 0; j < pn::OUT; ++j) {
+      const float gj = __ldg(go + b * pn::OUT + j);
+      g[j] = fmaf(gj, hv, g[j]);
+      a = fmaf(w[j], gj, a);
     }
-    for (int j = 0; j < pn::OUT; ++j) gfw[j * pn::FC_IN + k] = g[j];
+    gh[(size_t)b * pn::FC_IN + k] = a;
   }
+#pragma unroll
+  for (int j = 0; j < pn::OUT; ++j) part[((size_t)s * pn::OUT + j) * pn::FC_IN + k] = g[j];
   if (blockIdx.x == 0 && threadIdx.x < pn::OUT) {
     float a = 0.0f;
-    for (int b = 0; b < B; ++b) a += go[b * pn::OUT + threadIdx.x];
-    gfb[threadIdx.x] = a;
+    for (int b = b0; b < b1; ++b) a += go[b * pn::OUT + threadIdx.x];
+    bpart[s * pn::OUT + threadIdx.x] = a;
   }
 }
 
@@ -549,6 +826,74 @@ static int ensure_cap(ProposalNet* n, int B) {
   return EMC_OK;
 }
 
+// More than 48 KB of shared memory per block has to be asked for, once per device.
+template <typename Kernel>
+static int big_smem(emc_ctx* ctx, Kernel k, int bytes) {
+  EMC_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+  return EMC_OK;
+}
+
+static int conv_smem(emc_ctx* ctx) {
+  int rc = big_smem(ctx, conv_fwd_kernel<16>, ConvFwd<16>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_fwd_kernel<8>, ConvFwd<8>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_fwd_kernel<4>, ConvFwd<4>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_bwd_data_kernel<16>, ConvBwd<16>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_bwd_data_kernel<8>, ConvBwd<8>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_bwd_data_kernel<4>, ConvBwd<4>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_wgrad_kernel<16>, ConvWgrad<16>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_wgrad_kernel<8>, ConvWgrad<8>::SMEM);
+  if (!rc) rc = big_smem(ctx, conv_wgrad_kernel<4>, ConvWgrad<4>::SMEM);
+  return rc;
+}
+
+// Convolution l (64 input channels) to HO x HO outputs.
+template <int HO>
+static int conv_fwd(ProposalNet* n, int l, int B) {
+  emc_ctx* ctx = n->ctx;
+  conv_fwd_kernel<HO><<<ceil_div(B, ConvFwd<HO>::SPB), 256, ConvFwd<HO>::SMEM, ctx->stream>>>(
+      n->act[l], n->params + n->off_w[l], n->params + n->off_b[l], n->act[l + 1], B);
+  return after_launch(ctx, "conv_fwd_kernel");
+}
+
+static int grow_parts(ProposalNet* n, size_t need) {
+  emc_ctx* ctx = n->ctx;
+  if (need <= n->wpart_cap) return EMC_OK;
+  cudaFree(n->wpart);
+  n->wpart = nullptr;
+  n->wpart_cap = 0;
+  EMC_CUDA(ctx, cudaMalloc(&n->wpart, sizeof(float) * need));
+  n->wpart_cap = need;
+  return EMC_OK;
+}
+
+static int sum_parts(ProposalNet* n, const float* bpart, int S, int nw, int nb, size_t off_w,
+                     size_t off_b) {
+  emc_ctx* ctx = n->ctx;
+  sum_parts_kernel<<<ceil_div(nw + nb, 256), 256, 0, ctx->stream>>>(
+      n->wpart, bpart, S, nw, nb, n->grads + off_w, n->grads + off_b);
+  return after_launch(ctx, "sum_parts_kernel");
+}
+
+// Gradients of convolution l's weights and bias from g (d loss / d act[l + 1]), and
+// with gin of its input.
+template <int HO>
+static int conv_bwd(ProposalNet* n, int l, int B, const float* g, float* gin) {
+  emc_ctx* ctx = n->ctx;
+  int rc;
+  const int groups = pn::CH / pn::CC, per = ceil_div(B, pn::WG_BLOCKS / groups);
+  const int S = ceil_div(B, per), K = pn::CH * 9;
+  if ((rc = grow_parts(n, (size_t)S * pn::CH * (K + 1)))) return rc;
+  float* bpart = n->wpart + (size_t)S * pn::CH * K;
+  conv_wgrad_kernel<HO><<<dim3(groups, S), 256, ConvWgrad<HO>::SMEM, ctx->stream>>>(
+      g, n->act[l + 1], n->act[l], n->wpart, bpart, B, per);
+  if ((rc = after_launch(ctx, "conv_wgrad_kernel"))) return rc;
+  if ((rc = sum_parts(n, bpart, S, pn::CH * K, pn::CH, n->off_w[l], n->off_b[l]))) return rc;
+  using Bw = ConvBwd<HO>;
+  conv_bwd_data_kernel<HO><<<ceil_div(B, Bw::SPB) * Bw::PARTS, 256, Bw::SMEM, ctx->stream>>>(
+      g, n->act[l + 1], n->params + n->off_w[l], gin, B);
+  return after_launch(ctx, "conv_bwd_data_kernel");
+}
+
 // Forward pass of the B samples whose data rows are in n->idx (turned by
 // n->quarter when `turned`).
 static int forward(ProposalNet* n, int B, bool turned) {
@@ -558,13 +903,11 @@ static int forward(ProposalNet* n, int B, bool turned) {
   gather_rows_kernel<<<(unsigned)((e0 + 255) / 256), 256, 0, ctx->stream>>>(
       n->X, n->idx, turned ? n->quarter : nullptr, B, n->act[0]);
   if ((rc = after_launch(ctx, "gather_rows_kernel"))) return rc;
-  for (int l = 0; l < pn::NCONV; ++l) {
-    const int Hin = pn::hin(l), Ho = Hin / 2, ncol = B * Ho * Ho;
-    conv_fwd_kernel<<<ceil_div(ncol, pn::TILE), 256, 0, ctx->stream>>>(
-        n->act[l], n->params + n->off_w[l], n->params + n->off_b[l], n->act[l + 1], B, pn::cin(l),
-        Hin);
-    if ((rc = after_launch(ctx, "conv_fwd_kernel"))) return rc;
-  }
+  conv0_fwd_kernel<<<B * 4, 256, 0, ctx->stream>>>(n->act[0], n->params + n->off_w[0],
+                                                  n->params + n->off_b[0], n->act[1]);
+  if ((rc = after_launch(ctx, "conv0_fwd_kernel"))) return rc;
+  if ((rc = conv_fwd<16>(n, 1, B)) || (rc = conv_fwd<8>(n, 2, B)) || (rc = conv_fwd<4>(n, 3, B)))
+    return rc;
   fc_fwd_kernel<<<B, 256, 0, ctx->stream>>>(n->act[pn::NCONV], n->params + n->off_fw,
                                             n->params + n->off_fb, n->out);
   return after_launch(ctx, "fc_fwd_kernel");
@@ -576,40 +919,23 @@ static int backward(ProposalNet* n, int B) {
   int rc;
   float* gcur = n->g0;  // gradient of act[l + 1] (post-ReLU output of conv l)
   float* gnext = n->g1;
-  fc_bwd_kernel<<<ceil_div(pn::FC_IN, 256), 256, 0, ctx->stream>>>(
-      n->act[pn::NCONV], n->params + n->off_fw, n->gout, B, gcur, n->grads + n->off_fw,
-      n->grads + n->off_fb);
+  const int Sf = ceil_div(B, pn::FC_ROWS), nf = pn::OUT * pn::FC_IN;
+  if ((rc = grow_parts(n, (size_t)Sf * (nf + pn::OUT)))) return rc;
+  float* bpart = n->wpart + (size_t)Sf * nf;
+  fc_bwd_kernel<<<dim3(pn::FC_IN / 256, Sf), 256, 0, ctx->stream>>>(
+      n->act[pn::NCONV], n->params + n->off_fw, n->gout, B, gcur, n->wpart, bpart);
   if ((rc = after_launch(ctx, "fc_bwd_kernel"))) return rc;
-  for (int l = pn::NCONV - 1; l >= 0; --l) {
-    const int Hin = pn::hin(l), Ho = Hin / 2, Cin = pn::cin(l), K = Cin * 9;
-    const int ncol = B * Ho * Ho, S = ceil_div(ncol, pn::WG_COLS);
-    const size_t need = (size_t)S * pn::CH * K;
-    if (need > n->wpart_cap) {
-      cudaFree(n->wpart);
-      n->wpart = nullptr;
-      n->wpart_cap = 0;
-      EMC_CUDA(ctx, cudaMalloc(&n->wpart, sizeof(float) * need));
-      n->wpart_cap = need;
-    }
-    conv_wgrad_kernel<<<dim3(ceil_div(K, pn::TILE), S), 256, 0, ctx->stream>>>(
-        gcur, n->act[l + 1], n->act[l], n->wpart, B, Cin, Hin);
-    if ((rc = after_launch(ctx, "conv_wgrad_kernel"))) return rc;
-    sum_parts_kernel<<<ceil_div(pn::CH * K, 256), 256, 0, ctx->stream>>>(
-        n->wpart, S, pn::CH * K, n->grads + n->off_w[l]);
-    if ((rc = after_launch(ctx, "sum_parts_kernel"))) return rc;
-    conv_bgrad_kernel<<<pn::CH, 256, 0, ctx->stream>>>(gcur, n->act[l + 1], B, Ho * Ho,
-                                                        n->grads + n->off_b[l]);
-    if ((rc = after_launch(ctx, "conv_bgrad_kernel"))) return rc;
-    if (l > 0) {
-      const int nin = B * Hin * Hin;
-      conv_bwd_data_kernel<<<dim3(ceil_div(nin, pn::TILE), ceil_div(Cin, pn::TILE)), 256, 0,
-                             ctx->stream>>>(gcur, n->act[l + 1], n->params + n->off_w[l], gnext,
-                                            B, Cin, Hin);
-      if ((rc = after_launch(ctx, "conv_bwd_data_kernel"))) return rc;
-      std::swap(gcur, gnext);
-    }
-  }
-  return EMC_OK;
+  if ((rc = sum_parts(n, bpart, Sf, nf, pn::OUT, n->off_fw, n->off_fb))) return rc;
+  if ((rc = conv_bwd<4>(n, 3, B, gcur, gnext)) || (rc = conv_bwd<8>(n, 2, B, gnext, gcur)) ||
+      (rc = conv_bwd<16>(n, 1, B, gcur, gnext)))
+    return rc;
+  const int per = ceil_div(B, pn::WG_BLOCKS), S = ceil_div(B, per);
+  if ((rc = grow_parts(n, (size_t)S * pn::CH * 10))) return rc;
+  bpart = n->wpart + (size_t)S * pn::CH * 9;
+  conv0_wgrad_kernel<<<S, 256, 0, ctx->stream>>>(gnext, n->act[1], n->act[0], n->wpart, bpart, B,
+                                                 per);
+  if ((rc = after_launch(ctx, "conv0_wgrad_kernel"))) return rc;
+  return sum_parts(n, bpart, S, pn::CH * 9, pn::CH, n->off_w[0], n->off_b[0]);
 }
 
 // Loss of the batch in n->idx against labels (quaternions, data rows) and
@@ -661,6 +987,10 @@ extern "C" int emc_proposal_create(emc_ctx* ctx, unsigned long long seed, emc_pr
   if (!ctx || !out) return EMC_ERR_INVALID;
   emc_proposal* n = new emc_proposal();
   n->ctx = ctx;
+  if (const int rc = conv_smem(ctx)) {
+    delete n;
+    return rc;
+  }
   size_t o = 0;
   for (int l = 0; l < pn::NCONV; ++l) {
     n->off_w[l] = o;
