@@ -421,7 +421,10 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
 
 // The plane T = [0 < s < 1e-10] of the likelihood's rotation operands, in
 // the (rotation tile, 64-pixel block) pairs that hold such a value -- none in
-// most iterations: a block per rotation tile looks at its flags and exits.
+// most iterations: a rotation tile's eight blocks look at their flags and exit.
+// (With sharp atoms and trilinear slices most blocks hold one: 219 us at 96^3 and
+// 10,860 rotations with one block per rotation tile, 82 with eight.)
+constexpr int kTinyBlocks = 8;
 template <int INTERP>
 __global__ void __launch_bounds__(256) tiny_plane_kernel(
     const float* __restrict__ model, int side, const float* __restrict__ rot,
@@ -429,7 +432,7 @@ __global__ void __launch_bounds__(256) tiny_plane_kernel(
     const float* __restrict__ cz, int R, int Kp, const unsigned char* __restrict__ tiny, int nkb,
     __half* __restrict__ T) {
   const int rt = blockIdx.x;
-  for (int kb = 0; kb < nkb; ++kb) {
+  for (int kb = blockIdx.y; kb < nkb; kb += kTinyBlocks) {
     if (!__ldg(tiny + (size_t)rt * nkb + kb)) continue;  // uniform over the block
     for (int e = threadIdx.x; e < 128 * 64; e += blockDim.x) {
       const int r = rt * 128 + (e >> 6), q = kb * 64 + (e & 63);
@@ -1046,9 +1049,8 @@ int plan_respons_ready(emc_plan* p) {
 struct InsertCtx {
   float* model;
   float* weight;
-  unsigned long long* fix_m;
-  unsigned long long* fix_w;
-  float2* acc2;          // interleaved (model, weight) sums: one 8-byte atomic per point
+  ulonglong2* fix2;         // interleaved fixed-point (model, weight) sums
+  float2* acc2;             // interleaved (model, weight) sums: one 8-byte atomic per point
   const float2* fix_scale;  // {model, weight} fixed-point scales (deterministic mode)
   float* u;              // sorted mode: pair values [P_eff][ldu] instead of insertion
   int ldu;
@@ -1060,8 +1062,8 @@ struct InsertCtx {
 __device__ __forceinline__ void add_voxel(const InsertCtx& c, size_t v, float val, float w) {
   if (c.deterministic) {
     const float2 sc = __ldg(c.fix_scale);
-    atomicAdd(c.fix_m + v, (unsigned long long)fixed_from_float(__fmul_rn(val, sc.x)));
-    atomicAdd(c.fix_w + v, (unsigned long long)fixed_from_float(__fmul_rn(w, sc.y)));
+    atomicAdd(&c.fix2[v].x, (unsigned long long)fixed_from_float(__fmul_rn(val, sc.x)));
+    atomicAdd(&c.fix2[v].y, (unsigned long long)fixed_from_float(__fmul_rn(w, sc.y)));
   } else {
     atomicAdd(c.acc2 + v, make_float2(val, w));
   }
@@ -1233,21 +1235,21 @@ __global__ void insert_bounds_kernel(const double* __restrict__ row_mass,
 // emc_cuda.cu:758-768), from the fixed-point (deterministic) or the
 // interleaved float accumulators; part: the blocks' {sum, count} of its positive
 // voxels, for the normalisation.
-__global__ void finish_insert_kernel(const unsigned long long* __restrict__ fm,
-                                     const unsigned long long* __restrict__ fw,
+__global__ void finish_insert_kernel(const ulonglong2* __restrict__ fx,
                                      const float2* __restrict__ fix_scale,
                                      const float2* __restrict__ acc2, float* __restrict__ model,
                                      float* __restrict__ weight, long long n,
                                      double* __restrict__ part) {
-  const float2 sc = fm ? *fix_scale : make_float2(1.0f, 1.0f);
+  const float2 sc = fx ? *fix_scale : make_float2(1.0f, 1.0f);
   const double inv_m = 1.0 / (double)sc.x, inv_w = 1.0 / (double)sc.y;  // powers of two
   double s = 0.0, c = 0.0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
     float m, w;
-    if (fm) {
-      m = (float)((double)(long long)fm[v] * inv_m);
-      w = (float)((double)(long long)fw[v] * inv_w);
+    if (fx) {
+      const ulonglong2 u = fx[v];
+      m = (float)((double)(long long)u.x * inv_m);
+      w = (float)((double)(long long)u.y * inv_w);
     } else {
       const float2 a = acc2[v];
       m = a.x;
@@ -1297,18 +1299,18 @@ __global__ void lse_from_global_kernel(const double* __restrict__ lse_in, int N,
 
 // The inserted sums as floats (model sum of T_r x slice, weight sum of T_r),
 // exactly as finish_insert_kernel reads them.
-__global__ void sums_out_kernel(const unsigned long long* __restrict__ fm,
-                                     const unsigned long long* __restrict__ fw,
+__global__ void sums_out_kernel(const ulonglong2* __restrict__ fx,
                                 const float2* __restrict__ fix_scale,
                                 const float2* __restrict__ acc2,
                                 float* __restrict__ msum, float* __restrict__ wsum, long long n) {
-  const float2 sc = fm ? *fix_scale : make_float2(1.0f, 1.0f);
+  const float2 sc = fx ? *fix_scale : make_float2(1.0f, 1.0f);
   const double inv_m = 1.0 / (double)sc.x, inv_w = 1.0 / (double)sc.y;  // powers of two
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long v = (long long)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += stride) {
-    if (fm) {
-      msum[v] = (float)((double)(long long)fm[v] * inv_m);
-      wsum[v] = (float)((double)(long long)fw[v] * inv_w);
+    if (fx) {
+      const ulonglong2 u = fx[v];
+      msum[v] = (float)((double)(long long)u.x * inv_m);
+      wsum[v] = (float)((double)(long long)u.y * inv_w);
     } else {
       const float2 a = acc2[v];
       msum[v] = a.x;
@@ -1418,8 +1420,7 @@ extern "C" int emc_plan_create(emc_ctx* ctx, const emc_plan_desc* desc, emc_plan
   }
   if (!rc && d.precision == EMC_PREC_FP32) rc = alloc_n(p, &p->Q, (size_t)d.n_rot * p->Np);
   if (!rc && d.insert_mode == EMC_INSERT_DETERMINISTIC) {
-    rc = alloc_n(p, &p->fix_m, n3);
-    if (!rc) rc = alloc_n(p, &p->fix_w, n3);
+    rc = alloc_n(p, &p->fix2, n3);
   }
   if (!rc && d.insert_mode != EMC_INSERT_DETERMINISTIC) rc = alloc_n(p, &p->acc2, n3);
   if (rc) {
@@ -1604,7 +1605,7 @@ static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
           p->rot_cnt, p->rot_A, p->rot_ssum, ops);
   int rc = after_launch(ctx, "slice_rows_kernel");
   if (rc || !ops.tiny) return rc;
-  tiny_plane_kernel<INTERP><<<p->n_rt, 256, 0, ctx->stream>>>(
+  tiny_plane_kernel<INTERP><<<dim3(p->n_rt, kTinyBlocks), 256, 0, ctx->stream>>>(
       model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, ops.tiny, ops.nkb,
       tc_tiny_plane(p));
   return after_launch(ctx, "tiny_plane_kernel");
@@ -1651,8 +1652,7 @@ static InsertCtx make_insert_ctx(emc_plan* p, float* model, float* weight) {
   InsertCtx c;
   c.model = model;
   c.weight = weight;
-  c.fix_m = p->fix_m;
-  c.fix_w = p->fix_w;
+  c.fix2 = p->fix2;
   c.acc2 = p->acc2;
   c.fix_scale = reinterpret_cast<const float2*>(p->red + kRedFixScale);
   c.u = p->d.insert_mode == EMC_INSERT_SORTED ? p->ins_u : nullptr;
@@ -1745,7 +1745,7 @@ static int enqueue_lse(emc_plan* p) {
 }
 
 // responsibilities (mprep) and the M-step with insertion into the zeroed
-// accumulators (acc2, or fix_m / fix_w when deterministic); model / weight
+// accumulators (acc2, or fix2 when deterministic); model / weight
 // are the buffers the insertion context names (not written here)
 static int enqueue_mstep(emc_plan* p, float* d_model, float* d_weight) {
   emc_ctx* ctx = p->ctx;
@@ -1775,8 +1775,7 @@ static int enqueue_mstep(emc_plan* p, float* d_model, float* d_weight) {
         row_mass, row_bound, R, p->P_eff, p->red + kRedBoundM,
         reinterpret_cast<float2*>(p->red + kRedFixScale));
     if ((rc = after_launch(ctx, "insert_bounds_kernel"))) return rc;
-    EMC_CUDA(ctx, cudaMemsetAsync(p->fix_m, 0, sizeof(unsigned long long) * n3, ctx->stream));
-    EMC_CUDA(ctx, cudaMemsetAsync(p->fix_w, 0, sizeof(unsigned long long) * n3, ctx->stream));
+    EMC_CUDA(ctx, cudaMemsetAsync(p->fix2, 0, sizeof(ulonglong2) * n3, ctx->stream));
   } else if (p->d.insert_mode == EMC_INSERT_ATOMIC) {
     EMC_CUDA(ctx, cudaMemsetAsync(p->acc2, 0, sizeof(float2) * n3, ctx->stream));
   }  // sorted: the reduction writes every voxel of acc2
@@ -1797,7 +1796,7 @@ static int enqueue_finish(emc_plan* p, float* d_model, float* d_weight) {
   int rc;
   const int nb = mean_blocks(p, n3);
   finish_insert_kernel<<<nb, 256, 0, ctx->stream>>>(
-      det ? p->fix_m : nullptr, p->fix_w, reinterpret_cast<const float2*>(p->red + kRedFixScale),
+      det ? p->fix2 : nullptr, reinterpret_cast<const float2*>(p->red + kRedFixScale),
       p->acc2, d_model, d_weight, n3, mean_parts(p));
   if ((rc = after_launch(ctx, "finish_insert_kernel"))) return rc;
   if ((rc = mark_phase(p, 5))) return rc;
@@ -2210,7 +2209,7 @@ extern "C" int emc_rank_mstep(emc_plan* p, const double* d_lse, float* d_model_s
   if ((rc = enqueue_mstep(p, d_model_sum, d_weight_sum))) return rc;
   const bool det = p->d.insert_mode == EMC_INSERT_DETERMINISTIC;
   const int nb = (int)std::min<long long>(ceil_div(n3, 256), (long long)ctx->sm_count * 8);
-  sums_out_kernel<<<nb, 256, 0, ctx->stream>>>(det ? p->fix_m : nullptr, p->fix_w,
+  sums_out_kernel<<<nb, 256, 0, ctx->stream>>>(det ? p->fix2 : nullptr,
                                                 reinterpret_cast<const float2*>(p->red + kRedFixScale),
                                                 p->acc2, d_model_sum,
                                                 d_weight_sum, n3);

@@ -94,8 +94,7 @@ struct emc_plan {
   double* ll_part = nullptr;  // [N/32] sums of lse
   float* T = nullptr;      // [Rp] rotation totals
   double* red = nullptr;   // reduction scratch (small)
-  unsigned long long* fix_m = nullptr;  // [s^3] fixed-point model (deterministic insert)
-  unsigned long long* fix_w = nullptr;
+  ulonglong2* fix2 = nullptr;  // [s^3] fixed-point (model, weight) sums (deterministic insert)
   float2* acc2 = nullptr;  // [s^3] interleaved (model, weight) sums (float atomics)
   int* flags = nullptr;    // device status words
   float* sigma_dev = nullptr;  // [1] annealing width read by the E-step kernels

@@ -1211,8 +1211,7 @@ struct TcMstepArgs {
   int aggregate;  // 1: lanes hitting the same voxel combine before one atomic
   float* model;
   float* weight;
-  unsigned long long* fix_m;
-  unsigned long long* fix_w;
+  ulonglong2* fix2;
   float2* acc2;
   const float2* fix_scale;  // {model, weight} fixed-point scales (deterministic mode)
   float* u;                 // sorted mode: pair values [P_eff][ldu] instead of insertion
@@ -1234,8 +1233,8 @@ struct TcMstepArgs {
 __device__ __forceinline__ void tc_add(const TcMstepArgs& a, size_t v, float val, float w) {
   if (a.deterministic) {
     const float2 sc = __ldg(a.fix_scale);
-    atomicAdd(a.fix_m + v, (unsigned long long)fixed_from_float(__fmul_rn(val, sc.x)));
-    atomicAdd(a.fix_w + v, (unsigned long long)fixed_from_float(__fmul_rn(w, sc.y)));
+    atomicAdd(&a.fix2[v].x, (unsigned long long)fixed_from_float(__fmul_rn(val, sc.x)));
+    atomicAdd(&a.fix2[v].y, (unsigned long long)fixed_from_float(__fmul_rn(w, sc.y)));
   } else {
     atomicAdd(a.acc2 + v, make_float2(val, w));  // model and weight in one 8-byte atomic
   }
@@ -1269,24 +1268,58 @@ __device__ __forceinline__ void tc_insert_nearest(const TcMstepArgs& a, bool on,
   if (on) tc_add(a, (size_t)v, val, w);
 }
 
-// Trilinear insertion of one value.
-__device__ __forceinline__ void tc_insert_trilinear(const TcMstepArgs& a, const RotMat& R, float x,
-                                                    float y, float z, float val, float w) {
-  const int side = a.side;
+// Trilinear insertion of one value per lane; called by all 32 lanes.  What bounds
+// it is the L2 atomic unit, by the 32-byte sectors that an instruction touches: a
+// cell's eight corners at one lane's hands are eight sectors (sixteen with model and
+// weight in arrays of their own).  So the two corners of an x edge, neighbours in
+// memory, and with fixed-point sums the model and the weight of each, go to
+// neighbouring lanes of one instruction: 2 (float) or 4 (fixed) lanes take their
+// group's points in turn.  Fixed-point insertion of 10,860 slices of 7,236 pixels
+// (1.3e9 atomic additions): 6,790 us, now 3,070.
+__device__ __forceinline__ void tc_insert_trilinear(const TcMstepArgs& a, bool on, const RotMat& R,
+                                                    float x, float y, float z, float val,
+                                                    float w) {
+  const int side = a.side, lane = threadIdx.x & 31;
   const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
   const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
   const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
   const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
   const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
   const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
+  const unsigned n = (unsigned)side;
+  // bits 0, 1: x0 and x0 + 1 inside; 2, 3: y; 4, 5: z
+  unsigned in = 0;
+  if (on)
+    in = ((unsigned)x0 < n) | ((unsigned)x0 + 1 < n) << 1 | ((unsigned)y0 < n) << 2 |
+         ((unsigned)y0 + 1 < n) << 3 | ((unsigned)z0 < n) << 4 | ((unsigned)z0 + 1 < n) << 5;
+  const int base = on ? (z0 * side + y0) * side + x0 : 0;
+  const int group = a.deterministic ? 4 : 2;
+  const float2 sc = a.deterministic ? __ldg(a.fix_scale) : make_float2(1.0f, 1.0f);
+  for (int s = 0; s < group; ++s) {
+    const int src = (lane & ~(group - 1)) + s;
+    const unsigned pin = __shfl_sync(0xffffffffu, in, src);
+    const int pbase = __shfl_sync(0xffffffffu, base, src);
+    const float px = __shfl_sync(0xffffffffu, tx, src), py = __shfl_sync(0xffffffffu, ty, src);
+    const float pz = __shfl_sync(0xffffffffu, tz, src);
+    const float pv = __shfl_sync(0xffffffffu, val, src), pw = __shfl_sync(0xffffffffu, w, src);
+    const int hx = a.deterministic ? (lane >> 1) & 1 : lane & 1;
+    if (!((pin >> hx) & 1)) continue;
+    const float fx = hx ? px : 1.0f - px;
 #pragma unroll
-  for (int k = 0; k < 8; ++k) {
-    const int xi = x0 + (k & 1), yi = y0 + ((k >> 1) & 1), zi = z0 + (k >> 2);
-    if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
-    const float f = ((k & 1) ? tx : 1.0f - tx) * (((k >> 1) & 1) ? ty : 1.0f - ty) *
-                    ((k >> 2) ? tz : 1.0f - tz);
-    if (f <= 0.0f) continue;
-    tc_add(a, ((size_t)zi * side + yi) * side + xi, val * f, w * f);
+    for (int k = 0; k < 4; ++k) {
+      if (!((pin >> (2 + (k & 1))) & (pin >> (4 + (k >> 1))) & 1)) continue;
+      const float f = fx * ((k & 1) ? py : 1.0f - py) * ((k >> 1) ? pz : 1.0f - pz);
+      if (f <= 0.0f) continue;
+      const int v = pbase + hx + ((k & 1) + (k >> 1) * side) * side;
+      if (a.deterministic) {
+        const bool wt = lane & 1;
+        atomicAdd(wt ? &a.fix2[v].y : &a.fix2[v].x,
+                  (unsigned long long)fixed_from_float(
+                      __fmul_rn(wt ? pw * f : pv * f, wt ? sc.y : sc.x)));
+      } else {
+        atomicAdd(a.acc2 + v, make_float2(pv * f, pw * f));
+      }
+    }
   }
 }
 
@@ -1339,12 +1372,12 @@ __device__ __forceinline__ void ms_insert(const TcMstepArgs& a, uint32_t taddr, 
       }
 #pragma unroll
       for (int j = 0; j < 16; ++j) tc_insert_nearest(a, v[j] >= 0, v[j], u[j] * qs, Tr);
-    } else if (live) {
+    } else if (__any_sync(0xffffffffu, live)) {
 #pragma unroll
       for (int j = 0; j < 16; ++j)
         if (j < nc) {
           const float4 p = xyz[c0 + j];
-          tc_insert_trilinear(a, Rm, p.x, p.y, p.z, u[j] * qs, Tr);
+          tc_insert_trilinear(a, live, Rm, p.x, p.y, p.z, u[j] * qs, Tr);
         }
     }
   }
@@ -2188,8 +2221,7 @@ int tc_mstep(emc_plan* p, float* model, float* weight) {
   a.deterministic = p->d.insert_mode == EMC_INSERT_DETERMINISTIC;
   a.model = model;
   a.weight = weight;
-  a.fix_m = p->fix_m;
-  a.fix_w = p->fix_w;
+  a.fix2 = p->fix2;
   a.acc2 = p->acc2;
   a.q_lo = p->mstep_q_lo;
   a.aggregate = p->mstep_aggregate;
