@@ -33,6 +33,7 @@
 #include "geometry.cuh"
 #include "kernels.cuh"
 #include "plan.cuh"
+#include "ptx.cuh"
 
 namespace emc {
 
@@ -95,13 +96,13 @@ __global__ void pattern_norm_kernel(const float* __restrict__ images, const int*
 // count.  One block per (pattern, 256 compacted pixels), pixel blocks the
 // fast index so that a pattern's row stays in L2 while its blocks run; flags
 // and part[i][block] (the block's sum of k, FP64, fixed order) reduced by
-// warp shuffles and one barrier.  Kraw / Kt / K2 (FP32 path) may be null;
+// warp shuffles and one barrier.  Kraw / Kt (FP32 path) may be null;
 // with Kh non-null the kernel also writes the tensor path's FP16 counts
 // (the same values as tc_pattern_ops_kernel with the same scale).
 __global__ void pattern_ops_kernel(const float* __restrict__ images, const int* __restrict__ pix,
                                    const float* __restrict__ cnorm, int n2, int N, int Kp,
                                    float* __restrict__ Kraw, float* __restrict__ Kt,
-                                   float* __restrict__ K2, int* __restrict__ flags,
+                                   int* __restrict__ flags,
                                    const int* __restrict__ perm, double* __restrict__ part,
                                    __half* __restrict__ Kh, float count_scale) {
   const int nqb = (Kp + 255) / 256;
@@ -141,7 +142,6 @@ __global__ void pattern_ops_kernel(const float* __restrict__ images, const int* 
     if (Kraw) Kraw[o] = k;
     const float kt = k >= 1e-10f ? k : 0.0f;  // the reference's (double)k > 1e-10
     if (Kt) Kt[o] = kt;
-    if (K2) K2[o] = __fmul_rn(kt, kt);
     if (Kh) Kh[o] = scaled_count(v, count_scale);
   }
   __syncthreads();
@@ -181,7 +181,7 @@ __host__ __device__ inline size_t pattern_row_smem(int n2, int Kp) {
 __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
     const float* __restrict__ images, const int* __restrict__ pix, const float* __restrict__ cnorm,
     int n2, int N, int Kp, float* __restrict__ Kraw, float* __restrict__ Kt,
-    float* __restrict__ K2, int* __restrict__ flags, const int* __restrict__ perm,
+    int* __restrict__ flags, const int* __restrict__ perm,
     float* __restrict__ Ksum, __half* __restrict__ Kh, float count_scale) {
   extern __shared__ __align__(16) unsigned char row_smem[];
   float* srow = reinterpret_cast<float*>(row_smem);
@@ -229,7 +229,6 @@ __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
     const float kt0 = k[0] >= 1e-10f ? k[0] : 0.0f;  // the reference's (double)k > 1e-10
     const float kt1 = k[1] >= 1e-10f ? k[1] : 0.0f;
     if (Kt) *reinterpret_cast<float2*>(Kt + o) = make_float2(kt0, kt1);
-    if (K2) *reinterpret_cast<float2*>(K2 + o) = make_float2(__fmul_rn(kt0, kt0), __fmul_rn(kt1, kt1));
     if (Kh)
       *reinterpret_cast<__half2*>(Kh + o) =
           __halves2half2(scaled_count(v[0], count_scale), scaled_count(v[1], count_scale));
@@ -449,7 +448,15 @@ __global__ void __launch_bounds__(256) tiny_plane_kernel(
 }
 
 // --------------------------------------------------- FP32 E-step tile ----
-constexpr int BM = 128, BN = 128, BK = 16, TPB = 256, SP = BM + 4;
+// The FP32 contractions: 128 x 128 tiles, 16 steps of the reduction per stage and
+// two stages (one barrier each), 8 x 8 results per thread as packed pairs along
+// the second operand.  Bound by the FP32 pipe: with scalar
+// multiply-adds, two barriers per stage and the coverage as an operand of its own,
+// 3,240 rotations x 2,000 patterns at 64^3 took 5,451 us (E-step) and 1,214 (M-step),
+// now 4,122 and 1,086.
+constexpr int BM = 128, BN = 128, BK = 16, TPB = 256, STG = BK * BM;
+
+using ptx::f32x2;
 
 // Loads a [128 rows][16 cols] tile of a row-major matrix (leading dim ld,
 // ld % 4 == 0) into two float4 per thread; rows >= nrows read as zero.
@@ -465,25 +472,37 @@ __device__ __forceinline__ void ld_tile(const float* __restrict__ src, size_t ld
   }
 }
 
-// Transposed store of a loaded tile: dst[k][row] = op(v).
+// Transposed store of a loaded tile: dst[k][row] = op(v), the row with bits 3 and 4
+// flipped by k / 4: a warp's stores (8 rows x 4 quads) meet all banks.
 template <typename Op>
-__device__ __forceinline__ void st_tile_t(float (*dst)[SP], const float4 (&v)[2], Op op) {
+__device__ __forceinline__ void st_tile_t(float* dst, const float4 (&v)[2], Op op) {
 #pragma unroll
   for (int u = 0; u < 2; ++u) {
     const int f = threadIdx.x + u * TPB;
-    const int row = f >> 2, quad = f & 3;
-    dst[quad * 4 + 0][row] = op(v[u].x);
-    dst[quad * 4 + 1][row] = op(v[u].y);
-    dst[quad * 4 + 2][row] = op(v[u].z);
-    dst[quad * 4 + 3][row] = op(v[u].w);
+    const int quad = f & 3, at = quad * 4 * BM + ((f >> 2) ^ (quad << 3));
+    dst[at] = op(v[u].x);
+    dst[at + BM] = op(v[u].y);
+    dst[at + 2 * BM] = op(v[u].z);
+    dst[at + 3 * BM] = op(v[u].w);
   }
 }
 
-__device__ __forceinline__ void ld8(const float (*s)[SP], int k, int base, float (&o)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(&s[k][base]);
-  const float4 b = *reinterpret_cast<const float4*>(&s[k][64 + base]);
-  o[0] = a.x; o[1] = a.y; o[2] = a.z; o[3] = a.w;
-  o[4] = b.x; o[5] = b.y; o[6] = b.z; o[7] = b.w;
+// Eight values of row k of such a tile (base: a multiple of 4), as four pairs, or
+// each twice in a pair.
+__device__ __forceinline__ void ld_pairs(const float* s, int k, int base, f32x2 (&o)[4]) {
+  const float* row = s + k * BM + (base ^ ((k >> 2) << 3));
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row);
+  const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(row + 64);
+  o[0] = a.x; o[1] = a.y; o[2] = b.x; o[3] = b.y;
+}
+__device__ __forceinline__ void ld_twice(const float* s, int k, int base, f32x2 (&o)[8]) {
+  const float* row = s + k * BM + (base ^ ((k >> 2) << 3));
+  const float4 a = *reinterpret_cast<const float4*>(row);
+  const float4 b = *reinterpret_cast<const float4*>(row + 64);
+  o[0] = ptx::pack2(a.x, a.x); o[1] = ptx::pack2(a.y, a.y);
+  o[2] = ptx::pack2(a.z, a.z); o[3] = ptx::pack2(a.w, a.w);
+  o[4] = ptx::pack2(b.x, b.x); o[5] = ptx::pack2(b.y, b.y);
+  o[6] = ptx::pack2(b.z, b.z); o[7] = ptx::pack2(b.w, b.w);
 }
 
 __device__ __forceinline__ int micro_idx(int t4, int i) { return (i < 4 ? 0 : 64) + t4 + (i & 3); }
@@ -492,7 +511,6 @@ struct EstepArgs {
   const float* S;      // [Rp][Kp]
   const float* Kraw;   // [N][Kp]
   const float* Kt;
-  const float* K2;
   const float* Ksum;   // [N]
   const float* rot_cnt;
   const float* rot_ssum;
@@ -506,13 +524,11 @@ struct EstepArgs {
   int known_intensity;
 };
 
-// Writes L/phi of the micro-tile and the tile's (max, sum exp) per pattern.
-__device__ void estep_epilogue(const EstepArgs& a, float (&Lv)[8][8], float (&phi)[8][8],
-                               float* sred /* [16][128] */, float* scol /* [128] */) {
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+// out[r][n] of the micro-tile.
+__device__ __forceinline__ void store_tile(const EstepArgs& a, float* __restrict__ out,
+                                           const float (&v)[8][8]) {
+  const int ty4 = (threadIdx.x >> 4) * 4, tx4 = (threadIdx.x & 15) * 4;
   const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int ty4 = ty * 4, tx4 = tx * 4;
-  // stores
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = r0 + micro_idx(ty4, i);
@@ -520,22 +536,25 @@ __device__ void estep_epilogue(const EstepArgs& a, float (&Lv)[8][8], float (&ph
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
       const int n = n0 + h * 64 + tx4;
-      float* lp = a.L + (size_t)r * a.N + n;
-      float* pp = a.PHI + (size_t)r * a.N + n;
+      float* p = out + (size_t)r * a.N + n;
       if (n + 3 < a.N && ((a.N & 3) == 0)) {
-        *reinterpret_cast<float4*>(lp) =
-            make_float4(Lv[i][4 * h], Lv[i][4 * h + 1], Lv[i][4 * h + 2], Lv[i][4 * h + 3]);
-        *reinterpret_cast<float4*>(pp) =
-            make_float4(phi[i][4 * h], phi[i][4 * h + 1], phi[i][4 * h + 2], phi[i][4 * h + 3]);
+        *reinterpret_cast<float4*>(p) =
+            make_float4(v[i][4 * h], v[i][4 * h + 1], v[i][4 * h + 2], v[i][4 * h + 3]);
       } else {
+#pragma unroll
         for (int c = 0; c < 4; ++c)
-          if (n + c < a.N) {
-            lp[c] = Lv[i][4 * h + c];
-            pp[c] = phi[i][4 * h + c];
-          }
+          if (n + c < a.N) p[c] = v[i][4 * h + c];
       }
     }
   }
+}
+
+// Writes L of the micro-tile and the tile's (max, sum exp) per pattern.
+__device__ void estep_epilogue(const EstepArgs& a, float (&Lv)[8][8],
+                               float* sred /* [16][128] */, float* scol /* [128] */) {
+  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+  const int n0 = blockIdx.x * BN, tx4 = tx * 4;
+  store_tile(a, a.L, Lv);
   // per-pattern max over the tile's rotations
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
@@ -570,151 +589,118 @@ __device__ void estep_epilogue(const EstepArgs& a, float (&Lv)[8][8], float (&ph
   }
 }
 
-// Reference-"poisson" likelihood with per-pair scaling, two pixel passes.
+// Reference-"poisson" likelihood with per-pair scaling, two pixel passes: 1 + 3
+// multiply-adds per (rotation, pattern, pixel) where a tile's rotations cover all
+// 16 pixels of a stage (s >= 1e-10), 2 + 3 elsewhere.
 __global__ void __launch_bounds__(TPB, 1) estep_fp32_kernel(EstepArgs a) {
-  __shared__ __align__(16) float s0[BK][SP];
-  __shared__ __align__(16) float s1[BK][SP];
-  __shared__ __align__(16) float s2[BK][SP];
-  __shared__ __align__(16) float s3[BK][SP];
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const int ty4 = ty * 4, tx4 = tx * 4;
+  __shared__ __align__(16) float sS[2][STG], sG[2][STG], sK[2][STG];
+  const int ty4 = (threadIdx.x >> 4) * 4, tx4 = (threadIdx.x & 15) * 4;
   const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
 
-  float num[8][8], den[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) num[i][j] = den[i][j] = 0.0f;
-
-  float4 vr[2], vk2[2], vkt[2];
-  const int nk = a.Kp / BK;
-  if (!a.known_intensity) {
-    // ---- pass 1: num = sum Kt^2 [s > 1e-10], den = sum Kt s [s > 1e-10]
-    ld_tile(a.S, a.Kp, r0, a.R, 0, vr);
-    ld_tile(a.K2, a.Kp, n0, a.N, 0, vk2);
-    ld_tile(a.Kt, a.Kp, n0, a.N, 0, vkt);
-    for (int kb = 0; kb < nk; ++kb) {
-      // s >= 1e-10f is the reference's (double)s > 1e-10 for every float s
-      st_tile_t(s0, vr, [](float s) { return s >= 1e-10f ? 1.0f : 0.0f; });
-      st_tile_t(s1, vr, [](float s) { return s >= 1e-10f ? s : 0.0f; });
-      st_tile_t(s2, vk2, [](float v) { return v; });
-      st_tile_t(s3, vkt, [](float v) { return v; });
-      __syncthreads();
-      if (kb + 1 < nk) {
-        ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
-        ld_tile(a.K2, a.Kp, n0, a.N, (kb + 1) * BK, vk2);
-        ld_tile(a.Kt, a.Kp, n0, a.N, (kb + 1) * BK, vkt);
-      }
-#pragma unroll 4
-      for (int k = 0; k < BK; ++k) {
-        float ra[8], rb[8], pk2[8], pkt[8];
-        ld8(s0, k, ty4, ra);
-        ld8(s1, k, ty4, rb);
-        ld8(s2, k, tx4, pk2);
-        ld8(s3, k, tx4, pkt);
-#pragma unroll
-        for (int i = 0; i < 8; ++i)
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            num[i][j] = __fmaf_rn(pk2[j], ra[i], num[i][j]);
-            den[i][j] = __fmaf_rn(pkt[j], rb[i], den[i][j]);
-          }
-      }
-      __syncthreads();
-    }
-  }
-  // 1/phi into num, phi into den (phi = 1 when known or undefined)
-  int nbad = 0;
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float phi = 1.0f, iphi = 1.0f;
-      if (!a.known_intensity) {
-        const bool ok = num[i][j] > 0.0f && den[i][j] > 0.0f;
-        phi = ok ? __fdiv_rn(num[i][j], den[i][j]) : 1.0f;
-        iphi = ok ? __fdiv_rn(den[i][j], num[i][j]) : -1.0f;  // -1 marks invalid
-      }
-      num[i][j] = iphi;
-      den[i][j] = phi;
-    }
-  // ---- pass 2: acc = sum (s - k/phi)^2 / (s + c) over s > 0
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
-  ld_tile(a.S, a.Kp, r0, a.R, 0, vr);
-  ld_tile(a.Kraw, a.Kp, n0, a.N, 0, vk2);
-  for (int kb = 0; kb < nk; ++kb) {
-    st_tile_t(s0, vr, [](float s) { return s; });
-    st_tile_t(s1, vr, [](float s) { return s > 0.0f ? __frcp_rn(s + kPoisC) : 0.0f; });
-    st_tile_t(s2, vk2, [](float v) { return v; });
-    __syncthreads();
-    if (kb + 1 < nk) {
-      ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
-      ld_tile(a.Kraw, a.Kp, n0, a.N, (kb + 1) * BK, vk2);
-    }
-#pragma unroll 4
-    for (int k = 0; k < BK; ++k) {
-      float rs[8], rg[8], pk[8];
-      ld8(s0, k, ty4, rs);
-      ld8(s1, k, ty4, rg);
-      ld8(s2, k, tx4, pk);
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float d = __fmaf_rn(-pk[j], num[i][j], rs[i]);
-          const float t = __fmul_rn(d, rg[i]);
-          acc[i][j] = __fmaf_rn(t, d, acc[i][j]);
-        }
-    }
-    __syncthreads();
-  }
-  // ---- epilogue
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = r0 + micro_idx(ty4, i);
-    const bool rok = r < a.R;
-    const float cnt = rok ? __ldg(a.rot_cnt + r) : 0.0f;
-    const float lw = rok ? logf(__ldg(a.rotw + r)) : 0.0f;
-    const float sg = *a.sigma;
-    const float scale = cnt > 0.0f ? (1.0f / (2.0f * sg * sg)) / cnt : 0.0f;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int n = n0 + micro_idx(tx4, j);
-      const bool ok = rok && n < a.N && cnt > 0.0f && num[i][j] > 0.0f;
-      if (rok && n < a.N && !ok) nbad++;
-      acc[i][j] = ok ? lw - acc[i][j] * scale : -INFINITY;
-    }
-  }
-  if (nbad) atomicAdd(a.bad, nbad);
-  float* sred = &s0[0][0];  // 16 x 128 floats fit in s0..s3 (4 x 16 x 132)
-  float* scol = &s3[0][0];
-  estep_epilogue(a, acc, den, sred, scol);
-}
-
-// True-Poisson likelihood: L = log w + sum k log s + K log(K/S_r) - K.
-__global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
-  __shared__ __align__(16) float s0[BK][SP];
-  __shared__ __align__(16) float s2[BK][SP];
-  __shared__ __align__(16) float s4[BK][SP];
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const int ty4 = ty * 4, tx4 = tx * 4;
-  const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+  f32x2 iphi[8][4];
   float4 vr[2], vk[2];
   const int nk = a.Kp / BK;
+  int nbad = 0;
+  if (!a.known_intensity) {
+    // ---- pass 1: num = sum Kt^2 [s >= 1e-10], den = sum Kt s [s >= 1e-10]
+    // (s >= 1e-10f is the reference's (double)s > 1e-10 for every float s)
+    f32x2 num[8][4], den[8][4], all[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) num[i][j] = den[i][j] = 0;
+    ld_tile(a.S, a.Kp, r0, a.R, 0, vr);
+    ld_tile(a.Kt, a.Kp, n0, a.N, 0, vk);
+    for (int kb = 0; kb < nk; ++kb) {
+      float *s = sS[kb & 1], *t = sK[kb & 1];
+      int out = 0;  // a rotation of the tile with a pixel outside
+      st_tile_t(s, vr, [&](float v) {
+        const bool in = v >= 1e-10f;
+        out |= !in;
+        return in ? v : 0.0f;
+      });
+      st_tile_t(t, vk, [](float v) { return v; });
+      if (__syncthreads_or(out) == 0) {
+        if (kb + 1 < nk) {
+          ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
+          ld_tile(a.Kt, a.Kp, n0, a.N, (kb + 1) * BK, vk);
+        }
+#pragma unroll 8
+        for (int k = 0; k < BK; ++k) {
+          f32x2 rs[8], pk[4];
+          ld_twice(s, k, ty4, rs);
+          ld_pairs(t, k, tx4, pk);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) all[j] = ptx::add2(all[j], ptx::mul2(pk[j], pk[j]));
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) den[i][j] = ptx::fma2(pk[j], rs[i], den[i][j]);
+        }
+      } else {
+        if (kb + 1 < nk) {
+          ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
+          ld_tile(a.Kt, a.Kp, n0, a.N, (kb + 1) * BK, vk);
+        }
+#pragma unroll 4
+        for (int k = 0; k < BK; ++k) {
+          f32x2 rs[8], pk[4], p2[4];
+          ld_twice(s, k, ty4, rs);
+          ld_pairs(t, k, tx4, pk);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) p2[j] = ptx::mul2(pk[j], pk[j]);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const float m = ptx::unpack2(rs[i]).x > 0.0f ? 1.0f : 0.0f;
+            const f32x2 mm = ptx::pack2(m, m);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              num[i][j] = ptx::fma2(p2[j], mm, num[i][j]);
+              den[i][j] = ptx::fma2(pk[j], rs[i], den[i][j]);
+            }
+          }
+        }
+      }
+    }
+    float phi[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 u = ptx::unpack2(ptx::add2(num[i][j], all[j]));
+        const float2 d = ptx::unpack2(den[i][j]);
+        // phi = 1 where undefined; 1/phi = -1 marks it
+        const bool ox = u.x > 0.0f && d.x > 0.0f, oy = u.y > 0.0f && d.y > 0.0f;
+        phi[i][2 * j] = ox ? __fdiv_rn(u.x, d.x) : 1.0f;
+        phi[i][2 * j + 1] = oy ? __fdiv_rn(u.y, d.y) : 1.0f;
+        iphi[i][j] = ptx::pack2(ox ? __fdiv_rn(d.x, u.x) : -1.0f, oy ? __fdiv_rn(d.y, u.y) : -1.0f);
+      }
+    store_tile(a, a.PHI, phi);
+    __syncthreads();  // the last stage has been read
+  } else {
+    float phi[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        phi[i][j] = 1.0f;
+        iphi[i][j >> 1] = ptx::pack2(1.0f, 1.0f);
+      }
+    store_tile(a, a.PHI, phi);
+  }
+  // ---- pass 2: acc = sum (s - k/phi)^2 / (s + c) over s > 0
+  f32x2 acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   ld_tile(a.S, a.Kp, r0, a.R, 0, vr);
   ld_tile(a.Kraw, a.Kp, n0, a.N, 0, vk);
   for (int kb = 0; kb < nk; ++kb) {
-    st_tile_t(s0, vr, [](float s) { return logf(fmaxf(s, kSliceFloor)); });
-    st_tile_t(s2, vk, [](float v) { return v; });
+    float *s = sS[kb & 1], *g = sG[kb & 1], *t = sK[kb & 1];
+    st_tile_t(s, vr, [](float v) { return v; });
+    st_tile_t(g, vr, [](float v) { return v > 0.0f ? __frcp_rn(v + kPoisC) : 0.0f; });
+    st_tile_t(t, vk, [](float v) { return -v; });
     __syncthreads();
     if (kb + 1 < nk) {
       ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
@@ -722,17 +708,79 @@ __global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
     }
 #pragma unroll 4
     for (int k = 0; k < BK; ++k) {
-      float rl[8], pk[8];
-      ld8(s0, k, ty4, rl);
-      ld8(s2, k, tx4, pk);
+      f32x2 rs[8], rg[8], pk[4];
+      ld_twice(s, k, ty4, rs);
+      ld_twice(g, k, ty4, rg);
+      ld_pairs(t, k, tx4, pk);
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = __fmaf_rn(pk[j], rl[i], acc[i][j]);
+        for (int j = 0; j < 4; ++j) {
+          const f32x2 d = ptx::fma2(pk[j], iphi[i][j], rs[i]);
+          acc[i][j] = ptx::fma2(ptx::mul2(d, rg[i]), d, acc[i][j]);
+        }
     }
-    __syncthreads();
   }
-  float phi[8][8];
+  __syncthreads();  // sS and sK are free
+  // ---- epilogue
+  float Lv[8][8];
+  const float sg = *a.sigma;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int r = r0 + micro_idx(ty4, i);
+    const bool rok = r < a.R;
+    const float cnt = rok ? __ldg(a.rot_cnt + r) : 0.0f;
+    const float lw = rok ? logf(__ldg(a.rotw + r)) : 0.0f;
+    const float scale = cnt > 0.0f ? (1.0f / (2.0f * sg * sg)) / cnt : 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float2 e = ptx::unpack2(acc[i][j >> 1]), f = ptx::unpack2(iphi[i][j >> 1]);
+      const int n = n0 + micro_idx(tx4, j);
+      const bool ok = rok && n < a.N && cnt > 0.0f && ((j & 1) ? f.y : f.x) > 0.0f;
+      if (rok && n < a.N && !ok) nbad++;
+      Lv[i][j] = ok ? lw - ((j & 1) ? e.y : e.x) * scale : -INFINITY;
+    }
+  }
+  if (nbad) atomicAdd(a.bad, nbad);
+  estep_epilogue(a, Lv, &sS[0][0], &sK[0][0]);
+}
+
+// True-Poisson likelihood: L = log w + sum k log s + K log(K/S_r) - K.
+__global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
+  __shared__ __align__(16) float sS[2][STG], sK[2][STG];
+  const int ty4 = (threadIdx.x >> 4) * 4, tx4 = (threadIdx.x & 15) * 4;
+  const int r0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
+  f32x2 acc[8][4];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
+  float4 vr[2], vk[2];
+  const int nk = a.Kp / BK;
+  ld_tile(a.S, a.Kp, r0, a.R, 0, vr);
+  ld_tile(a.Kraw, a.Kp, n0, a.N, 0, vk);
+  for (int kb = 0; kb < nk; ++kb) {
+    float *s = sS[kb & 1], *t = sK[kb & 1];
+    st_tile_t(s, vr, [](float v) { return logf(fmaxf(v, kSliceFloor)); });
+    st_tile_t(t, vk, [](float v) { return v; });
+    __syncthreads();
+    if (kb + 1 < nk) {
+      ld_tile(a.S, a.Kp, r0, a.R, (kb + 1) * BK, vr);
+      ld_tile(a.Kraw, a.Kp, n0, a.N, (kb + 1) * BK, vk);
+    }
+#pragma unroll 8
+    for (int k = 0; k < BK; ++k) {
+      f32x2 rl[8], pk[4];
+      ld_twice(s, k, ty4, rl);
+      ld_pairs(t, k, tx4, pk);
+#pragma unroll
+      for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = ptx::fma2(pk[j], rl[i], acc[i][j]);
+    }
+  }
+  __syncthreads();  // sS and sK are free
+  float Lv[8][8], phi[8][8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int r = r0 + micro_idx(ty4, i);
@@ -741,26 +789,27 @@ __global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
     const float Sr = rok ? __ldg(a.rot_ssum + r) : 1.0f;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
+      const float2 e2 = ptx::unpack2(acc[i][j >> 1]);
+      const float e = (j & 1) ? e2.y : e2.x;
       const int n = n0 + micro_idx(tx4, j);
       const float Ki = n < a.N ? __ldg(a.Ksum + n) : 0.0f;
       float l, f;
       if (a.known_intensity) {
         f = 1.0f;
-        l = lw + acc[i][j] - Sr;
+        l = lw + e - Sr;
       } else if (Ki > 0.0f) {
         f = Ki / Sr;
-        l = lw + acc[i][j] + Ki * logf(f) - Ki;
+        l = lw + e + Ki * logf(f) - Ki;
       } else {
         f = 0.0f;
         l = lw;
       }
-      acc[i][j] = rok && n < a.N ? l : -INFINITY;
+      Lv[i][j] = rok && n < a.N ? l : -INFINITY;
       phi[i][j] = f;
     }
   }
-  float* sred = &s0[0][0];
-  float* scol = &s4[0][0];
-  estep_epilogue(a, acc, phi, sred, scol);
+  store_tile(a, a.PHI, phi);
+  estep_epilogue(a, Lv, &sS[0][0], &sK[0][0]);
 }
 
 // ------------------------------------------------------- normalise -------
@@ -1069,34 +1118,36 @@ __device__ __forceinline__ void add_voxel(const InsertCtx& c, size_t v, float va
   }
 }
 
-// Inserts value `val` with weight `w` at the detector point (x, y, z) rotated
-// by R: nearest voxel with the reference's insertion bounds (>= 0,
-// emc_atomic.cu:67-69) or a trilinear splat.
-__device__ __forceinline__ void insert_point(const InsertCtx& c, const RotMat& R, float x, float y,
-                                             float z, float val, float w) {
+// The voxel nearest to the detector point (x, y, z) rotated by R, -1 outside the
+// reference's insertion bounds (>= 0, emc_atomic.cu:67-69).
+__device__ __forceinline__ long long nearest_voxel(const InsertCtx& c, const RotMat& R, float x,
+                                                   float y, float z) {
   const int side = c.side;
-  if (c.interp == EMC_INTERP_NEAREST) {
-    const long ix = voxel_round(voxel_coord(side, rotate_row(R, 0, x, y, z)));
-    const long iy = voxel_round(voxel_coord(side, rotate_row(R, 1, x, y, z)));
-    const long iz = voxel_round(voxel_coord(side, rotate_row(R, 2, x, y, z)));
-    if (ix < 0 || ix >= side || iy < 0 || iy >= side || iz < 0 || iz >= side) return;
-    add_voxel(c, ((size_t)iz * side + iy) * side + ix, val, w);
-  } else {
-    const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
-    const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
-    const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
-    const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
-    const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-    const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
+  const long ix = voxel_round(voxel_coord(side, rotate_row(R, 0, x, y, z)));
+  const long iy = voxel_round(voxel_coord(side, rotate_row(R, 1, x, y, z)));
+  const long iz = voxel_round(voxel_coord(side, rotate_row(R, 2, x, y, z)));
+  if (ix < 0 || ix >= side || iy < 0 || iy >= side || iz < 0 || iz >= side) return -1;
+  return ((long long)iz * side + iy) * side + ix;
+}
+
+// Trilinear splat of value `val` with weight `w` at the rotated point.
+__device__ __forceinline__ void splat_point(const InsertCtx& c, const RotMat& R, float x, float y,
+                                            float z, float val, float w) {
+  const int side = c.side;
+  const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
+  const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
+  const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
+  const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
+  const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
+  const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-      const int xi = x0 + (k & 1), yi = y0 + ((k >> 1) & 1), zi = z0 + (k >> 2);
-      if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
-      const float f = ((k & 1) ? tx : 1.0f - tx) * (((k >> 1) & 1) ? ty : 1.0f - ty) *
-                      ((k >> 2) ? tz : 1.0f - tz);
-      if (f <= 0.0f) continue;
-      add_voxel(c, ((size_t)zi * side + yi) * side + xi, val * f, w * f);
-    }
+  for (int k = 0; k < 8; ++k) {
+    const int xi = x0 + (k & 1), yi = y0 + ((k >> 1) & 1), zi = z0 + (k >> 2);
+    if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
+    const float f = ((k & 1) ? tx : 1.0f - tx) * (((k >> 1) & 1) ? ty : 1.0f - ty) *
+                    ((k >> 2) ? tz : 1.0f - tz);
+    if (f <= 0.0f) continue;
+    add_voxel(c, ((size_t)zi * side + yi) * side + xi, val * f, w * f);
   }
 }
 
@@ -1111,23 +1162,22 @@ struct MstepArgs {
   InsertCtx ins;
 };
 
-// U = Q K for a 128-rotation x 128-pixel tile, inserted in the epilogue.
-__global__ void __launch_bounds__(TPB, 1) mstep_fp32_kernel(MstepArgs a) {
-  __shared__ __align__(16) float sq[BK][SP];
-  __shared__ __align__(16) float sk[BK][SP];
+// U = Q K for a 128-rotation x 128-pixel tile, inserted in the epilogue (slice =
+// U / T_r with weight T_r: U itself goes to the model sum).
+__global__ void __launch_bounds__(TPB, 2) mstep_fp32_kernel(MstepArgs a) {
+  __shared__ __align__(16) float sq[2][STG], sk[2][STG];
   __shared__ RotMat sR[BM];
-  const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
-  const int ty4 = ty * 4, tx4 = tx * 4;
+  const int ty4 = (threadIdx.x >> 4) * 4, tx4 = (threadIdx.x & 15) * 4;
   const int r0 = blockIdx.y * BM, q0 = blockIdx.x * BN;
   if (threadIdx.x < BM) {
     const int r = r0 + threadIdx.x;
     if (r < a.R) sR[threadIdx.x] = quat_to_matrix(a.rot + 4 * (size_t)r);
   }
-  float acc[8][8];
+  f32x2 acc[8][4];
 #pragma unroll
   for (int i = 0; i < 8; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.0f;
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0;
   float4 vq[2], vk[2];
   const int nk = (a.N + BK - 1) / BK;
   auto ld_k = [&](int kb) {
@@ -1141,19 +1191,20 @@ __global__ void __launch_bounds__(TPB, 1) mstep_fp32_kernel(MstepArgs a) {
                       : make_float4(0.f, 0.f, 0.f, 0.f);
     }
   };
-  auto st_k = [&]() {
+  auto st_k = [&](float* dst) {  // with the columns' bits flipped as in st_tile_t
 #pragma unroll
     for (int u = 0; u < 2; ++u) {
       const int f = threadIdx.x + u * TPB;
-      const int row = f >> 5, c4 = f & 31;
-      *reinterpret_cast<float4*>(&sk[row][c4 * 4]) = vk[u];
+      const int row = f >> 5, c = (f & 31) * 4;
+      *reinterpret_cast<float4*>(dst + row * BN + (c ^ ((row >> 2) << 3))) = vk[u];
     }
   };
   ld_tile(a.Q, a.ldq, r0, a.R, 0, vq);
   ld_k(0);
   for (int kb = 0; kb < nk; ++kb) {
-    st_tile_t(sq, vq, [](float v) { return v; });
-    st_k();
+    float *s = sq[kb & 1], *t = sk[kb & 1];
+    st_tile_t(s, vq, [](float v) { return v; });
+    st_k(t);
     __syncthreads();
     if (kb + 1 < nk) {
       ld_tile(a.Q, a.ldq, r0, a.R, (kb + 1) * BK, vq);
@@ -1161,42 +1212,58 @@ __global__ void __launch_bounds__(TPB, 1) mstep_fp32_kernel(MstepArgs a) {
     }
 #pragma unroll 4
     for (int k = 0; k < BK; ++k) {
-      float rq[8], pk[8];
-      ld8(sq, k, ty4, rq);
-      ld8(sk, k, tx4, pk);
+      f32x2 rq[8], pk[4];
+      ld_twice(s, k, ty4, rq);
+      ld_pairs(t, k, tx4, pk);
 #pragma unroll
       for (int i = 0; i < 8; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j] = __fmaf_rn(rq[i], pk[j], acc[i][j]);
+        for (int j = 0; j < 4; ++j) acc[i][j] = ptx::fma2(pk[j], rq[i], acc[i][j]);
     }
-    __syncthreads();
   }
-  // ---- epilogue: slice = U / T_r, insert T_r * slice with weight T_r
+  // ---- epilogue
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     const int rl = micro_idx(ty4, i);
     const int r = r0 + rl;
     if (r >= a.R) continue;
     const float t = __ldg(a.T + r);
+    const bool live = t > 1e-10f;
+    float u[8];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 v = ptx::unpack2(acc[i][j]);
+      u[2 * j] = v.x;
+      u[2 * j + 1] = v.y;
+    }
     if (a.ins.u) {  // sorted mode: the pair values, 0 where the rotation inserts nothing
-      const bool live = t > 1e-10f;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int q = q0 + micro_idx(tx4, j);
-        if (q < a.P_eff)
-          a.ins.u[(size_t)q * a.ins.ldu + r] = live ? __fmul_rn(t, __fdiv_rn(acc[i][j], t)) : 0.0f;
+        if (q < a.P_eff) a.ins.u[(size_t)q * a.ins.ldu + r] = live ? u[j] : 0.0f;
       }
       continue;
     }
-    if (!(t > 1e-10f)) continue;
+    if (!live) continue;
     const RotMat R = sR[rl];
+    if (a.ins.interp == EMC_INTERP_NEAREST) {
+      long long v[8];  // all voxels before the first atomic
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int q = q0 + micro_idx(tx4, j);
+        v[j] = q < a.P_eff ? nearest_voxel(a.ins, R, __ldg(a.cx + q), __ldg(a.cy + q), __ldg(a.cz + q))
+                           : -1;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (v[j] >= 0) add_voxel(a.ins, (size_t)v[j], u[j], t);
+      continue;
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const int q = q0 + micro_idx(tx4, j);
-      if (q >= a.P_eff) continue;
-      const float slice = __fdiv_rn(acc[i][j], t);
-      insert_point(a.ins, R, __ldg(a.cx + q), __ldg(a.cy + q), __ldg(a.cz + q),
-                   __fmul_rn(t, slice), t);
+      if (q < a.P_eff)
+        splat_point(a.ins, R, __ldg(a.cx + q), __ldg(a.cy + q), __ldg(a.cz + q), u[j], t);
     }
   }
 }
@@ -1458,7 +1525,7 @@ int emc::pattern_side(emc_plan* p, const int* d_perm, bool with_tc) {
   pattern_norm_kernel<<<ceil_div(N, 128), 128, 0, ctx->stream>>>(
       p->images, p->mask, n2, N, p->d.normalize_images, p->cnorm, d_perm);
   if ((rc = after_launch(ctx, "pattern_norm_kernel"))) return rc;
-  // Kt / K2 exist only for the FP32 path (null: not written).
+  // Kt exists only for the FP32 path (null: not written).
   const int nqb = ceil_div(p->Kp, 256);
   // once the tensor-core operands exist, their FP16 counts come from the same
   // pass at the current scale (bind re-runs them if the new counts need
@@ -1468,14 +1535,14 @@ int emc::pattern_side(emc_plan* p, const int* d_perm, bool with_tc) {
   const size_t row_smem = pattern_row_smem(n2, p->Kp);
   if (row_smem <= (size_t)kRowSmemMax) {
     pattern_row_kernel<<<N, kRowThreads, row_smem, ctx->stream>>>(
-        p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->K2, p->flags, d_perm,
+        p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->flags, d_perm,
         p->Ksum, fused ? p->Kh : nullptr, p->count_scale);
     if ((rc = after_launch(ctx, "pattern_row_kernel"))) return rc;
     if (with_tc && p->tc) return tc_pattern_side(p, d_perm, fused);
     return EMC_OK;
   }
   pattern_ops_kernel<<<(unsigned)N * (unsigned)nqb, 256, 0, ctx->stream>>>(
-      p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->K2, p->flags, d_perm,
+      p->images, p->pix, p->cnorm, n2, N, p->Kp, p->Kraw, p->Kt, p->flags, d_perm,
       p->ksum_part, fused ? p->Kh : nullptr, p->count_scale);
   if ((rc = after_launch(ctx, "pattern_ops_kernel"))) return rc;
   pattern_sums_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(p->ksum_part, N, nqb, p->Ksum);
@@ -1543,7 +1610,6 @@ extern "C" int emc_plan_bind(emc_plan* p, const float* d_images, const int* d_ma
   if (!rc && p->d.precision == EMC_PREC_FP32) rc = alloc_n(p, &p->S, (size_t)p->Rp * p->Kp);
   if (!rc && p->d.precision == EMC_PREC_FP32) {
     rc = alloc_n(p, &p->Kt, (size_t)N * p->Kp);
-    if (!rc) rc = alloc_n(p, &p->K2, (size_t)N * p->Kp);
   }
   // rows R..Rp of the slices stay zero: the expand writes rows < R only
   if (!rc && p->S) {
@@ -1626,7 +1692,6 @@ static int plan_estep_fp32(emc_plan* p) {
   a.S = p->S;
   a.Kraw = p->Kraw;
   a.Kt = p->Kt;
-  a.K2 = p->K2;
   a.Ksum = p->Ksum;
   a.rot_cnt = p->rot_cnt;
   a.rot_ssum = p->rot_ssum;

@@ -46,7 +46,6 @@ struct emc_plan {
   std::vector<int> h_mask, h_pix;  // the bound mask and its compacted pixels (re-binds)
   float fused_scale = 0.0f;  // count_scale of FP16 counts written by the pattern pass (0: none)
   float* Kt = nullptr;    // k if k > 1e-10 else 0
-  float* K2 = nullptr;    // Kt^2
   float* Ksum = nullptr;  // [N] sum_p k
   float* cnorm = nullptr; // [N] c_i (1 when not normalising)
 

@@ -27,6 +27,7 @@
 #include "emc_gb300.h"
 #include "geometry.cuh"
 #include "plan.cuh"
+#include "ptx.cuh"
 
 namespace emc {
 namespace pn {
@@ -159,8 +160,8 @@ __global__ void gather_rows_kernel(const float* __restrict__ X, const int* __res
 // so that a value from shared memory serves eight multiply-adds; what bounds them
 // is FP32 issue.  The GEMM form before, with 4 x 4 sums per thread and every
 // element of the implicit column matrix addressed by divisions, reached 14 TFLOP/s
-// forward: 4,107 us for 2,250 patterns, now 1,456 (47 TFLOP/s in the layer with 16 x
-// 16 outputs); the gradients of 250 patterns took 3,271 us, now 590.
+// forward: 4,107 us for 2,250 patterns, now 1,406 (49 TFLOP/s in the layer with 16 x
+// 16 outputs); the gradients of 250 patterns took 3,271 us, now 560.
 
 // A stride-2 row of the input in shared memory: the even columns 0, 2, .. at 0,
 // the odd ones -1, 1, 3, .. at HO, so that the eight outputs of a thread read
@@ -186,6 +187,10 @@ struct ConvPatch {
 __device__ __forceinline__ int own_channel(int cg, int i) {
   return (i & 4) * 8 + cg * 4 + (i & 3);
 }
+
+using ptx::f32x2;
+
+__device__ __forceinline__ f32x2 twice(float x) { return ptx::pack2(x, x); }
 
 __device__ __forceinline__ float4 relu_grad(float4 out, float4 g) {
   return make_float4(out.x > 0.0f ? g.x : 0.0f, out.y > 0.0f ? g.y : 0.0f,
@@ -261,11 +266,11 @@ __global__ void __launch_bounds__(256, 2) conv_fwd_kernel(const float* __restric
   const int oy = g / (HO / PX), ox = (g % (HO / PX)) * PX;
   const int b0 = blockIdx.x * F::SPB;
   for (int e = threadIdx.x; e < F::X; e += 256) sX[e] = 0.0f;  // the borders stay zero
-  float acc[8][PX];
+  f32x2 acc[4][PX];  // pairs of output channels
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < PX; ++j) acc[i][j] = 0.0f;
+    for (int j = 0; j < PX; ++j) acc[i][j] = 0;
   for (int c0 = 0; c0 < pn::CH; c0 += pn::CC) {
     __syncthreads();
     constexpr int Q = HI * HI / 4;
@@ -292,26 +297,26 @@ __global__ void __launch_bounds__(256, 2) conv_fwd_kernel(const float* __restric
 #pragma unroll
       for (int ky = 0; ky < 3; ++ky) {
         const float* row = sX + (c * F::SPB + smp) * Patch::SIZE + (2 * oy + ky) * Patch::RS + ox;
-        float ev[PX], od[PX + 1];
+        f32x2 ev[PX], od[PX + 1];
 #pragma unroll
         for (int j = 0; j < PX; j += 4) {
           const float4 a = *reinterpret_cast<const float4*>(row + j);
           const float4 o = *reinterpret_cast<const float4*>(row + HO + j);
-          ev[j] = a.x; ev[j + 1] = a.y; ev[j + 2] = a.z; ev[j + 3] = a.w;
-          od[j] = o.x; od[j + 1] = o.y; od[j + 2] = o.z; od[j + 3] = o.w;
+          ev[j] = twice(a.x); ev[j + 1] = twice(a.y); ev[j + 2] = twice(a.z); ev[j + 3] = twice(a.w);
+          od[j] = twice(o.x); od[j + 1] = twice(o.y); od[j + 2] = twice(o.z); od[j + 3] = twice(o.w);
         }
-        od[PX] = row[HO + PX];
+        od[PX] = twice(row[HO + PX]);
 #pragma unroll
         for (int kx = 0; kx < 3; ++kx) {
           const float* wp = sW + (c * 9 + ky * 3 + kx) * pn::WS + cg * 4;
-          const float4 w0 = *reinterpret_cast<const float4*>(wp);
-          const float4 w1 = *reinterpret_cast<const float4*>(wp + 32);
-          const float w[8] = {w0.x, w0.y, w0.z, w0.w, w1.x, w1.y, w1.z, w1.w};
+          const ulonglong2 w0 = *reinterpret_cast<const ulonglong2*>(wp);
+          const ulonglong2 w1 = *reinterpret_cast<const ulonglong2*>(wp + 32);
+          const f32x2 w[4] = {w0.x, w0.y, w1.x, w1.y};
 #pragma unroll
-          for (int i = 0; i < 8; ++i)
+          for (int i = 0; i < 4; ++i)
 #pragma unroll
             for (int j = 0; j < PX; ++j)
-              acc[i][j] = fmaf(w[i], kx == 1 ? ev[j] : od[j + (kx >> 1)], acc[i][j]);
+              acc[i][j] = ptx::fma2(w[i], kx == 1 ? ev[j] : od[j + (kx >> 1)], acc[i][j]);
         }
       }
     }
@@ -323,11 +328,14 @@ __global__ void __launch_bounds__(256, 2) conv_fwd_kernel(const float* __restric
     const int co = own_channel(cg, i);
     const float bi = bias[co];
     float* dst = out + (((size_t)b * pn::CH + co) * HO + oy) * HO + ox;
+    auto value = [&](int j) {
+      const float2 v = ptx::unpack2(acc[i >> 1][j]);
+      return fmaxf(((i & 1) ? v.y : v.x) + bi, 0.0f);
+    };
 #pragma unroll
     for (int j = 0; j < PX; j += 4)
       *reinterpret_cast<float4*>(dst + j) =
-          make_float4(fmaxf(acc[i][j] + bi, 0.0f), fmaxf(acc[i][j + 1] + bi, 0.0f),
-                      fmaxf(acc[i][j + 2] + bi, 0.0f), fmaxf(acc[i][j + 3] + bi, 0.0f));
+          make_float4(value(j), value(j + 1), value(j + 2), value(j + 3));
   }
 }
 
@@ -362,13 +370,14 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_data_kernel(const float* __re
   const int ry = g / (HO / 4), px = (g % (HO / 4)) * 4;
   const int b0 = (blockIdx.x / F::PARTS) * F::SPB, y0 = (blockIdx.x % F::PARTS) * F::ROWS;
   for (int e = threadIdx.x; e < F::DSZ; e += 256) sD[e] = 0.0f;  // the borders stay zero
-  float acc[4][4][4];  // pixel (2 y, 2 x), (2 y, 2 x + 1), (2 y + 1, 2 x), (2 y + 1, 2 x + 1)
+  // pairs of input channels; pixel (2 y, 2 x), (2 y, 2 x + 1), (2 y + 1, 2 x), ..
+  f32x2 acc[2][4][4];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < 2; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int u = 0; u < 4; ++u) acc[i][j][u] = 0.0f;
+      for (int u = 0; u < 4; ++u) acc[i][j][u] = 0;
   for (int c0 = 0; c0 < pn::CH; c0 += pn::CC) {
     __syncthreads();
     for (int e = threadIdx.x; e < pn::CC * F::SPB * (F::ROWS + 1) * (HO / 4); e += 256) {
@@ -392,19 +401,21 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_data_kernel(const float* __re
       const float* r1 = r0 + F::RS;
       const float4 e0 = *reinterpret_cast<const float4*>(r0);
       const float4 e1 = *reinterpret_cast<const float4*>(r1);
-      const float d0[5] = {e0.x, e0.y, e0.z, e0.w, r0[4]};
-      const float d1[5] = {e1.x, e1.y, e1.z, e1.w, r1[4]};
+      const f32x2 d0[5] = {twice(e0.x), twice(e0.y), twice(e0.z), twice(e0.w), twice(r0[4])};
+      const f32x2 d1[5] = {twice(e1.x), twice(e1.y), twice(e1.z), twice(e1.w), twice(r1[4])};
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
-        const float4 w0 = *reinterpret_cast<const float4*>(sW + (c * 9 + t) * pn::WS + cg * 4);
-        const float w[4] = {w0.x, w0.y, w0.z, w0.w};
+        const ulonglong2 w0 =
+            *reinterpret_cast<const ulonglong2*>(sW + (c * 9 + t) * pn::WS + cg * 4);
+        const f32x2 w[2] = {w0.x, w0.y};
         const int ky = t / 3, kx = t % 3;
         const int cls = (ky != 1 ? 2 : 0) + (kx != 1 ? 1 : 0);
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            acc[i][j][cls] = fmaf(w[i], (ky == 0 ? d1 : d0)[j + (kx == 0 ? 1 : 0)], acc[i][j][cls]);
+            acc[i][j][cls] =
+                ptx::fma2(w[i], (ky == 0 ? d1 : d0)[j + (kx == 0 ? 1 : 0)], acc[i][j][cls]);
       }
     }
   }
@@ -413,12 +424,16 @@ __global__ void __launch_bounds__(256, 2) conv_bwd_data_kernel(const float* __re
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
     float* dst = gin + (((size_t)b * pn::CH + cg * 4 + i) * HI + 2 * (y0 + ry)) * HI + 2 * px;
+    auto value = [&](int j, int u) {
+      const float2 v = ptx::unpack2(acc[i >> 1][j][u]);
+      return (i & 1) ? v.y : v.x;
+    };
 #pragma unroll
     for (int j = 0; j < 4; j += 2) {
       *reinterpret_cast<float4*>(dst + 2 * j) =
-          make_float4(acc[i][j][0], acc[i][j][1], acc[i][j + 1][0], acc[i][j + 1][1]);
+          make_float4(value(j, 0), value(j, 1), value(j + 1, 0), value(j + 1, 1));
       *reinterpret_cast<float4*>(dst + HI + 2 * j) =
-          make_float4(acc[i][j][2], acc[i][j][3], acc[i][j + 1][2], acc[i][j + 1][3]);
+          make_float4(value(j, 2), value(j, 3), value(j + 1, 2), value(j + 1, 3));
     }
   }
 }
@@ -451,11 +466,11 @@ __global__ void __launch_bounds__(256, 2) conv_wgrad_kernel(const float* __restr
   const int cg = threadIdx.x & 7, ci = (threadIdx.x >> 3) & 7, sp = threadIdx.x >> 6;
   const int c0 = blockIdx.x * pn::CC, s = blockIdx.y;
   const int bend = min(B, (s + 1) * per);
-  float acc[8][9];
+  f32x2 acc[4][9];  // pairs of output channels
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int t = 0; t < 9; ++t) acc[i][t] = 0.0f;
+    for (int t = 0; t < 9; ++t) acc[i][t] = 0;
   float bsum = 0.0f;  // block 0: channel threadIdx.x & 63, split sp of the pixels
   for (int e = threadIdx.x; e < F::X; e += 256) sX[e] = 0.0f;
   for (int b = s * per; b < bend; ++b) {
@@ -479,26 +494,26 @@ __global__ void __launch_bounds__(256, 2) conv_wgrad_kernel(const float* __restr
     __syncthreads();
     for (int oy = sp; oy < HO; oy += 4) {
       const float* row = sX + ci * Patch::SIZE + 2 * oy * Patch::RS;
-      float lft[3];
+      f32x2 lft[3];
 #pragma unroll
-      for (int ky = 0; ky < 3; ++ky) lft[ky] = row[ky * Patch::RS + HO];
+      for (int ky = 0; ky < 3; ++ky) lft[ky] = twice(row[ky * Patch::RS + HO]);
 #pragma unroll 2
       for (int ox = 0; ox < HO; ++ox) {
         const float* dp = sD + (oy * HO + ox) * pn::WS + cg * 4;
-        const float4 a = *reinterpret_cast<const float4*>(dp);
-        const float4 c = *reinterpret_cast<const float4*>(dp + 32);
-        const float d[8] = {a.x, a.y, a.z, a.w, c.x, c.y, c.z, c.w};
-        float x[9];
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(dp);
+        const ulonglong2 c = *reinterpret_cast<const ulonglong2*>(dp + 32);
+        const f32x2 d[4] = {a.x, a.y, c.x, c.y};
+        f32x2 x[9];
 #pragma unroll
         for (int ky = 0; ky < 3; ++ky) {
           x[3 * ky] = lft[ky];
-          x[3 * ky + 1] = row[ky * Patch::RS + ox];
-          x[3 * ky + 2] = lft[ky] = row[ky * Patch::RS + HO + ox + 1];
+          x[3 * ky + 1] = twice(row[ky * Patch::RS + ox]);
+          x[3 * ky + 2] = lft[ky] = twice(row[ky * Patch::RS + HO + ox + 1]);
         }
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
+        for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int t = 0; t < 9; ++t) acc[i][t] = fmaf(d[i], x[t], acc[i][t]);
+          for (int t = 0; t < 9; ++t) acc[i][t] = ptx::fma2(d[i], x[t], acc[i][t]);
       }
     }
     if (blockIdx.x == 0)
@@ -506,11 +521,15 @@ __global__ void __launch_bounds__(256, 2) conv_wgrad_kernel(const float* __restr
   }
   __syncthreads();
   const int lane64 = threadIdx.x & 63;
+  auto value = [&](int i, int t) {
+    const float2 v = ptx::unpack2(acc[i >> 1][t]);
+    return (i & 1) ? v.y : v.x;
+  };
   if (sp > 0) {
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
-      for (int t = 0; t < 9; ++t) sm[((sp - 1) * 72 + i * 9 + t) * 64 + lane64] = acc[i][t];
+      for (int t = 0; t < 9; ++t) sm[((sp - 1) * 72 + i * 9 + t) * 64 + lane64] = value(i, t);
   }
   __syncthreads();
   if (sp == 0) {
@@ -518,7 +537,7 @@ __global__ void __launch_bounds__(256, 2) conv_wgrad_kernel(const float* __restr
     for (int i = 0; i < 8; ++i)
 #pragma unroll
       for (int t = 0; t < 9; ++t) {
-        float v = acc[i][t];
+        float v = value(i, t);
 #pragma unroll
         for (int u = 0; u < 3; ++u) v += sm[(u * 72 + i * 9 + t) * 64 + lane64];
         part[((size_t)s * pn::CH + own_channel(cg, i)) * K + (c0 + ci) * 9 + t] = v;
