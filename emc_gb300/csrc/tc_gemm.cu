@@ -1001,27 +1001,43 @@ __global__ void __launch_bounds__(es::THREADS, 1)
 // L_ri = log w_r + c_i sum_p k_ip log s~_rp + K_i log(K_i / S_r) - K_i,
 // s~ = max(s, floor), K_i = c_i sum_p k_ip, S_r = sum_p s~_rp, phi = K_i / S_r
 // (known intensity: phi = 1, L = log w_r + c_i sum k log s~ - S_r), as the
-// FP32 path.  One contraction K . (log S~)^T with log S~ as FP16 hi + lo;
-// one CTA owns 128 patterns x 256 rotations (TMEM columns 0-255) and writes
-// one (max, sum exp) partial per 128-rotation half.
+// FP32 path.  One contraction K . (log S~)^T with log S~ as FP16 hi + lo, over the
+// pattern tile's 64-pixel blocks with counts (the others' products are zero).
+// Persistent: a CTA (pair) takes tiles first, first + grid, ..; the stage ring runs
+// on across tiles and the accumulator is double-buffered in TMEM, so that a tile's
+// epilogue -- 256 columns of logarithms, exponentials and stores -- overlaps the
+// next one's MMAs.  Bound by the tensor pipe in pairs (48 KB per CTA and 64 pixels,
+// 47 B/clk), by L2 reads in single CTAs (80 KB for the same time).  Each 128-rotation
+// half of a tile leaves one (max, sum exp) partial.  All blocks, single CTAs of 32
+// pixels a stage and no overlap before: 112^3, 10,860 rotations, 10,000 patterns
+// 3,210 us, now 943; 128^3 pruned 2,428, now 1,124.
 namespace ep {
-constexpr int BM = 128;   // patterns per tile (TMEM lanes)
-constexpr int BN = 256;   // rotations per tile
-constexpr int BK = 32;    // pixels per stage (64 B rows, 64B swizzle)
-constexpr int STAGES = 4;
-constexpr int A_BYTES = BM * BK * 2;  // 8 KB
-constexpr int B_BYTES = BN * BK * 2;  // 16 KB
-constexpr int STAGE_BYTES = A_BYTES + 2 * B_BYTES;
-constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 256 + 2 * BN * 4 + 1024;
-constexpr int EPI_WARPS = 8;  // two per TMEM lane quarter, one per 128-column half
+constexpr int BM = 128;  // patterns per CTA (TMEM lanes)
+constexpr int BN = 256;  // rotations per tile
+constexpr int BK = 64;   // pixels per block
+constexpr int EPI_WARPS = 16;  // four per TMEM lane quarter, 64 columns each
 constexpr int THREADS = 64 + 32 * EPI_WARPS;
+// A pair (256 patterns x 256 rotations, each CTA half of the log-slices) takes a
+// block per stage; a single CTA half a block, so that more of them are in flight.
+template <bool PAIR>
+struct Ring {
+  static constexpr int kPix = PAIR ? 64 : 32;  // 128 B rows, 128B swizzle; 64 B, 64B
+  static constexpr int kA = BM * kPix * 2, kB = (PAIR ? BN / 2 : BN) * kPix * 2;
+  static constexpr int kStage = kA + 2 * kB;
+  static constexpr int kStages = PAIR ? 4 : 5;
+  // barriers, two rows of BN floats, the (max, sum exp) of the odd column parts
+  static constexpr int kSmem = kStages * kStage + 256 + 2 * BN * 4 + 2 * BM * 8 + 1024;
+  static_assert(kSmem <= 232448, "shared memory of the true-Poisson likelihood");
+};
 }  // namespace ep
 
 struct TcEstepPoisArgs {
-  int N, R, n_pt, n_rt, nkb;
+  int N, R, n_pt, n_rt, nkb;  // n_pt: pattern tiles (pairs of tiles)
   int raster;             // tile order (raster_tile)
-  int tile0;              // CTA b runs tile tile0 + b of the order
-  const int2* tiles;      // pruned iteration: (pattern tile, 256-rotation tile) per CTA
+  int tile0, n_tiles;     // the tiles tile0 .. + n_tiles of the order
+  const int2* tiles;      // pruned iteration: n_tiles of (pattern tile, 256-rotation tile)
+  const uint32_t* list;   // [n_pt][nkb] blocks with counts << 8, ascending
+  const int* list_n;      // at least one
   int n_part;             // 128-rotation partial tiles
   const float* rot_ssum;  // S_r
   const float* rotw;
@@ -1035,154 +1051,266 @@ struct TcEstepPoisArgs {
   uint32_t spin;  // polls per pipeline wait
 };
 
+template <bool PAIR>
 __global__ void __launch_bounds__(ep::THREADS, 1)
     tc_estep_pois_kernel(const __grid_constant__ CUtensorMap mK,
                          const __grid_constant__ CUtensorMap mLh,
                          const __grid_constant__ CUtensorMap mLl, TcEstepPoisArgs a) {
   using namespace ep;
+  using Rg = Ring<PAIR>;
+  constexpr int STAGES = Rg::kStages, STAGE_BYTES = Rg::kStage;
+  constexpr int SUB = BK / Rg::kPix;  // stages per block
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + STAGES * STAGE_BYTES);
   uint64_t* empty = full + STAGES;
-  uint64_t* accum = empty + STAGES;
-  uint64_t* drain = accum + 1;  // the MMA issuer's own completion wait before TMEM is freed
+  uint64_t* tfull = empty + STAGES;  // [2] accumulator ready
+  uint64_t* tempty = tfull + 2;      // [2] (rank 0) accumulator drained
+  uint64_t* drain = tempty + 2;  // the MMA issuer's own completion wait before TMEM is freed
   uint32_t* tmem_slot = (uint32_t*)(drain + 1);
   float* s_ss = (float*)(smem + STAGES * STAGE_BYTES + 256);
   float* s_lw = s_ss + BN;
+  float2* s_half = (float2*)(s_lw + BN);  // [2][BM]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  int pt, rt;
-  if (a.tiles) {  // pruned: the listed tiles only
-    const int2 t = a.tiles[blockIdx.x];
-    pt = t.x;
-    rt = t.y;
-  } else {
-    raster_tile(blockIdx.x + a.tile0, a.raster, a.n_pt, a.n_rt, pt, rt);
-  }
-  const int n0 = pt * BM, r0 = rt * BN;
+  const uint32_t rank = PAIR ? ptx::cluster_ctarank() : 0u;
+  const int first = (int)(PAIR ? blockIdx.x >> 1 : blockIdx.x);
+  const int step = (int)(PAIR ? gridDim.x >> 1 : gridDim.x);
+  auto tile = [&](int t, int& pt, int& rt) {
+    if (!PAIR && a.tiles) {  // pruned: the listed tiles only
+      const int2 v = __ldg(a.tiles + t);
+      pt = v.x;
+      rt = v.y;
+    } else {
+      raster_tile(t + a.tile0, a.raster, a.n_pt, a.n_rt, pt, rt);
+    }
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
       ptx::mbar_init(&full[s], 1);
       ptx::mbar_init(&empty[s], 1);
     }
-    ptx::mbar_init(accum, 1);
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(&tfull[b], 1);
+      ptx::mbar_init(&tempty[b], (PAIR ? 2 : 1) * EPI_WARPS);
+    }
     ptx::mbar_init(drain, 1);
     ptx::fence_mbar_init();
   }
-  for (int c = threadIdx.x; c < BN; c += blockDim.x) {
-    const int r = r0 + c;
-    s_ss[c] = r < a.R ? a.rot_ssum[r] : 1.0f;
-    s_lw[c] = r < a.R ? logf(a.rotw[r]) : 0.0f;
-  }
   if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, BN);
-    ptx::tmem_relinquish();
+    if (PAIR) {
+      ptx::tmem_alloc_pair(tmem_slot, 512);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(tmem_slot, 512);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if (PAIR) ptx::cluster_sync();  // both CTAs' barriers initialised and TMEM allocated
   ptx::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
   if (warp == 0) {
-    // ------------------------------------------------ TMA producer
+    // ------------------------------------------------ TMA producer (both CTAs of a pair)
     if (ptx::elect_one()) {
-      int kb = 0;
-      for (; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 8, a.spin)) break;
-        ptx::mbar_arrive_expect_tx(&full[s], STAGE_BYTES);
-        unsigned char* st = smem + s * STAGE_BYTES;
-        ptx::tma_load_2d(st, &mK, kb * BK, n0, &full[s]);
-        ptx::tma_load_2d(st + A_BYTES, &mLh, kb * BK, r0, &full[s]);
-        ptx::tma_load_2d(st + A_BYTES + B_BYTES, &mLl, kb * BK, r0, &full[s]);
+      const uint32_t full0 = ptx::smem_u32(full);
+      const uint32_t fb0 = PAIR ? ptx::mapa_shared(full0, 0) : full0;
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = first; t < a.n_tiles && ok; t += step) {
+        int pt, rt;
+        tile(t, pt, rt);
+        // a pair's second pattern tile may be past the last (zeros)
+        const int n0 = (PAIR ? 2 * pt + (int)rank : pt) * BM;
+        const int r0 = rt * BN + (PAIR ? BN / 2 * (int)rank : 0);
+        const uint32_t* list = a.list + (size_t)pt * a.nkb;
+        const int cnt = a.list_n[pt];
+        uint32_t next = __ldg(list);
+        for (int u = 0; u < cnt * SUB; ++u, ++it) {
+          const int x = (int)(next >> 8) * BK + (u % SUB) * Rg::kPix;
+          if (u % SUB == SUB - 1 && u + 1 < cnt * SUB) next = __ldg(list + u / SUB + 1);
+          const uint32_t s = it % STAGES;
+          if (!ptx::mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, a.status, 8, a.spin)) {
+            ok = false;
+            break;
+          }
+          // rank 0's barriers count both CTAs' bytes
+          if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], STAGE_BYTES * (PAIR ? 2 : 1));
+          unsigned char* st = smem + s * STAGE_BYTES;
+          if (PAIR) {
+            ptx::tma_load_2d_pair(st, &mK, x, n0, fb0 + 8 * s);
+            ptx::tma_load_2d_pair(st + Rg::kA, &mLh, x, r0, fb0 + 8 * s);
+            ptx::tma_load_2d_pair(st + Rg::kA + Rg::kB, &mLl, x, r0, fb0 + 8 * s);
+          } else {
+            ptx::tma_load_2d(st, &mK, x, n0, fb0 + 8 * s);
+            ptx::tma_load_2d(st + Rg::kA, &mLh, x, r0, fb0 + 8 * s);
+            ptx::tma_load_2d(st + Rg::kA + Rg::kB, &mLl, x, r0, fb0 + 8 * s);
+          }
+        }
       }
-      ptx::drain_loads(full, STAGES, (uint32_t)kb, a.status, 11);  // none in flight at exit
+      if (rank == 0) ptx::drain_loads(full, STAGES, it, a.status, 11);  // none in flight at exit
     }
   } else if (warp == 1) {
-    // ------------------------------------------------ MMA issuer
-    if (ptx::elect_one()) {
-      constexpr uint32_t idesc = ptx::idesc_f16(BM, BN);
-      for (int kb = 0; kb < a.nkb; ++kb) {
-        const int s = kb % STAGES;
-        const uint32_t ph = (kb / STAGES) & 1;
-        if (!ptx::mbar_wait(&full[s], ph, a.status, 9, a.spin)) break;
+    // ------------------------------------------------ MMA issuer (rank 0 of a pair)
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::idesc_f16(PAIR ? 2 * BM : BM, BN);
+      uint32_t it = 0;
+      bool ok = true;
+      int j = 0;
+      for (int t = first; t < a.n_tiles && ok; t += step, ++j) {
+        const int b = j & 1;
+        const uint32_t d = tmem + (uint32_t)(b * BN);
+        int pt, rt;
+        tile(t, pt, rt);
+        const int n = a.list_n[pt] * SUB;
+        if (!ptx::mbar_wait_cluster(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin)) break;
         ptx::tc_fence_after();
-        const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
+        for (int u = 0; u < n; ++u, ++it) {
+          const uint32_t s = it % STAGES;
+          if (!ptx::mbar_wait(&full[s], (it / STAGES) & 1, a.status, 9, a.spin)) {
+            ok = false;
+            break;
+          }
+          ptx::tc_fence_after();
+          const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
 #pragma unroll
-        for (int ks = 0; ks < BK / 16; ++ks) {
-          const uint64_t aK = ptx::smem_desc(base + ks * 32, 512, 4);
-          const uint64_t bh = ptx::smem_desc(base + A_BYTES + ks * 32, 512, 4);
-          const uint64_t bl = ptx::smem_desc(base + A_BYTES + B_BYTES + ks * 32, 512, 4);
-          ptx::mma_f16(tmem, aK, bh, idesc, (kb | ks) ? 1u : 0u);
-          ptx::mma_f16(tmem, aK, bl, idesc, 1u);
+          for (int ks = 0; ks < Rg::kPix / 16; ++ks) {
+            constexpr int sbo = PAIR ? 1024 : 512, sw = PAIR ? 2 : 4;
+            const uint64_t aK = ptx::smem_desc(base + ks * 32, sbo, sw);
+            const uint64_t bh = ptx::smem_desc(base + Rg::kA + ks * 32, sbo, sw);
+            const uint64_t bl = ptx::smem_desc(base + Rg::kA + Rg::kB + ks * 32, sbo, sw);
+            if (PAIR) {
+              ptx::mma_f16_pair(d, aK, bh, idesc, (u | ks) ? 1u : 0u);
+              ptx::mma_f16_pair(d, aK, bl, idesc, 1u);
+            } else {
+              ptx::mma_f16(d, aK, bh, idesc, (u | ks) ? 1u : 0u);
+              ptx::mma_f16(d, aK, bl, idesc, 1u);
+            }
+          }
+          if (PAIR)
+            ptx::mma_commit_pair(&empty[s], 0x3);
+          else
+            ptx::mma_commit(&empty[s]);
         }
-        ptx::mma_commit(&empty[s]);
+        if (PAIR)
+          ptx::mma_commit_pair(&tfull[b], 0x3);
+        else
+          ptx::mma_commit(&tfull[b]);
       }
-      ptx::mma_commit(accum);
-      ptx::mma_commit(drain);  // TMEM is freed only after these MMAs have completed
+      if (PAIR)
+        ptx::mma_commit_pair(drain, 0x1);  // both CTAs' TMEM is written by these MMAs
+      else
+        ptx::mma_commit(drain);
       ptx::mbar_wait(drain, 0, a.status, 12);
     }
   } else {
-    // ------------------------------------------------ epilogue (warps 2-9)
-    const int quarter = warp & 3;
+    // ------------------------------------------------ epilogue
+    const int quarter = warp & 3;      // TMEM lanes this warp may access
+    const int part = (warp - 2) >> 2;  // which of the tile's columns
     const int row = quarter * 32 + lane;
-    const int n = n0 + row;
-    const bool nok = n < a.N;
-    const float ci = nok ? a.cnorm[n] : 1.0f;
-    const float Ki = nok ? a.Ksum[n] : 0.0f;
-    const bool waited = ptx::mbar_wait_sleep(accum, 0, a.status, 10, 256, a.spin);
-    if (waited) ptx::tc_fence_after();
-    const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
-    {
-      const int h = (warp - 2) >> 2;  // the 128-rotation half this warp evaluates
+    const int c_beg = part * (BN / 4), c_end = c_beg + BN / 4;
+    bool ok = true;
+    int j = 0;
+    for (int t = first; t < a.n_tiles; t += step, ++j) {
+      const int b = j & 1;
+      int pt, rt;
+      tile(t, pt, rt);
+      const int n = (PAIR ? 2 * pt + (int)rank : pt) * BM + row, r0 = rt * BN;
+      const bool nok = n < a.N;
+      const float ci = nok ? a.cnorm[n] : 1.0f;
+      const float Ki = nok ? a.Ksum[n] : 0.0f;
+      const int e = (int)threadIdx.x - 64;
+      if (e < BN) {  // the last tile's readers have passed its second barrier
+        const int r = r0 + e;
+        s_ss[e] = r < a.R ? a.rot_ssum[r] : 1.0f;
+        s_lw[e] = r < a.R ? logf(a.rotw[r]) : 0.0f;
+      }
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+      // after a wait that gave up the warp only keeps the other warps' barriers going
+      ok = ok && ptx::mbar_wait_sleep(&tfull[b], (j >> 1) & 1, a.status, 10, 128, a.spin);
       float m = -INFINITY, ssum = 0.0f;
-      for (int c0 = h * 128; waited && c0 < h * 128 + 128; c0 += 16) {
-        float v[16];
-        ptx::tmem_ld16(lane_addr + c0, v);
-        ptx::tmem_wait_ld();
+      if (ok) {
+        ptx::tc_fence_after();
+        const uint32_t col = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * BN);
+        constexpr int CG = 8;
+        for (int c0 = c_beg; c0 < c_end; c0 += CG) {
+          float v[CG];
+          ptx::tmem_ld8(col + c0, v);
+          ptx::tmem_wait_ld();
+          const int jn = nok ? min(CG, a.R - (r0 + c0)) : 0;  // columns that are pairs
+          float* Lp = a.L + (size_t)(r0 + c0) * a.N + n;
+          float* Pp = a.PHI + (size_t)(r0 + c0) * a.N + n;
+          float mx = m;
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int cl = c0 + j;
-          const int r = r0 + cl;
-          const float acc = ci * v[j];
-          float l, f;
-          if (a.known_intensity) {
-            f = 1.0f;
-            l = s_lw[cl] + acc - s_ss[cl];
-          } else if (Ki > 0.0f) {
-            f = Ki / s_ss[cl];
-            l = s_lw[cl] + acc + Ki * logf(f) - Ki;
-          } else {
-            f = 0.0f;
-            l = s_lw[cl];
+          for (int i = 0; i < CG; ++i) {
+            const float acc = ci * v[i], lw = s_lw[c0 + i], Sr = s_ss[c0 + i];
+            float l, f;
+            if (a.known_intensity) {
+              f = 1.0f;
+              l = lw + acc - Sr;
+            } else if (Ki > 0.0f) {
+              f = Ki / Sr;
+              l = lw + acc + Ki * logf(f) - Ki;
+            } else {
+              f = 0.0f;
+              l = lw;
+            }
+            if (i < jn) {
+              *Lp = l;
+              *Pp = f;
+            } else {
+              l = -INFINITY;
+            }
+            Lp += a.N;
+            Pp += a.N;
+            v[i] = l;
+            mx = fmaxf(mx, l);
           }
-          const bool ok = nok && r < a.R;
-          if (ok) {
-            a.L[(size_t)r * a.N + n] = l;
-            a.PHI[(size_t)r * a.N + n] = f;
-          }
-          const float L = ok ? l : -INFINITY;
-          if (L > m) {
-            ssum = ssum * expf(m - L) + 1.0f;
-            m = L;
-          } else if (L > -INFINITY) {
-            ssum += expf(L - m);
+          if (mx > -INFINITY) {
+            float s = 0.0f;
+#pragma unroll
+            for (int i = 0; i < CG; ++i) s += expf(v[i] - mx);
+            ssum = ssum * expf(m - mx) + s;
+            m = mx;
           }
         }
       }
-      const int t = 2 * rt + h;
-      if (nok && t < a.n_part) a.part[(size_t)t * a.N + n] = make_float2(m, ssum);
+      // this warp's reads of buffer b are complete: hand it back to the MMA warp
+      ptx::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) {
+        if (PAIR && rank != 0)
+          ptx::mbar_arrive_cluster(ptx::mapa_shared(ptx::smem_u32(&tempty[b]), 0));
+        else
+          ptx::mbar_arrive(&tempty[b]);
+      }
+      // one partial per 128-rotation half: parts 0 and 1, 2 and 3
+      if (part & 1) s_half[(part >> 1) * BM + row] = make_float2(m, ssum);
+      asm volatile("bar.sync 1, %0;" ::"n"(EPI_WARPS * 32) : "memory");
+      const int tp = 2 * rt + (part >> 1);
+      if (!(part & 1) && nok && tp < a.n_part) {
+        const float2 o = s_half[(part >> 1) * BM + row];
+        const float M = fmaxf(m, o.x);
+        float S = 0.0f;
+        if (M > -INFINITY) S = ssum * expf(m - M) + o.y * expf(o.x - M);
+        a.part[(size_t)tp * a.N + n] = make_float2(M, S);
+      }
     }
   }
   ptx::tc_fence_before();
   __syncthreads();
+  if (PAIR) ptx::cluster_sync();  // the pair's MMAs and barrier traffic are over in both CTAs
   if (threadIdx.x == 32) ptx::settle_after_timeout(a.status);
   __syncthreads();
   if (warp == 1) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc(tmem, BN);
+    if (PAIR)
+      ptx::tmem_dealloc_pair(tmem, 512);
+    else
+      ptx::tmem_dealloc(tmem, 512);
   }
 }
 
@@ -1768,7 +1896,8 @@ struct TcState {
   CUtensorMap mK, mJ, mJl, mQh, mQl, mKt;
   CUtensorMap mKt128;  // K^T in 128-row boxes (pair M-step halves)
   CUtensorMap mMS, mHh, mHl, mIv, mTv;  // rotation operands: 64-row boxes
-  CUtensorMap mLh, mLl;  // true Poisson: log-slices hi / lo, 256-row boxes
+  CUtensorMap mLh, mLl;  // true Poisson, single CTAs: log-slices hi / lo, 256 rows x 32
+  CUtensorMap mK64, mLh64, mLl64;  // and pairs: 128 rows x 64
   __half *MS, *Hh, *Hl, *Iv, *Tv, *Lh, *Ll;
   int* status;
 };
@@ -1842,6 +1971,9 @@ int tc_bind(emc_plan* p) {
       if (!rc) rc = make_map(ctx, &st->mK, p->Kh, Np, Kp, 128, 32);
       if (!rc) rc = make_map(ctx, &st->mLh, st->Lh, Rp, Kp, 256, 32);
       if (!rc) rc = make_map(ctx, &st->mLl, st->Ll, Rp, Kp, 256, 32);
+      if (!rc) rc = make_map(ctx, &st->mK64, p->Kh, Np, Kp, 128, 64);
+      if (!rc) rc = make_map(ctx, &st->mLh64, st->Lh, Rp, Kp, 128, 64);
+      if (!rc) rc = make_map(ctx, &st->mLl64, st->Ll, Rp, Kp, 128, 64);
     } else {
       if (!rc) rc = make_map(ctx, &st->mK, p->Kh, Np, Kp, 128, 64);
       if (!rc) rc = make_map(ctx, &st->mJ, p->Jh, Np, Kp, 128, 64);
@@ -1859,8 +1991,12 @@ int tc_bind(emc_plan* p) {
     EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel<true>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        es::SMEM_BYTES));
-    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pois_kernel,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, ep::SMEM_BYTES));
+    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pois_kernel<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       ep::Ring<false>::kSmem));
+    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pois_kernel<true>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       ep::Ring<true>::kSmem));
     EMC_CUDA(ctx, cudaFuncSetAttribute(tc_mstep_kernel<0>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        MsRing<0>::kSmem));
@@ -1936,16 +2072,36 @@ int tc_ensure_qlo(emc_plan* p) {
   return make_map(ctx, &state(p)->mQl, p->Ql, p->Rp, p->Np, 128, 64);
 }
 
-// The likelihood kernels over tiles [first, first + count) of the full
+// A kernel on clusters of two CTAs.
+template <typename... P, typename... A>
+static cudaError_t launch_pairs(emc_ctx* ctx, void (*kernel)(P...), int pairs, int threads, int smem,
+                                const A&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * pairs);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+// The true-Poisson likelihood over tiles [first, first + count) of the full
 // (pattern tile, rotation tile) grid in the order `raster`, or over the plan's
-// pruned tile list (full == false and a list exists; first/count ignored).
+// pruned tile list (full == false and a list exists; first/count ignored).  Full
+// scans run on CTA pairs unless those are switched off: half the reads of the
+// log-slices per pattern; the pruned lists name single pattern tiles.
 static int estep_pois_launch(emc_plan* p, int raster, int first, int count, bool full) {
   emc_ctx* ctx = p->ctx;
   TcState* st = state(p);
   TcEstepPoisArgs a;
   a.N = p->d.n_images;
   a.R = p->d.n_rot;
-  a.n_pt = p->Np / ep::BM;
   a.n_rt = ceil_div(p->Rp, ep::BN);
   a.nkb = p->Kp / ep::BK;
   a.raster = raster;
@@ -1961,13 +2117,35 @@ static int estep_pois_launch(emc_plan* p, int raster, int first, int count, bool
   a.part = p->part;
   a.status = st->status;
   a.spin = p->debug_spin ? p->debug_spin : ptx::kSpinLimit;
+  const int n_pt = p->Np / ep::BM;
+  if (p->estep_pair && !a.tiles) {
+    a.n_pt = (n_pt + 1) / 2;
+    a.list = p->pp_list;
+    a.list_n = p->pp_n;
+    const int total = a.n_pt * a.n_rt;
+    a.tile0 = std::max(0, std::min(first, total));
+    a.n_tiles = std::min(total - a.tile0, count);
+    if (a.n_tiles == 0) return EMC_OK;
+    const cudaError_t e =
+        launch_pairs(ctx, tc_estep_pois_kernel<true>, std::min(a.n_tiles, ctx->sm_count / 2),
+                     ep::THREADS, ep::Ring<true>::kSmem, st->mK64, st->mLh64, st->mLl64, a);
+    if (e == cudaSuccess) return after_launch(ctx, "tc_estep_pois_kernel (pairs)");
+    // as in estep_launch: no pairs on this device, single CTAs from now on
+    (void)cudaGetLastError();
+    p->estep_pair = 0;
+    first *= 2;
+    count = count > INT_MAX / 2 ? INT_MAX : 2 * count;
+  }
+  a.n_pt = n_pt;
+  a.list = p->pt_list;
+  a.list_n = p->pt_n;
   const int total = a.n_pt * a.n_rt;
-  first = a.tiles ? 0 : std::max(0, std::min(first, total));
-  const int grid = a.tiles ? p->prune_n_tiles : std::min(total - first, count);
-  a.tile0 = first;
-  if (grid == 0) return EMC_OK;
-  tc_estep_pois_kernel<<<grid, ep::THREADS, ep::SMEM_BYTES, ctx->stream>>>(st->mK, st->mLh,
-                                                                           st->mLl, a);
+  a.tile0 = a.tiles ? 0 : std::max(0, std::min(first, total));
+  a.n_tiles = a.tiles ? p->prune_n_tiles : std::min(total - a.tile0, count);
+  if (a.n_tiles == 0) return EMC_OK;
+  tc_estep_pois_kernel<false>
+      <<<std::min(a.n_tiles, ctx->sm_count), ep::THREADS, ep::Ring<false>::kSmem, ctx->stream>>>(
+          st->mK, st->mLh, st->mLl, a);
   return after_launch(ctx, "tc_estep_pois_kernel");
 }
 
@@ -2018,20 +2196,9 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     const int pairs = std::min(total - first, count);
     a.tile0 = first;
     if (pairs == 0) return EMC_OK;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * pairs);
-    cfg.blockDim = dim3(es::THREADS);
-    cfg.dynamicSmemBytes = es::SMEM_BYTES;
-    cfg.stream = ctx->stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, tc_estep_kernel<true>, st->mK, st->mJ, st->mJl,
-                                             st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
+    const cudaError_t e =
+        launch_pairs(ctx, tc_estep_kernel<true>, pairs, es::THREADS, es::SMEM_BYTES, st->mK, st->mJ,
+                     st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
     if (e == cudaSuccess) return after_launch(ctx, "tc_estep_kernel (pairs)");
     // a refused launch configuration (a GPU or partition that cannot
     // co-schedule the pairs) is not a sticky error: single CTAs from now on
@@ -2080,11 +2247,6 @@ RotOps tc_rot_ops(emc_plan* p) {
   return o;
 }
 
-// Full scans of the reference likelihood run on CTA pairs unless switched off.
-static bool estep_uses_pair(const emc_plan* p) {
-  return p->estep_pair && p->d.diff != EMC_DIFF_TRUE_POISSON;
-}
-
 // One timed launch of the likelihood kernel over tiles [first, first + count)
 // of the order `raster` (CUDA events on the plan's stream; synchronises).  The
 // rotation operands are those of the last expansion.
@@ -2109,8 +2271,8 @@ int tc_time_estep(emc_plan* p, int raster, int first, int count, float* ms) {
 // CTA-pair tiles for the pair kernel.
 int tc_estep_tiles(emc_plan* p) {
   const int n_pt = p->Np / 128;
-  if (p->d.diff == EMC_DIFF_TRUE_POISSON) return n_pt * ceil_div(p->Rp, ep::BN);
-  return (estep_uses_pair(p) ? (n_pt + 1) / 2 : n_pt) * (p->Rp / es::BN);
+  return (p->estep_pair ? (n_pt + 1) / 2 : n_pt) *
+         (p->d.diff == EMC_DIFF_TRUE_POISSON ? ceil_div(p->Rp, ep::BN) : p->Rp / es::BN);
 }
 
 // Raster autotuner.  The likelihood kernel streams two operand panels per
@@ -2131,7 +2293,7 @@ int tc_autotune(emc_plan* p, int waves, int* best, float* best_ms) {
   emc_ctx* ctx = p->ctx;
   int rc = EMC_OK;
   const bool pois = p->d.diff == EMC_DIFF_TRUE_POISSON;
-  const bool pair = !pois && estep_uses_pair(p);
+  const bool pair = p->estep_pair != 0;
   const int n_pt = pair ? (p->Np / 128 + 1) / 2 : p->Np / 128;
   const int n_rt = pois ? ceil_div(p->Rp, ep::BN) : p->Rp / es::BN;
   const int total = n_pt * n_rt;

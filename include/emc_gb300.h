@@ -462,8 +462,8 @@ int emc_batch_destroy(emc_batch* batch);
  * running through all rotation tiles.  |g| <= 4096.  Results do not depend on
  * it; L2 reuse of the operand panels does. */
 #define EMC_OPT_ESTEP_RASTER 6
-/* EMC_OPT_ESTEP_PAIR: 1 (default) runs full scans of the reference
- * likelihood on clusters of two CTAs with 256-row MMAs (each CTA stores half
+/* EMC_OPT_ESTEP_PAIR: 1 (default) runs full scans of the tensor-core
+ * likelihoods on clusters of two CTAs with 256-row MMAs (each CTA stores half
  * of the rotation-side operands); 0 runs every scan on single CTAs.
  * emc_plan_autotune may switch it off where single CTAs are faster.  Pruned
  * iterations always use single CTAs.  The log-likelihoods agree to FP32
