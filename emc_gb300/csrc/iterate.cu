@@ -28,6 +28,7 @@
 #include <cstring>
 #include <vector>
 
+#include <cooperative_groups.h>
 #include <cuda_fp16.h>
 
 #include "geometry.cuh"
@@ -813,6 +814,8 @@ __global__ void __launch_bounds__(TPB, 1) estep_pois_fp32_kernel(EstepArgs a) {
 }
 
 // ------------------------------------------------------- normalise -------
+constexpr float kLog2E = 1.4426950408889634f;
+
 // Per pattern, over the rotation tiles' (max, sum exp) pairs: M = the largest max
 // and s = sum_t s_t exp(m_t - M), FP64.  A block takes 32 patterns; its eight
 // warps share the tiles (one thread per pattern left a small problem on a few
@@ -846,13 +849,35 @@ __device__ __forceinline__ void lse_tiles(const float2* __restrict__ part, int n
     for (int w = 0; w < kLseWarps; ++w) s += ss[w][lane];
 }
 
-// lse_i = M + log(s), FP64, also as two floats hi + lo (hi = fl(lse), lo =
-// fl(lse - hi)) so that consumers form L - lse in FP32 to the same accuracy.
+// A pattern's lse in the forms its consumers read: FP64; two floats hi + lo (hi =
+// fl(lse), lo = fl(lse - hi)), so that L - lse is formed in FP32 to the same accuracy;
+// and in four copies, copy h from pattern h on, hi and -lo log2(e) in arrays of their
+// own: the rows [R][N] of the likelihood start at any 4-byte boundary, and reading
+// them by 16 bytes, mprep_hi_kernel finds their lse by 16 bytes as well.
+struct LseOut {
+  double* lse;
+  float2* lse2;
+  float* shifted;  // [4][2][ld]
+  int ld;
+  __device__ __forceinline__ void store(int n, double l) const {
+    const bool ok = isfinite(l);
+    const float hi = (float)l, lo = ok ? (float)(l - (double)hi) : 0.0f;
+    lse[n] = l;
+    lse2[n] = make_float2(hi, lo);
+#pragma unroll
+    for (int h = 0; h < 4; ++h)
+      if (n >= h) {
+        shifted[(size_t)(2 * h) * ld + n - h] = ok ? hi : INFINITY;  // P = 0
+        shifted[(size_t)(2 * h + 1) * ld + n - h] = -lo * kLog2E;
+      }
+  }
+};
+
+// lse_i = M + log(s), FP64.
 // Patterns with no valid pair get lse = +inf (all responsibilities 0).
 // ll_part[block] = the sum of the block's finite lse.
 __global__ void __launch_bounds__(32 * kLseWarps) lse_combine_kernel(
-    const float2* __restrict__ part, int n_rt, int N, double* __restrict__ lse,
-    float2* __restrict__ lse2, double* __restrict__ ll_part) {
+    const float2* __restrict__ part, int n_rt, int N, LseOut out, double* __restrict__ ll_part) {
   const int n = blockIdx.x * 32 + (threadIdx.x & 31);
   float M;
   double s;
@@ -861,9 +886,7 @@ __global__ void __launch_bounds__(32 * kLseWarps) lse_combine_kernel(
   double l = INFINITY;
   if (n < N) {
     if (M > -INFINITY) l = (double)M + log(s);
-    lse[n] = l;
-    const float hi = (float)l;
-    lse2[n] = make_float2(hi, isfinite(l) ? (float)(l - (double)hi) : 0.0f);
+    out.store(n, l);
   }
   double t = isfinite(l) ? l : 0.0;
 #pragma unroll
@@ -888,170 +911,329 @@ __global__ void __launch_bounds__(1024) finite_sum_kernel(const double* __restri
   if (threadIdx.x == 0) out[0] = s;
 }
 
-// One block per rotation row: P = exp(L - lse) (in place), Q = P / phi,
-// T_r = sum_i P, the row's captured mass and the inserted-mass bound
-// sum_i Q_ri K_i.  Element math is FP32 (L - lse with lse as float hi + lo,
-// since FP64 arithmetic is scarce on this GPU); per-thread sums are FP32 and
-// the block sums FP64.
-//   FP32 M-step: Q [R][ldq] (zero padded).
-//   Tensor M-step (Qh != nullptr): Q' = P c_i / phi (phi holds c_i num/den,
-//   the tensor M-step multiplies raw counts) as FP16 hi [R][ldq] (and lo,
-//   when Ql != nullptr), each row scaled by 2^e_r so its largest entry sits
-//   near 2^14 (qscale_r = 2^-e_r); with stage, the row is kept in shared
-//   memory between the two passes, else the second pass re-reads it.
-constexpr int kMprepThreads = 512;  // two blocks per SM (at most 64 registers per thread)
-constexpr int kMprepStageMax = 30720;  // patterns whose row of Q fits shared memory (120 KB)
+// ---- responsibilities -> M-step operand --------------------------------
+// One block per rotation row: P = exp(L - lse), Q = P / phi, T_r = sum_i P, the
+// row's captured mass and the inserted-mass bound sum_i Q_ri K_i.  Element math is
+// FP32 (L - lse with lse as float hi + lo, since FP64 arithmetic is scarce on this
+// GPU); per-thread sums are FP32 and the block sums FP64.
 
-__global__ void __launch_bounds__(kMprepThreads, 2) mprep_kernel(
-    float* __restrict__ L, const float* __restrict__ PHI, const float2* __restrict__ lse2,
-    const float* __restrict__ Ksum, const float* __restrict__ cnorm, int R, int N,
-    float* __restrict__ Q, __half* __restrict__ Qh, __half* __restrict__ Ql,
-    float* __restrict__ qscale, int ldq, float* __restrict__ T, double* __restrict__ row_mass,
-    double* __restrict__ row_bound, int stage, const unsigned char* __restrict__ tstate,
-    int n_rt, double* __restrict__ row_margin, int write_p) {
-  extern __shared__ float qrow[];  // [N] when stage: the row's P c_i / phi
-  const int r = blockIdx.x;
-  // pruned iteration: tstate[pattern tile][rotation tile] = 0 not evaluated
-  // (P = 0), 1 evaluated, 2 evaluated margin tile (its mass is summed)
-  const unsigned char* ts = tstate ? tstate + (r >> 7) : nullptr;
-  float t = 0.0f, b = 0.0f, qmax = 0.0f, mg = 0.0f;
-  const bool fast = Qh != nullptr && Ql == nullptr;  // M-step operand FP16 hi only
-  // one element: P = exp(L - lse) (0 outside the evaluated tiles), q = P / phi
-  // (x c_i for the FP16 operand); returns q and stores P
-  auto elem = [&](int i, int st, float l, float f, float2 li, float ks, float cn) -> float {
-    float P = 0.0f;
-    if (st) {
-      // an M-step operand of FP16 hi only takes P through an 11-bit rounding:
-      // the hardware exponential (2^-21 relative) serves it; Q hi + lo and the
-      // FP32 path keep expf
-      if (isfinite(li.x) && l > -INFINITY) {
-        const float x = (l - li.x) - li.y;
-        P = fast ? __expf(x) : expf(x);
-      }
-      if (st == 2) mg += P;
-    } else {
-      f = 0.0f;
-    }
-    // q = P / phi correctly rounded, except for an FP16 hi-only operand, which
-    // a 2-ulp quotient changes at most in rare ties of its rounding
-    float q = f > 0.0f ? (fast ? __fdividef(P, f) : __fdiv_rn(P, f)) : 0.0f;
-    t += P;
-    b = __fmaf_rn(q, ks, b);
-    if (Qh) q = __fmul_rn(q, cn);
-    qmax = fmaxf(qmax, q);
-    if (Q) Q[(size_t)r * ldq + i] = q;
-    if (stage) qrow[i] = q;
-    return P;
-  };
-  if ((N & 3) == 0) {
-    // 16-byte rows: four elements per load keep enough bytes in flight to
-    // approach HBM bandwidth (4-tuples never straddle a 128-pattern tile)
-    float4* L4 = reinterpret_cast<float4*>(L + (size_t)r * N);
-    const float4* F4 = reinterpret_cast<const float4*>(PHI + (size_t)r * N);
-    const float4* S4 = reinterpret_cast<const float4*>(lse2);
-    const float4* K4 = reinterpret_cast<const float4*>(Ksum);
-    const float4* C4 = reinterpret_cast<const float4*>(cnorm);
-    // two 4-tuples per thread and pass (j and j + blockDim, in that order, as
-    // one tuple per pass would take them): both tuples' row loads are in
-    // flight together
-    const int n4 = N / 4, bd = (int)blockDim.x;
-    auto tuple = [&](int j, int st, const float4& l, const float4& f) {
-      const int i = 4 * j;
-      const float4 s01 = S4[2 * j], s23 = S4[2 * j + 1];
-      const float4 ks = __ldg(K4 + j), cn = __ldg(C4 + j);
-      float4 P;
-      P.x = elem(i, st, l.x, f.x, make_float2(s01.x, s01.y), ks.x, cn.x);
-      P.y = elem(i + 1, st, l.y, f.y, make_float2(s01.z, s01.w), ks.y, cn.y);
-      P.z = elem(i + 2, st, l.z, f.z, make_float2(s23.x, s23.y), ks.z, cn.z);
-      P.w = elem(i + 3, st, l.w, f.w, make_float2(s23.z, s23.w), ks.w, cn.w);
-      if (write_p) L4[j] = P;
-    };
-    const float4 z4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    for (int j = threadIdx.x; j < n4; j += 2 * bd) {
-      const int j2 = j + bd;
-      const bool two = j2 < n4;
-      const int st = ts ? ts[(size_t)((4 * j) >> 7) * n_rt] : 1;
-      const int st2 = two ? (ts ? ts[(size_t)((4 * j2) >> 7) * n_rt] : 1) : 0;
-      const float4 l = L4[j];
-      const float4 f = st ? F4[j] : z4;
-      const float4 l2 = two ? L4[j2] : z4;
-      const float4 f2 = st2 ? F4[j2] : z4;
-      tuple(j, st, l, f);
-      if (two) tuple(j2, st2, l2, f2);
-    }
-  } else {
-    for (int i = threadIdx.x; i < N; i += blockDim.x) {
-      const size_t e = (size_t)r * N + i;
-      const int st = ts ? ts[(size_t)(i >> 7) * n_rt] : 1;
-      const float l = L[e];
-      const float f = st ? PHI[e] : 0.0f;
-      const float P = elem(i, st, l, f, lse2[i], __ldg(Ksum + i), __ldg(cnorm + i));
-      if (write_p) L[e] = P;
-    }
-  }
-  if (Q)
-    for (int i = N + threadIdx.x; i < ldq; i += blockDim.x) Q[(size_t)r * ldq + i] = 0.0f;
-  // row sums and maximum: FP32 warp shuffles over the threads' FP32
-  // partials, then the 32 warp sums in FP64 on warp 0 -- a block tree over
-  // 1,024 shared FP64 slots took 28 KB of shared memory (one block per SM
-  // with the staged row) and ten block barriers, and FP64 shuffles in every
-  // warp cost more than they saved (FP64 runs at a small fraction of the
-  // FP32 rate on this GPU)
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float f0 = t, f1 = b, f2 = mg, rmx = qmax;
-  for (int o = 16; o > 0; o >>= 1) {
-    f0 += __shfl_down_sync(0xffffffffu, f0, o);
-    f1 += __shfl_down_sync(0xffffffffu, f1, o);
-    f2 += __shfl_down_sync(0xffffffffu, f2, o);
-    rmx = fmaxf(rmx, __shfl_down_sync(0xffffffffu, rmx, o));
-  }
-  double r0s = (double)f0, r1s = (double)f1, r2s = (double)f2;
-  __shared__ double wsum[3][kMprepThreads / 32];
-  __shared__ float wmax[kMprepThreads / 32];
+// Row sums (t, b, m) and maximum over the block, in thread 0 (mx in every thread):
+// FP32 warp shuffles over the threads' FP32 partials, then the warps' sums in FP64
+// on warp 0 (FP64 runs at a small fraction of the FP32 rate).
+__device__ __forceinline__ void row_sums(float t, float b, float m, float& mx, double& st,
+                                         double& sb, double& sm) {
+  __shared__ double wsum[3][32];
+  __shared__ float wmax[32];
   __shared__ float row_max;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (int)(blockDim.x >> 5);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    t += __shfl_down_sync(0xffffffffu, t, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+    m += __shfl_down_sync(0xffffffffu, m, o);
+    mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
+  }
   if (lane == 0) {
-    wsum[0][warp] = r0s;
-    wsum[1][warp] = r1s;
-    wsum[2][warp] = r2s;
-    wmax[warp] = rmx;
+    wsum[0][warp] = (double)t;
+    wsum[1][warp] = (double)b;
+    wsum[2][warp] = (double)m;
+    wmax[warp] = mx;
   }
   __syncthreads();
   if (warp == 0) {
-    const int nw = (int)(blockDim.x >> 5);
-    r0s = lane < nw ? wsum[0][lane] : 0.0;
-    r1s = lane < nw ? wsum[1][lane] : 0.0;
-    r2s = lane < nw ? wsum[2][lane] : 0.0;
-    rmx = lane < nw ? wmax[lane] : 0.0f;
+    st = lane < nw ? wsum[0][lane] : 0.0;
+    sb = lane < nw ? wsum[1][lane] : 0.0;
+    sm = lane < nw ? wsum[2][lane] : 0.0;
+    mx = lane < nw ? wmax[lane] : 0.0f;
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      r0s += __shfl_down_sync(0xffffffffu, r0s, o);
-      r1s += __shfl_down_sync(0xffffffffu, r1s, o);
-      r2s += __shfl_down_sync(0xffffffffu, r2s, o);
-      rmx = fmaxf(rmx, __shfl_down_sync(0xffffffffu, rmx, o));
+      st += __shfl_down_sync(0xffffffffu, st, o);
+      sb += __shfl_down_sync(0xffffffffu, sb, o);
+      sm += __shfl_down_sync(0xffffffffu, sm, o);
+      mx = fmaxf(mx, __shfl_down_sync(0xffffffffu, mx, o));
     }
-    if (lane == 0) {
-      T[r] = (float)r0s;
-      row_mass[r] = r0s;
-      row_bound[r] = r1s;
-      if (row_margin) row_margin[r] = r2s;
-      row_max = rmx;
+    if (lane == 0) row_max = mx;
+  }
+  __syncthreads();
+  mx = row_max;
+}
+
+// The power of two that brings a row whose largest entry is mx near 2^14.
+__device__ __forceinline__ int row_exponent(float mx) {
+  const int ex = mx > 0.0f ? 14 - ilogbf(mx) - 1 : 0;
+  return max(-100, min(100, ex));
+}
+
+struct MprepArgs {
+  float* L;
+  const float* PHI;
+  const float2* lse2;
+  const float* lse_shifted;  // LseOut, ld = ldq
+  const float* Ksum;   // null: no mass bound wanted
+  const float* cnorm;  // null: 1
+  int N, ldq, n_rt;
+  float* Q;            // FP32 M-step
+  __half *Qh, *Ql;     // tensor M-step
+  float* qscale;
+  float* T;
+  double *row_mass, *row_bound, *row_margin;
+  const unsigned char* tstate;  // pruned iteration: [pattern tile][rotation tile] = 0 not
+                                // evaluated (P = 0), 1 evaluated, 2 evaluated margin tile
+                                // (its mass is summed); null: all evaluated
+  int chunk;    // patterns per CTA of a row's cluster (mprep_hi_kernel)
+  int stage;    // the row's P c_i / phi is kept in shared memory between the passes
+  int write_p;  // P over L
+};
+
+// The tensor M-step's operand as FP16 hi only: Q' = P c_i / phi (phi holds c_i
+// num/den, the M-step multiplies raw counts), [R][ldq], each row scaled by 2^e_r so
+// that its largest entry sits near 2^14 (qscale_r = 2^-e_r).  Taking P through an
+// 11-bit rounding, it is served by the hardware exponential (2^-21 relative; results
+// below 2^-126 are 0) and reciprocal.  Bound by HBM and by issue: 8 bytes read and 2
+// written per pair, and phi only where P is not 0.  A row is kept in shared memory
+// between the two passes, shared by a cluster of 1 to 8 CTAs of `chunk` patterns, so
+// that four CTAs fit an SM and one's reads overlap another's writes; a row too long
+// for that is formed again.  With 50 to 90 instructions per pair instead of 30, of
+// which phi's load waited for L's, 10,860 x 50,000 pairs took 2,988 us (1,531 now),
+// 25,680 x 20,000 1,537 (1,000), 10,860 x 10,000 376 (197), 10,860 x 4,999 377 (166).
+constexpr int kMprepChunk = 14208;     // patterns per CTA, 55.5 KB
+constexpr int kMprepChunkMax = 56832;  // where eight CTAs per row do not suffice, 222 KB
+constexpr int kMprepStageLo = 30720;   // of mprep_kernel, two blocks per SM (120 KB)
+
+template <bool PLAIN>
+__global__ void __launch_bounds__(512, 2) mprep_hi_kernel(MprepArgs a) {
+  extern __shared__ __align__(16) float smem_row[];  // [chunk + 4] when stage
+  const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  const int ctas = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int r = (int)blockIdx.x / ctas, bd = (int)blockDim.x;
+  const int i0 = rank * a.chunk;                               // this CTA's patterns
+  const int n = max(0, min(a.N - i0, a.chunk));                // of the row,
+  const int n_out = max(0, min(a.ldq - i0, a.chunk));          // and of the operand
+  const unsigned char* ts =
+      !PLAIN && a.tstate ? a.tstate + (size_t)(i0 >> 7) * a.n_rt + (r >> 7) : nullptr;
+  float* Lr = a.L + (size_t)r * a.N + i0;
+  const float* Fr = a.PHI + (size_t)r * a.N + i0;
+  const float* hi0 = a.lse_shifted + i0;
+  // patterns before the first 16-byte boundary of the row; the row in shared memory
+  // has the same alignment
+  const int head = min(n, (int)(((4 - (((size_t)r * a.N + i0) & 3)) & 3)));
+  float* qrow = smem_row + ((4 - head) & 3);
+  float t = 0.0f, b = 0.0f, qmax = 0.0f, mg = 0.0f;
+  auto state = [&](int i) { return ts ? (int)ts[(size_t)(i >> 7) * a.n_rt] : 1; };
+  auto prob = [](float l, float hi, float lo) {  // exp(l - lse)
+    float p;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(__fmaf_rn(l - hi, kLog2E, lo)));
+    return p;
+  };
+  auto over = [](float P, float f) {
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(f));
+    return P * rf;
+  };
+  auto weigh = [&](int i, float q) {  // P / phi: its part of the mass bound, times c_i
+    if (PLAIN) return q;
+    if (a.Ksum) b = __fmaf_rn(q, __ldg(a.Ksum + i0 + i), b);
+    return a.cnorm ? __fmul_rn(q, __ldg(a.cnorm + i0 + i)) : q;
+  };
+  auto one = [&](int i) {
+    const int st = state(i);
+    const float P = st ? prob(Lr[i], hi0[i], hi0[a.ldq + i]) : 0.0f;
+    if (!PLAIN && a.write_p) Lr[i] = P;
+    const float f = P > 0.0f ? __ldg(Fr + i) : 0.0f;
+    const float q = weigh(i, f > 0.0f ? over(P, f) : 0.0f);
+    t += P;
+    if (st == 2) mg += P;
+    qmax = fmaxf(qmax, q);
+    if (a.stage) qrow[i] = q;
+  };
+  if (ts && head) {  // a 4-tuple may lie in two pattern tiles
+    for (int i = threadIdx.x; i < n; i += bd) one(i);
+  } else {
+    const int n4 = (n - head) / 4, rest = n - 4 * n4;
+    if ((int)threadIdx.x < rest) one((int)threadIdx.x < head ? threadIdx.x : 4 * n4 + threadIdx.x);
+    float4* L4 = reinterpret_cast<float4*>(Lr + head);
+    const float4* F4 = reinterpret_cast<const float4*>(Fr + head);
+    const float* sh = hi0 + (size_t)(2 * head) * a.ldq;  // from pattern i0 + head on
+    const float4* H4 = reinterpret_cast<const float4*>(sh);
+    const float4* O4 = reinterpret_cast<const float4*>(sh + a.ldq);
+    float4* Q4 = reinterpret_cast<float4*>(qrow + head);
+    // two 4-tuples per thread and turn, their loads in flight together; phi is not
+    // waited for where the last turn needed it
+    const float4 none = make_float4(-INFINITY, -INFINITY, -INFINITY, -INFINITY);
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f), ones = make_float4(1.0f, 1.0f, 1.0f, 1.0f);
+    bool eager = true;
+    for (int j0 = threadIdx.x; j0 < n4; j0 += 2 * bd) {
+      float4 l[2], hi[2], lo[2], f[2];
+      int st[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + h * bd;
+        st[h] = j < n4 ? state(head + 4 * j) : 0;
+        l[h] = none;
+        hi[h] = lo[h] = zero;
+        f[h] = ones;
+        if (st[h]) {
+          l[h] = L4[j];
+          if (eager) f[h] = __ldg(F4 + j);
+          hi[h] = __ldg(H4 + j);
+          lo[h] = __ldg(O4 + j);
+        }
+      }
+      bool any[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        l[h].x = prob(l[h].x, hi[h].x, lo[h].x);
+        l[h].y = prob(l[h].y, hi[h].y, lo[h].y);
+        l[h].z = prob(l[h].z, hi[h].z, lo[h].z);
+        l[h].w = prob(l[h].w, hi[h].w, lo[h].w);
+        const float sum = (l[h].x + l[h].y) + (l[h].z + l[h].w);
+        any[h] = sum > 0.0f;
+        t += sum;
+        if (!PLAIN && st[h] == 2) mg += sum;
+        if (any[h] && !eager) f[h] = __ldg(F4 + j0 + h * bd);
+      }
+      eager = any[0] || any[1];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int j = j0 + h * bd, i = head + 4 * j;
+        if (j >= n4) break;
+        if (!PLAIN && a.write_p) L4[j] = l[h];
+        float4 q = zero;
+        if (any[h]) {
+          q = make_float4(over(l[h].x, f[h].x), over(l[h].y, f[h].y), over(l[h].z, f[h].z),
+                          over(l[h].w, f[h].w));
+          if (!(fminf(fminf(f[h].x, f[h].y), fminf(f[h].z, f[h].w)) > 0.0f)) {
+            // patterns without counts (true Poisson: phi = 0)
+            q.x = f[h].x > 0.0f ? q.x : 0.0f;
+            q.y = f[h].y > 0.0f ? q.y : 0.0f;
+            q.z = f[h].z > 0.0f ? q.z : 0.0f;
+            q.w = f[h].w > 0.0f ? q.w : 0.0f;
+          }
+          if (!PLAIN) {
+            q.x = weigh(i, q.x);
+            q.y = weigh(i + 1, q.y);
+            q.z = weigh(i + 2, q.z);
+            q.w = weigh(i + 3, q.w);
+          }
+          qmax = fmaxf(fmaxf(qmax, fmaxf(q.x, q.y)), fmaxf(q.z, q.w));
+        }
+        if (a.stage) Q4[j] = q;
+      }
     }
   }
-  if (!Qh) return;
-  __syncthreads();
-  const float mx = row_max;
-  int ex = mx > 0.0f ? 14 - ilogbf(mx) - 1 : 0;
-  ex = max(-100, min(100, ex));
+  if (a.stage)
+    for (int i = n + threadIdx.x; i < n_out; i += bd) qrow[i] = 0.0f;
+  double r0s = 0.0, r1s = 0.0, r2s = 0.0;
+  row_sums(t, b, mg, qmax, r0s, r1s, r2s);
+  __shared__ double part[3];
+  __shared__ float part_max;
+  if (ctas > 1) {  // the other CTAs' parts, in rank order
+    if (threadIdx.x == 0) {
+      part[0] = r0s;
+      part[1] = r1s;
+      part[2] = r2s;
+      part_max = qmax;
+    }
+    cluster.sync();
+    for (int k = 0; k < ctas; ++k) qmax = fmaxf(qmax, *cluster.map_shared_rank(&part_max, k));
+    if (threadIdx.x == 0 && rank == 0)
+      for (int k = 1; k < ctas; ++k) {
+        const double* o = cluster.map_shared_rank(part, k);
+        r0s += o[0];
+        r1s += o[1];
+        r2s += o[2];
+      }
+  }
+  const int ex = row_exponent(qmax);
+  if (threadIdx.x == 0 && rank == 0) {
+    a.T[r] = (float)r0s;
+    a.row_mass[r] = r0s;
+    a.row_bound[r] = r1s;
+    if (a.row_margin) a.row_margin[r] = r2s;
+    a.qscale[r] = ldexpf(1.0f, -ex);
+  }
+  const float up = ldexpf(1.0f, ex);
+  auto again = [&](int i) -> float {  // the row's entry, formed once more
+    if (i >= n || !state(i)) return 0.0f;
+    const float P = a.write_p ? Lr[i] : prob(Lr[i], hi0[i], hi0[a.ldq + i]);
+    const float f = P > 0.0f ? __ldg(Fr + i) : 0.0f;
+    return weigh(i, f > 0.0f ? over(P, f) : 0.0f);
+  };
+  // ldq and chunk are multiples of 128
+  __half* out = a.Qh + (size_t)r * a.ldq + i0;
+  if (a.stage && !head) {  // eight FP16 values (16 bytes) per store
+    for (int j = threadIdx.x; j < n_out / 8; j += bd) {
+      const float4 x = *reinterpret_cast<const float4*>(qrow + 8 * j);
+      const float4 y = *reinterpret_cast<const float4*>(qrow + 8 * j + 4);
+      union {
+        __half2 h[4];
+        uint4 u;
+      } p;
+      p.h[0] = __floats2half2_rn(__fmul_rn(x.x, up), __fmul_rn(x.y, up));
+      p.h[1] = __floats2half2_rn(__fmul_rn(x.z, up), __fmul_rn(x.w, up));
+      p.h[2] = __floats2half2_rn(__fmul_rn(y.x, up), __fmul_rn(y.y, up));
+      p.h[3] = __floats2half2_rn(__fmul_rn(y.z, up), __fmul_rn(y.w, up));
+      reinterpret_cast<uint4*>(out)[j] = p.u;
+    }
+  } else {
+    for (int j = threadIdx.x; j < n_out / 2; j += bd) {
+      const float x = a.stage ? qrow[2 * j] : again(2 * j);
+      const float y = a.stage ? qrow[2 * j + 1] : again(2 * j + 1);
+      reinterpret_cast<__half2*>(out)[j] = __floats2half2_rn(__fmul_rn(x, up), __fmul_rn(y, up));
+    }
+  }
+  if (ctas > 1) cluster.sync();  // no CTA leaves while another reads its part
+}
+
+// The general form: Q in FP32 (FP32 M-step, [R][ldq], zero padded) or as FP16 hi +
+// lo, with the correctly rounded exponential and quotient.
+__global__ void __launch_bounds__(512, 2) mprep_kernel(MprepArgs a) {
+  extern __shared__ __align__(16) float qrow[];
+  const int r = blockIdx.x, N = a.N;
+  const unsigned char* ts = a.tstate ? a.tstate + (r >> 7) : nullptr;
+  float t = 0.0f, b = 0.0f, qmax = 0.0f, mg = 0.0f;
+  for (int i = threadIdx.x; i < N; i += blockDim.x) {
+    const size_t e = (size_t)r * N + i;
+    const int st = ts ? ts[(size_t)(i >> 7) * a.n_rt] : 1;
+    const float2 li = a.lse2[i];
+    const float l = a.L[e];
+    float P = 0.0f;
+    if (st && isfinite(li.x) && l > -INFINITY) P = expf((l - li.x) - li.y);
+    if (st == 2) mg += P;
+    const float f = st ? a.PHI[e] : 0.0f;
+    float q = f > 0.0f ? __fdiv_rn(P, f) : 0.0f;
+    t += P;
+    if (a.Ksum) b = __fmaf_rn(q, __ldg(a.Ksum + i), b);
+    if (a.Qh && a.cnorm) q = __fmul_rn(q, __ldg(a.cnorm + i));
+    qmax = fmaxf(qmax, q);
+    if (a.Q) a.Q[(size_t)r * a.ldq + i] = q;
+    if (a.stage) qrow[i] = q;
+    if (a.write_p) a.L[e] = P;
+  }
+  if (a.Q)
+    for (int i = N + threadIdx.x; i < a.ldq; i += blockDim.x) a.Q[(size_t)r * a.ldq + i] = 0.0f;
+  double r0s = 0.0, r1s = 0.0, r2s = 0.0;
+  row_sums(t, b, mg, qmax, r0s, r1s, r2s);
+  if (threadIdx.x == 0) {
+    a.T[r] = (float)r0s;
+    a.row_mass[r] = r0s;
+    a.row_bound[r] = r1s;
+    if (a.row_margin) a.row_margin[r] = r2s;
+  }
+  if (!a.Qh) return;
+  const int ex = row_exponent(qmax);
   const float up = ldexpf(1.0f, ex);
   auto qval = [&](int i) -> float {
     if (i >= N) return 0.0f;
-    if (stage) return __fmul_rn(qrow[i], up);
+    if (a.stage) return __fmul_rn(qrow[i], up);
     // re-read the row (L now holds P)
     const size_t e = (size_t)r * N + i;
-    const float f = PHI[e];
-    return f > 0.0f ? __fmul_rn(__fmul_rn(__fdiv_rn(L[e], f), __ldg(cnorm + i)), up) : 0.0f;
+    const float f = a.PHI[e];
+    const float q = f > 0.0f ? __fdiv_rn(a.L[e], f) : 0.0f;
+    return __fmul_rn(a.cnorm ? __fmul_rn(q, __ldg(a.cnorm + i)) : q, up);
   };
   // ldq is a multiple of 128: four FP16 values (8 bytes) per store
-  for (int j = threadIdx.x; j < ldq / 4; j += blockDim.x) {
+  for (int j = threadIdx.x; j < a.ldq / 4; j += blockDim.x) {
     const int i = 4 * j;
     union Pack4 {
       __half h[4];
@@ -1062,10 +1244,10 @@ __global__ void __launch_bounds__(kMprepThreads, 2) mprep_kernel(
       hi.h[c] = __float2half_rn(q);
       lo.h[c] = __float2half_rn(q - __half2float(hi.h[c]));
     }
-    *reinterpret_cast<uint2*>(Qh + (size_t)r * ldq + i) = hi.u;
-    if (Ql) *reinterpret_cast<uint2*>(Ql + (size_t)r * ldq + i) = lo.u;
+    *reinterpret_cast<uint2*>(a.Qh + (size_t)r * a.ldq + i) = hi.u;
+    *reinterpret_cast<uint2*>(a.Ql + (size_t)r * a.ldq + i) = lo.u;
   }
-  if (threadIdx.x == 0) qscale[r] = ldexpf(1.0f, -ex);
+  if (threadIdx.x == 0) a.qscale[r] = ldexpf(1.0f, -ex);
 }
 
 // P = exp(L - lse) in place over the plan's [R][N] rows, with mprep's own
@@ -1355,13 +1537,9 @@ __global__ void __launch_bounds__(32 * kLseWarps) rank_partial_kernel(
 // The normaliser combined over all ranks, in the plan's own form (FP64 and
 // float hi + lo).
 __global__ void lse_from_global_kernel(const double* __restrict__ lse_in, int N,
-                                       double* __restrict__ lse, float2* __restrict__ lse2) {
+                                       LseOut out) {
   const int n = blockIdx.x * blockDim.x + threadIdx.x;
-  if (n >= N) return;
-  const double l = lse_in[n];
-  lse[n] = l;
-  const float hi = (float)l;
-  lse2[n] = make_float2(hi, isfinite(l) ? (float)(l - (double)hi) : 0.0f);
+  if (n < N) out.store(n, lse_in[n]);
 }
 
 // The inserted sums as floats (model sum of T_r x slice, weight sum of T_r),
@@ -1451,10 +1629,17 @@ extern "C" int emc_plan_create(emc_ctx* ctx, const emc_plan_desc* desc, emc_plan
   if (!rc) rc = alloc_n(p, &p->part, (size_t)p->n_rt * d.n_images);
   if (!rc) rc = alloc_n(p, &p->lse, d.n_images);
   if (!rc) rc = alloc_n(p, &p->lse2, d.n_images);
+  if (!rc) rc = alloc_n(p, &p->lse_shifted, (size_t)8 * p->Np);
   if (!rc) rc = alloc_n(p, &p->ll_part, ceil_div(d.n_images, 32));
   if (!rc) {
     cudaError_t e = cudaFuncSetAttribute(mprep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(float) * kMprepStageMax));
+                                         (int)(sizeof(float) * kMprepStageLo));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(mprep_hi_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(sizeof(float) * (kMprepChunkMax + 4)));
+    if (e == cudaSuccess)
+      e = cudaFuncSetAttribute(mprep_hi_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               (int)(sizeof(float) * (kMprepChunkMax + 4)));
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "plan_create: mprep smem");
   }
   if (!rc) {
@@ -1796,17 +1981,52 @@ static int enqueue_estep(emc_plan* p, float* d_model) {
 }
 
 // the normaliser lse_i from the per-tile partials, and the total log-likelihood
+static LseOut lse_out(emc_plan* p) { return {p->lse, p->lse2, p->lse_shifted, p->Np}; }
+
 static int enqueue_lse(emc_plan* p) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images;
   int rc;
   const int nb = ceil_div(N, 32);
-  lse_combine_kernel<<<nb, 32 * kLseWarps, 0, ctx->stream>>>(p->part, p->n_rt, N, p->lse, p->lse2,
+  lse_combine_kernel<<<nb, 32 * kLseWarps, 0, ctx->stream>>>(p->part, p->n_rt, N, lse_out(p),
                                                              p->ll_part);
   if ((rc = after_launch(ctx, "lse_combine_kernel"))) return rc;
   finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->ll_part, nb, p->red + kRedLL);
   if ((rc = after_launch(ctx, "finite_sum_kernel"))) return rc;
   return mark_phase(p, 3);
+}
+
+// Rows of mprep_hi_kernel: the fewest CTAs that keep `chunk` at kMprepChunk.
+static int launch_mprep_hi(emc_plan* p, MprepArgs a) {
+  emc_ctx* ctx = p->ctx;
+  const int N = p->d.n_images;
+  int ctas = 1;
+  while (ctas < 8 && N > ctas * kMprepChunk) ctas *= 2;
+  for (;; ctas = 1) {
+    a.chunk = ceil_div(ceil_div(N, ctas), 128) * 128;
+    a.stage = a.chunk <= kMprepChunkMax;
+    // a thread for eight pairs of a short row
+    const int threads = a.chunk <= 1024 ? 128 : a.chunk <= kMprepChunk ? 256 : 512;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)p->d.n_rot * (unsigned)ctas);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = a.stage ? sizeof(float) * (a.chunk + 4) : 0;
+    cfg.stream = ctx->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool plain = !a.Ksum && !a.cnorm && !a.tstate && !a.write_p;
+    const cudaError_t e =
+        cudaLaunchKernelEx(&cfg, plain ? mprep_hi_kernel<true> : mprep_hi_kernel<false>, a);
+    if (e == cudaSuccess) break;
+    if (ctas == 1) return cuda_fail(ctx, e, "mprep_hi_kernel launch");
+    (void)cudaGetLastError();  // a device that cannot co-schedule the cluster
+  }
+  return after_launch(ctx, "mprep_hi_kernel");
 }
 
 // responsibilities (mprep) and the M-step with insertion into the zeroed
@@ -1820,17 +2040,39 @@ static int enqueue_mstep(emc_plan* p, float* d_model, float* d_weight) {
   double* row_mass = p->red + kRedSlots;
   double* row_bound = row_mass + p->Rp;
   const bool tcm = p->d.precision == EMC_PREC_MIXED;
-  const int stage = tcm && N <= kMprepStageMax;
+  const bool hi_only = tcm && !p->mstep_q_lo;
+  const int stage = tcm && N <= (hi_only ? 8 * kMprepChunkMax : kMprepStageLo);
   // P is written over L only where it is read back: by the pruning of the
-  // next iteration, or by mprep's own second pass when the row of Q does not
-  // fit shared memory.  Otherwise the responsibilities are formed on request
+  // next iteration, or by mprep_kernel's own second pass when the row of Q does
+  // not fit shared memory.  Otherwise the responsibilities are formed on request
   // (emc_plan_results, emc_plan_best_quaternions: plan_respons_ready).
-  const int write_p = (p->prune != nullptr || (tcm && !stage)) ? 1 : 0;
-  mprep_kernel<<<R, kMprepThreads, stage ? sizeof(float) * N : 0, ctx->stream>>>(
-      p->L, p->PHI, p->lse2, p->Ksum, p->cnorm, R, N, tcm ? nullptr : p->Q,
-      tcm ? p->Qh : nullptr, tcm && p->mstep_q_lo ? p->Ql : nullptr, p->qscale, p->Np, p->T,
-      row_mass, row_bound,
-      stage, p->prune_tiles ? p->prune_state : nullptr, p->n_rt, p->prune_margin, write_p);
+  const int write_p = (p->prune != nullptr || (tcm && !hi_only && !stage)) ? 1 : 0;
+  MprepArgs ma;
+  ma.L = p->L;
+  ma.PHI = p->PHI;
+  ma.lse2 = p->lse2;
+  ma.lse_shifted = p->lse_shifted;
+  ma.Ksum = p->d.insert_mode == EMC_INSERT_DETERMINISTIC ? p->Ksum : nullptr;
+  ma.cnorm = p->d.normalize_images ? p->cnorm : nullptr;
+  ma.N = N;
+  ma.ldq = p->Np;
+  ma.n_rt = p->n_rt;
+  ma.Q = tcm ? nullptr : p->Q;
+  ma.Qh = tcm ? p->Qh : nullptr;
+  ma.Ql = tcm && p->mstep_q_lo ? p->Ql : nullptr;
+  ma.qscale = p->qscale;
+  ma.T = p->T;
+  ma.row_mass = row_mass;
+  ma.row_bound = row_bound;
+  ma.row_margin = p->prune_margin;
+  ma.tstate = p->prune_tiles ? p->prune_state : nullptr;
+  ma.stage = stage;
+  ma.write_p = write_p;
+  if (hi_only) {
+    if ((rc = launch_mprep_hi(p, ma))) return rc;
+  } else {
+    mprep_kernel<<<R, 512, stage ? sizeof(float) * N : 0, ctx->stream>>>(ma);
+  }
   p->p_written = write_p != 0;
   if ((rc = after_launch(ctx, "mprep_kernel"))) return rc;
   if ((rc = mark_phase(p, 4))) return rc;
@@ -2265,7 +2507,7 @@ extern "C" int emc_rank_mstep(emc_plan* p, const double* d_lse, float* d_model_s
   EMC_REQUIRE(ctx, !p->prune, "rank_mstep: pruning is not supported on a rotation split");
   const int N = p->d.n_images;
   const long long n3 = (long long)p->d.side * p->d.side * p->d.side;
-  lse_from_global_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(d_lse, N, p->lse, p->lse2);
+  lse_from_global_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(d_lse, N, lse_out(p));
   int rc = after_launch(ctx, "lse_from_global_kernel");
   if (rc) return rc;
   finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->lse, N, p->red + kRedLL);

@@ -90,6 +90,7 @@ struct emc_plan {
   float2* part = nullptr;  // [n_rt][N] (max, sumexp) per rotation tile
   double* lse = nullptr;   // [N]
   float2* lse2 = nullptr;  // [N] lse as float hi + lo
+  float* lse_shifted = nullptr;  // [4][2][Np] the same in four alignments (LseOut)
   double* ll_part = nullptr;  // [N/32] sums of lse
   float* T = nullptr;      // [Rp] rotation totals
   double* red = nullptr;   // reduction scratch (small)
