@@ -175,8 +175,12 @@ __global__ void pattern_ops_kernel(const float* __restrict__ images, const int* 
 constexpr int kRowThreads = 512;
 constexpr int kRowSmemMax = 200 * 1024;
 
+// the row, then the warps' FP64 sums (8-byte aligned: n2 may be odd)
+__host__ __device__ inline size_t pattern_row_bytes(int n2) {
+  return ((size_t)n2 + (n2 & 1)) * sizeof(float);
+}
 __host__ __device__ inline size_t pattern_row_smem(int n2, int Kp) {
-  return (size_t)n2 * sizeof(float) + (size_t)((Kp + 255) / 256) * 8 * sizeof(double);
+  return pattern_row_bytes(n2) + (size_t)((Kp + 255) / 256) * 8 * sizeof(double);
 }
 
 __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
@@ -186,7 +190,7 @@ __global__ void __launch_bounds__(kRowThreads) pattern_row_kernel(
     float* __restrict__ Ksum, __half* __restrict__ Kh, float count_scale) {
   extern __shared__ __align__(16) unsigned char row_smem[];
   float* srow = reinterpret_cast<float*>(row_smem);
-  double* wsum = reinterpret_cast<double*>(row_smem + (size_t)n2 * sizeof(float));
+  double* wsum = reinterpret_cast<double*>(row_smem + pattern_row_bytes(n2));
   const int i = blockIdx.x;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const float* img = images + (size_t)(perm ? perm[i] : i) * n2;
