@@ -273,6 +273,19 @@ __global__ void pattern_sums_kernel(const double* __restrict__ part, int N, int 
 // ------------------------------------------------------------ expand -----
 constexpr float kSliceFloor = 1e-6f;  // true-Poisson floor for unknown voxels
 
+// Index arithmetic of the samples without conversion instructions (roundf, floorf
+// and the casts run at an eighth of the rate of an addition): adding 2^23 (rounding
+// down for the trilinear cell: 1.5 x 2^23) leaves the integer in the low bits.
+
+// The voxel voxel_round(v) where that is 1 .. n, else 0: v + 1/2 rounded towards
+// zero does not reach the next integer, and truncates to it.  Values outside, and
+// NaN, give bits outside the range.
+__device__ __forceinline__ unsigned slice_voxel(float v, unsigned n) {
+  const unsigned i =
+      __float_as_uint(__fadd_rz(__fadd_rz(v, 0.5f), 8388608.0f)) - 0x4B000000u;
+  return i - 1u < n ? i : 0u;
+}
+
 template <int INTERP>
 __device__ __forceinline__ float plan_sample(const float* __restrict__ model, int side,
                                              const RotMat& R, float x, float y, float z);
@@ -281,11 +294,11 @@ template <>
 __device__ __forceinline__ float plan_sample<EMC_INTERP_NEAREST>(const float* __restrict__ model,
                                                                   int side, const RotMat& R,
                                                                   float x, float y, float z) {
-  const long ix = voxel_round(voxel_coord(side, rotate_row(R, 0, x, y, z)));
-  const long iy = voxel_round(voxel_coord(side, rotate_row(R, 1, x, y, z)));
-  const long iz = voxel_round(voxel_coord(side, rotate_row(R, 2, x, y, z)));
-  if (ix > 0 && ix < side && iy > 0 && iy < side && iz > 0 && iz < side)
-    return __ldg(model + ((size_t)iz * side + iy) * side + ix);
+  const unsigned n = (unsigned)side - 1;  // 1 .. side - 1: the reference's bounds
+  const unsigned ix = slice_voxel(voxel_coord(side, rotate_row(R, 0, x, y, z)), n);
+  const unsigned iy = slice_voxel(voxel_coord(side, rotate_row(R, 1, x, y, z)), n);
+  const unsigned iz = slice_voxel(voxel_coord(side, rotate_row(R, 2, x, y, z)), n);
+  if (ix && iy && iz) return __ldg(model + ((iz * side + iy) * side + ix));
   return -1.0f;
 }
 
@@ -293,20 +306,31 @@ template <>
 __device__ __forceinline__ float plan_sample<EMC_INTERP_TRILINEAR>(const float* __restrict__ model,
                                                                     int side, const RotMat& R,
                                                                     float x, float y, float z) {
-  const float cx = voxel_coord(side, rotate_row(R, 0, x, y, z));
-  const float cy = voxel_coord(side, rotate_row(R, 1, x, y, z));
-  const float cz = voxel_coord(side, rotate_row(R, 2, x, y, z));
-  const float fx0 = floorf(cx), fy0 = floorf(cy), fz0 = floorf(cz);
-  const int x0 = (int)fx0, y0 = (int)fy0, z0 = (int)fz0;
-  const float tx = cx - fx0, ty = cy - fy0, tz = cz - fz0;
+  constexpr float kMagic = 12582912.0f;  // 1.5 x 2^23
+  const float c[3] = {voxel_coord(side, rotate_row(R, 0, x, y, z)),
+                      voxel_coord(side, rotate_row(R, 1, x, y, z)),
+                      voxel_coord(side, rotate_row(R, 2, x, y, z))};
+  int i0[3];
+  float f1[3], f0[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    const float t = __fadd_rd(c[d], kMagic);
+    // a coordinate this far out (or NaN) meets no voxel: neither 2^30 nor 2^30 + 1 does
+    const bool near = fabsf(c[d]) < 4194304.0f;
+    i0[d] = near ? __float_as_int(t) - __float_as_int(kMagic) : 1 << 30;
+    f1[d] = c[d] - (t - kMagic);
+    f0[d] = 1.0f - f1[d];
+  }
+  const unsigned n = (unsigned)side;
+  const float xy[4] = {f0[0] * f0[1], f1[0] * f0[1], f0[0] * f1[1], f1[0] * f1[1]};
   float acc = 0.0f, wsum = 0.0f;
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const int xi = x0 + (c & 1), yi = y0 + ((c >> 1) & 1), zi = z0 + (c >> 2);
-    if (xi < 0 || xi >= side || yi < 0 || yi >= side || zi < 0 || zi >= side) continue;
-    const float w = ((c & 1) ? tx : 1.0f - tx) * (((c >> 1) & 1) ? ty : 1.0f - ty) *
-                    ((c >> 2) ? tz : 1.0f - tz);
-    const float v = __ldg(model + ((size_t)zi * side + yi) * side + xi);
+  for (int e = 0; e < 8; ++e) {
+    const unsigned xi = (unsigned)(i0[0] + (e & 1)), yi = (unsigned)(i0[1] + ((e >> 1) & 1)),
+                   zi = (unsigned)(i0[2] + (e >> 2));
+    if (xi >= n || yi >= n || zi >= n) continue;
+    const float w = xy[e & 3] * ((e >> 2) ? f1[2] : f0[2]);
+    const float v = __ldg(model + ((zi * n + yi) * n + xi));
     if (v < 0.0f || w <= 0.0f) continue;
     acc = __fmaf_rn(w, v, acc);
     wsum += w;
@@ -315,15 +339,22 @@ __device__ __forceinline__ float plan_sample<EMC_INTERP_TRILINEAR>(const float* 
 }
 
 // The compacted slice rows S[r][0..Kp) (or their FP16 operands) of
-// kSliceRows rotations per block and the per-rotation sums: count_r (s > 0),
-// A_r = sum s^2/(s+c) and the floored slice sum of the true-Poisson
-// likelihood.
+// kSliceRows rotations per block and the per-rotation sums: count_r (s > 0) and
+// A_r = sum s^2/(s+c) of the reference likelihood, the floored slice sum of the
+// true-Poisson one.  Bound by issue while the model fits near L1 -- with all three
+// sums and a division in either case, conversions in the index and every test on every
+// pixel a sample took up to 110 instructions: 64^3, 6,300 rotations 56 us, now 42;
+// 112^3, 10,860, true Poisson 378, now 302; 96^3 trilinear 1,217, now 1,067 -- and by
+// the latency of the gathers in an 8 MB model (128^3, 25,680: 1,116 and 1,113, true
+// Poisson 1,078 and 985; two rotations per block with more blocks spill: 1,676).
+enum SliceMode { kSliceFp32, kSliceTc, kSliceTcPois };
+
 // rotations per expand block: four with nearest sampling, two with the
 // eight-voxel trilinear gather (registers)
 template <int INTERP>
 __host__ __device__ constexpr int slice_rows_per_block() { return INTERP == EMC_INTERP_NEAREST ? 4 : 2; }
 
-template <int INTERP>
+template <int INTERP, int MODE>
 __global__ void __launch_bounds__(256) slice_rows_kernel(
     const float* __restrict__ model, int side, const float* __restrict__ rot,
     const int* __restrict__ pix, const float* __restrict__ cx, const float* __restrict__ cy,
@@ -354,7 +385,8 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
     const int pv[4] = {pp.x, pp.y, pp.z, pp.w};
     const float xv[4] = {X.x, X.y, X.z, X.w}, yv[4] = {Y.x, Y.y, Y.z, Y.w},
                 zv[4] = {Z.x, Z.y, Z.z, Z.w};
-    const bool live = ops.live && __ldg(ops.live + (q >> 6)) != 0;
+    const bool pixels = (pp.x | pp.y | pp.z | pp.w) >= 0;  // none is padding
+    const bool live = MODE != kSliceFp32 && __ldg(ops.live + (q >> 6)) != 0;
     int odd = 0;  // bit 0: an s <= 0, bit 1: one in (0, 1e-10)
 #pragma unroll
     for (int k = 0; k < kSliceRows; ++k) {
@@ -363,29 +395,48 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
       float sv[4], hv[4];
 #pragma unroll
       for (int u = 0; u < 4; ++u)
-        sv[u] = pv[u] >= 0 ? plan_sample<INTERP>(model, side, Rm, xv[u], yv[u], zv[u]) : 0.0f;
+        sv[u] = pixels || pv[u] >= 0 ? plan_sample<INTERP>(model, side, Rm, xv[u], yv[u], zv[u])
+                                     : 0.0f;
+      const size_t e = (size_t)(r0 + k) * Kp + q;
+      if (MODE != kSliceTc) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        // one division per pixel: h = 1 / (s + c) serves A = s^2 h and the operands
-        hv[u] = sv[u] > 0.0f ? 1.0f / (sv[u] + kPoisC) : 0.0f;
-        if (pv[u] >= 0) {
-          if (!(sv[u] >= 1e-10f)) odd |= sv[u] > 0.0f ? 2 : 1;
-          if (sv[u] > 0.0f) {
-            cnt[k] += 1.0f;
-            A[k] += sv[u] * sv[u] * hv[u];
+        for (int u = 0; u < 4; ++u)
+          if (pixels || pv[u] >= 0) ss[k] += fmaxf(sv[u], kSliceFloor);
+      }
+      if (MODE == kSliceTcPois) {
+        if (live) rot_ops_store_pois4(ops, e, sv);
+        continue;
+      }
+      const float lo = fminf(fminf(sv[0], sv[1]), fminf(sv[2], sv[3]));
+      const bool covered = pixels && lo >= 1e-10f;
+      if (covered) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          hv[u] = inverse(sv[u] + kPoisC);  // serves A = s^2 h and the operands
+          A[k] = __fmaf_rn(sv[u] * sv[u], hv[u], A[k]);
+        }
+        cnt[k] += 4.0f;
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          hv[u] = sv[u] > 0.0f ? inverse(sv[u] + kPoisC) : 0.0f;
+          if (pv[u] >= 0) {
+            if (!(sv[u] >= 1e-10f)) odd |= sv[u] > 0.0f ? 2 : 1;
+            if (sv[u] > 0.0f) {
+              cnt[k] += 1.0f;
+              A[k] = __fmaf_rn(sv[u] * sv[u], hv[u], A[k]);
+            }
           }
-          ss[k] += fmaxf(sv[u], kSliceFloor);
         }
       }
       // the tensor path takes its FP16 operands straight from s; the FP32
       // path keeps the slices
-      const size_t e = (size_t)(r0 + k) * Kp + q;
-      if (ops.live)
-        rot_ops_store4(ops, e, sv, hv, live, q < hl_end);
+      if (MODE == kSliceTc)
+        rot_ops_store4(ops, e, sv, hv, covered, live, q < hl_end);
       else
         *reinterpret_cast<float4*>(S + e) = make_float4(sv[0], sv[1], sv[2], sv[3]);
     }
-    if (ops.inv && odd) {  // races store the same value
+    if (MODE == kSliceTc && odd) {  // races store the same value
       const size_t f = (size_t)(r0 >> 7) * ops.nkb + (q >> 6);
       if (odd & 1) ops.inv[f] = 1;
       if (odd & 2) ops.tiny[f] = 1;
@@ -1854,10 +1905,17 @@ extern "C" int emc_plan_bind(emc_plan* p, const float* d_images, const int* d_ma
 template <int INTERP>
 static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
   emc_ctx* ctx = p->ctx;
-  slice_rows_kernel<INTERP>
-      <<<ceil_div(p->d.n_rot, slice_rows_per_block<INTERP>()), 256, 0, ctx->stream>>>(
-          model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S,
-          p->rot_cnt, p->rot_A, p->rot_ssum, ops);
+  // the block size that leaves the fewest threads without pixels in the last turn
+  const int n4 = p->Kp / 4;
+  int threads = 256;
+  for (int t = 224; t >= 128; t -= 32)
+    if (ceil_div(n4, t) * t < ceil_div(n4, threads) * threads) threads = t;
+  auto kernel = !ops.live ? slice_rows_kernel<INTERP, kSliceFp32>
+                : ops.Lh  ? slice_rows_kernel<INTERP, kSliceTcPois>
+                          : slice_rows_kernel<INTERP, kSliceTc>;
+  kernel<<<ceil_div(p->d.n_rot, slice_rows_per_block<INTERP>()), threads, 0, ctx->stream>>>(
+      model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S, p->rot_cnt,
+      p->rot_A, p->rot_ssum, ops);
   int rc = after_launch(ctx, "slice_rows_kernel");
   if (rc || !ops.tiny) return rc;
   tiny_plane_kernel<INTERP><<<dim3(p->n_rt, kTinyBlocks), 256, 0, ctx->stream>>>(
