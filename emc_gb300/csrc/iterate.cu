@@ -1722,7 +1722,8 @@ extern "C" int emc_plan_create(emc_ctx* ctx, const emc_plan_desc* desc, emc_plan
     if (!rc) rc = blur_prepare(ctx, d.side, d.blur_sigma, ba, bb, bg, bk, &p->blur);
   }
   if (!rc) {
-    cudaError_t e = cudaMemsetAsync(p->flags, 0, 16 * sizeof(int), ctx->stream);
+    cudaError_t e = cudaHostAlloc((void**)&p->report, sizeof(IterReport), cudaHostAllocDefault);
+    if (e == cudaSuccess) e = cudaMemsetAsync(p->flags, 0, 16 * sizeof(int), ctx->stream);
     if (e != cudaSuccess) rc = cuda_fail(ctx, e, "plan_create");
   }
   if (!rc && d.precision == EMC_PREC_FP32) rc = alloc_n(p, &p->Q, (size_t)d.n_rot * p->Np);
@@ -1749,6 +1750,7 @@ extern "C" int emc_plan_destroy(emc_plan* p) {
     if (e) cudaEventDestroy(e);
   if (p->tc) tc_free(p);
   for (void* a : p->allocs) cudaFree(a);
+  if (p->report) cudaFreeHost(p->report);
   delete p;
   return EMC_OK;
 }
@@ -2220,42 +2222,59 @@ extern "C" int emc_iterate_async(emc_plan* p, float* d_model, float* d_weight, f
 // Synchronises, then reports what the device recorded since the last wait:
 // a pipeline wait that timed out, slice values outside the FP16 operand
 // range; fills stats (of the last iteration) and clears the status words.
-extern "C" int emc_plan_wait(emc_plan* p, emc_iter_stats* stats) {
-  if (!p) return EMC_ERR_INVALID;
-  emc_ctx* ctx = p->ctx;
-  const int R = p->d.n_rot, N = p->d.n_images;
-  int hflags[8] = {0};
-  int tcs = 0;
-  int* dtc = tc_status(p);
-  double h[kRedSlots];
-  std::vector<double> mass(stats ? R : 0);
-  EMC_CUDA(ctx, cudaMemcpyAsync(hflags, p->flags, sizeof(hflags), cudaMemcpyDeviceToHost,
-                                ctx->stream));
-  if (dtc)
-    EMC_CUDA(ctx, cudaMemcpyAsync(&tcs, dtc, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-  if (stats) {
-    EMC_CUDA(ctx, cudaMemcpyAsync(h, p->red, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
-    EMC_CUDA(ctx, cudaMemcpyAsync(mass.data(), p->red + kRedSlots, sizeof(double) * R,
-                                  cudaMemcpyDeviceToHost, ctx->stream));
+__global__ void __launch_bounds__(1024) report_kernel(const int* __restrict__ flags,
+                                                      const int* __restrict__ status,
+                                                      const double* __restrict__ red,
+                                                      const double* __restrict__ row_mass,
+                                                      const double* __restrict__ margin, int R,
+                                                      IterReport* __restrict__ out) {
+  double m = 0.0, g = 0.0;
+  for (int r = threadIdx.x; r < R; r += blockDim.x) {
+    m += row_mass[r];
+    if (margin) g += margin[r];
   }
+  block_sum2(m, g);
+  if (threadIdx.x == 0) {
+    out->mass = m;
+    out->margin = g;
+    out->status = status ? *status : 0;
+  }
+  if (threadIdx.x < 8) out->flags[threadIdx.x] = flags[threadIdx.x];
+  if (threadIdx.x < kRedSlots) out->red[threadIdx.x] = red[threadIdx.x];
+  __threadfence_system();
+}
+
+// Waits for the iteration; margin: per-rotation masses whose sum goes to
+// *margin_sum (may both be null).
+int emc::plan_wait(emc_plan* p, emc_iter_stats* stats, const double* margin, double* margin_sum) {
+  emc_ctx* ctx = p->ctx;
+  int* dtc = tc_status(p);
+  report_kernel<<<1, 1024, 0, ctx->stream>>>(p->flags, dtc, p->red, p->red + kRedSlots, margin,
+                                             stats || margin ? p->d.n_rot : 0, p->report);
+  const int rc = after_launch(ctx, "report_kernel");
+  if (rc) return rc;
   EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
-  if (dtc && tcs) EMC_CUDA(ctx, cudaMemsetAsync(dtc, 0, sizeof(int), ctx->stream));
-  if (hflags[0] & 4) EMC_CUDA(ctx, cudaMemsetAsync(p->flags, 0, sizeof(int), ctx->stream));
-  if (tcs)
+  const IterReport h = *p->report;
+  if (h.status) EMC_CUDA(ctx, cudaMemsetAsync(dtc, 0, sizeof(int), ctx->stream));
+  if (h.flags[0] & 4) EMC_CUDA(ctx, cudaMemsetAsync(p->flags, 0, sizeof(int), ctx->stream));
+  if (h.status)
     return fail(ctx, EMC_ERR_TIMEOUT, "iterate: tensor-core pipeline wait timed out (status 0x%x)",
-                tcs);
-  if (hflags[0] & 4)
+                h.status);
+  if (h.flags[0] & 4)
     return fail(ctx, EMC_ERR_UNSUPPORTED, "iterate: slice values exceed the FP16 operand range");
   if (stats) {
-    double m = 0.0;
-    for (double v : mass) m += v;
-    stats->total_loglik = h[kRedLL];
-    stats->model_mean_before = h[kRedMean + 1] > 0 ? h[kRedMean] / h[kRedMean + 1] : 0.0;
-    stats->captured_mass = m / (double)N;
-    stats->bad_pairs = hflags[4];
+    stats->total_loglik = h.red[kRedLL];
+    stats->model_mean_before = h.red[kRedMean + 1] > 0 ? h.red[kRedMean] / h.red[kRedMean + 1] : 0.0;
+    stats->captured_mass = h.mass / (double)p->d.n_images;
+    stats->bad_pairs = h.flags[4];
     stats->reserved = 0;
   }
+  if (margin_sum) *margin_sum = h.margin;
   return EMC_OK;
+}
+
+extern "C" int emc_plan_wait(emc_plan* p, emc_iter_stats* stats) {
+  return p ? plan_wait(p, stats, nullptr, nullptr) : EMC_ERR_INVALID;
 }
 
 extern "C" int emc_iterate(emc_plan* p, float* d_model, float* d_weight, float sigma,

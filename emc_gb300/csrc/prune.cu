@@ -51,6 +51,11 @@ struct PruneState {
   float *d_rot = nullptr, *d_rotw = nullptr;
   const float *rot_in = nullptr, *rotw_in = nullptr;
   double* d_margin = nullptr;
+  // page-locked copies of state, tiles, kb_off and kb_list: their transfers are
+  // enqueued without a wait (the next ones follow a wait for the device)
+  unsigned char* h_state = nullptr;
+  int2* h_tiles = nullptr;
+  int *h_kb_off = nullptr, *h_kb_list = nullptr;
   emc_prune_info info{};
 };
 
@@ -119,7 +124,8 @@ __global__ void best_rotation_kernel(const float* __restrict__ P, int R, int N,
   best[i] = br;
 }
 
-// core[newpos[i] / 128][rt] = 1 when pattern i's mass in rotation tile rt > tau.
+// core[newpos[i] / 128][rt] = 1 when pattern i's mass in rotation tile rt > tau
+// (newpos null: i itself).
 __global__ void tile_mass_kernel(const float* __restrict__ P, int R, int N, int n_rt,
                                  const int* __restrict__ newpos, float tau,
                                  unsigned char* __restrict__ core) {
@@ -129,7 +135,7 @@ __global__ void tile_mass_kernel(const float* __restrict__ P, int R, int N, int 
   const int r1 = min(R, (rt + 1) * 128);
   float m = 0.0f;
   for (int r = rt * 128; r < r1; ++r) m += P[(size_t)r * N + i];
-  if (m > tau) core[(size_t)(newpos[i] >> 7) * n_rt + rt] = 1;
+  if (m > tau) core[(size_t)((newpos ? newpos[i] : i) >> 7) * n_rt + rt] = 1;
 }
 
 // state = 1 for core tiles, 2 for tiles adjacent to a core tile of the same
@@ -242,6 +248,18 @@ static int prune_alloc(emc_plan* p, PruneState* ps) {
   if (!rc) rc = plan_alloc(p, (void**)&ps->d_kb_list, sizeof(int) * 2 * (size_t)n_pt * n_rt);
   if (!rc) rc = plan_alloc(p, (void**)&ps->d_rot, sizeof(float) * 4 * (size_t)R);
   if (!rc) rc = plan_alloc(p, (void**)&ps->d_rotw, sizeof(float) * (size_t)R);
+  const size_t cells = (size_t)n_pt * n_rt;
+  unsigned char* h = nullptr;
+  if (!rc)
+    EMC_CUDA(p->ctx, cudaHostAlloc((void**)&h, cells * (sizeof(int2) + 2 * sizeof(int) + 1) +
+                                                   sizeof(int) * ((size_t)n_rt + 1),
+                                   cudaHostAllocDefault));
+  if (h) {
+    ps->h_tiles = (int2*)h;
+    ps->h_kb_list = (int*)(ps->h_tiles + cells);
+    ps->h_kb_off = ps->h_kb_list + 2 * cells;
+    ps->h_state = (unsigned char*)(ps->h_kb_off + n_rt + 1);
+  }
   return rc;
 }
 
@@ -338,8 +356,7 @@ static int prune_prepare(emc_plan* p, PruneState* ps, bool reorder) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images, R = p->d.n_rot, n_rt = p->n_rt, n_pt = p->Np / 128;
   int rc;
-  std::vector<int> newpos(N), new_perm = ps->h_perm;
-  std::iota(newpos.begin(), newpos.end(), 0);
+  std::vector<int> newpos(reorder ? N : 0), new_perm = ps->h_perm;
   if ((rc = plan_respons_ready(p))) return rc;
   if (reorder) {
     best_rotation_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(p->L, R, N, ps->d_best);
@@ -354,12 +371,12 @@ static int prune_prepare(emc_plan* p, PruneState* ps, bool reorder) {
       new_perm[j] = ps->h_perm[order[j]];
       newpos[order[j]] = j;
     }
+    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_newpos, newpos.data(), sizeof(int) * N,
+                                  cudaMemcpyHostToDevice, ctx->stream));
   }
-  EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_newpos, newpos.data(), sizeof(int) * N,
-                                cudaMemcpyHostToDevice, ctx->stream));
   EMC_CUDA(ctx, cudaMemsetAsync(ps->d_core, 0, (size_t)n_pt * n_rt, ctx->stream));
   tile_mass_kernel<<<dim3(ceil_div(N, 256), n_rt), 256, 0, ctx->stream>>>(
-      p->L, R, N, n_rt, ps->d_newpos, ps->tau, ps->d_core);
+      p->L, R, N, n_rt, reorder ? ps->d_newpos : nullptr, ps->tau, ps->d_core);
   if ((rc = after_launch(ctx, "tile_mass_kernel"))) return rc;
   return prune_finish(p, ps, new_perm);
 }
@@ -379,9 +396,9 @@ static int prune_finish(emc_plan* p, PruneState* ps, const std::vector<int>& new
   dilate_kernel<<<ceil_div(n_pt * n_rt, 256), 256, 0, ctx->stream>>>(ps->d_core, ps->d_adj, n_pt,
                                                                      n_rt, ps->d_state);
   if ((rc = after_launch(ctx, "dilate_kernel"))) return rc;
-  std::vector<unsigned char> state((size_t)n_pt * n_rt);
-  EMC_CUDA(ctx, cudaMemcpyAsync(state.data(), ps->d_state, state.size(), cudaMemcpyDeviceToHost,
-                                ctx->stream));
+  unsigned char* state = ps->h_state;
+  const size_t cells = (size_t)n_pt * n_rt;
+  EMC_CUDA(ctx, cudaMemcpyAsync(state, ps->d_state, cells, cudaMemcpyDeviceToHost, ctx->stream));
   EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   if (probe_stride > 0) {
     for (int pt = 0; pt < n_pt; ++pt)
@@ -389,8 +406,7 @@ static int prune_finish(emc_plan* p, PruneState* ps, const std::vector<int>& new
         unsigned char& st = state[(size_t)pt * n_rt + rt];
         if (!st) st = 2;
       }
-    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_state, state.data(), state.size(), cudaMemcpyHostToDevice,
-                                  ctx->stream));
+    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_state, state, cells, cudaMemcpyHostToDevice, ctx->stream));
   }
   // The true-Poisson E-step evaluates 256 rotations per CTA: both 128-row
   // halves of a pair take the stronger state, so that every evaluated row is
@@ -408,49 +424,48 @@ static int prune_finish(emc_plan* p, PruneState* ps, const std::vector<int>& new
         }
         a[0] = s;
       }
-    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_state, state.data(), state.size(), cudaMemcpyHostToDevice,
-                                  ctx->stream));
+    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_state, state, cells, cudaMemcpyHostToDevice, ctx->stream));
   }
   // tile list in the E-step's grouped raster: 8 rotation tiles share a pattern tile
-  std::vector<int2> tiles;
+  int n_tiles = 0;
   long long rows = 0;  // evaluated 128-rotation row tiles
   for (int g0 = 0; g0 < n_rt; g0 += 8 * span)
     for (int pt = 0; pt < n_pt; ++pt)
       for (int rt = g0; rt < std::min(n_rt, g0 + 8 * span); rt += span)
         if (state[(size_t)pt * n_rt + rt]) {
-          tiles.push_back(make_int2(pt, rt / span));
+          ps->h_tiles[n_tiles++] = make_int2(pt, rt / span);
           rows += std::min(span, n_rt - rt);
         }
-  ps->n_tiles = (int)tiles.size();
+  ps->n_tiles = n_tiles;
   ps->info.active_fraction = (double)rows / ((double)n_pt * n_rt);
   // M-step: per rotation tile, the 64-pattern k-blocks of its evaluated pattern tiles
-  std::vector<int> kb_off(n_rt + 1), kb_list;
+  int n_kb = 0;
   for (int rt = 0; rt < n_rt; ++rt) {
-    kb_off[rt] = (int)kb_list.size();
+    ps->h_kb_off[rt] = n_kb;
     for (int pt = 0; pt < n_pt; ++pt)
       if (state[(size_t)pt * n_rt + rt]) {
-        kb_list.push_back(2 * pt);
-        kb_list.push_back(2 * pt + 1);
+        ps->h_kb_list[n_kb++] = 2 * pt;
+        ps->h_kb_list[n_kb++] = 2 * pt + 1;
       }
   }
-  kb_off[n_rt] = (int)kb_list.size();
-  EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_kb_off, kb_off.data(), sizeof(int) * (n_rt + 1),
+  ps->h_kb_off[n_rt] = n_kb;
+  EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_kb_off, ps->h_kb_off, sizeof(int) * (n_rt + 1),
                                 cudaMemcpyHostToDevice, ctx->stream));
-  if (!kb_list.empty())
-    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_kb_list, kb_list.data(), sizeof(int) * kb_list.size(),
+  if (n_kb)
+    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_kb_list, ps->h_kb_list, sizeof(int) * n_kb,
                                   cudaMemcpyHostToDevice, ctx->stream));
   ps->info.core_fraction =
-      (double)std::count(state.begin(), state.end(), (unsigned char)1) / ((double)n_pt * n_rt);
-  if (!tiles.empty())
-    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_tiles, tiles.data(), sizeof(int2) * tiles.size(),
+      (double)std::count(state, state + cells, (unsigned char)1) / (double)cells;
+  if (n_tiles)
+    EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_tiles, ps->h_tiles, sizeof(int2) * n_tiles,
                                   cudaMemcpyHostToDevice, ctx->stream));
   if (new_perm != ps->h_perm) {
     EMC_CUDA(ctx, cudaMemcpyAsync(ps->d_perm, new_perm.data(), sizeof(int) * N,
                                   cudaMemcpyHostToDevice, ctx->stream));
     if ((rc = pattern_side(p, ps->d_perm, true))) return rc;
+    EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // new_perm is staged
     ps->h_perm = new_perm;
   }
-  EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));  // host vectors above are staged
   // a dense mask is cheaper as a full scan
   ps->ready = arm || (ps->info.active_fraction < 0.75 &&
                       !(ps->full_every > 0 && ps->since_full + 1 >= ps->full_every));
@@ -470,6 +485,11 @@ int prune_reset(emc_plan* p) {
 }
 
 void prune_free(emc_plan* p) {
+  if (PruneState* ps = pstate(p))
+    if (ps->h_tiles) {
+      cudaStreamSynchronize(p->ctx->stream);
+      cudaFreeHost(ps->h_tiles);
+    }
   delete pstate(p);
   p->prune = nullptr;
 }
@@ -481,7 +501,7 @@ int prune_iterate(emc_plan* p, float* model, float* weight, float sigma, emc_ite
   *handled = false;
   if (!ps || !p->bound || !model || !weight) return EMC_OK;
   *handled = true;
-  const int N = p->d.n_images, R = p->d.n_rot;
+  const int N = p->d.n_images;
   const size_t n3 = (size_t)p->d.side * p->d.side * p->d.side;
   int rc;
   ps->h_perm_results = ps->h_perm;
@@ -510,13 +530,8 @@ int prune_iterate(emc_plan* p, float* model, float* weight, float sigma, emc_ite
   p->prune_kb_off = nullptr;
   p->prune_kb_list = nullptr;
   if (rc) return rc;
-  if ((rc = emc_plan_wait(p, stats))) return rc;
-  std::vector<double> margin(R);
-  EMC_CUDA(ctx, cudaMemcpyAsync(margin.data(), ps->d_margin, sizeof(double) * R,
-                                cudaMemcpyDeviceToHost, ctx->stream));
-  EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   double mg = 0.0;
-  for (double v : margin) mg += v;
+  if ((rc = plan_wait(p, stats, ps->d_margin, &mg))) return rc;
   ps->info.margin_mass = mg / (double)N;
   ps->info.pruned = 1;
   if (ps->info.margin_mass > 1.0 - (double)ps->min_mass) {
