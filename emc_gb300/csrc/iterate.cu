@@ -955,17 +955,6 @@ __global__ void fill_part_kernel(float2* __restrict__ part, size_t n) {
     part[e] = make_float2(-INFINITY, 0.0f);
 }
 
-// Deterministic FP64 sum of the finite entries of x[0..n) into out[0]
-// (one block; the order of additions is fixed).
-__global__ void __launch_bounds__(1024) finite_sum_kernel(const double* __restrict__ x, int n,
-                                                          double* __restrict__ out) {
-  double s = 0.0, none = 0.0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x)
-    if (isfinite(x[i])) s += x[i];
-  block_sum2(s, none);
-  if (threadIdx.x == 0) out[0] = s;
-}
-
 // ---- responsibilities -> M-step operand --------------------------------
 // One block per rotation row: P = exp(L - lse), Q = P / phi, T_r = sum_i P, the
 // row's captured mass and the inserted-mass bound sum_i Q_ri K_i.  Element math is
@@ -1929,8 +1918,6 @@ static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
 static int plan_expand(emc_plan* p, const float* model) {
   emc_ctx* ctx = p->ctx;
   const RotOps ops = tc_rot_ops(p);
-  if (ops.inv)
-    EMC_CUDA(ctx, cudaMemsetAsync(p->rot_flags, 0, 2 * (size_t)p->n_rt * ops.nkb, ctx->stream));
   return p->d.interp == EMC_INTERP_NEAREST ? expand_launch<EMC_INTERP_NEAREST>(p, model, ops)
                                            : expand_launch<EMC_INTERP_TRILINEAR>(p, model, ops);
 }
@@ -2028,7 +2015,6 @@ static int enqueue_estep(emc_plan* p, float* d_model) {
   const int N = p->d.n_images;
   int rc;
   if ((rc = mark_phase(p, 0))) return rc;
-  EMC_CUDA(ctx, cudaMemsetAsync(p->flags + 4, 0, sizeof(int), ctx->stream));
   if (p->prune_tiles) {  // skipped tiles contribute (max, sum exp) = (-inf, 0)
     fill_part_kernel<<<ctx->sm_count * 4, 256, 0, ctx->stream>>>(p->part,
                                                                 (size_t)p->n_rt * N);
@@ -2047,6 +2033,13 @@ static int enqueue_estep(emc_plan* p, float* d_model) {
 // the normaliser lse_i from the per-tile partials, and the total log-likelihood
 static LseOut lse_out(emc_plan* p) { return {p->lse, p->lse2, p->lse_shifted, p->Np}; }
 
+// The terms of the total log-likelihood that plan_wait adds: the partials of
+// lse_combine_kernel (or, after a rank's M-step, every pattern's lse).
+static void own_loglik(emc_plan* p) {
+  p->ll_src = p->ll_part;
+  p->ll_n = ceil_div(p->d.n_images, 32);
+}
+
 static int enqueue_lse(emc_plan* p) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images;
@@ -2055,8 +2048,7 @@ static int enqueue_lse(emc_plan* p) {
   lse_combine_kernel<<<nb, 32 * kLseWarps, 0, ctx->stream>>>(p->part, p->n_rt, N, lse_out(p),
                                                              p->ll_part);
   if ((rc = after_launch(ctx, "lse_combine_kernel"))) return rc;
-  finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->ll_part, nb, p->red + kRedLL);
-  if ((rc = after_launch(ctx, "finite_sum_kernel"))) return rc;
+  own_loglik(p);
   return mark_phase(p, 3);
 }
 
@@ -2200,13 +2192,30 @@ static int iterate_enqueue(emc_plan* p, float* d_model, float* d_weight) {
 // copy: a copy would queue on the copy engine behind any bulk host copy that
 // another stream has issued (the next patterns, uploaded while this iteration
 // runs) and hold the iteration back until that copy ends.
-__global__ void set_float_kernel(float* __restrict__ dst, float v) { *dst = v; }
+// Start of an iteration, before its graph or its first kernel: the annealing width,
+// and zeros in the invalid-pair counter and the expand's block flags.
+__global__ void begin_kernel(float* __restrict__ sigma, float v, int* __restrict__ bad,
+                             uint4* __restrict__ flags, int n16) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e == 0) {
+    *sigma = v;
+    *bad = 0;
+  }
+  if (e < n16) flags[e] = make_uint4(0, 0, 0, 0);
+}
+
+static int begin_iteration(emc_plan* p, float sigma, cudaStream_t stream) {
+  const size_t bytes = p->rot_flags ? 2 * (size_t)p->n_rt * (p->Kp / 64) : 0;
+  const int n16 = (int)((bytes + 15) / 16);  // rot_flags is allocated in whole 16 bytes
+  begin_kernel<<<std::max(1, ceil_div(n16, 256)), 256, 0, stream>>>(
+      p->sigma_dev, sigma, p->flags + 4, reinterpret_cast<uint4*>(p->rot_flags), n16);
+  return after_launch(p->ctx, "begin_kernel");
+}
 
 static int set_sigma(emc_plan* p, float sigma) {
   emc_ctx* ctx = p->ctx;
   EMC_REQUIRE(ctx, sigma > 0.0f && std::isfinite(sigma), "iterate: bad sigma");
-  set_float_kernel<<<1, 1, 0, ctx->stream>>>(p->sigma_dev, sigma);
-  return after_launch(ctx, "set_float_kernel");
+  return begin_iteration(p, sigma, ctx->stream);
 }
 
 extern "C" int emc_iterate_async(emc_plan* p, float* d_model, float* d_weight, float sigma) {
@@ -2227,6 +2236,7 @@ __global__ void __launch_bounds__(1024) report_kernel(const int* __restrict__ fl
                                                       const double* __restrict__ red,
                                                       const double* __restrict__ row_mass,
                                                       const double* __restrict__ margin, int R,
+                                                      const double* __restrict__ ll, int n_ll,
                                                       IterReport* __restrict__ out) {
   double m = 0.0, g = 0.0;
   for (int r = threadIdx.x; r < R; r += blockDim.x) {
@@ -2234,9 +2244,15 @@ __global__ void __launch_bounds__(1024) report_kernel(const int* __restrict__ fl
     if (margin) g += margin[r];
   }
   block_sum2(m, g);
+  double l = 0.0, none = 0.0;  // the finite entries
+  for (int i = threadIdx.x; i < n_ll; i += blockDim.x)
+    if (isfinite(ll[i])) l += ll[i];
+  __syncthreads();
+  block_sum2(l, none);
   if (threadIdx.x == 0) {
     out->mass = m;
     out->margin = g;
+    out->loglik = l;
     out->status = status ? *status : 0;
   }
   if (threadIdx.x < 8) out->flags[threadIdx.x] = flags[threadIdx.x];
@@ -2250,7 +2266,8 @@ int emc::plan_wait(emc_plan* p, emc_iter_stats* stats, const double* margin, dou
   emc_ctx* ctx = p->ctx;
   int* dtc = tc_status(p);
   report_kernel<<<1, 1024, 0, ctx->stream>>>(p->flags, dtc, p->red, p->red + kRedSlots, margin,
-                                             stats || margin ? p->d.n_rot : 0, p->report);
+                                             stats || margin ? p->d.n_rot : 0, p->ll_src,
+                                             stats ? p->ll_n : 0, p->report);
   const int rc = after_launch(ctx, "report_kernel");
   if (rc) return rc;
   EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -2263,7 +2280,7 @@ int emc::plan_wait(emc_plan* p, emc_iter_stats* stats, const double* margin, dou
   if (h.flags[0] & 4)
     return fail(ctx, EMC_ERR_UNSUPPORTED, "iterate: slice values exceed the FP16 operand range");
   if (stats) {
-    stats->total_loglik = h.red[kRedLL];
+    stats->total_loglik = h.loglik;
     stats->model_mean_before = h.red[kRedMean + 1] > 0 ? h.red[kRedMean] / h.red[kRedMean + 1] : 0.0;
     stats->captured_mass = h.mass / (double)p->d.n_images;
     stats->bad_pairs = h.flags[4];
@@ -2333,6 +2350,7 @@ extern "C" int emc_plan_replay(emc_plan* p, float sigma) {
   int rc = set_sigma(p, sigma);
   if (rc) return rc;
   EMC_CUDA(ctx, cudaGraphLaunch(p->graph_exec, ctx->stream));
+  own_loglik(p);
   return EMC_OK;
 }
 
@@ -2380,8 +2398,8 @@ extern "C" int emc_batch_run(emc_batch* b, const float* sigmas) {
   for (size_t k = 0; k < b->plans.size(); ++k) {
     const float sg = sigmas[k];
     EMC_REQUIRE(ctx, sg > 0.0f && std::isfinite(sg), "batch_run: bad sigma %zu", k);
-    set_float_kernel<<<1, 1, 0, ctx->stream>>>(b->plans[k]->sigma_dev, sg);
-    int rc = after_launch(ctx, "set_float_kernel");
+    const int rc = begin_iteration(b->plans[k], sg, ctx->stream);
+    own_loglik(b->plans[k]);
     if (rc) return rc;
   }
   EMC_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
@@ -2591,8 +2609,8 @@ extern "C" int emc_rank_mstep(emc_plan* p, const double* d_lse, float* d_model_s
   lse_from_global_kernel<<<ceil_div(N, 256), 256, 0, ctx->stream>>>(d_lse, N, lse_out(p));
   int rc = after_launch(ctx, "lse_from_global_kernel");
   if (rc) return rc;
-  finite_sum_kernel<<<1, 1024, 0, ctx->stream>>>(p->lse, N, p->red + kRedLL);
-  if ((rc = after_launch(ctx, "finite_sum_kernel"))) return rc;
+  p->ll_src = p->lse;
+  p->ll_n = N;
   if ((rc = mark_phase(p, 3))) return rc;
   if ((rc = enqueue_mstep(p, d_model_sum, d_weight_sum))) return rc;
   const bool det = p->d.insert_mode == EMC_INSERT_DETERMINISTIC;

@@ -95,6 +95,8 @@ struct emc_plan {
   double* lse = nullptr;   // [N]
   float2* lse2 = nullptr;  // [N] lse as float hi + lo
   float* lse_shifted = nullptr;  // [4][2][Np] the same in four alignments (LseOut)
+  const double* ll_src = nullptr;  // what the report adds (own_loglik)
+  int ll_n = 0;
   double* ll_part = nullptr;  // [N/32] sums of lse
   float* T = nullptr;      // [Rp] rotation totals
   double* red = nullptr;   // reduction scratch (small)
@@ -152,7 +154,6 @@ namespace emc {
 
 // Voxel-sum upper bound and fixed-point scale slots in plan->red.
 enum RedSlot {
-  kRedLL = 0,        // total log-likelihood
   kRedMass = 1,      // captured responsibility mass
   kRedBad = 2,       // invalid pairs
   kRedBoundM = 3,    // upper bound of inserted model mass
@@ -317,6 +318,7 @@ int tc_mstep(emc_plan* p, float* model, float* weight);
 struct IterReport {
   double red[kRedSlots];
   double mass, margin;  // sums over the rotations
+  double loglik;        // of the patterns' lse
   int flags[8];
   int status;  // of the tensor-core pipelines
 };

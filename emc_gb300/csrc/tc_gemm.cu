@@ -1950,7 +1950,7 @@ int tc_bind(emc_plan* p) {
       if (!rc) rc = plan_alloc(p, (void**)&p->ktot, (size_t)Np * 4);
       if (!rc) rc = plan_alloc(p, (void**)&p->k2tot, (size_t)Np * 4);
       if (!rc) rc = plan_alloc(p, (void**)&p->lo_kb, sizeof(int) * (n_pt + 1));
-      if (!rc) rc = plan_alloc(p, (void**)&p->rot_flags, 2 * (size_t)p->n_rt * nkb);
+      if (!rc) rc = plan_alloc(p, (void**)&p->rot_flags, (2 * (size_t)p->n_rt * nkb + 15) / 16 * 16);
     }
     __half** pois_ops[] = {&st->Lh, &st->Ll};
     __half** rot_ops[] = {&st->MS, &st->Hh, &st->Hl, &st->Iv, &st->Tv};
