@@ -405,8 +405,8 @@ static_assert(EPI_WARP0 % 4 == 0, "epilogue warp w reads TMEM lane quarter w % 4
 constexpr int kList = 1100;
 constexpr uint32_t kInv = 16, kTiny = 32;  // flags of the rotation tile in an entry
 constexpr uint32_t kNJ = 64;               // of all entries: the tile needs n_J
-// barriers, per-rotation rows (3 x 128 floats), epilogue parts, list
-constexpr int EXTRA = 256 + 3 * BN * 4 + (EPI_PARTS - 1) * BM * 8 + kList * 4 + 16;
+// barriers, per-rotation rows (128 float4), epilogue parts, list
+constexpr int EXTRA = 256 + BN * 16 + (EPI_PARTS - 1) * BM * 8 + kList * 4 + 16;
 constexpr int SMEM_BYTES = CHUNKS * CHUNK + EXTRA + 1024;
 static_assert(SMEM_BYTES <= 232448, "shared memory of the likelihood kernel");
 }  // namespace es
@@ -520,7 +520,7 @@ __device__ __forceinline__ uint32_t es_entry(const uint32_t* list, const unsigne
 // division, whose range checks num and den do not need.
 __device__ __forceinline__ float quotient(float a, float b) {
   float r;
-  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(b));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(b));
   const float q = a * r;
   return __fmaf_rn(__fmaf_rn(-q, b, a), r, q);
 }
@@ -531,8 +531,8 @@ __device__ __forceinline__ float quotient(float a, float b) {
 // the tile's (max, sum exp) per pattern.
 template <bool PAIR>
 __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tmem, uint64_t* accum,
-                                               uint64_t* jdone, uint32_t jfree, const float* s_A, const float* s_scale,
-                                               const float* s_lw, float2* s_half, int warp,
+                                               uint64_t* jdone, uint32_t jfree, const float4* s_rot,
+                                               float2* s_half, int warp,
                                                int lane, int n0, int r0, int rt, uint32_t seen) {
   using namespace es;
   const int quarter = warp & 3;  // TMEM lanes this warp may access
@@ -597,8 +597,9 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
       // eight independent chains, then their exponentials: the running
       // (max, sum exp) is updated once per eight columns
       const int jn = nok ? min(CG, a.R - (r0 + c0)) : 0;  // columns that are pairs
-      float* Lp = a.L + (size_t)(r0 + c0) * a.N + n;
-      float* Pp = a.PHI + (size_t)(r0 + c0) * a.N + n;
+      const size_t o0 = (size_t)(r0 + c0) * a.N + n;
+      float* const Lp = a.L + o0;
+      float* const Pp = a.PHI + o0;
       float vq[CG];  // n_J
       if (nj) {      // this thread's own stores, all loads in flight together
 #pragma unroll
@@ -613,25 +614,26 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
         const float kh = (full_h ? vh[j] + vd[j] : vh[j]) * a.k_inv;
         const float B = __fmaf_rn(-kPoisC, kh, ktot - n1);
         const float Cc = have_j || nj ? __fmaf_rn(vj[j], a.k_inv, kh) : kh;
-        const float sc = s_scale[c0 + j];
-        bool ok = j < jn && sc > 0.0f;
+        const float4 rc = s_rot[c0 + j];  // A_r, 1 / (2 sigma^2 count_r), log w_r
+        bool ok = true;
         float iphi = 1.0f, phi = 1.0f;
         if (!a.known_intensity) {
           const float num = nj ? __fmaf_rn(-a.k_inv, vq[j], k2tot - n1) : k2tot - n1;
           const float den = vd[j] * (256.0f * a.k_inv);
-          ok = ok && num > 0.0f && den > 0.0f;
+          ok = num > 0.0f && den > 0.0f;
           iphi = quotient(den, num);
           phi = quotient(ci * num, den);
         }
-        const float Sig = __fmaf_rn(__fmaf_rn(Cc, iphi, -2.0f * B), iphi, s_A[c0 + j]);
-        const float L = ok ? __fmaf_rn(-Sig, sc, s_lw[c0 + j]) : -INFINITY;
+        ok = ok && rc.y > 0.0f;
+        const float Sig = __fmaf_rn(__fmaf_rn(Cc, iphi, -2.0f * B), iphi, rc.x);
+        float L = ok ? __fmaf_rn(-Sig, rc.y, rc.z) : -INFINITY;
         if (j < jn) {
           nbad += ok ? 0 : 1;
-          *Lp = L;
-          *Pp = ok ? phi : 1.0f;
+          Lp[(size_t)j * a.N] = L;
+          Pp[(size_t)j * a.N] = ok ? phi : 1.0f;
+        } else {
+          L = -INFINITY;
         }
-        Lp += a.N;
-        Pp += a.N;
         vh[j] = L;
         mx = fmaxf(mx, L);
       }
@@ -680,10 +682,8 @@ __global__ void __launch_bounds__(es::THREADS, 1)
   uint64_t* jdone = drain + 1;  // pass A's products are complete
   uint64_t* jfree = jdone + 1;  // (rank 0) J.H and n_J have been moved out of TMEM
   uint32_t* tmem_slot = (uint32_t*)(jfree + 1);
-  float* s_A = (float*)(smem + CHUNKS * CHUNK + 256);
-  float* s_scale = s_A + BN;
-  float* s_lw = s_scale + BN;
-  float2* s_half = (float2*)(s_lw + BN);  // [EPI_PARTS-1][BM] (max, sum exp) of column parts 1..
+  float4* s_rot = (float4*)(smem + CHUNKS * CHUNK + 256);
+  float2* s_half = (float2*)(s_rot + BN);  // [EPI_PARTS-1][BM] (max, sum exp) of column parts 1..
   uint32_t* s_list = (uint32_t*)(s_half + (EPI_PARTS - 1) * BM);  // [kList]
   uint32_t* s_seen = s_list + kList;  // the bits of all entries; entries passes A and C look at
 
@@ -733,9 +733,9 @@ __global__ void __launch_bounds__(es::THREADS, 1)
   if (threadIdx.x < BN) {
     const int r = r0 + threadIdx.x;
     const float c = r < a.R ? a.rot_cnt[r] : 0.0f;
-    s_A[threadIdx.x] = r < a.R ? a.rot_A[r] : 0.0f;
-    s_scale[threadIdx.x] = c > 0.0f ? inv2s2 / c : -1.0f;  // < 0: invalid rotation
-    s_lw[threadIdx.x] = r < a.R ? logf(a.rotw[r]) : 0.0f;
+    // scale < 0: invalid rotation
+    s_rot[threadIdx.x] = make_float4(r < a.R ? a.rot_A[r] : 0.0f, c > 0.0f ? inv2s2 / c : -1.0f,
+                                     r < a.R ? logf(a.rotw[r]) : 0.0f, 0.0f);
   }
   if (warp == MMA_WARP) {
     if (PAIR) {
@@ -980,7 +980,7 @@ __global__ void __launch_bounds__(es::THREADS, 1)
     }
   } else {
     // ------------------------------------------------ epilogue
-    estep_epilogue<PAIR>(a, tmem, accum, jdone, ptx::mapa_shared(ptx::smem_u32(jfree), 0), s_A, s_scale, s_lw, s_half, warp, lane, n0, r0, rt,
+    estep_epilogue<PAIR>(a, tmem, accum, jdone, ptx::mapa_shared(ptx::smem_u32(jfree), 0), s_rot, s_half, warp, lane, n0, r0, rt,
                          *s_seen);
   }
   ptx::tc_fence_before();
