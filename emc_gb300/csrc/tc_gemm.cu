@@ -1525,6 +1525,40 @@ __device__ __forceinline__ void ms_tile(const TcMstepArgs& a, int t, int& r0, in
 // across tiles, and the accumulator is double-buffered in TMEM (columns
 // 0-255 and 256-511), so the insertion epilogue of one tile overlaps the
 // MMAs of the next.
+// The k-blocks of (rotation tile rt, pixel tile qt): those with counts in the pixel
+// tile, of all pattern blocks or (pruned) of the rotation tile's list, of which the
+// first is always taken, so that the accumulator is written.  Called by a whole warp,
+// which looks at 32 entries at a time (one thread on its own waited for two dependent
+// loads per entry, longer than a block's products); f(kb) is called by all lanes and
+// returns false, in all, to stop.
+template <typename F>
+__device__ __forceinline__ bool ms_each_block(const TcMstepArgs& a, int rt, int qt, F&& f) {
+  const int lane = threadIdx.x & 31;
+  const int* list = a.kb_off ? a.kb_list + a.kb_off[rt] : a.ms_list + (size_t)qt * a.nkb;
+  const int n = a.kb_off ? a.kb_off[rt + 1] - a.kb_off[rt] : a.ms_n[qt];
+  const unsigned char* map = a.kb_off ? a.ms_map + (size_t)qt * a.nkb : nullptr;
+  for (int j0 = 0; j0 < n; j0 += 32) {
+    const int j = j0 + lane, kb = j < n ? __ldg(list + j) : 0;
+    unsigned m = __ballot_sync(0xffffffffu, j < n && (!map || j == 0 || __ldg(map + kb)));
+    for (; m; m &= m - 1)
+      if (!f(__shfl_sync(0xffffffffu, kb, __ffs(m) - 1))) return false;
+  }
+  return true;
+}
+__device__ __forceinline__ int ms_block_count(const TcMstepArgs& a, int rt, int qt) {
+  if (!a.kb_off) return a.ms_n[qt];
+  const int lane = threadIdx.x & 31;
+  const int* list = a.kb_list + a.kb_off[rt];
+  const int n = a.kb_off[rt + 1] - a.kb_off[rt];
+  int c = 0;
+  for (int j0 = 0; j0 < n; j0 += 32) {
+    const int j = j0 + lane;
+    const bool on = j < n && (j == 0 || __ldg(a.ms_map + (size_t)qt * a.nkb + __ldg(list + j)));
+    c += __popc(__ballot_sync(0xffffffffu, on));
+  }
+  return c;
+}
+
 // Stage ring of the single-CTA M-step: Q hi (+ Q lo) and the 256 K^T rows of
 // a 64-pattern k-block.  Without the Q lo slot a stage is 48 KB and four fit
 // where three of 64 KB do: a third more bytes in flight for the same ring.
@@ -1552,17 +1586,6 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
   uint64_t* drain = tempty + 2;      // the MMA issuer's own completion wait before TMEM is freed
   uint32_t* tmem_slot = (uint32_t*)(drain + 1);
   float4* s_xyz = (float4*)(smem + Ring::kStages * Ring::kStageBytes + 256);
-  // the k-blocks of tile (rt, qt): those with counts, of all or (pruned) of the
-  // rotation tile's; the first one always, so that the accumulator is written
-  auto blocks = [&](int rt, int qt) {
-    return a.kb_off ? a.kb_off[rt + 1] - a.kb_off[rt] : a.ms_n[qt];
-  };
-  auto block = [&](int rt, int qt, int j) {  // -1: passed over
-    if (!a.kb_off) return a.ms_list[(size_t)qt * a.nkb + j];
-    const int kb = a.kb_list[a.kb_off[rt] + j];
-    return j == 0 || a.ms_map[(size_t)qt * a.nkb + kb] ? kb : -1;
-  };
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
     for (int s = 0; s < Ring::kStages; ++s) {
@@ -1587,54 +1610,53 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer
-    if (ptx::elect_one()) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x) {
-        int r0, q0;
-        ms_tile(a, t, r0, q0);
-        const int nk = blocks(r0 / BM, q0 / BN);
-        for (int j = 0; j < nk; ++j) {
-          const int kb = block(r0 / BM, q0 / BN, j);
-          if (kb < 0) continue;
+    uint32_t it = 0;
+    bool ok = true;
+    for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x) {
+      int r0, q0;
+      ms_tile(a, t, r0, q0);
+      ok = ms_each_block(a, r0 / BM, q0 / BN, [&](int kb) {
+        bool go = true;
+        if (ptx::elect_one()) {
           const int s = it % Ring::kStages;
-          const uint32_t ph = (it / Ring::kStages) & 1;
-          if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 4, a.spin)) {
-            ok = false;
-            break;
+          go = ptx::mbar_wait(&empty[s], ((it / Ring::kStages) & 1) ^ 1, a.status, 4, a.spin);
+          if (go) {
+            ptx::mbar_arrive_expect_tx(&full[s], Ring::kStageBytes);
+            unsigned char* st = smem + s * Ring::kStageBytes;
+            ptx::tma_load_2d(st, &mQh, kb * BK, r0, &full[s]);
+            if (QLO) ptx::tma_load_2d(st + A_BYTES, &mQl, kb * BK, r0, &full[s]);
+            ptx::tma_load_2d(st + Ring::kOffK, &mKt, kb * BK, q0, &full[s]);
           }
-          ptx::mbar_arrive_expect_tx(&full[s], Ring::kStageBytes);
-          unsigned char* st = smem + s * Ring::kStageBytes;
-          ptx::tma_load_2d(st, &mQh, kb * BK, r0, &full[s]);
-          if (QLO) ptx::tma_load_2d(st + A_BYTES, &mQl, kb * BK, r0, &full[s]);
-          ptx::tma_load_2d(st + Ring::kOffK, &mKt, kb * BK, q0, &full[s]);
-          ++it;
         }
-      }
-      ptx::drain_loads(full, Ring::kStages, it, a.status, 11);  // none in flight at exit
+        go = __all_sync(0xffffffffu, go);
+        it += go;
+        return go;
+      });
     }
+    if (ptx::elect_one())
+      ptx::drain_loads(full, Ring::kStages, it, a.status, 11);  // none in flight at exit
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer
-    if (ptx::elect_one()) {
-      constexpr uint32_t idesc = ptx::idesc_f16(BM, BN);
-      uint32_t it = 0;
-      bool ok = true;
-      int j = 0;
-      for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x, ++j) {
-        const int b = j & 1;
-        const uint32_t d = tmem + (uint32_t)(b * BN);
-        if (!ptx::mbar_wait(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin)) break;
-        ptx::tc_fence_after();
-        int r0t, q0t;
-        ms_tile(a, t, r0t, q0t);
-        // a tile with no k-block leaves the buffer as it was: its rotations
-        // have no responsibility (T_r = 0), so the epilogue inserts nothing
-        const int nk = blocks(r0t / BM, q0t / BN);
-        for (int j2 = 0; j2 < nk; ++j2) {
-          if (a.kb_off && block(r0t / BM, q0t / BN, j2) < 0) continue;
-          const int s = it % Ring::kStages;
-          const uint32_t ph = (it / Ring::kStages) & 1;
-          if (!ptx::mbar_wait(&full[s], ph, a.status, 5, a.spin)) {
+    constexpr uint32_t idesc = ptx::idesc_f16(BM, BN);
+    uint32_t it = 0;
+    bool ok = true;
+    int j = 0;
+    for (int t = blockIdx.x; t < a.n_tiles && ok; t += gridDim.x, ++j) {
+      const int b = j & 1;
+      const uint32_t d = tmem + (uint32_t)(b * BN);
+      int r0t, q0t;
+      ms_tile(a, t, r0t, q0t);
+      // a tile with no k-block leaves the buffer as it was: its rotations
+      // have no responsibility (T_r = 0), so the epilogue inserts nothing
+      const int nk = ms_block_count(a, r0t / BM, q0t / BN);
+      if (ptx::elect_one()) {
+        const bool drained = ptx::mbar_wait(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin);
+        if (drained) ptx::tc_fence_after();
+        ok = drained;
+        for (int kb = 0; kb < nk && ok; ++kb) {
+          const uint32_t i = it + (uint32_t)kb;
+          const int s = i % Ring::kStages;
+          if (!ptx::mbar_wait(&full[s], (i / Ring::kStages) & 1, a.status, 5, a.spin)) {
             ok = false;
             break;
           }
@@ -1645,14 +1667,17 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
             const uint64_t dQh = ptx::smem_desc(base + ks * 32, 1024, 2);
             const uint64_t dQl = ptx::smem_desc(base + A_BYTES + ks * 32, 1024, 2);
             const uint64_t dK = ptx::smem_desc(base + Ring::kOffK + ks * 32, 1024, 2);
-            ptx::mma_f16(d, dQh, dK, idesc, (j2 | ks) ? 1u : 0u);
+            ptx::mma_f16(d, dQh, dK, idesc, (kb | ks) ? 1u : 0u);
             if (QLO) ptx::mma_f16(d, dQl, dK, idesc, 1u);
           }
-          ++it;
           ptx::mma_commit(&empty[s]);
         }
-        ptx::mma_commit(&tfull[b]);  // fires when this tile's MMAs have completed
+        if (drained) ptx::mma_commit(&tfull[b]);  // fires when this tile's MMAs have completed
       }
+      ok = __all_sync(0xffffffffu, ok);
+      it += (uint32_t)nk;
+    }
+    if (ptx::elect_one()) {
       ptx::mma_commit(drain);  // TMEM is freed only after every MMA issued here has completed
       ptx::mbar_wait(drain, 0, a.status, 12);
     }
@@ -1772,40 +1797,37 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 
   if (warp == 0) {
     // ------------------------------------------------ TMA producer (both CTAs)
-    if (ptx::elect_one()) {
-      uint32_t it = 0;
-      bool ok = true;
-      const uint32_t bytes = STAGE_BYTES;
-      for (int t = cl; t < n_tiles && ok; t += ncl) {
-        int qt, rp;
-        raster_tile(t, a.raster, a.n_qt, n_rp, qt, rp);
-        const int r0 = (2 * rp + (int)rank) * BM, q0 = qt * BN + 128 * (int)rank;
-        const int nk = a.ms_n[qt];
-        const int* list = a.ms_list + (size_t)qt * a.nkb;
-        int kb_next = __ldg(list);
-        for (int j = 0; j < nk; ++j, ++it) {
-          const int kb = kb_next;
-          if (j + 1 < nk) kb_next = __ldg(list + j + 1);
+    uint32_t it = 0;
+    bool ok = true;
+    for (int t = cl; t < n_tiles && ok; t += ncl) {
+      int qt, rp;
+      raster_tile(t, a.raster, a.n_qt, n_rp, qt, rp);
+      const int r0 = (2 * rp + (int)rank) * BM, q0 = qt * BN + 128 * (int)rank;
+      ok = ms_each_block(a, 2 * rp, qt, [&](int kb) {
+        bool go = true;
+        if (ptx::elect_one()) {
           const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!ptx::mbar_wait(&empty[s], ph ^ 1, a.status, 4, a.spin)) {
-            ok = false;
-            break;
+          go = ptx::mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, a.status, 4, a.spin);
+          if (go) {
+            // both CTAs' loads
+            if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * STAGE_BYTES);
+            const uint32_t fb = ptx::mapa_shared(ptx::smem_u32(&full[s]), 0);
+            unsigned char* st = smem + s * STAGE_BYTES;
+            ptx::tma_load_2d_pair(st, &mQh, kb * BK, r0, fb);
+            if (QLO) ptx::tma_load_2d_pair(st + ms2::A_BYTES, &mQl, kb * BK, r0, fb);
+            ptx::tma_load_2d_pair(st + OFF_K, &mKt128, kb * BK, q0, fb);
           }
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&full[s], 2 * bytes);  // both CTAs' loads
-          const uint32_t fb = ptx::mapa_shared(ptx::smem_u32(&full[s]), 0);
-          unsigned char* st = smem + s * STAGE_BYTES;
-          ptx::tma_load_2d_pair(st, &mQh, kb * BK, r0, fb);
-          if (QLO) ptx::tma_load_2d_pair(st + ms2::A_BYTES, &mQl, kb * BK, r0, fb);
-          ptx::tma_load_2d_pair(st + OFF_K, &mKt128, kb * BK, q0, fb);
         }
-      }
-      // rank 0's barriers count both CTAs' bytes of the stages it armed
-      if (rank == 0) ptx::drain_loads(full, STAGES, it, a.status, 11);
+        go = __all_sync(0xffffffffu, go);
+        it += go;
+        return go;
+      });
     }
+    // rank 0's barriers count both CTAs' bytes of the stages it armed
+    if (rank == 0 && ptx::elect_one()) ptx::drain_loads(full, STAGES, it, a.status, 11);
   } else if (warp == 1) {
     // ------------------------------------------------ MMA issuer (rank 0)
-    if (rank == 0 && ptx::elect_one()) {
+    if (rank == 0) {
       constexpr uint32_t idesc = ptx::idesc_f16(2 * BM, BN);  // 256 x 256
       uint32_t it = 0;
       bool ok = true;
@@ -1815,32 +1837,40 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
         const uint32_t d = tmem + (uint32_t)(b * BN);
         int qt, rp;
         raster_tile(t, a.raster, a.n_qt, n_rp, qt, rp);
-        const int nk = a.ms_n[qt];
-        if (!ptx::mbar_wait_cluster(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin)) break;
-        ptx::tc_fence_after();
-        for (int kb = 0; kb < nk; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1;
-          if (!ptx::mbar_wait(&full[s], ph, a.status, 5, a.spin)) {
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
+        const int nk = ms_block_count(a, 2 * rp, qt);
+        if (ptx::elect_one()) {
+          const bool drained =
+              ptx::mbar_wait_cluster(&tempty[b], ((j >> 1) & 1) ^ 1, a.status, 7, a.spin);
+          if (drained) ptx::tc_fence_after();
+          ok = drained;
+          for (int kb = 0; kb < nk && ok; ++kb) {
+            const uint32_t i = it + (uint32_t)kb;
+            const int s = i % STAGES;
+            if (!ptx::mbar_wait(&full[s], (i / STAGES) & 1, a.status, 5, a.spin)) {
+              ok = false;
+              break;
+            }
+            ptx::tc_fence_after();
+            const uint32_t base = ptx::smem_u32(smem + s * STAGE_BYTES);
 #pragma unroll
-          for (int ks = 0; ks < BK / 16; ++ks) {
-            const uint64_t dQh = ptx::smem_desc(base + ks * 32, 1024, 2);
-            const uint64_t dQl = ptx::smem_desc(base + ms2::A_BYTES + ks * 32, 1024, 2);
-            const uint64_t dK = ptx::smem_desc(base + OFF_K + ks * 32, 1024, 2);
-            ptx::mma_f16_pair(d, dQh, dK, idesc, (kb | ks) ? 1u : 0u);
-            if (QLO) ptx::mma_f16_pair(d, dQl, dK, idesc, 1u);
+            for (int ks = 0; ks < BK / 16; ++ks) {
+              const uint64_t dQh = ptx::smem_desc(base + ks * 32, 1024, 2);
+              const uint64_t dQl = ptx::smem_desc(base + ms2::A_BYTES + ks * 32, 1024, 2);
+              const uint64_t dK = ptx::smem_desc(base + OFF_K + ks * 32, 1024, 2);
+              ptx::mma_f16_pair(d, dQh, dK, idesc, (kb | ks) ? 1u : 0u);
+              if (QLO) ptx::mma_f16_pair(d, dQl, dK, idesc, 1u);
+            }
+            ptx::mma_commit_pair(&empty[s], 0x3);
           }
-          ptx::mma_commit_pair(&empty[s], 0x3);
+          if (drained) ptx::mma_commit_pair(&tfull[b], 0x3);  // when this tile's MMAs have completed
         }
-        ptx::mma_commit_pair(&tfull[b], 0x3);  // fires when this tile's MMAs have completed
+        ok = __all_sync(0xffffffffu, ok);
+        it += (uint32_t)nk;
       }
-      ptx::mma_commit_pair(drain, 0x1);  // both CTAs' TMEM is written by these MMAs
-      ptx::mbar_wait(drain, 0, a.status, 12);
+      if (ptx::elect_one()) {
+        ptx::mma_commit_pair(drain, 0x1);  // both CTAs' TMEM is written by these MMAs
+        ptx::mbar_wait(drain, 0, a.status, 12);
+      }
     }
   } else {
     // ------------------------------------------------ insertion epilogue
@@ -2398,7 +2428,10 @@ int tc_mstep(emc_plan* p, float* model, float* weight) {
   a.status = st->status;
   a.spin = p->debug_spin ? p->debug_spin : ptx::kSpinLimit;
   a.n_tiles = a.n_qt * a.n_rt;
-  if (p->mstep_pair && !a.kb_off && a.n_rt > 1 && ctx->sm_count >= 2) {
+  // pruned: the pair's two rotation tiles have one list in true-Poisson plans, whose
+  // masks span 256 rotations (prune_finish)
+  const bool one_list = !a.kb_off || p->d.diff == EMC_DIFF_TRUE_POISSON;
+  if (p->mstep_pair && one_list && a.n_rt > 1 && ctx->sm_count >= 2) {
     // CTA pairs, persistent: one cluster per two SMs
     const int tiles = ((a.n_rt + 1) / 2) * a.n_qt;
     const int clusters = std::min(tiles, ctx->sm_count / 2);
