@@ -635,8 +635,7 @@ def finish(args, prob, workspace, ctx, ws, rank, precision, value, ms_step, st, 
     p_eff = int(prob.mask.sum())
     if args.diff == "poisson":
         flops = 8.0 * p_eff * pairs  # 4 GEMM-equivalents (num, den, B, C) x 2 FLOP
-        kernel = ("tc_estep_pair_kernel" if args.estep_pair else "tc_estep_kernel") \
-            if precision == "mixed" else "estep_fp32_kernel"
+        kernel = "tc_estep_kernel" if precision == "mixed" else "estep_fp32_kernel"
     else:
         flops = 2.0 * p_eff * pairs  # one GEMM-equivalent (counts x log slice) x 2 FLOP
         kernel = "tc_estep_pois_kernel" if precision == "mixed" else "estep_pois_fp32_kernel"
@@ -648,6 +647,9 @@ def finish(args, prob, workspace, ctx, ws, rank, precision, value, ms_step, st, 
                 "peak_source": f"bf16_tflops of {peaks['source']} peaks",
                 "flops_per_launch": flops, "ms_per_launch": est,
                 "traffic": traffic}
+    if precision == "mixed":
+        roofline["note"] = ("flops_per_launch are those of the dense contractions; the kernel "
+                            "multiplies the pixel blocks in which a tile of patterns has counts")
     if precision == "fp32":
         roofline["note"] = ("plain FP32 SIMT kernel; against the FP32 FMA pipe "
                             "(152 SMs x 128 lanes x 2 x sm clock) it runs at "
@@ -668,9 +670,10 @@ def finish(args, prob, workspace, ctx, ws, rank, precision, value, ms_step, st, 
                            diff="poisson (reference)" if args.diff == "poisson"
                            else "true poisson (counts x log slice)",
                            mstep_q="fp16 hi+lo" if args.mstep_qlo else "fp16 hi",
-                           estep_gh={-1: "G fp16 hi+lo, H fp16 hi", 3: "G, H fp16 hi+lo",
-                                     2: "G hi, H hi+lo", 1: "G hi+lo, H hi",
-                                     0: "G, H fp16 hi"}[args.estep_ghlo],
+                           estep_gh={-1: "H fp16 hi, hi+lo in K.H before the count tail",
+                                     3: "H fp16 hi+lo", 2: "H fp16 hi+lo",
+                                     1: "H fp16 hi, hi+lo in K.H before the count tail",
+                                     0: "H fp16 hi"}[args.estep_ghlo],
                            mstep_atomics="warp-aggregated" if args.mstep_aggregate else "per pair",
                            estep_kernel="CTA pairs (256-row MMAs)" if args.estep_pair
                            else "single CTAs",

@@ -1810,7 +1810,7 @@ extern "C" int emc_plan_bind(emc_plan* p, const float* d_images, const int* d_ma
     // Compacted pixels in one-pixel bands of detector radius, each band in
     // order of angle.  By radius: the bright low-q pixels, the only ones whose
     // k^2 needs a second FP16 term, share a few k-blocks of the tensor-core
-    // E-step, and the dim outer blocks form the count tail where the G lo
+    // E-step, and the dim outer blocks form the count tail where the H lo
     // term is dropped.  By angle within a band: the 32 pixels of a warp are
     // neighbours on the ring, so the expand's model gathers of a warp touch
     // neighbouring voxels.  (The order is otherwise free: every compacted

@@ -436,10 +436,10 @@ int emc_batch_run(emc_batch* batch, const float* sigmas);
 int emc_batch_wait(emc_batch* batch, emc_iter_stats* stats);
 int emc_batch_destroy(emc_batch* batch);
 /* Precision knobs of the tensor-core kernels.
- * EMC_OPT_ESTEP_GHLO: which of the likelihood's rotation-side factors
- * G = s/(s+c) (bit 0) and H = 1/(s+c) (bit 1) carry an FP16 lo term besides
- * their FP16 hi term (one 128-column MMA per 16-pixel step each, ~2^-12
- * relative rounding of a factor without it).  -1 (default): G always, H too
+ * EMC_OPT_ESTEP_GHLO: where the likelihood's rotation-side factor
+ * H = 1/(s+c) carries an FP16 lo term besides its FP16 hi term (~2^-12
+ * relative rounding without it): bit 0 in K.H before the count tail
+ * (EMC_OPT_GLO_TAIL), bit 1 in every product.  -1 (default): bit 0, and both
  * when known_intensity fixes the scaling at 1; 0..3 set the bits. */
 #define EMC_OPT_ESTEP_GHLO 3
 /* EMC_OPT_MSTEP_QLO: 0 (default) multiplies responsibility/scaling as FP16
@@ -496,12 +496,12 @@ int emc_batch_destroy(emc_batch* batch);
  * The two shapes' models agree to FP32 accumulation rounding (1e-5
  * relative). */
 #define EMC_OPT_MSTEP_PAIR 10
-/* EMC_OPT_GLO_TAIL: the likelihood's G lo term (the FP16 lo half of
- * G = s/(s+c) in B = K.G^T) is applied per 128-pattern tile up to the last
- * 32-pixel block after which at most value / 1e6 of each pattern's counts
- * remain (pixels are ordered by detector radius, so the dropped blocks are
- * the dim outer ones): the term dropped there is below 2^-12 x value / 1e6
- * of B.  Default 1000 (0.1 %); 0 applies it on every block.  Recomputed at
+/* EMC_OPT_GLO_TAIL: the lo term of H in K.H (EMC_OPT_ESTEP_GHLO bit 0) is
+ * applied per 128-pattern tile up to the last 64-pixel block after which at
+ * most 300 x value / 1e6 of each pattern's counts remain (pixels are ordered
+ * by detector radius, so the others are the dim outer ones).  Default 1000
+ * (30 %): the log-likelihood is then as accurate as with the lo term
+ * everywhere to its third digit; 0 applies it on every block.  Recomputed at
  * once when the plan is bound. */
 #define EMC_OPT_GLO_TAIL 11
 int emc_plan_set_option(emc_plan* plan, int option, int value);
