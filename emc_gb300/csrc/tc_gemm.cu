@@ -364,12 +364,15 @@ __global__ void transpose_h_kernel(const __half* __restrict__ in, int rows, int 
 // photons 4.4 products of 128 columns per block, 1.1 to 2.3 here.
 //
 // TMEM has room for four of the five sums: den and K.H in columns 0-255, n_1 and
-// J.H in 256-383 and 384-511.  Where a tile needs n_J, J x [H | I] runs first (pass
-// A, columns 256-511), and the epilogue warps move both sums out into the tile's
-// own part of phi and L, which they overwrite at the end.  One CTA owns 128 patterns x 128 rotations, or (PAIR) a cluster of
+// J.H in 256-383 and 384-511.  Where a tile needs n_J, J x H and J x I run first
+// (pass A): J.H stays where it is, and the epilogue warps move n_J, whose columns
+// n_1 takes, out into the tile's own part of L, which they overwrite at the end
+// (with J x [H | I] as one product both sums had to go: 7,795 -> 7,620 us at 128^3
+// with 80 photons per pattern, 17,790 -> 17,450 with 5,000, 2,332 -> 2,263 at 96^3).
+// One CTA owns 128 patterns x 128 rotations, or (PAIR) a cluster of
 // two 256 x 128 with 256-row MMAs issued by rank 0: each CTA then holds its own
-// 128 patterns and 64 of the 128 rows of every rotation operand, [M'S | H] (and
-// [H | I]) side by side, so the columns of such a 256-column product come in
+// 128 patterns and 64 of the 128 rows of every rotation operand, [M'S | H] side by
+// side, so the columns of that 256-column product come in
 // quarters (den 0-63, K.H 0-63, den 64-127, K.H 64-127).  Per 64-pixel block and
 // CTA that is 32 KB for a 256 x 256 x 64 product (the M-step's ratio).
 //
@@ -470,7 +473,7 @@ struct TcEstepArgs {
 template <bool PAIR>
 struct EsStages {
   static constexpr int RC = PAIR ? 1 : 2;
-  // pass A: J, [H | I]; then what few tiles have: J lo, [H lo | 0], K, [0 | T]
+  // pass A: J, H, I; then what few tiles have: J lo, H lo, K, T
   static constexpr int aJ = 0, aH = 2, aI = 2 + RC;
   int aJl, aHl, aK, aT;
   // pass B: K, [M'S (or H lo) | H], I; in tiles without pass A: J, J lo, H lo
@@ -487,11 +490,11 @@ struct EsStages {
     aJl = o;
     o += jl;
     aHl = o;
-    o += jh ? 2 * RC : 0;
+    o += jh ? RC : 0;
     aK = o;
     o += (seen & es::kTiny) ? 2 : 0;
     aT = o;
-    o += (seen & es::kTiny) ? 2 * RC : 0;
+    o += (seen & es::kTiny) ? RC : 0;
     const bool j = !nj && (seen & es::kJ);
     int q = bI + ((seen & es::kInv) ? RC : 0);
     bJ = q;
@@ -544,22 +547,19 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
   const float ktot = nok ? a.ktot[n] : 0.0f, k2tot = nok ? a.k2tot[n] : 0.0f;
   const bool full_h = a.known_intensity && (a.gh_lo & 2);
   // which of the sums received a product (their columns hold old data otherwise)
-  const bool nj = seen & kNJ, have_j = !nj && (seen & kJ), have_1 = seen & kInv;
+  const bool nj = seen & kNJ, have_j = seen & kJ, have_1 = seen & kInv;
   const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
   const int cbeg = half * (BN / EPI_PARTS), cend = cbeg + BN / EPI_PARTS;
   if (nj) {
-    // pass A's J.H to phi and n_J to L; the columns go back before the stores,
+    // pass A's n_J to L; the columns, which n_1 takes, go back before the stores,
     // whose completion the arrival would otherwise wait for
     constexpr int CN = BN / EPI_PARTS;
-    float vj[CN], vn[CN];
+    float vn[CN];
     const bool got = ptx::mbar_wait_sleep(jdone, 0, a.status, 13, 64, a.spin);
     if (got) {
       ptx::tc_fence_after();
-      const int cj = 256 + (PAIR ? cbeg + (cbeg & 64) : cbeg);
-      ptx::tmem_ld16(lane_addr + cj, reinterpret_cast<float(&)[16]>(vj[0]));
-      ptx::tmem_ld16(lane_addr + cj + 16, reinterpret_cast<float(&)[16]>(vj[16]));
-      ptx::tmem_ld16(lane_addr + cj + (PAIR ? 64 : 128), reinterpret_cast<float(&)[16]>(vn[0]));
-      ptx::tmem_ld16(lane_addr + cj + (PAIR ? 80 : 144), reinterpret_cast<float(&)[16]>(vn[16]));
+      ptx::tmem_ld16(lane_addr + 256 + cbeg, reinterpret_cast<float(&)[16]>(vn[0]));
+      ptx::tmem_ld16(lane_addr + 256 + cbeg + 16, reinterpret_cast<float(&)[16]>(vn[16]));
       ptx::tmem_wait_ld();
       ptx::tc_fence_before();
     }
@@ -568,15 +568,10 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
     if (got) {
       const int jn = nok ? min(CN, a.R - (r0 + cbeg)) : 0;
       float* Lp = a.L + (size_t)(r0 + cbeg) * a.N + n;
-      float* Pp = a.PHI + (size_t)(r0 + cbeg) * a.N + n;
 #pragma unroll
       for (int j = 0; j < CN; ++j) {
-        if (j < jn) {
-          *Lp = vn[j];
-          *Pp = vj[j];
-        }
+        if (j < jn) *Lp = vn[j];
         Lp += a.N;
-        Pp += a.N;
       }
     }
   }
@@ -603,17 +598,14 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
       float vq[CG];  // n_J
       if (nj) {      // this thread's own stores, all loads in flight together
 #pragma unroll
-        for (int j = 0; j < CG; ++j) {
-          vq[j] = j < jn ? Lp[(size_t)j * a.N] : 0.0f;
-          vj[j] = j < jn ? Pp[(size_t)j * a.N] : 0.0f;
-        }
+        for (int j = 0; j < CG; ++j) vq[j] = j < jn ? Lp[(size_t)j * a.N] : 0.0f;
       }
 #pragma unroll
       for (int j = 0; j < CG; ++j) {
         const float n1 = have_1 ? vn[j] * a.k_inv : 0.0f;
         const float kh = (full_h ? vh[j] + vd[j] : vh[j]) * a.k_inv;
         const float B = __fmaf_rn(-kPoisC, kh, ktot - n1);
-        const float Cc = have_j || nj ? __fmaf_rn(vj[j], a.k_inv, kh) : kh;
+        const float Cc = have_j ? __fmaf_rn(vj[j], a.k_inv, kh) : kh;
         const float4 rc = s_rot[c0 + j];  // A_r, 1 / (2 sigma^2 count_r), log w_r
         bool ok = true;
         float iphi = 1.0f, phi = 1.0f;
@@ -680,7 +672,7 @@ __global__ void __launch_bounds__(es::THREADS, 1)
   uint64_t* accum = empty + NB;
   uint64_t* drain = accum + 1;  // the MMA issuer's own completion wait before TMEM is freed
   uint64_t* jdone = drain + 1;  // pass A's products are complete
-  uint64_t* jfree = jdone + 1;  // (rank 0) J.H and n_J have been moved out of TMEM
+  uint64_t* jfree = jdone + 1;  // (rank 0) n_J has been moved out of TMEM
   uint32_t* tmem_slot = (uint32_t*)(jfree + 1);
   float4* s_rot = (float4*)(smem + CHUNKS * CHUNK + 256);
   float2* s_half = (float2*)(s_rot + BN);  // [EPI_PARTS-1][BM] (max, sum exp) of column parts 1..
@@ -813,7 +805,7 @@ __global__ void __launch_bounds__(es::THREADS, 1)
         const uint32_t e = entry(u);
         if (!(e & (kJ | kTiny))) continue;
         const bool j = e & kJ, jl = j && (e & kJlo), hl = j && jh, t = e & kTiny;
-        if (!open((j ? 2 + 2 * RC : 0) + (jl ? 2 : 0) + (hl ? 2 * RC : 0) + (t ? 2 + 2 * RC : 0)))
+        if (!open((j ? 2 + 2 * RC : 0) + (jl ? 2 : 0) + (hl ? RC : 0) + (t ? 2 + RC : 0)))
           break;
         if (warp == 0) {
           if (j) ld(st.aJ, &mJ, e, n0);
@@ -822,11 +814,9 @@ __global__ void __launch_bounds__(es::THREADS, 1)
         } else if (warp == 1) {
           if (j) ldr(st.aH, &mHh, e);
           if (hl) ldr(st.aHl, &mHl, e);
-          if (t) ldz(st.aT, &mTv, e);
         } else {
           if (j) ldr(st.aI, &mIv, e);
-          if (hl) ldz(st.aHl + RC, &mHl, e);
-          if (t) ldr(st.aT + RC, &mTv, e);
+          if (t) ldr(st.aT, &mTv, e);
         }
         next();
       }
@@ -905,23 +895,25 @@ __global__ void __launch_bounds__(es::THREADS, 1)
           phase ^= 1;
         }
       };
-      uint32_t accA = 0;  // pass A's columns hold a product
+      uint32_t accJ = 0, accN = 0;  // J.H, n_J hold a product
       for (uint32_t u = n_a; u-- > 0;) {
         const uint32_t e = entry(u);
         if (!(e & (kJ | kTiny))) continue;
         if (!open()) break;
         const bool j = e & kJ, jl = j && (e & kJlo);
         if (j) {
-          mma4(t256, st.aJ, st.aH, idesc2, accA);  // J.H | n_J
-          accA = 1;
-          if (jl) mma4(t256, st.aJl, st.aH, idesc2, 1u);
-          if (jh) mma4(t256, st.aJ, st.aHl, idesc2, 1u);
+          mma4(t384, st.aJ, st.aH, idesc1, accJ);  // J.H
+          if (jl) mma4(t384, st.aJl, st.aH, idesc1, 1u);
+          if (jh) mma4(t384, st.aJ, st.aHl, idesc1, 1u);
+          mma4(t256, st.aJ, st.aI, idesc1, accN);  // n_J
+          if (jl) mma4(t256, st.aJl, st.aI, idesc1, 1u);
+          accJ = accN = 1;
         }
         if (e & kTiny) {
-          mma4(t256, st.aK, st.aT, idesc2, accA);
-          accA = 1;
-          if (j) mma4(t256, st.aJ, st.aT, idesc2, 1u);
-          if (jl) mma4(t256, st.aJl, st.aT, idesc2, 1u);
+          mma4(t256, st.aK, st.aT, idesc1, accN);
+          if (j) mma4(t256, st.aJ, st.aT, idesc1, 1u);
+          if (jl) mma4(t256, st.aJl, st.aT, idesc1, 1u);
+          accN = 1;
         }
         close();
       }
@@ -940,15 +932,15 @@ __global__ void __launch_bounds__(es::THREADS, 1)
         accB = 1;
         close();
       }
-      uint32_t accJ = 0, acc1 = 0;  // J.H, n_1 hold a product of this pass
-      bool taken = nj;              // pass A's sums are still there
+      uint32_t acc1 = 0;  // n_1 holds a product
+      bool taken = nj;    // pass A's n_J is still there
       for (uint32_t u = n_b; run && u-- > 0;) {
         const uint32_t e = entry(u);
         const bool j = !nj && (e & kJ);
         if (!open()) break;
         mma4(tmem, st.bK, st.bMS, idesc2, accB);  // den | K.H
         accB = 1;
-        if (taken && (j || (e & kInv))) {
+        if (taken && (e & kInv)) {
           if (!ptx::mbar_wait_cluster(jfree, 0, a.status, 13, a.spin)) break;
           ptx::tc_fence_after();
           taken = false;
