@@ -407,8 +407,9 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
         if (live) rot_ops_store_pois4(ops, e, sv);
         continue;
       }
-      const float lo = fminf(fminf(sv[0], sv[1]), fminf(sv[2], sv[3]));
-      const bool covered = pixels && lo >= 1e-10f;
+      // each value for itself: a minimum would pass over a NaN, which is not covered
+      const bool covered = pixels && sv[0] >= 1e-10f && sv[1] >= 1e-10f && sv[2] >= 1e-10f &&
+                           sv[3] >= 1e-10f;
       if (covered) {
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -1066,10 +1067,10 @@ __global__ void __launch_bounds__(512, 2) mprep_hi_kernel(MprepArgs a) {
   float* qrow = smem_row + ((4 - head) & 3);
   float t = 0.0f, b = 0.0f, qmax = 0.0f, mg = 0.0f;
   auto state = [&](int i) { return ts ? (int)ts[(size_t)(i >> 7) * a.n_rt] : 1; };
-  auto prob = [](float l, float hi, float lo) {  // exp(l - lse)
+  auto prob = [](float l, float hi, float lo) {  // exp(l - lse), 0 for a NaN
     float p;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(__fmaf_rn(l - hi, kLog2E, lo)));
-    return p;
+    return fmaxf(p, 0.0f);
   };
   auto over = [](float P, float f) {
     float rf;

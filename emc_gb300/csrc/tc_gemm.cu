@@ -626,7 +626,7 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
         } else {
           L = -INFINITY;
         }
-        vh[j] = L;
+        vh[j] = fmaxf(L, -INFINITY);  // a NaN (a rotation weight that is none) is left out
         mx = fmaxf(mx, L);
       }
       if (mx > -INFINITY) {
@@ -1258,7 +1258,7 @@ __global__ void __launch_bounds__(ep::THREADS, 1)
             }
             Lp += a.N;
             Pp += a.N;
-            v[i] = l;
+            v[i] = fmaxf(l, -INFINITY);  // a NaN (a rotation weight that is none) is left out
             mx = fmaxf(mx, l);
           }
           if (mx > -INFINITY) {
