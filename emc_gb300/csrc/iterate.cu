@@ -347,7 +347,7 @@ __device__ __forceinline__ float plan_sample<EMC_INTERP_TRILINEAR>(const float* 
 // 112^3, 10,860, true Poisson 378, now 302; 96^3 trilinear 1,217, now 1,067 -- and by
 // the latency of the gathers in an 8 MB model (128^3, 25,680: 1,116 and 1,113, true
 // Poisson 1,078 and 985; two rotations per block with more blocks spill: 1,676).
-enum SliceMode { kSliceFp32, kSliceTc, kSliceTcPois };
+enum SliceMode { kSliceFp32, kSliceTc, kSliceTcBright, kSliceTcPois };
 
 // rotations per expand block: four with nearest sampling, two with the
 // eight-voxel trilinear gather (registers)
@@ -367,6 +367,7 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
   // model gathers of several rotations are in flight together; the operands
   // go out as 8-byte stores (Kp is a multiple of 128)
   constexpr int kSliceRows = slice_rows_per_block<INTERP>();
+  constexpr bool kTc = MODE == kSliceTc || MODE == kSliceTcBright;
   const int r0 = blockIdx.x * kSliceRows;
   const int hl_end = ops.hl_end ? 64 * __ldg(ops.hl_end) : Kp;  // H lo pixels
   const int nr = min(kSliceRows, R - r0);
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
         sv[u] = pixels || pv[u] >= 0 ? plan_sample<INTERP>(model, side, Rm, xv[u], yv[u], zv[u])
                                      : 0.0f;
       const size_t e = (size_t)(r0 + k) * Kp + q;
-      if (MODE != kSliceTc) {
+      if (!kTc) {
 #pragma unroll
         for (int u = 0; u < 4; ++u)
           if (pixels || pv[u] >= 0) ss[k] += fmaxf(sv[u], kSliceFloor);
@@ -432,12 +433,12 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
       }
       // the tensor path takes its FP16 operands straight from s; the FP32
       // path keeps the slices
-      if (MODE == kSliceTc)
-        rot_ops_store4(ops, e, sv, hv, covered, live, q < hl_end);
+      if (kTc)
+        rot_ops_store4<MODE == kSliceTcBright>(ops, e, sv, hv, covered, live, q < hl_end);
       else
         *reinterpret_cast<float4*>(S + e) = make_float4(sv[0], sv[1], sv[2], sv[3]);
     }
-    if (MODE == kSliceTc && odd) {  // races store the same value
+    if (kTc && odd) {  // races store the same value
       const size_t f = (size_t)(r0 >> 7) * ops.nkb + (q >> 6);
       if (odd & 1) ops.inv[f] = 1;
       if (odd & 2) ops.tiny[f] = 1;
@@ -1907,9 +1908,10 @@ static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
   int threads = 256;
   for (int t = 224; t >= 128 && ops.live && !ops.Lh; t -= 32)
     if (ceil_div(n4, t) * t < ceil_div(n4, threads) * threads) threads = t;
-  auto kernel = !ops.live ? slice_rows_kernel<INTERP, kSliceFp32>
-                : ops.Lh  ? slice_rows_kernel<INTERP, kSliceTcPois>
-                          : slice_rows_kernel<INTERP, kSliceTc>;
+  auto kernel = !ops.live    ? slice_rows_kernel<INTERP, kSliceFp32>
+                : ops.Lh     ? slice_rows_kernel<INTERP, kSliceTcPois>
+                : ops.bright ? slice_rows_kernel<INTERP, kSliceTcBright>
+                             : slice_rows_kernel<INTERP, kSliceTc>;
   kernel<<<ceil_div(p->d.n_rot, slice_rows_per_block<INTERP>()), threads, 0, ctx->stream>>>(
       model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S, p->rot_cnt,
       p->rot_A, p->rot_ssum, ops);

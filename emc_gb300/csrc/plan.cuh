@@ -58,6 +58,10 @@ struct emc_plan {
   __half* Jh = nullptr;      // fp16(j), j = k (k - 1): written in blocks with a count above 1
   __half* Jl = nullptr;      // j - Jh: written in blocks where it is not 0
   float *ktot = nullptr, *k2tot = nullptr;  // [Np] sum k, sum k^2 (exact, then rounded)
+  // some pattern's sum k^2 or count is beyond FP32 differences (found at bind; the
+  // likelihood then sums over the covered pixels): the device's word for it, ours
+  int* d_bright = nullptr;
+  bool bright = false;
   unsigned char* blk_bits = nullptr;  // [Np/128][Kp/64] what the block holds (es::kJ ..)
   // the blocks each pattern tile (and pair of tiles) has counts in, with their
   // bits: index << 8 | bits, in order; never empty
@@ -221,8 +225,9 @@ constexpr float kPoisC = 0.02f;  // emc_cuda.cu:205
 // Rotation-side FP16 operands of the tensor-core likelihood, written by the
 // expand kernel straight from each slice value s (no FP32 slice buffer).
 // Reference likelihood: M'S = [s >= 1e-10] s 2^-8, H = 1 / (s + 0.02) with 0
-// where s <= 0 (its lo half in Hl where that is read), I = [s <= 0], and the
-// flags of the 64-pixel blocks that hold such pixels or an s in (0, 1e-10);
+// where s <= 0 (its lo half in Hl where that is read), I = [s <= 0] (bright counts:
+// V = [s >= 1e-10] in its place), and the flags of the 64-pixel blocks that hold
+// pixels with s <= 0 or an s in (0, 1e-10);
 // true Poisson: log max(s, 1e-6) as hi + lo in Lh / Ll.  Blocks in which no pattern counts are not
 // written (nothing reads them).  flags[0] |= 4 when M'S leaves the FP16 range.
 struct RotOps {
@@ -230,6 +235,7 @@ struct RotOps {
   __half *Lh = nullptr, *Ll = nullptr;
   int* flags = nullptr;
   const unsigned char* live = nullptr;  // [nkb] (null: no tensor path)
+  bool bright = false;                  // V instead of I
   unsigned char *inv = nullptr, *tiny = nullptr;  // [n_rt][nkb]
   int nkb = 0;
   // device int: H lo is read (and written) only in the 64-pixel blocks below
@@ -239,6 +245,8 @@ struct RotOps {
 
 // The operands of four neighbouring pixels e .. e + 3 (e a multiple of 4) as
 // 8-byte stores; hv = 1 / (s + 0.02) where s > 0, else 0, computed by the caller.
+// BRIGHT: V in I's place.
+template <bool BRIGHT>
 __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const float (&sv)[4],
                                                const float (&hv)[4], bool covered, bool live,
                                                bool h_lo) {
@@ -261,8 +269,11 @@ __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const 
   ms4.h[1] = __floats2half2_rn(ms[2], ms[3]);
   hh4.h[0] = __floats2half2_rn(hv[0], hv[1]);
   hh4.h[1] = __floats2half2_rn(hv[2], hv[3]);
-  iv4.u = make_uint2(0, 0);
-  if (!covered) {
+  iv4.h[0] = iv4.h[1] = __float2half2_rn(BRIGHT ? 1.0f : 0.0f);
+  if (BRIGHT && !covered) {
+    iv4.h[0] = __floats2half2_rn(sv[0] >= 1e-10f ? 1.0f : 0.0f, sv[1] >= 1e-10f ? 1.0f : 0.0f);
+    iv4.h[1] = __floats2half2_rn(sv[2] >= 1e-10f ? 1.0f : 0.0f, sv[3] >= 1e-10f ? 1.0f : 0.0f);
+  } else if (!covered) {
     iv4.h[0] = __floats2half2_rn(sv[0] > 0.0f ? 0.0f : 1.0f, sv[1] > 0.0f ? 0.0f : 1.0f);
     iv4.h[1] = __floats2half2_rn(sv[2] > 0.0f ? 0.0f : 1.0f, sv[3] > 0.0f ? 0.0f : 1.0f);
   }

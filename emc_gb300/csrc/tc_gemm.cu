@@ -193,19 +193,22 @@ __global__ void __launch_bounds__(256) tc_count_blocks_kernel(
 // rounded once), and the last 64-pixel block b whose suffix (blocks b ..) still
 // holds more than eps of the row's counts: lo_kb[n / 128] (zeroed before)
 // becomes the largest b + 1 over the tile's rows, lo_kb[n_pt] the largest of
-// all.  Lane l takes a contiguous run of blocks: run sums, a warp prefix scan,
+// all.  bright (zeroed before) is set where k2tot is not exact in FP32 or a count's
+// k (k - 1) not in two FP16 terms.  Lane l takes a contiguous run of blocks: run sums, a warp prefix scan,
 // then a second walk over its run.
 __global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __restrict__ Kh, int Kp,
                                                             int nkb, int N, float scale, float eps,
                                                             float* __restrict__ ktot,
                                                             float* __restrict__ k2tot,
-                                                            int* __restrict__ lo_kb) {
+                                                            int* __restrict__ lo_kb,
+                                                            int* __restrict__ bright) {
   const int n = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
   if (n >= N) return;  // whole warps
   const float inv = 1.0f / scale;
   const __half* k = Kh + (size_t)n * Kp;
   const int per = (nkb + 31) / 32;
   const int b0 = min(lane * per, nkb), b1 = min(b0 + per, nkb);
+  unsigned most = 0;
   auto block = [&](int b, unsigned long long& s2) {  // the block's sum of k; k^2 added to s2
     const uint4* v = reinterpret_cast<const uint4*>(k + 64 * (size_t)b);
     unsigned s = 0;
@@ -219,6 +222,7 @@ __global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __rest
         const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[h]));
         const unsigned x = (unsigned)(f.x * inv), y = (unsigned)(f.y * inv);
         s += x + y;
+        most = max(most, max(x, y));
         s2 += (unsigned long long)x * x + (unsigned long long)y * y;
       }
     }
@@ -234,6 +238,7 @@ __global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __rest
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) s2 += __shfl_xor_sync(0xffffffffu, s2, o);
+  most = __reduce_max_sync(0xffffffffu, most);
   const unsigned long long total = __shfl_sync(0xffffffffu, incl, 31);
   const float lim = eps * (float)total;
   unsigned long long pre = incl - c;  // the counts of the blocks before b0
@@ -247,6 +252,7 @@ __global__ void __launch_bounds__(256) tc_count_rows_kernel(const __half* __rest
   if (lane == 0) {
     ktot[n] = (float)total;
     k2tot[n] = (float)s2;
+    if (s2 >= 1ull << 24 || most > 2048u) *bright = 1;  // races store the same value
     if (last >= 0) {
       atomicMax(lo_kb + n / 128, last + 1);
       atomicMax(lo_kb + (N + 127) / 128, last + 1);
@@ -356,6 +362,14 @@ __global__ void transpose_h_kernel(const __half* __restrict__ in, int rows, int 
 //   n_1 = K . I^T                      n_J = J . I^T
 // with k_tot and k2_tot summed exactly at bind (a pixel with 0 < s < 1e-10
 // counts in B and C but not in num: its k^2 is added to n_J through a plane T).
+// These are differences of whole numbers, exact while sum k^2 stays below 2^24 and
+// the counts below 2,049 (k (k - 1) in 22 bits).  Where some pattern of the plan
+// exceeds that (a beam spot or hot pixels, which may lie outside every slice) the
+// differences would keep rounding of what they take out, so the plane of I holds V =
+// [s >= 1e-10] instead, and a tile with an invalid pixel sums what is covered:
+//   num = K . V^T + J . V^T      B = K . V^T + K . T^T - c (K . H^T)
+// over all its blocks, K . V^T and K . T^T in n_1's columns and num in n_J's.
+// (A tile without invalid pixels takes nothing out, and keeps k_tot and k2_tot.)
 // What each 64-pixel block of a pattern tile needs is decided at bind too:
 // nothing where no pattern of the tile counts, K x [M'S | H] where every count
 // is 0 or 1 (J = 0), J x H where one is larger, the products with I only where
@@ -473,18 +487,19 @@ struct TcEstepArgs {
 template <bool PAIR>
 struct EsStages {
   static constexpr int RC = PAIR ? 1 : 2;
-  // pass A: J, H, I; then what few tiles have: J lo, H lo, K, T
+  // pass A: J, H, I (or V); then what few tiles have: J lo, H lo, K, T
   static constexpr int aJ = 0, aH = 2, aI = 2 + RC;
   int aJl, aHl, aK, aT;
-  // pass B: K, [M'S (or H lo) | H], I; in tiles without pass A: J, J lo, H lo
+  // pass B: K, [M'S (or H lo) | H], I (or V); in tiles without pass A: J, J lo, H lo;
+  // beside V: T
   static constexpr int bK = 0, bMS = 2, bH = 2 + RC, bI = 2 + 2 * RC;
-  int bJ, bJl, bHl;
+  int bJ, bJl, bHl, bT;
   // pass C: K, [0 | H lo] (256 columns: a pair's K.H lies in two column quarters
   // that one 128-column product cannot reach, and den starts from the 0)
   static constexpr int cK = 0, cZ = 2, cHl = 2 + RC;
   int size, slots;
-  // jh: J x H lo as well; full_h: H lo in M'S's place
-  __device__ __forceinline__ EsStages(uint32_t seen, bool nj, bool jh, bool full_h) {
+  // jh: J x H lo as well; full_h: H lo in M'S's place; vis: sums over V
+  __device__ __forceinline__ EsStages(uint32_t seen, bool nj, bool jh, bool full_h, bool vis) {
     const int jl = (seen & es::kJlo) ? 2 : 0;
     int o = aI + RC;
     aJl = o;
@@ -492,17 +507,19 @@ struct EsStages {
     aHl = o;
     o += jh ? RC : 0;
     aK = o;
-    o += (seen & es::kTiny) ? 2 : 0;
+    o += vis || (seen & es::kTiny) ? 2 : 0;
     aT = o;
-    o += (seen & es::kTiny) ? RC : 0;
+    o += !vis && (seen & es::kTiny) ? RC : 0;
     const bool j = !nj && (seen & es::kJ);
-    int q = bI + ((seen & es::kInv) ? RC : 0);
+    int q = bI + (vis || (seen & es::kInv) ? RC : 0);
     bJ = q;
     q += j ? 2 : 0;
     bJl = q;
     q += j ? jl : 0;
     bHl = q;
     q += j && jh && !full_h ? RC : 0;
+    bT = q;
+    q += vis && (seen & es::kTiny) ? RC : 0;
     size = max(q, nj ? o : 0);
     slots = min(es::NB, es::CHUNKS / size);
   }
@@ -536,7 +553,8 @@ template <bool PAIR>
 __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tmem, uint64_t* accum,
                                                uint64_t* jdone, uint32_t jfree, const float4* s_rot,
                                                float2* s_half, int warp,
-                                               int lane, int n0, int r0, int rt, uint32_t seen) {
+                                               int lane, int n0, int r0, int rt, uint32_t seen,
+                                               bool vis) {
   using namespace es;
   const int quarter = warp & 3;  // TMEM lanes this warp may access
   const int half = (warp - EPI_WARP0) >> 2;  // column part
@@ -544,10 +562,12 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
   const int n = n0 + row;
   const bool nok = n < a.N;
   const float ci = nok ? a.cnorm[n] : 1.0f;
-  const float ktot = nok ? a.ktot[n] : 0.0f, k2tot = nok ? a.k2tot[n] : 0.0f;
+  // what n_1 and n_J are taken from, and with which sign (vis: they are the sums)
+  const float ktot = nok && !vis ? a.ktot[n] : 0.0f, k2tot = nok && !vis ? a.k2tot[n] : 0.0f;
+  const float k_1 = vis ? a.k_inv : -a.k_inv, k2_1 = vis ? 0.0f : -a.k_inv;
   const bool full_h = a.known_intensity && (a.gh_lo & 2);
   // which of the sums received a product (their columns hold old data otherwise)
-  const bool nj = seen & kNJ, have_j = seen & kJ, have_1 = seen & kInv;
+  const bool nj = seen & kNJ, have_j = seen & kJ, have_1 = vis || (seen & kInv);
   const uint32_t lane_addr = tmem + ((uint32_t)(quarter * 32) << 16);
   const int cbeg = half * (BN / EPI_PARTS), cend = cbeg + BN / EPI_PARTS;
   if (nj) {
@@ -602,15 +622,16 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
       }
 #pragma unroll
       for (int j = 0; j < CG; ++j) {
-        const float n1 = have_1 ? vn[j] * a.k_inv : 0.0f;
+        const float n1 = have_1 ? vn[j] : 0.0f;
         const float kh = (full_h ? vh[j] + vd[j] : vh[j]) * a.k_inv;
-        const float B = __fmaf_rn(-kPoisC, kh, ktot - n1);
+        const float B = __fmaf_rn(-kPoisC, kh, __fmaf_rn(k_1, n1, ktot));
         const float Cc = have_j ? __fmaf_rn(vj[j], a.k_inv, kh) : kh;
         const float4 rc = s_rot[c0 + j];  // A_r, 1 / (2 sigma^2 count_r), log w_r
         bool ok = true;
         float iphi = 1.0f, phi = 1.0f;
         if (!a.known_intensity) {
-          const float num = nj ? __fmaf_rn(-a.k_inv, vq[j], k2tot - n1) : k2tot - n1;
+          const float rest = __fmaf_rn(k2_1, n1, k2tot);
+          const float num = nj ? __fmaf_rn(k_1, vq[j], rest) : rest;
           const float den = vd[j] * (256.0f * a.k_inv);
           ok = num > 0.0f && den > 0.0f;
           iphi = quotient(den, num);
@@ -657,7 +678,11 @@ __device__ __forceinline__ void estep_epilogue(const TcEstepArgs& a, uint32_t tm
   if (nbad) atomicAdd(a.bad, nbad);
 }
 
-template <bool PAIR>
+// BRIGHT: the plan's I operand is V (bright counts).  A variant of its own: the branches
+// slow the threads that issue loads and products, 3.7 % of an iteration at 96^3.  A tile
+// that sums over V takes more products: 4,000 patterns x 6,300 rotations at 96^3 with
+// 2,000 counts at pixels outside the volume, 1,308 us, without such counts 519.
+template <bool PAIR, bool BRIGHT>
 __global__ void __launch_bounds__(es::THREADS, 1)
     tc_estep_kernel(const __grid_constant__ CUtensorMap mK, const __grid_constant__ CUtensorMap mJ,
                     const __grid_constant__ CUtensorMap mJl, const __grid_constant__ CUtensorMap mMS,
@@ -718,7 +743,8 @@ __global__ void __launch_bounds__(es::THREADS, 1)
     if (b < kList) s_list[b] = e;
     seen |= e & 0xff;
     // n_J is needed: invalid pixels where counts exceed 1, or an s in (0, 1e-10)
-    if (((e & (kJ | kInv)) == (kJ | kInv) || (e & kTiny)) && !a.known_intensity) seen |= kNJ;
+    const bool takes = (e & kInv) && (BRIGHT || (e & kJ));
+    if ((takes || (e & kTiny)) && !a.known_intensity) seen |= kNJ;
     if (e & (kJ | kTiny)) last_a = b + 1;
     if (e & kHlo) last_c = b + 1;
   }
@@ -755,9 +781,11 @@ __global__ void __launch_bounds__(es::THREADS, 1)
   const bool jh = (a.gh_lo & 2) != 0;  // H lo in every product
   const uint32_t all = *s_seen;
   const bool nj = all & kNJ;  // the tile has a pass A
-  const EsStages<PAIR> st(known ? all & ~kTiny : all, nj, jh, full_h);
-  // entries of each pass: A those with J (or T), B all, C those before the count tail
-  const uint32_t n_a = nj ? s_seen[1] : 0u, n_b = (uint32_t)cnt;
+  const bool vis = BRIGHT && (all & (kInv | kTiny));  // sums over the covered pixels
+  const EsStages<PAIR> st(known && !vis ? all & ~kTiny : all, nj, jh, full_h, vis);
+  // entries of each pass: A those with J (or T; all with V), B all, C those before the
+  // count tail
+  const uint32_t n_b = (uint32_t)cnt, n_a = !nj ? 0u : vis ? n_b : s_seen[1];
   const uint32_t n_c = full_h || !a.gh_lo ? 0u : (jh ? n_b : s_seen[2]);
   const uint32_t in_c = jh ? ~0u : kHlo;
 
@@ -803,19 +831,20 @@ __global__ void __launch_bounds__(es::THREADS, 1)
       };
       for (uint32_t u = n_a; u-- > 0;) {  // pass A
         const uint32_t e = entry(u);
-        if (!(e & (kJ | kTiny))) continue;
-        const bool j = e & kJ, jl = j && (e & kJlo), hl = j && jh, t = e & kTiny;
-        if (!open((j ? 2 + 2 * RC : 0) + (jl ? 2 : 0) + (hl ? RC : 0) + (t ? 2 + RC : 0)))
+        if (!vis && !(e & (kJ | kTiny))) continue;
+        const bool j = e & kJ, jl = j && (e & kJlo), hl = j && jh, t = !vis && (e & kTiny);
+        if (!open((j ? 2 + RC : 0) + (j || vis ? RC : 0) + (jl ? 2 : 0) + (hl ? RC : 0) +
+                  (t || vis ? 2 : 0) + (t ? RC : 0)))
           break;
         if (warp == 0) {
           if (j) ld(st.aJ, &mJ, e, n0);
           if (jl) ld(st.aJl, &mJl, e, n0);
-          if (t) ld(st.aK, &mK, e, n0);
+          if (t || vis) ld(st.aK, &mK, e, n0);
         } else if (warp == 1) {
           if (j) ldr(st.aH, &mHh, e);
           if (hl) ldr(st.aHl, &mHl, e);
         } else {
-          if (j) ldr(st.aI, &mIv, e);
+          if (j || vis) ldr(st.aI, &mIv, e);
           if (t) ldr(st.aT, &mTv, e);
         }
         next();
@@ -836,8 +865,9 @@ __global__ void __launch_bounds__(es::THREADS, 1)
       for (uint32_t u = n_b; run && u-- > 0;) {  // pass B
         const uint32_t e = entry(u);
         const bool j = !nj && (e & kJ), jl = j && (e & kJlo);
-        const bool hl = j && jh && !full_h;
-        if (!open(2 + 2 * RC + ((e & kInv) ? RC : 0) + (j ? 2 : 0) + (jl ? 2 : 0) + (hl ? RC : 0)))
+        const bool hl = j && jh && !full_h, i = vis || (e & kInv), t = vis && (e & kTiny);
+        if (!open(2 + 2 * RC + (i ? RC : 0) + (j ? 2 : 0) + (jl ? 2 : 0) + (hl ? RC : 0) +
+                  (t ? RC : 0)))
           break;
         if (warp == 0) {
           ld(st.bK, &mK, e, n0);
@@ -848,7 +878,8 @@ __global__ void __launch_bounds__(es::THREADS, 1)
           if (j) ld(st.bJ, &mJ, e, n0);
         } else {
           ldr(st.bH, &mHh, e);
-          if (e & kInv) ldr(st.bI, &mIv, e);
+          if (i) ldr(st.bI, &mIv, e);
+          if (t) ldr(st.bT, &mTv, e);
         }
         next();
       }
@@ -898,7 +929,7 @@ __global__ void __launch_bounds__(es::THREADS, 1)
       uint32_t accJ = 0, accN = 0;  // J.H, n_J hold a product
       for (uint32_t u = n_a; u-- > 0;) {
         const uint32_t e = entry(u);
-        if (!(e & (kJ | kTiny))) continue;
+        if (!vis && !(e & (kJ | kTiny))) continue;
         if (!open()) break;
         const bool j = e & kJ, jl = j && (e & kJlo);
         if (j) {
@@ -909,7 +940,10 @@ __global__ void __launch_bounds__(es::THREADS, 1)
           if (jl) mma4(t256, st.aJl, st.aI, idesc1, 1u);
           accJ = accN = 1;
         }
-        if (e & kTiny) {
+        if (vis) {
+          mma4(t256, st.aK, st.aI, idesc1, accN);
+          accN = 1;
+        } else if (e & kTiny) {
           mma4(t256, st.aK, st.aT, idesc1, accN);
           if (j) mma4(t256, st.aJ, st.aT, idesc1, 1u);
           if (jl) mma4(t256, st.aJl, st.aT, idesc1, 1u);
@@ -940,7 +974,8 @@ __global__ void __launch_bounds__(es::THREADS, 1)
         if (!open()) break;
         mma4(tmem, st.bK, st.bMS, idesc2, accB);  // den | K.H
         accB = 1;
-        if (taken && (e & kInv)) {
+        const bool i = vis || (e & kInv);
+        if (taken && i) {
           if (!ptx::mbar_wait_cluster(jfree, 0, a.status, 13, a.spin)) break;
           ptx::tc_fence_after();
           taken = false;
@@ -951,9 +986,10 @@ __global__ void __launch_bounds__(es::THREADS, 1)
           if (e & kJlo) mma4(t384, st.bJl, st.bH, idesc1, 1u);
           if (jh) mma4(t384, st.bJ, full_h ? st.bMS : st.bHl, idesc1, 1u);
         }
-        if (e & kInv) {
+        if (i) {
           mma4(t256, st.bK, st.bI, idesc1, acc1);
           acc1 = 1;
+          if (vis && (e & kTiny)) mma4(t256, st.bK, st.bT, idesc1, 1u);
         }
         close();
       }
@@ -972,8 +1008,8 @@ __global__ void __launch_bounds__(es::THREADS, 1)
     }
   } else {
     // ------------------------------------------------ epilogue
-    estep_epilogue<PAIR>(a, tmem, accum, jdone, ptx::mapa_shared(ptx::smem_u32(jfree), 0), s_rot, s_half, warp, lane, n0, r0, rt,
-                         *s_seen);
+    estep_epilogue<PAIR>(a, tmem, accum, jdone, ptx::mapa_shared(ptx::smem_u32(jfree), 0), s_rot,
+                         s_half, warp, lane, n0, r0, rt, *s_seen, vis);
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -1971,7 +2007,8 @@ int tc_bind(emc_plan* p) {
       if (!rc) rc = plan_alloc(p, (void**)&p->Jl, pk * 2);
       if (!rc) rc = plan_alloc(p, (void**)&p->ktot, (size_t)Np * 4);
       if (!rc) rc = plan_alloc(p, (void**)&p->k2tot, (size_t)Np * 4);
-      if (!rc) rc = plan_alloc(p, (void**)&p->lo_kb, sizeof(int) * (n_pt + 1));
+      if (!rc) rc = plan_alloc(p, (void**)&p->lo_kb, sizeof(int) * (n_pt + 2));
+      p->d_bright = p->lo_kb + n_pt + 1;
       if (!rc) rc = plan_alloc(p, (void**)&p->rot_flags, (2 * (size_t)p->n_rt * nkb + 15) / 16 * 16);
     }
     __half** pois_ops[] = {&st->Lh, &st->Ll};
@@ -2007,12 +2044,10 @@ int tc_bind(emc_plan* p) {
     if (!rc) rc = make_map(ctx, &st->mKt, p->KhT, Kp, Np, 256, 64);
     if (!rc) rc = make_map(ctx, &st->mKt128, p->KhT, Kp, Np, 128, 64);
     if (rc) return rc;
-    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel<false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       es::SMEM_BYTES));
-    EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_kernel<true>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       es::SMEM_BYTES));
+    for (auto* k : {tc_estep_kernel<false, false>, tc_estep_kernel<false, true>,
+                    tc_estep_kernel<true, false>, tc_estep_kernel<true, true>})
+      EMC_CUDA(ctx, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         es::SMEM_BYTES));
     EMC_CUDA(ctx, cudaFuncSetAttribute(tc_estep_pois_kernel<false>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        ep::Ring<false>::kSmem));
@@ -2034,7 +2069,16 @@ int tc_bind(emc_plan* p) {
   }
   if (p->mstep_q_lo && (rc = tc_ensure_qlo(p))) return rc;
   // counts already in FP16 from the bind's pattern pass when its scale holds
-  return tc_pattern_side(p, nullptr, p->fused_scale == p->count_scale);
+  if ((rc = tc_pattern_side(p, nullptr, p->fused_scale == p->count_scale))) return rc;
+  p->bright = false;
+  if (p->d_bright) {  // which kernels the iterations launch
+    int bright = 0;
+    EMC_CUDA(ctx, cudaMemcpyAsync(&bright, p->d_bright, sizeof(int), cudaMemcpyDeviceToHost,
+                                  ctx->stream));
+    EMC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    p->bright = bright != 0;
+  }
+  return EMC_OK;
 }
 
 // FP16 pattern operands for the pattern order perm (position -> input
@@ -2069,10 +2113,10 @@ int tc_block_lists(emc_plan* p) {
   const int nkb = p->Kp / es::BK, n_pt = p->Np / es::BM;
   int rc;
   if (p->lo_kb) {
-    EMC_CUDA(ctx, cudaMemsetAsync(p->lo_kb, 0, sizeof(int) * (size_t)(n_pt + 1), ctx->stream));
+    EMC_CUDA(ctx, cudaMemsetAsync(p->lo_kb, 0, sizeof(int) * (size_t)(n_pt + 2), ctx->stream));
     tc_count_rows_kernel<<<ceil_div(p->d.n_images, 8), 256, 0, ctx->stream>>>(
         p->Kh, p->Kp, nkb, p->d.n_images, p->count_scale, (float)p->glo_tail_ppm * 3e-4f, p->ktot,
-        p->k2tot, p->lo_kb);
+        p->k2tot, p->lo_kb, p->d_bright);
     if ((rc = after_launch(ctx, "tc_count_rows_kernel"))) return rc;
   }
   const int n_qt = ceil_div(p->Kp, ms::BN);
@@ -2218,9 +2262,10 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     const int pairs = std::min(total - first, count);
     a.tile0 = first;
     if (pairs == 0) return EMC_OK;
+    auto* kernel = p->bright ? tc_estep_kernel<true, true> : tc_estep_kernel<true, false>;
     const cudaError_t e =
-        launch_pairs(ctx, tc_estep_kernel<true>, pairs, es::THREADS, es::SMEM_BYTES, st->mK, st->mJ,
-                     st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
+        launch_pairs(ctx, kernel, pairs, es::THREADS, es::SMEM_BYTES, st->mK, st->mJ, st->mJl,
+                     st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
     if (e == cudaSuccess) return after_launch(ctx, "tc_estep_kernel (pairs)");
     // a refused launch configuration (a GPU or partition that cannot
     // co-schedule the pairs) is not a sticky error: single CTAs from now on
@@ -2236,7 +2281,8 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
   const int grid = a.tiles ? p->prune_n_tiles : std::min(total - first, count);
   a.tile0 = first;
   if (grid == 0) return EMC_OK;
-  tc_estep_kernel<false><<<grid, es::THREADS, es::SMEM_BYTES, ctx->stream>>>(
+  auto* kernel = p->bright ? tc_estep_kernel<false, true> : tc_estep_kernel<false, false>;
+  kernel<<<grid, es::THREADS, es::SMEM_BYTES, ctx->stream>>>(
       st->mK, st->mJ, st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tc_estep_kernel launch");
@@ -2262,6 +2308,7 @@ RotOps tc_rot_ops(emc_plan* p) {
   o.MS = st->MS;
   o.Hh = st->Hh;
   o.Iv = st->Iv;
+  o.bright = p->bright;
   o.inv = p->rot_flags;
   o.tiny = p->rot_flags + (size_t)p->n_rt * o.nkb;
   o.Hl = gh ? st->Hl : nullptr;
