@@ -2452,6 +2452,7 @@ extern "C" int emc_plan_get_option(const emc_plan* p, int option, int* value) {
     case EMC_OPT_DEBUG_SPIN: *value = (int)p->debug_spin; return EMC_OK;
     case EMC_OPT_MSTEP_PAIR: *value = p->mstep_pair; return EMC_OK;
     case EMC_OPT_GLO_TAIL: *value = p->glo_tail_ppm; return EMC_OK;
+    case EMC_OPT_HLO_TAIL: *value = p->hlo_tail_ppm; return EMC_OK;
     default: return fail(ctx, EMC_ERR_INVALID, "plan_get_option: unknown option %d", option);
   }
 }
@@ -2502,9 +2503,10 @@ extern "C" int emc_plan_set_option(emc_plan* p, int option, int value) {
     p->counts_round = value;
     return EMC_OK;
   }
-  if (option == EMC_OPT_GLO_TAIL) {
-    EMC_REQUIRE(ctx, value >= 0 && value <= 1000000, "plan_set_option: G lo tail %d", value);
-    p->glo_tail_ppm = value;
+  if (option == EMC_OPT_GLO_TAIL || option == EMC_OPT_HLO_TAIL) {
+    EMC_REQUIRE(ctx, value >= 0 && value <= 1000000, "plan_set_option: lo tail %d", value);
+    p->hlo_tail_ppm = value;
+    if (option == EMC_OPT_GLO_TAIL) p->glo_tail_ppm = value;
     return p->tc ? tc_block_lists(p) : EMC_OK;
   }
   if (option == EMC_OPT_MSTEP_QLO) {

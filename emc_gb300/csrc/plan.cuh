@@ -73,10 +73,11 @@ struct emc_plan {
   unsigned char *sub_any = nullptr, *ms_map = nullptr;
   int *ms_list = nullptr, *ms_n = nullptr;
   // [Np/128 + 1] K . H takes H's lo half on the 64-pixel blocks below lo_kb[pt]:
-  // the blocks after it hold at most 300 glo_tail_ppm / 1e6 of every pattern's
-  // counts (EMC_OPT_GLO_TAIL; 0: every block); lo_kb[Np/128] is the largest
+  // the blocks after it hold at most hlo_tail_ppm / 1e6 of every pattern's
+  // counts (EMC_OPT_HLO_TAIL; 0: every block); lo_kb[Np/128] is the largest
   int* lo_kb = nullptr;
-  int glo_tail_ppm = 1000;
+  int hlo_tail_ppm = 300000;
+  int glo_tail_ppm = 1000;  // what EMC_OPT_GLO_TAIL reads: its last value set
   // [2][Rp/128][Kp/64] per iteration: a slice value s <= 0 / in (0, 1e-10) among
   // the tile's rotations and the block's pixels
   unsigned char* rot_flags = nullptr;

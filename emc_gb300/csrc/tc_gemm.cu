@@ -2115,7 +2115,7 @@ int tc_block_lists(emc_plan* p) {
   if (p->lo_kb) {
     EMC_CUDA(ctx, cudaMemsetAsync(p->lo_kb, 0, sizeof(int) * (size_t)(n_pt + 2), ctx->stream));
     tc_count_rows_kernel<<<ceil_div(p->d.n_images, 8), 256, 0, ctx->stream>>>(
-        p->Kh, p->Kp, nkb, p->d.n_images, p->count_scale, (float)p->glo_tail_ppm * 3e-4f, p->ktot,
+        p->Kh, p->Kp, nkb, p->d.n_images, p->count_scale, (float)p->hlo_tail_ppm * 1e-6f, p->ktot,
         p->k2tot, p->lo_kb, p->d_bright);
     if ((rc = after_launch(ctx, "tc_count_rows_kernel"))) return rc;
   }
