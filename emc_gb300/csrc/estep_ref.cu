@@ -25,6 +25,8 @@
 // conversions) took 59 ms for the likelihood and 2.9 ms for the scaling of 2,000
 // patterns x 180 rotations of 64 x 64; the forms below give the same roundings
 // from FP32 multiply-adds.
+#include <algorithm>
+
 #include "common.cuh"
 
 namespace emc {
@@ -34,6 +36,8 @@ constexpr int kRotPerCta = 4;  // rotations of a block
 constexpr int kImgScal = 4;    // images of a scaling block
 constexpr int kImgResp = 8;    // images of a likelihood block
 constexpr int kPairsPerFold = kVT / 32;
+// Rotations per launch (the grid's second dimension ends at 65,535), and per call.
+constexpr int kChunkLaunch = 65535 * kRotPerCta, kChunkMax = 65535 * 8;
 
 // Folds 16 pairs' 512-wide partials with the reference's tree, data[t] +=
 // data[t + s] for s = 256, 128, ..., 1: the partials go through shared memory to
@@ -282,12 +286,17 @@ extern "C" int emc_update_scaling_full(emc_ctx* ctx, const float* d_images,
   EMC_REQUIRE(ctx, N_2d > 0 && N_images >= 0 && slice_start >= 0 && slice_chunk >= 0,
               "update_scaling_full: bad sizes");
   if (N_images == 0 || slice_chunk == 0) return EMC_OK;
-  const int gy = emc::ceil_div(slice_chunk, emc::kRotPerCta);
-  EMC_REQUIRE(ctx, gy <= 65535, "update_scaling_full: chunk too large");
-  dim3 grid(emc::ceil_div(N_images, emc::kImgScal), gy);
-  emc::scaling_ref_kernel<<<grid, emc::kVT, 0, ctx->stream>>>(
-      d_images, d_slices, d_mask, d_scaling, N_2d, N_images, slice_start, slice_chunk);
-  return emc::after_launch(ctx, "scaling_ref_kernel");
+  EMC_REQUIRE(ctx, slice_chunk <= emc::kChunkMax, "update_scaling_full: chunk too large");
+  for (int r0 = 0; r0 < slice_chunk; r0 += emc::kChunkLaunch) {
+    const int n = std::min(slice_chunk - r0, emc::kChunkLaunch);
+    dim3 grid(emc::ceil_div(N_images, emc::kImgScal), emc::ceil_div(n, emc::kRotPerCta));
+    emc::scaling_ref_kernel<<<grid, emc::kVT, 0, ctx->stream>>>(
+        d_images, d_slices + (size_t)r0 * N_2d, d_mask, d_scaling, N_2d, N_images,
+        slice_start + r0, n);
+    const int rc = emc::after_launch(ctx, "scaling_ref_kernel");
+    if (rc) return rc;
+  }
+  return EMC_OK;
 }
 
 extern "C" int emc_calculate_responsabilities(emc_ctx* ctx, const float* d_slices,
@@ -304,19 +313,18 @@ extern "C" int emc_calculate_responsabilities(emc_ctx* ctx, const float* d_slice
   EMC_REQUIRE(ctx, diff == EMC_DIFF_ABSOLUTE || diff == EMC_DIFF_POISSON || diff == EMC_DIFF_RELATIVE,
               "calculate_responsabilities: diff %d is not a reference diff type", diff);
   if (N_images == 0 || slice_chunk == 0) return EMC_OK;
-  const int gy = emc::ceil_div(slice_chunk, emc::kRotPerCta);
-  EMC_REQUIRE(ctx, gy <= 65535, "calculate_responsabilities: chunk too large");
-  dim3 grid(emc::ceil_div(N_images, emc::kImgResp), gy);
-#define EMC_LAUNCH_RESP(D)                                                                    \
-  emc::respons_ref_kernel<D><<<grid, emc::kVT, 0, ctx->stream>>>(                             \
-      d_slices, d_images, d_mask, sigma, d_scaling, d_respons, d_weights, N_2d, N_images,     \
-      slice_start, slice_chunk)
-  if (diff == EMC_DIFF_POISSON)
-    EMC_LAUNCH_RESP(EMC_DIFF_POISSON);
-  else if (diff == EMC_DIFF_ABSOLUTE)
-    EMC_LAUNCH_RESP(EMC_DIFF_ABSOLUTE);
-  else
-    EMC_LAUNCH_RESP(EMC_DIFF_RELATIVE);
-#undef EMC_LAUNCH_RESP
-  return emc::after_launch(ctx, "respons_ref_kernel");
+  EMC_REQUIRE(ctx, slice_chunk <= emc::kChunkMax, "calculate_responsabilities: chunk too large");
+  auto* kernel = diff == EMC_DIFF_POISSON    ? emc::respons_ref_kernel<EMC_DIFF_POISSON>
+                 : diff == EMC_DIFF_ABSOLUTE ? emc::respons_ref_kernel<EMC_DIFF_ABSOLUTE>
+                                             : emc::respons_ref_kernel<EMC_DIFF_RELATIVE>;
+  for (int r0 = 0; r0 < slice_chunk; r0 += emc::kChunkLaunch) {
+    const int n = std::min(slice_chunk - r0, emc::kChunkLaunch);
+    dim3 grid(emc::ceil_div(N_images, emc::kImgResp), emc::ceil_div(n, emc::kRotPerCta));
+    kernel<<<grid, emc::kVT, 0, ctx->stream>>>(d_slices + (size_t)r0 * N_2d, d_images, d_mask,
+                                               sigma, d_scaling, d_respons, d_weights, N_2d,
+                                               N_images, slice_start + r0, n);
+    const int rc = emc::after_launch(ctx, "respons_ref_kernel");
+    if (rc) return rc;
+  }
+  return EMC_OK;
 }
