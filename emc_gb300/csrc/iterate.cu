@@ -2331,9 +2331,17 @@ extern "C" int emc_plan_capture(emc_plan* p, float* d_model, float* d_weight) {
     p->graph = nullptr;
   }
   const bool prof = p->profiling;
-  p->profiling = false;  // no event records inside the graph
   EMC_CUDA(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+  p->profiling = false;  // no event records inside the graph
+  // recording runs nothing: what the last iteration left stays described as it was
+  const bool p_written = p->p_written;
+  const double* const ll_src = p->ll_src;
+  const int ll_n = p->ll_n;
   const int rc = iterate_enqueue(p, d_model, d_weight);
+  const bool graph_p_written = p->p_written;
+  p->p_written = p_written;
+  p->ll_src = ll_src;
+  p->ll_n = ll_n;
   cudaGraph_t g = nullptr;
   const cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   p->profiling = prof;
@@ -2348,6 +2356,7 @@ extern "C" int emc_plan_capture(emc_plan* p, float* d_model, float* d_weight) {
     return cuda_fail(ctx, ei, "plan_capture: instantiate");
   }
   p->graph = g;
+  p->graph_p_written = graph_p_written;
   return EMC_OK;
 }
 
@@ -2359,6 +2368,7 @@ extern "C" int emc_plan_replay(emc_plan* p, float sigma) {
   if (rc) return rc;
   EMC_CUDA(ctx, cudaGraphLaunch(p->graph_exec, ctx->stream));
   own_loglik(p);
+  p->p_written = p->graph_p_written;
   return EMC_OK;
 }
 
@@ -2368,6 +2378,7 @@ extern "C" int emc_plan_replay(emc_plan* p, float sigma) {
 // between them, so the GPU runs them concurrently.
 struct emc_batch {
   std::vector<emc_plan*> plans;
+  std::vector<bool> p_written;  // each plan's, after a run
   emc_ctx* ctx = nullptr;  // stream of the launches (the first plan's context)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
@@ -2385,6 +2396,7 @@ extern "C" int emc_batch_create(emc_plan** plans, float** d_models, float** d_we
   }
   emc_batch* b = new emc_batch();
   b->plans.assign(plans, plans + n);
+  for (emc_plan* p : b->plans) b->p_written.push_back(p->graph_p_written);
   b->ctx = ctx;
   cudaError_t e = cudaGraphCreate(&b->graph, 0);
   for (int k = 0; k < n && e == cudaSuccess; ++k) {
@@ -2407,10 +2419,13 @@ extern "C" int emc_batch_run(emc_batch* b, const float* sigmas) {
     const float sg = sigmas[k];
     EMC_REQUIRE(ctx, sg > 0.0f && std::isfinite(sg), "batch_run: bad sigma %zu", k);
     const int rc = begin_iteration(b->plans[k], sg, ctx->stream);
-    own_loglik(b->plans[k]);
     if (rc) return rc;
   }
   EMC_CUDA(ctx, cudaGraphLaunch(b->exec, ctx->stream));
+  for (size_t k = 0; k < b->plans.size(); ++k) {
+    own_loglik(b->plans[k]);
+    b->plans[k]->p_written = b->p_written[k];
+  }
   return EMC_OK;
 }
 

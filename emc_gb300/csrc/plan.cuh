@@ -126,6 +126,7 @@ struct emc_plan {
   emc::IterReport* report = nullptr;  // page-locked host memory, written by the device
 
   // one captured iteration (emc_plan_capture / emc_plan_replay)
+  bool graph_p_written = true;  // p_written after one of its replays
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t graph_exec = nullptr;
 
