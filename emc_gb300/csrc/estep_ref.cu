@@ -142,7 +142,9 @@ __device__ __forceinline__ bool in_range(float x, float lo, float hi) {
 // per rotation and pixel, the square, product and sum exact to their low
 // halves), which rounds to the same float except where the FP64 result lies
 // within 2^-21 of an ulp of a tie.  Pixels outside the range where the pairs
-// hold (checked) take the reference's own operations.
+// hold (checked) take the reference's own operations: a term stays below (2^51)^2 x 50
+// < 2^108, so that a thread's sum (2^20 terms for 2^29 pixels) does not reach infinity,
+// where a pair's low half would be NaN.
 template <int DIFF>
 __global__ void __launch_bounds__(kVT, 1) respons_ref_kernel(
     const float* __restrict__ slices, const float* __restrict__ images,
@@ -171,7 +173,7 @@ __global__ void __launch_bounds__(kVT, 1) respons_ref_kernel(
     // k / inf = 0 (a denominator truncated to 0 everywhere) is k (1 / inf) with residual k * 0
     const bool inf = isinf(phi);
     s_phi[threadIdx.x] = inf ? make_float2(1.0f, 0.0f) : make_float2(phi, __frcp_rn(phi));
-    bad = !inf && !in_range(phi, 0x1p-30f, 0x1p60f);
+    bad = !inf && !in_range(phi, 0x1p-25f, 0x1p60f);
   }
   if (threadIdx.x < kRotPerCta) s_cnt[threadIdx.x] = 0;
   const bool phi_ok = !__syncthreads_or(bad);
@@ -188,13 +190,13 @@ __global__ void __launch_bounds__(kVT, 1) respons_ref_kernel(
 #pragma unroll
     for (int i = 0; i < kImgResp; ++i) {
       k[i] = __ldg(img[i] + p);
-      ok = ok && (k[i] == 0.0f || in_range(k[i], 0x1p-60f, 0x1p30f));
+      ok = ok && (k[i] == 0.0f || in_range(k[i], 0x1p-60f, 0x1p25f));
     }
 #pragma unroll
     for (int j = 0; j < kRotPerCta; ++j) {
       s[j] = __ldg(sl[j] + p);
       cnt[j] += s[j] > 0.0f;
-      ok = ok && (!(s[j] > 0.0f) || in_range(s[j], 0x1p-50f, 0x1p60f));
+      ok = ok && (!(s[j] > 0.0f) || in_range(s[j], 0x1p-50f, 0x1p50f));
     }
     if (ok) {
 #pragma unroll
