@@ -57,8 +57,9 @@ def parse():
     ap.add_argument("--mstep-aggregate", type=int, choices=[0, 1], default=0,
                     help="tensor M-step: warp-aggregated atomics for nearest insertion")
     ap.add_argument("--estep-ghlo", type=int, choices=[-1, 0, 1, 2, 3], default=-1,
-                    help="tensor E-step: lo terms of G (bit 0) and H (bit 1); -1: the library's "
-                         "default (G, and H when the intensity is known)")
+                    help="tensor E-step: lo term of H in K.H before the count tail (bit 0) and "
+                         "in every product (bit 1); -1: the library's default (bit 0, both when "
+                         "the intensity is known)")
     ap.add_argument("--counts-round", type=int, choices=[-1, 0, 1], default=-1,
                     help="tensor path: round counts above 2,048 to the nearest FP16 value "
                          "(relative change <= 2^-12 on those pixels); without it such "

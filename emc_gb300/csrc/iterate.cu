@@ -1036,8 +1036,9 @@ struct MprepArgs {
 // The tensor M-step's operand as FP16 hi only: Q' = P c_i / phi (phi holds c_i
 // num/den, the M-step multiplies raw counts), [R][ldq], each row scaled by 2^e_r so
 // that its largest entry sits near 2^14 (qscale_r = 2^-e_r).  Taking P through an
-// 11-bit rounding, it is served by the hardware exponential (2^-21 relative; results
-// below 2^-126 are 0) and reciprocal.  Bound by HBM and by issue: 8 bytes read and 2
+// 11-bit rounding, it is served by the hardware exponential and reciprocal, both to a
+// unit or two in the last place; P = 2^x also takes the rounding of x, which is
+// relative 2^-25 |x| at most (2^-18 where P nears 2^-126, below which it is 0).  Bound by HBM and by issue: 8 bytes read and 2
 // written per pair, and phi only where P is not 0.  A row is kept in shared memory
 // between the two passes, shared by a cluster of 1 to 8 CTAs of `chunk` patterns, so
 // that four CTAs fit an SM and one's reads overlap another's writes; a row too long
@@ -1354,8 +1355,9 @@ __global__ void __launch_bounds__(512, 2) mprep_kernel(MprepArgs a) {
   if (threadIdx.x == 0) a.qscale[r] = ldexpf(1.0f, -ex);
 }
 
-// P = exp(L - lse) in place over the plan's [R][N] rows, with mprep's own
-// expression for an evaluated pair (bit-identical to an eagerly written P).
+// P = exp(L - lse) in place over the plan's [R][N] rows, with mprep_kernel's
+// expression for an evaluated pair.  (mprep_hi_kernel, which writes P itself where
+// pruning reads it, takes the hardware exponential: see its bound.)
 __global__ void respons_from_loglik_kernel(float* __restrict__ L, const float2* __restrict__ lse2,
                                            int N, long long total) {
   const long long stride = (long long)gridDim.x * blockDim.x;
@@ -2094,7 +2096,6 @@ static int enqueue_estep(emc_plan* p, float* d_model) {
   return mark_phase(p, 2);
 }
 
-// the normaliser lse_i from the per-tile partials, and the total log-likelihood
 static LseOut lse_out(emc_plan* p) { return {p->lse, p->lse2, p->lse_shifted, p->Np}; }
 
 // The terms of the total log-likelihood that plan_wait adds: the partials of
@@ -2104,6 +2105,8 @@ static void own_loglik(emc_plan* p) {
   p->ll_n = ceil_div(p->d.n_images, 32);
 }
 
+// the normaliser lse_i from the per-tile partials, and the terms of the total
+// log-likelihood
 static int enqueue_lse(emc_plan* p) {
   emc_ctx* ctx = p->ctx;
   const int N = p->d.n_images;
@@ -2252,12 +2255,12 @@ static int iterate_enqueue(emc_plan* p, float* d_model, float* d_weight) {
   return enqueue_finish(p, d_model, d_weight);
 }
 
-// Writes one float on a stream with a kernel rather than a host-to-device
-// copy: a copy would queue on the copy engine behind any bulk host copy that
-// another stream has issued (the next patterns, uploaded while this iteration
-// runs) and hold the iteration back until that copy ends.
 // Start of an iteration, before its graph or its first kernel: the annealing width,
-// and zeros in the invalid-pair counter and the expand's block flags.
+// and zeros in the invalid-pair counter and the expand's block flags.  The width is
+// written by a kernel rather than a host-to-device copy: a copy would queue on the
+// copy engine behind any bulk host copy that another stream has issued (the next
+// patterns, uploaded while this iteration runs) and hold the iteration back until
+// that copy ends.
 __global__ void begin_kernel(float* __restrict__ sigma, float v, int* __restrict__ bad,
                              uint4* __restrict__ flags, int n16) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2292,9 +2295,7 @@ extern "C" int emc_iterate_async(emc_plan* p, float* d_model, float* d_weight, f
   return iterate_enqueue(p, d_model, d_weight);
 }
 
-// Synchronises, then reports what the device recorded since the last wait:
-// a pipeline wait that timed out, slice values outside the FP16 operand
-// range; fills stats (of the last iteration) and clears the status words.
+// What plan_wait reads, in one launch and one write to host memory.
 __global__ void __launch_bounds__(1024) report_kernel(const int* __restrict__ flags,
                                                       const int* __restrict__ status,
                                                       const double* __restrict__ red,
@@ -2324,8 +2325,10 @@ __global__ void __launch_bounds__(1024) report_kernel(const int* __restrict__ fl
   __threadfence_system();
 }
 
-// Waits for the iteration; margin: per-rotation masses whose sum goes to
-// *margin_sum (may both be null).
+// Synchronises, then reports what the device recorded since the last wait:
+// a pipeline wait that timed out, slice values outside the FP16 operand
+// range; fills stats (of the last iteration) and clears the status words.
+// margin: per-rotation masses whose sum goes to *margin_sum (may both be null).
 int emc::plan_wait(emc_plan* p, emc_iter_stats* stats, const double* margin, double* margin_sum) {
   emc_ctx* ctx = p->ctx;
   int* dtc = tc_status(p);

@@ -14,16 +14,17 @@
 // tile's rotations: the per-tile LSE partials that the FP64 normaliser
 // combines.
 //
-// M-step.  U = Q K^T over the patterns for a tile of 128 rotations x 256
-// pixels, Q = P / phi split hi + lo in FP16 with a per-rotation power-of-two
-// scale, K the exact FP16 counts; the epilogue inserts T_r * (U / T_r) at
-// the rotated pixel (nearest or trilinear) with weight T_r -- the slice never
-// reaches HBM (emc_atomic.cu:88-132, 183-200).
+// M-step.  U = Q K^T over the patterns for a tile of 128 (a pair of CTAs: 256)
+// rotations x 256 pixels, Q = P / phi as FP16 hi (or hi + lo) with a per-rotation
+// power-of-two scale, K the exact FP16 counts; the epilogue inserts U, which is T_r
+// times the slice, at the rotated pixel (nearest or trilinear) with weight T_r -- the
+// slice never reaches HBM (emc_atomic.cu:88-132, 183-200).
 //
-// Pipeline: warp 0 issues TMA loads into a ring of shared-memory stages
-// (mbarrier full/empty handshake), warp 1 owns TMEM and issues tcgen05.mma
-// from one lane, warps 2-5 run the epilogue.  Every wait is bounded and
-// reports through a device status word (EMC_ERR_TIMEOUT on the host).
+// Pipeline: one warp (three in the reference likelihood) issues TMA loads into a
+// ring of shared-memory stages (mbarrier full/empty handshake), the next owns TMEM
+// and issues tcgen05.mma from one elected lane, sixteen run the epilogue.  Every
+// wait is bounded and reports through a device status word (EMC_ERR_TIMEOUT on the
+// host).
 #include <cuda.h>
 #include <cuda_fp16.h>
 
@@ -1549,10 +1550,6 @@ __device__ __forceinline__ void ms_tile(const TcMstepArgs& a, int t, int& r0, in
   q0 = qt * ms::BN;
 }
 
-// Persistent: CTA b takes tiles b, b + grid, ...  The k-block ring runs on
-// across tiles, and the accumulator is double-buffered in TMEM (columns
-// 0-255 and 256-511), so the insertion epilogue of one tile overlaps the
-// MMAs of the next.
 // The k-blocks of (rotation tile rt, pixel tile qt): those with counts in the pixel
 // tile, of all pattern blocks or (pruned) of the rotation tile's list, of which the
 // first is always taken, so that the accumulator is written.  Called by a whole warp,
@@ -1599,6 +1596,10 @@ struct MsRing {
   static_assert(kSmem <= 232448, "shared memory of the M-step ring");
 };
 
+// Persistent: CTA b takes tiles b, b + grid, ...  The k-block ring runs on
+// across tiles, and the accumulator is double-buffered in TMEM (columns
+// 0-255 and 256-511), so the insertion epilogue of one tile overlaps the
+// MMAs of the next.
 template <int QLO>
 __global__ void __launch_bounds__(ms::THREADS, 1)
     tc_mstep_kernel(const __grid_constant__ CUtensorMap mQh, const __grid_constant__ CUtensorMap mQl,
@@ -1761,7 +1762,8 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 // overlaps the MMAs of the next.  Both CTAs' loads complete on rank 0's
 // `full` barriers; rank 0's commits multicast to both CTAs' `empty` and
 // `tfull`; the epilogue warps of both CTAs hand a buffer back on rank 0's
-// `tempty`.  Full scans only (a pruned M-step runs single CTAs).
+// `tempty`.  Full scans, and pruned ones whose lists span the pair's 256 rotations
+// (true Poisson); the pruned reference likelihood's M-step runs single CTAs.
 namespace ms2 {
 constexpr int A_BYTES = ms::BM * ms::BK * 2;  // 16 KB: 128 rotations x 64 patterns
 constexpr int B_BYTES = 128 * ms::BK * 2;     // 16 KB: 128 pixels x 64 patterns
@@ -2512,8 +2514,9 @@ void tc_free(emc_plan* p) {
 // ------------------------------------------------------- self-test -------
 // One CTA computes D[128 x BN] = A[128 x K] B[BN x K]^T with the same TMA,
 // shared-memory descriptor, MMA and TMEM-load code as the iteration kernels,
-// for the tile shapes they use: (BN = 128, 64B swizzle, 32-wide k-blocks)
-// and (BN = 256, 128B swizzle, 64-wide k-blocks).  Single-stage pipeline.
+// in their two operand layouts: (BN = 128) 64B swizzle with 32-wide k-blocks, as the
+// true-Poisson likelihood's single CTAs load, and (BN = 256) 128B swizzle with 64-wide
+// k-blocks, as all others do.  Single-stage pipeline.
 template <int BN, int BK>
 __global__ void __launch_bounds__(128, 1)
     tc_gemm_selftest_kernel(const __grid_constant__ CUtensorMap mA,
@@ -2583,9 +2586,8 @@ __global__ void __launch_bounds__(128, 1)
 }  // namespace emc
 
 // Diagnostic: D[128 x n] = A[128 x k] B[n x k]^T (FP16 in, FP32 out, device
-// pointers) through the tcgen05 building blocks; n = 128 uses the E-step's
-// 64B-swizzled 32-wide k-blocks, n = 256 the M-step's 128B-swizzled 64-wide
-// k-blocks.  k must be a multiple of the k-block.
+// pointers) through the tcgen05 building blocks; n = 128 uses 64B-swizzled 32-wide
+// k-blocks, n = 256 128B-swizzled 64-wide ones.  k must be a multiple of the k-block.
 extern "C" int emc_tc_gemm_selftest(emc_ctx* ctx, const void* d_a, const void* d_b, float* d_d,
                                     int n, int k) {
   using namespace emc;

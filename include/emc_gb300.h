@@ -487,11 +487,12 @@ int emc_batch_destroy(emc_batch* batch);
  * frees its TMEM and exits, so no copy or MMA is in flight when a CTA leaves.
  * The next iteration with the default is unaffected. */
 #define EMC_OPT_DEBUG_SPIN 9
-/* EMC_OPT_MSTEP_PAIR: 1 (default) runs the full-scan tensor-core M-step on
+/* EMC_OPT_MSTEP_PAIR: 1 (default) runs the tensor-core M-step on
  * clusters of two CTAs (256 rotations x 256 pixels per pair, 256-row MMAs,
  * half of the pixel-side operand per CTA), 0 on single CTAs (128 x 256); at
- * 128^3 the pairs measured 6.7 ms against 8.4 ms.  Pruned iterations always
- * use single CTAs;
+ * 128^3 the pairs measured 6.7 ms against 8.4 ms.  Pruned iterations of the
+ * reference likelihood always use single CTAs (their tile lists are those of
+ * 128 rotations; the true-Poisson likelihood's span 256);
  * where a cluster launch is refused the plan falls back to single CTAs.
  * The two shapes' models agree to FP32 accumulation rounding (1e-5
  * relative). */
@@ -545,8 +546,9 @@ int emc_plan_set_profiling(emc_plan* plan, int on);
 int emc_plan_phase_ms(emc_plan* plan, float* ms, int n);
 /* Diagnostic of the tensor-core building blocks (TMA, shared-memory
  * descriptors, tcgen05.mma, TMEM loads): D[128 x n] = A[128 x k] B[n x k]^T,
- * FP16 A and B (row-major, device), FP32 D.  n = 128 exercises the E-step
- * tile shape, n = 256 the M-step's.  No counterpart in the reference. */
+ * FP16 A and B (row-major, device), FP32 D.  n = 128 exercises 64B-swizzled
+ * operands of 32 columns, n = 256 128B-swizzled ones of 64 columns.  No
+ * counterpart in the reference. */
 int emc_tc_gemm_selftest(emc_ctx* ctx, const void* d_a, const void* d_b, float* d_d, int n, int k);
 /* Device pointers into the plan's workspace (valid until the next call):
  * the normalised responsibilities [R*N] (rotation-major) and scaling [R*N]
