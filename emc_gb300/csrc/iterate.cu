@@ -347,7 +347,14 @@ __device__ __forceinline__ float plan_sample<EMC_INTERP_TRILINEAR>(const float* 
 // 112^3, 10,860, true Poisson 378, now 302; 96^3 trilinear 1,217, now 1,067 -- and by
 // the latency of the gathers in an 8 MB model (128^3, 25,680: 1,116 and 1,113, true
 // Poisson 1,078 and 985; two rotations per block with more blocks spill: 1,676).
-enum SliceMode { kSliceFp32, kSliceTc, kSliceTcBright, kSliceTcPois };
+enum SliceMode {
+  kSliceFp32,
+  kSliceTcPois,
+  kSliceTc,  // and with bright counts, or with M'S lo, or both:
+  kSliceTcBright,
+  kSliceTcLo,
+  kSliceTcBrightLo
+};
 
 // rotations per expand block: four with nearest sampling, two with the
 // eight-voxel trilinear gather (registers)
@@ -367,7 +374,9 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
   // model gathers of several rotations are in flight together; the operands
   // go out as 8-byte stores (Kp is a multiple of 128)
   constexpr int kSliceRows = slice_rows_per_block<INTERP>();
-  constexpr bool kTc = MODE == kSliceTc || MODE == kSliceTcBright;
+  constexpr bool kTc = MODE >= kSliceTc;
+  constexpr bool kBright = MODE == kSliceTcBright || MODE == kSliceTcBrightLo;
+  constexpr bool kMsLo = MODE == kSliceTcLo || MODE == kSliceTcBrightLo;
   const int r0 = blockIdx.x * kSliceRows;
   const int hl_end = ops.hl_end ? 64 * __ldg(ops.hl_end) : Kp;  // H lo pixels
   const int nr = min(kSliceRows, R - r0);
@@ -434,7 +443,7 @@ __global__ void __launch_bounds__(256) slice_rows_kernel(
       // the tensor path takes its FP16 operands straight from s; the FP32
       // path keeps the slices
       if (kTc)
-        rot_ops_store4<MODE == kSliceTcBright>(ops, e, sv, hv, covered, live, q < hl_end);
+        rot_ops_store4<kBright, kMsLo>(ops, e, sv, hv, covered, live, q < hl_end);
       else
         *reinterpret_cast<float4*>(S + e) = make_float4(sv[0], sv[1], sv[2], sv[3]);
     }
@@ -1968,7 +1977,9 @@ static int expand_launch(emc_plan* p, const float* model, const RotOps& ops) {
     if (ceil_div(n4, t) * t < ceil_div(n4, threads) * threads) threads = t;
   auto kernel = !ops.live    ? slice_rows_kernel<INTERP, kSliceFp32>
                 : ops.Lh     ? slice_rows_kernel<INTERP, kSliceTcPois>
-                : ops.bright ? slice_rows_kernel<INTERP, kSliceTcBright>
+                : ops.bright ? (ops.MSl ? slice_rows_kernel<INTERP, kSliceTcBrightLo>
+                                        : slice_rows_kernel<INTERP, kSliceTcBright>)
+                : ops.MSl    ? slice_rows_kernel<INTERP, kSliceTcLo>
                              : slice_rows_kernel<INTERP, kSliceTc>;
   kernel<<<ceil_div(p->d.n_rot, slice_rows_per_block<INTERP>()), threads, 0, ctx->stream>>>(
       model, p->d.side, p->rot, p->pix, p->cx, p->cy, p->cz, p->d.n_rot, p->Kp, p->S, p->rot_cnt,
@@ -2537,7 +2548,7 @@ extern "C" int emc_plan_set_option(emc_plan* p, int option, int value) {
   if (option == EMC_OPT_ESTEP_GHLO) {
     EMC_REQUIRE(ctx, value >= -1 && value <= 3, "plan_set_option: gh_lo %d", value);
     p->estep_gh_lo = value;
-    return EMC_OK;
+    return tc_ensure_mslo(p);
   }
   if (option == EMC_OPT_ESTEP_RASTER) {
     EMC_REQUIRE(ctx, value != 0 && value >= -4096 && value <= 4096,

@@ -219,6 +219,7 @@ void prune_free(emc_plan* p);
 int prune_reset(emc_plan* p);
 int tc_pattern_side(emc_plan* p, const int* d_perm, bool counts_done = false);
 int tc_ensure_qlo(emc_plan* p);
+int tc_ensure_mslo(emc_plan* p);  // M'S lo, where EMC_OPT_ESTEP_GHLO asks for it
 int tc_block_lists(emc_plan* p);  // count sums, lo_kb and block lists from the bound counts
 __half* tc_tiny_plane(emc_plan* p);  // 1 where 0 < s < 1e-10 (blocks flagged tiny)
 int pattern_side(emc_plan* p, const int* d_perm, bool with_tc);
@@ -227,13 +228,13 @@ constexpr float kPoisC = 0.02f;  // emc_cuda.cu:205
 // Rotation-side FP16 operands of the tensor-core likelihood, written by the
 // expand kernel straight from each slice value s (no FP32 slice buffer).
 // Reference likelihood: M'S = [s >= 1e-10] s 2^-8, H = 1 / (s + 0.02) with 0
-// where s <= 0 (its lo half in Hl where that is read), I = [s <= 0] (bright counts:
+// where s <= 0 (their lo halves in MSl and Hl where those are read), I = [s <= 0] (bright counts:
 // V = [s >= 1e-10] in its place), and the flags of the 64-pixel blocks that hold
 // pixels with s <= 0 or an s in (0, 1e-10);
 // true Poisson: log max(s, 1e-6) as hi + lo in Lh / Ll.  Blocks in which no pattern counts are not
 // written (nothing reads them).  flags[0] |= 4 when M'S leaves the FP16 range.
 struct RotOps {
-  __half *MS = nullptr, *Hh = nullptr, *Hl = nullptr, *Iv = nullptr;
+  __half *MS = nullptr, *MSl = nullptr, *Hh = nullptr, *Hl = nullptr, *Iv = nullptr;
   __half *Lh = nullptr, *Ll = nullptr;
   int* flags = nullptr;
   const unsigned char* live = nullptr;  // [nkb] (null: no tensor path)
@@ -247,8 +248,8 @@ struct RotOps {
 
 // The operands of four neighbouring pixels e .. e + 3 (e a multiple of 4) as
 // 8-byte stores; hv = 1 / (s + 0.02) where s > 0, else 0, computed by the caller.
-// BRIGHT: V in I's place.
-template <bool BRIGHT>
+// BRIGHT: V in I's place; MS_LO: M'S lo too.
+template <bool BRIGHT, bool MS_LO>
 __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const float (&sv)[4],
                                                const float (&hv)[4], bool covered, bool live,
                                                bool h_lo) {
@@ -282,6 +283,13 @@ __device__ __forceinline__ void rot_ops_store4(const RotOps& o, size_t e, const 
   *reinterpret_cast<uint2*>(o.MS + e) = ms4.u;
   *reinterpret_cast<uint2*>(o.Hh + e) = hh4.u;
   *reinterpret_cast<uint2*>(o.Iv + e) = iv4.u;
+  if (MS_LO) {
+    H4 ml4;
+    const float2 a = __half22float2(ms4.h[0]), b = __half22float2(ms4.h[1]);
+    ml4.h[0] = __floats2half2_rn(ms[0] - a.x, ms[1] - a.y);
+    ml4.h[1] = __floats2half2_rn(ms[2] - b.x, ms[3] - b.y);
+    *reinterpret_cast<uint2*>(o.MSl + e) = ml4.u;
+  }
   if (o.Hl && h_lo) {
     H4 hl4;
     const float2 a = __half22float2(hh4.h[0]), b = __half22float2(hh4.h[1]);

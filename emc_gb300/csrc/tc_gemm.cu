@@ -471,6 +471,7 @@ struct TcEstepArgs {
   const float* ktot;    // [N] sum k
   const float* k2tot;   // [N] sum k^2
   float k_inv;          // 1 / count_scale of the K and J operands
+  int ms_lo;            // pass C multiplies M'S lo
   int zrow;             // a row past the rotation operands: TMA reads it as zeros
   const float* sigma;   // [1] annealing width (device memory)
   int known_intensity;
@@ -496,7 +497,8 @@ struct EsStages {
   static constexpr int bK = 0, bMS = 2, bH = 2 + RC, bI = 2 + 2 * RC;
   int bJ, bJl, bHl, bT;
   // pass C: K, [0 | H lo] (256 columns: a pair's K.H lies in two column quarters
-  // that one 128-column product cannot reach, and den starts from the 0)
+  // that one 128-column product cannot reach, and den starts from the 0, or with lo
+  // terms in every product from K x M'S lo)
   static constexpr int cK = 0, cZ = 2, cHl = 2 + RC;
   int size, slots;
   // jh: J x H lo as well; full_h: H lo in M'S's place; vis: sums over V
@@ -689,7 +691,7 @@ __global__ void __launch_bounds__(es::THREADS, 1)
                     const __grid_constant__ CUtensorMap mJl, const __grid_constant__ CUtensorMap mMS,
                     const __grid_constant__ CUtensorMap mHh, const __grid_constant__ CUtensorMap mHl,
                     const __grid_constant__ CUtensorMap mIv, const __grid_constant__ CUtensorMap mTv,
-                    TcEstepArgs a) {
+                    const __grid_constant__ CUtensorMap mMSl, TcEstepArgs a) {
   using namespace es;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -857,7 +859,10 @@ __global__ void __launch_bounds__(es::THREADS, 1)
         if (warp == 0) {
           ld(st.cK, &mK, e, n0);
         } else if (warp == 1) {
-          ldz(st.cZ, &mHl, e);
+          if (a.ms_lo)
+            ldr(st.cZ, &mMSl, e);
+          else
+            ldz(st.cZ, &mHl, e);
         } else {
           ldr(st.cHl, &mHl, e);
         }
@@ -1955,10 +1960,10 @@ __global__ void __launch_bounds__(ms::THREADS, 1)
 struct TcState {
   CUtensorMap mK, mJ, mJl, mQh, mQl, mKt;
   CUtensorMap mKt128;  // K^T in 128-row boxes (pair M-step halves)
-  CUtensorMap mMS, mHh, mHl, mIv, mTv;  // rotation operands: 64-row boxes
+  CUtensorMap mMS, mHh, mHl, mIv, mTv, mMSl;  // rotation operands: 64-row boxes
   CUtensorMap mLh, mLl;  // true Poisson, single CTAs: log-slices hi / lo, 256 rows x 32
   CUtensorMap mK64, mLh64, mLl64;  // and pairs: 128 rows x 64
-  __half *MS, *Hh, *Hl, *Iv, *Tv, *Lh, *Ll;
+  __half *MS, *Hh, *Hl, *Iv, *Tv, *MSl, *Lh, *Ll;
   int* status;
 };
 
@@ -2070,6 +2075,7 @@ int tc_bind(emc_plan* p) {
                                        ms2::Ring<1>::kSmem));
   }
   if (p->mstep_q_lo && (rc = tc_ensure_qlo(p))) return rc;
+  if ((rc = tc_ensure_mslo(p))) return rc;
   // counts already in FP16 from the bind's pattern pass when its scale holds
   if ((rc = tc_pattern_side(p, nullptr, p->fused_scale == p->count_scale))) return rc;
   p->bright = false;
@@ -2138,6 +2144,27 @@ int tc_ensure_qlo(emc_plan* p) {
   if (rc) return rc;
   EMC_CUDA(ctx, cudaMemsetAsync(p->Ql, 0, bytes, ctx->stream));
   return make_map(ctx, &state(p)->mQl, p->Ql, p->Rp, p->Np, 128, 64);
+}
+
+// M'S in every product as hi + lo: with H lo everywhere, where a scaling is fitted.
+static bool estep_ms_lo(const emc_plan* p) {
+  return p->d.diff != EMC_DIFF_TRUE_POISSON && !p->d.known_intensity && p->estep_gh_lo >= 0 &&
+         (p->estep_gh_lo & 2);
+}
+
+// Its plane and tensor map, allocated the first time it is asked for.
+int tc_ensure_mslo(emc_plan* p) {
+  if (!p->tc || !estep_ms_lo(p) || state(p)->MSl) return EMC_OK;
+  emc_ctx* ctx = p->ctx;
+  const size_t bytes = (size_t)p->Rp * p->Kp * 2;
+  __half* plane = nullptr;
+  int rc = plan_alloc(p, (void**)&plane, bytes);
+  if (rc) return rc;
+  // rows R..Rp stay zero, as those of the other operands
+  EMC_CUDA(ctx, cudaMemsetAsync(plane, 0, bytes, ctx->stream));
+  if ((rc = make_map(ctx, &state(p)->mMSl, plane, p->Rp, p->Kp, 64, 64))) return rc;
+  state(p)->MSl = plane;
+  return EMC_OK;
 }
 
 // A kernel on clusters of two CTAs.
@@ -2246,6 +2273,7 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
   a.ktot = p->ktot;
   a.k2tot = p->k2tot;
   a.k_inv = 1.0f / p->count_scale;
+  a.ms_lo = estep_ms_lo(p) && st->MSl;
   a.zrow = p->Rp;
   a.sigma = p->sigma_dev;
   a.known_intensity = p->d.known_intensity;
@@ -2267,7 +2295,7 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
     auto* kernel = p->bright ? tc_estep_kernel<true, true> : tc_estep_kernel<true, false>;
     const cudaError_t e =
         launch_pairs(ctx, kernel, pairs, es::THREADS, es::SMEM_BYTES, st->mK, st->mJ, st->mJl,
-                     st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
+                     st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, st->mMSl, a);
     if (e == cudaSuccess) return after_launch(ctx, "tc_estep_kernel (pairs)");
     // a refused launch configuration (a GPU or partition that cannot
     // co-schedule the pairs) is not a sticky error: single CTAs from now on
@@ -2285,7 +2313,7 @@ static int estep_launch(emc_plan* p, int raster, int first, int count, bool full
   if (grid == 0) return EMC_OK;
   auto* kernel = p->bright ? tc_estep_kernel<false, true> : tc_estep_kernel<false, false>;
   kernel<<<grid, es::THREADS, es::SMEM_BYTES, ctx->stream>>>(
-      st->mK, st->mJ, st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, a);
+      st->mK, st->mJ, st->mJl, st->mMS, st->mHh, st->mHl, st->mIv, st->mTv, st->mMSl, a);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(ctx, e, "tc_estep_kernel launch");
   return after_launch(ctx, "tc_estep_kernel");
@@ -2314,6 +2342,7 @@ RotOps tc_rot_ops(emc_plan* p) {
   o.inv = p->rot_flags;
   o.tiny = p->rot_flags + (size_t)p->n_rt * o.nkb;
   o.Hl = gh ? st->Hl : nullptr;
+  o.MSl = estep_ms_lo(p) ? st->MSl : nullptr;
   if (gh == 1) o.hl_end = p->lo_kb + p->Np / es::BM;
   return o;
 }

@@ -439,8 +439,10 @@ int emc_batch_destroy(emc_batch* batch);
  * EMC_OPT_ESTEP_GHLO: where the likelihood's rotation-side factor
  * H = 1/(s+c) carries an FP16 lo term besides its FP16 hi term (~2^-12
  * relative rounding without it): bit 0 in K.H before the count tail
- * (EMC_OPT_HLO_TAIL), bit 1 in every product.  -1 (default): bit 0, and both
- * when known_intensity fixes the scaling at 1; 0..3 set the bits. */
+ * (EMC_OPT_HLO_TAIL), bit 1 in every product, and with a fitted scaling s too
+ * in its denominator (an operand of n_rot x pixels FP16 values more).  -1
+ * (default): bit 0, and both when known_intensity fixes the scaling at 1; 0..3
+ * set the bits. */
 #define EMC_OPT_ESTEP_GHLO 3
 /* EMC_OPT_MSTEP_QLO: 0 (default) multiplies responsibility/scaling as FP16
  * hi only (~2^-12 relative rounding per term), 1 as FP16 hi + lo (twice the
