@@ -36,9 +36,10 @@ def radius(prob, values):
 
 @pytest.mark.parametrize("pair", [1, 0], ids=["pairs", "single"])
 @pytest.mark.parametrize("outside", [-1.0, 0.0, 5e-11], ids=["unknown", "zeros", "tiny"])
-@pytest.mark.parametrize("pixels,count", [(1, 60000), (1, 30000), (4, 60000), (1, 3001), (5, 2000),
-                                          (40, 2000)])
-def test_scaling_over_covered_pixels(ctx, cuda, prob, pixels, count, outside, pair):
+@pytest.mark.parametrize("pixels,count,ghlo", [(1, 60000, -1), (1, 30000, -1), (4, 60000, -1),
+                                               (1, 3001, -1), (5, 2000, -1), (40, 2000, -1),
+                                               (4, 60000, 3), (40, 2000, 0)])
+def test_scaling_over_covered_pixels(ctx, cuda, prob, pixels, count, ghlo, outside, pair):
     s, R, N = prob.cfg.side, prob.quats.shape[0], prob.images.shape[0]
     rng = np.random.default_rng(pixels * count)
     r2 = radius(prob, 2)
@@ -52,6 +53,7 @@ def test_scaling_over_covered_pixels(ctx, cuda, prob, pixels, count, outside, pa
     m0[radius(prob, 3) > 14.0] = outside
     plan = E.Plan(ctx, s, N, R, precision=E.PREC_MIXED)
     plan.set_option(E.Plan.OPT_ESTEP_PAIR, pair)
+    plan.set_option(E.Plan.OPT_ESTEP_GHLO, ghlo)
     if count > 2048:
         plan.set_option(E.Plan.OPT_COUNTS_ROUND, 1)
         im = im.astype(np.float16).astype(np.float32)  # the counts that the plan takes
@@ -72,10 +74,11 @@ def test_scaling_over_covered_pixels(ctx, cuda, prob, pixels, count, outside, pa
         assert np.abs(P - want["respons"]).max() < TOL_RESP
 
 
+@pytest.mark.parametrize("pair", [1, 0], ids=["pairs", "single"])
 @pytest.mark.parametrize("outside", [-1.0, 5e-11], ids=["unknown", "tiny"])
-def test_known_intensity(ctx, cuda, prob, outside):
-    """phi = 1: the sums over the covered pixels stay exact beside 1,000 counts of 60,000
-    that only some rotations cover not at all."""
+def test_known_intensity(ctx, cuda, prob, outside, pair):
+    """phi = 1: the sums over the covered pixels stay exact beside 60,000 counts at every
+    pixel outside the volume (single CTAs with a tiny s: the largest stage, one slot)."""
     s, R, N = prob.cfg.side, prob.quats.shape[0], prob.images.shape[0]
     rng = np.random.default_rng(4)
     r2 = radius(prob, 2)
@@ -87,6 +90,7 @@ def test_known_intensity(ctx, cuda, prob, outside):
     m0 = (prob.init_model + 0.05).astype(np.float32)
     m0[radius(prob, 3) > 14.0] = outside
     plan = E.Plan(ctx, s, N, R, precision=E.PREC_MIXED, known_intensity=1)
+    plan.set_option(E.Plan.OPT_ESTEP_PAIR, pair)
     plan.set_option(E.Plan.OPT_COUNTS_ROUND, 1)
     plan.bind(T(im, cuda), T(mask, cuda, torch.int32), T(prob.x, cuda), T(prob.y, cuda),
               T(prob.z, cuda), T(prob.quats, cuda), T(prob.weights, cuda))
